@@ -26,6 +26,12 @@ namespace {
 
 constexpr uint32_t kStatsCapMax = 1u << 20;
 
+// Planes the x / y tables are sized for: one per (slice, input), also where
+// a slice has a single plane (xy_plane) and the rest of its share stays
+// unused, so that a memory budget admits the same models and queries for
+// every substep count.
+uint64_t table_planes(const GridInfo& g) { return static_cast<uint64_t>(g.slices) * g.M; }
+
 // Reference wrap_angle (model.hpp:14-24).
 double wrap_angle(double x) {
     constexpr double kPi = 3.14159265358979323846;
@@ -101,6 +107,7 @@ int grid_from_model(const gsc_model_desc* m, GridInfo* g, std::string* err) {
     g->T = m->sample_time;
     g->K = m->integration_substeps;
     g->dt = m->sample_time / static_cast<double>(m->integration_substeps);
+    g->xy_planes = xy_planes_of(g->K, g->M);
     g->S = total;
     g->ps[0] = 1;
     for (int d = 1; d < 4; ++d) g->ps[d] = g->ps[d - 1] * (g->n[d - 1] + 1);
@@ -113,7 +120,9 @@ int grid_from_model(const gsc_model_desc* m, GridInfo* g, std::string* err) {
     g->rows = static_cast<uint64_t>(g->n[1]) * g->n[2] * g->n[3];
     g->slices = g->n[2] * g->n[3];
     g->magic_n1 = fdiv_magic(g->n[1]);
-    g->magic_nw = fdiv_magic(g->n[1] * g->W);
+    g->sw = (g->n[1] * g->W + 3) & ~3u;
+    g->n1p = (g->n[1] + 3) & ~3u;
+    g->magic_sw4 = fdiv_magic(g->sw / 4);
     return GSC_OK;
 }
 
@@ -231,7 +240,7 @@ int abstraction_enqueue(gsc_abstraction* a, cudaStream_t st, std::vector<std::pa
             vf[static_cast<size_t>(i3) * g.ma + ja] = v;
         }
     }
-    const uint64_t planes = static_cast<uint64_t>(g.slices) * g.M;
+    const uint64_t planes = table_planes(g);
     void* q = nullptr;
     GSC_TRY(device_alloc(ctx, a->pool, a->allocs, a->bytes, &q, planes * g.n[0] * 8));
     a->xn = static_cast<double*>(q);
@@ -581,6 +590,17 @@ namespace {
 
 namespace gsc_api {
 
+// Whether the satisfaction test reads a representative's (theta, v) window
+// of D' itself (nz * nv words per staged word) rather than one word of a
+// dilated copy that a kernel of its own brings up to date every iteration.
+static bool reads_windows_directly(const GridInfo& g, const PlanRecord& pl) {
+    // Offsets into the dilated copies are 32-bit.
+    if (static_cast<uint64_t>(pl.dil.nk) * pl.dil.nl * __builtin_popcount(pl.ylevels | 1u) * g.slices * g.sw >=
+        0xFFFFFFFFull)
+        return true;
+    return pl.rep_rows <= 4 * pl.reps && (pl.rep_rows - pl.reps) * g.sw * 4ull <= 32ull << 20;
+}
+
 int problem_stage1(gsc_problem* p, const gsc_query_desc* qd) {
     gsc_context* ctx = p->ctx;
     const GridInfo& g = p->g;
@@ -622,9 +642,9 @@ int problem_stage1(gsc_problem* p, const gsc_query_desc* qd) {
     GSC_TRY(palloc(p, &p->valid, g.S));
     GSC_TRY(palloc(p, &p->cand, g.S));
     GSC_TRY(palloc(p, &p->counts, 8));
-    GSC_TRY(palloc(p, &p->flags, 1));
+    GSC_TRY(palloc(p, &p->flags, 2));
     GSC_CU(ctx, cudaMemsetAsync(p->counts, 0, 8 * sizeof(unsigned long long), st));
-    GSC_CU(ctx, cudaMemsetAsync(p->flags, 0, sizeof(unsigned int), st));
+    GSC_CU(ctx, cudaMemsetAsync(p->flags, 0, 2 * sizeof(unsigned int), st));
     if (p->time_h2d) GSC_CU(ctx, cudaEventRecord(ctx->pev[0], st));
     if (qd->obstacle_count) {
         GSC_TRY(palloc(p, &p->obstacles, 8ull * qd->obstacle_count));
@@ -658,11 +678,9 @@ int problem_stage1(gsc_problem* p, const gsc_query_desc* qd) {
     GSC_CU(ctx, launch_masks(g, q, ma, st));
 
     // Per-axis boxes.
-    const uint64_t planes = static_cast<uint64_t>(g.slices) * g.M;
+    const uint64_t planes = table_planes(g);
     GSC_TRY(palloc(p, &p->xt, planes * g.n[0]));
-    // y tables, class records and dilated rows are read by 16-byte aligned
-    // bulk copies up to three words past their last entry: four spare words.
-    GSC_TRY(palloc(p, &p->yt, planes * g.n[1] + 4));
+    GSC_TRY(palloc(p, &p->yt, planes * g.n1p));
     GSC_TRY(palloc(p, &p->zt, static_cast<uint64_t>(g.n[2]) * g.mw));
     GSC_TRY(palloc(p, &p->wt, static_cast<uint64_t>(g.n[3]) * g.ma));
     GSC_CU(ctx, launch_axis_tables(g, q, p->abs->xn, p->abs->yn, p->abs->thf, p->abs->vf, p->xt, p->yt, p->zt, p->wt,
@@ -672,10 +690,13 @@ int problem_stage1(gsc_problem* p, const gsc_query_desc* qd) {
     GSC_TRY(palloc(p, &p->dplan, 1));
     GSC_CU(ctx, cudaMemsetAsync(p->dplan, 0, sizeof(PlanRecord), st));
     if (p->fused_candidate) {
-        GSC_TRY(palloc(p, &p->xcls, planes * class_words(g) + 4));
+        GSC_TRY(palloc(p, &p->xcls, planes * class_words(g)));
         GSC_CU(ctx, launch_x_classes(g, p->xt, p->xcls, st));
         GSC_TRY(palloc(p, &p->xrep, planes));
         GSC_CU(ctx, launch_plane_reps(g, p->xt, p->yt, p->wt, p->xrep, &p->dplan->max_reps, st));
+        GSC_TRY(palloc(p, &p->reps, planes));
+        GSC_TRY(palloc(p, &p->nreps, g.slices));
+        GSC_CU(ctx, launch_slice_reps(g, p->xt, p->yt, p->zt, p->wt, p->xrep, p->reps, p->nreps, p->dplan, st));
         GSC_TRY(palloc(p, &p->kidx, static_cast<uint64_t>(g.n[2]) + 1));
         GSC_TRY(palloc(p, &p->lidx, static_cast<uint64_t>(g.n[3]) + 1));
     }
@@ -706,11 +727,16 @@ int problem_plan(gsc_problem* p) {
     if (fused_ok) {
         p->max_reps = pl.max_reps;
         p->dil = pl.dil;
-        // dilated-row offsets are 32-bit in the satisfaction kernel
         if (static_cast<uint64_t>(pl.dil.nk) * pl.dil.nl * g.rows * g.W >= 0xFFFFFFFFull) fused_ok = false;
-        if (fused_smem_bytes(g, class_words(g), p->need_valid, p->max_reps, true) > kFusedSmemMax ||
-            fused_smem_bytes(g, class_words(g), p->need_valid, p->max_reps, false) > kFusedSmemMax)
-            fused_ok = false;
+        const size_t admitted = fused_admission_bytes(g, p->need_valid, p->max_reps);
+        if (admitted > kFusedSmemMax) fused_ok = false;
+        p->direct = reads_windows_directly(g, pl);
+        p->pass = fused_pass(g, pl.slice_reps);
+        p->sat_threads = fused_sat_threads(g, pl.slice_reps);
+        p->tile = dilate_tile_of(g, pl.dil, pl.ylevels);
+        uint32_t rank = 0;
+        for (uint32_t l = 0; l < static_cast<uint32_t>(kYLevels); ++l)
+            if ((p->tile.levels >> l) & 1u) p->ylev[l] = static_cast<uint32_t>(rank++ * pl.dil.nk * pl.dil.nl * g.slices * g.sw);
     }
     uint32_t method = p->method;
     if (method == GSC_METHOD_AUTO) method = fused_ok ? GSC_METHOD_FUSED : (stored_ok ? GSC_METHOD_STORED : 0);
@@ -777,27 +803,24 @@ int problem_stage2(gsc_problem* p) {
         GSC_CU(ctx, cudaMemsetAsync(p->pd, 0, g.tsize * 4, st));
         return GSC_OK;
     }
-    const uint64_t words = g.rows * g.W;
+    const uint64_t words = static_cast<uint64_t>(g.slices) * g.sw;
     GSC_TRY(palloc(p, &p->validb, words));
     GSC_TRY(palloc(p, &p->unsafeb, words));
     GSC_TRY(palloc(p, &p->srcb, words));
     GSC_TRY(palloc(p, &p->candb, words));
-    GSC_TRY(palloc(p, &p->dp, words));
+    GSC_TRY(palloc(p, &p->dp[0], words));
+    GSC_TRY(palloc(p, &p->dp[1], words));
     GSC_TRY(palloc(p, &p->reach0, words));
-    // One reachable set, updated in place by the finalize: no iteration reads
-    // another's reachable words (the satisfaction test reads D' only), so
-    // reach1 names the same buffer and every parity choice picks it.
+    // One reachable set, updated in place: no iteration reads another slice's
+    // reachable words (the satisfaction test reads D' only), so reach1 names
+    // the same buffer and every parity choice picks it.
     p->reach1 = p->reach0;
     GSC_TRY(palloc(p, &p->active, words));
-    GSC_TRY(palloc(p, &p->hit, words));
-    GSC_TRY(palloc(p, &p->best, g.S));
-    const uint64_t combos = static_cast<uint64_t>(p->dil.nk) * p->dil.nl;
-    GSC_TRY(palloc(p, &p->dzw, combos * words + 4));
+    const uint64_t copies = static_cast<uint64_t>(p->dil.nk) * p->dil.nl * __builtin_popcount(p->tile.levels);
+    if (!p->direct) GSC_TRY(palloc(p, &p->dzw, copies * words));
     p->rl_words = g.slices * ((g.n[1] + 31) / 32) + 1;
     GSC_TRY(palloc(p, &p->rowlost, 2ull * p->rl_words));
-    GSC_TRY(palloc(p, &p->offz, static_cast<uint64_t>(g.n[2]) * g.mw));
-    GSC_TRY(palloc(p, &p->offv, static_cast<uint64_t>(g.n[3]) * g.ma));
-    GSC_CU(ctx, launch_sat_offsets(g, p->zt, p->wt, p->kidx, p->lidx, p->dil.nl, p->offz, p->offv, st));
+    GSC_CU(ctx, launch_rep_boxes(g, p->kidx, p->lidx, p->dil.nl, fused_args(p, 0, 0), p->reps, st));
     GSC_CU(ctx, launch_pack_bits(g, 0, p->valid, nullptr, p->validb, st));
     GSC_CU(ctx, launch_pack_bits(g, 0, p->cand, nullptr, p->candb, st));
     if (!p->safe) {
@@ -811,8 +834,12 @@ int problem_stage2(gsc_problem* p) {
         GSC_CU(ctx, launch_pack_bits(g, 4, p->valid, p->safe, p->srcb, st));
     }
     if (p->need_valid) {
-        GSC_TRY(palloc(p, &p->vzw, combos * words + 4));
-        GSC_CU(ctx, launch_dilate(g, p->validb, p->vzw, p->dil, nullptr, nullptr, 0, st));
+        GSC_TRY(palloc(p, &p->vzw, copies * words));
+        GSC_CU(ctx, launch_dilate(g, p->validb, p->validb, p->vzw, p->dil, p->tile, nullptr, nullptr, 0, st));
+        uint32_t* rowvoid = nullptr;
+        GSC_TRY(palloc(p, &rowvoid, static_cast<uint64_t>(p->rl_words)));
+        GSC_TRY(palloc(p, &p->needv, static_cast<uint64_t>(g.slices) * g.M * ((g.n[1] + 31) / 32)));
+        GSC_CU(ctx, launch_need_valid(g, fused_args(p, 0, 0), rowvoid, p->reps, p->needv, st));
     }
     return GSC_OK;
 }
@@ -849,40 +876,36 @@ FusedFixArgs fused_args(const gsc_problem* p, cudaGraphConditionalHandle cond, i
     FusedFixArgs a{};
     a.xt = p->xt;
     a.yt = p->yt;
-    a.zt = p->zt;
-    a.wt = p->wt;
     a.validb = p->validb;
     a.unsafeb = p->unsafeb;
     a.srcb = p->srcb;
     a.candb = p->candb;
-    a.dp = p->dp;
+    a.dp[0] = p->dp[0];
+    a.dp[1] = p->dp[1];
     a.reach0 = p->reach0;
-    a.reach1 = p->reach1;
     a.active = p->active;
-    a.hit = p->hit;
-    a.best = p->best;
     a.controller = p->controller;
     a.reach_step = p->reach_step;
     a.fc = p->fc;
     a.stats = p->stats;
     a.need_valid = p->need_valid;
     a.xcls = p->xcls;
-    a.xrep = p->xrep;
     a.cls_words = class_words(p->g);
-    a.max_reps = p->max_reps;
-    a.sat_threads = fused_sat_threads(p->g, p->max_reps);
+    a.reps = p->reps;
+    a.nreps = p->nreps;
+    a.pass = p->pass;
+    a.sat_threads = p->sat_threads;
+    a.direct = p->direct ? 1u : 0u;
     a.dzw = p->dzw;
     a.rowlost = p->rowlost;
     a.shard_begin = p->shard_begin;
     a.shard_slices = p->shard_slices;
     a.rl_words = p->rl_words;
     a.vzw = p->vzw;
-    a.kidx = p->kidx;
-    a.lidx = p->lidx;
-    a.nl = p->dil.nl;
+    a.needv = p->needv;
     a.dil = p->dil;
-    a.offz = p->offz;
-    a.offv = p->offv;
+    a.tile = p->tile;
+    for (int l = 0; l < kYLevels; ++l) a.ylev[l] = p->ylev[l];
     a.cond = cond;
     a.use_cond = use_cond;
     a.mirror = p->mirror;
@@ -989,7 +1012,7 @@ int gsc_problem_create(gsc_context* ctx, const gsc_abstraction* abs, const gsc_q
     p->timings.method = p->method;
     if (p->method == GSC_METHOD_FUSED) {
         p->timings.max_reps = p->max_reps;
-        p->timings.sat_threads = fused_sat_threads(p->g, p->max_reps);
+        p->timings.sat_threads = p->sat_threads;
     }
     *out = p.release();
     return GSC_OK;
@@ -1012,7 +1035,7 @@ int gsc_problem_solve(gsc_problem* p, uint32_t flags) {
     uint32_t launches = 0;
     double sat_ms = 0.0, scan_ms = 0.0;
     uint32_t sat_launches = 0;
-    const uint32_t per_iter = (p->method == GSC_METHOD_STORED) ? prefix4_launches(p->g) + 2 : 3;
+    const uint32_t per_iter = (p->method == GSC_METHOD_STORED) ? prefix4_launches(p->g) + 2 : fused_launches(p->direct);
     if (flags & GSC_SOLVE_PROFILE) {
         GSC_CU(ctx, enqueue_init(p));
         launches += 2;
@@ -1132,7 +1155,7 @@ int gsc_problem_solve(gsc_problem* p, uint32_t flags) {
         aux += hs[kStatsCols * i + 3];
     }
     if (hfc.message == kMsgDeviceTimeout)
-        return fail(ctx, GSC_ERR_TIMEOUT, "a bounded device wait for staged rows gave up; the solve stopped");
+        return fail(ctx, GSC_ERR_TIMEOUT, "a bounded device wait for staged tables gave up; the solve stopped");
     p->timings.iterations = hfc.iter;
     p->timings.pair_tests = tests;
     p->timings.aux_count = aux;
@@ -1188,8 +1211,8 @@ int gsc_problem_shard_step(gsc_problem* p, uint64_t counts[2]) {
 int gsc_problem_shard_words(const gsc_problem* p, void** dprime_words, uint64_t* words_per_slice) {
     if (!p || !dprime_words || !words_per_slice) return GSC_ERR_INVALID_ARGUMENT;
     if (p->method != GSC_METHOD_FUSED) return GSC_ERR_UNSUPPORTED;
-    *dprime_words = p->dp;
-    *words_per_slice = static_cast<uint64_t>(p->g.n[1]) * p->g.W;
+    *dprime_words = p->dp[0];
+    *words_per_slice = p->g.sw;
     return GSC_OK;
 }
 
@@ -1358,16 +1381,17 @@ int gsc_problem_phase_timings(const gsc_problem* p, gsc_phase_timings* out) {
                           static_cast<const void*>(p->zt), static_cast<const void*>(p->wt),
                           static_cast<const void*>(p->boxes), static_cast<const void*>(p->boxes16),
                           static_cast<const void*>(p->xcls),
-                          static_cast<const void*>(p->xrep), static_cast<const void*>(p->offz),
-                          static_cast<const void*>(p->offv), static_cast<const void*>(p->kidx),
+                          static_cast<const void*>(p->xrep), static_cast<const void*>(p->reps),
+                          static_cast<const void*>(p->nreps), static_cast<const void*>(p->kidx),
                           static_cast<const void*>(p->lidx), static_cast<const void*>(p->unsafe2),
                           static_cast<const void*>(p->unsafe4), static_cast<const void*>(p->safe),
                           static_cast<const void*>(p->obstacles)})
         boxes += alloc_bytes(p, q);
     uint64_t prefix = 0;
     for (const void* q : {static_cast<const void*>(p->pd), static_cast<const void*>(p->pvalid),
-                          static_cast<const void*>(p->dzw), static_cast<const void*>(p->vzw),
-                          static_cast<const void*>(p->dp), static_cast<const void*>(p->rowlost)})
+                          static_cast<const void*>(p->dzw), static_cast<const void*>(p->needv), static_cast<const void*>(p->vzw),
+                          static_cast<const void*>(p->dp[0]), static_cast<const void*>(p->dp[1]),
+                          static_cast<const void*>(p->rowlost)})
         prefix += alloc_bytes(p, q);
     out->abstraction_bytes = p->abs->bytes + boxes;
     out->prefix_bytes = prefix;

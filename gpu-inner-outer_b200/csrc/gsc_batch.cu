@@ -6,7 +6,7 @@
 // records) in the middle; all device memory comes from one growable pool.
 // The fixpoint is the batched kernels of gsc_batch_kernels.cu over every
 // instance, optionally as one CUDA graph: [init] -> while (any running)
-// { dilate, satisfaction, finalize, status }.  An instance that fills the
+// { dilate, satisfaction, status }.  An instance that fills the
 // GPU on its own (is_big_instance) iterates with the one-problem kernels
 // inside the same step and shares only init and status.  Launch shapes come
 // from the options, or from a small autotuner that times candidate shapes
@@ -38,37 +38,48 @@ InstanceDesc make_instance(const gsc_problem* p) {
     d.counts = p->counts;
     d.max_iterations = p->q.max_iterations;
     d.stats_cap = p->stats_cap;
-    d.sat_tasks = p->g.slices * p->g.mw;
-    d.words = static_cast<uint32_t>(p->g.rows * p->g.W);
+    d.words = p->g.slices * p->g.sw;
     return d;
 }
 
 size_t instance_smem(const gsc_problem* p) {
-    return fused_smem_bytes(p->g, class_words(p->g), p->need_valid, p->max_reps, false);
+    return fused_admission_bytes(p->g, p->need_valid, p->max_reps);
+}
+
+std::vector<BatchClass> batch_classes(const std::vector<const gsc_problem*>& probs) {
+    std::vector<BatchClass> out;
+    for (uint32_t k = 0; k < probs.size(); ++k) {
+        const gsc_problem* p = probs[k];
+        if (out.empty() || out.back().W != p->g.W) out.push_back(BatchClass{p->g.W, k, k, 0, 0});
+        BatchClass& c = out.back();
+        c.end = k + 1;
+        c.tasks += p->g.slices;
+        c.smem = std::max(c.smem, fused_smem_bytes(p->g, p->pass));
+    }
+    return out;
 }
 
 void build_work_list(const std::vector<const gsc_problem*>& probs, const std::vector<uint32_t>& slots,
                      uint32_t chunk, std::vector<uint32_t>& buf, WorkTotals& tot) {
     const size_t n = slots.size();
-    buf.assign(n + 4 * (n + 1), 0);
+    tot.dil_smem = 0;
+    buf.assign(work_list_words(n), 0);
     uint32_t* slot = buf.data();
     uint32_t* sat = slot + n;
     uint32_t* dil = sat + n + 1;
-    uint32_t* fin = dil + n + 1;
-    uint32_t* ini = fin + n + 1;
+    uint32_t* ini = dil + n + 1;
     for (size_t k = 0; k < n; ++k) {
         const gsc_problem* p = probs[k];
-        const uint64_t words = p->g.rows * p->g.W;
+        const uint64_t words = static_cast<uint64_t>(p->g.slices) * p->g.sw;
         const uint64_t span = std::max<uint64_t>({words, p->g.S, static_cast<uint64_t>(kStatsCols) * p->stats_cap});
         slot[k] = slots[k];
-        sat[k + 1] = sat[k] + p->g.slices * p->g.mw;
-        dil[k + 1] = dil[k] + static_cast<uint32_t>((words + chunk - 1) / chunk);
-        fin[k + 1] = fin[k] + static_cast<uint32_t>((words + chunk - 1) / chunk);
+        sat[k + 1] = sat[k] + p->g.slices;
+        dil[k + 1] = dil[k] + (p->direct ? 0u : p->g.slices * p->tile.tiles);
+        if (!p->direct) tot.dil_smem = std::max(tot.dil_smem, p->tile.smem);
         ini[k + 1] = ini[k] + static_cast<uint32_t>((span + chunk - 1) / chunk);
     }
     tot.sat = sat[n];
     tot.dil = dil[n];
-    tot.fin = fin[n];
     tot.ini = ini[n];
 }
 
@@ -77,16 +88,13 @@ WorkList device_work_list(const uint32_t* dbuf, uint32_t n, uint32_t chunk, FixC
     wl.slot = dbuf;
     wl.sat_off = dbuf + n;
     wl.dil_off = wl.sat_off + n + 1;
-    wl.fin_off = wl.dil_off + n + 1;
-    wl.ini_off = wl.fin_off + n + 1;
+    wl.ini_off = wl.dil_off + n + 1;
     wl.n = n;
     wl.chunk = chunk;
     wl.status = status;
     wl.running = running;
     return wl;
 }
-
-uint32_t wmax_of(uint32_t w) { return w <= 1 ? 1 : w == 2 ? 2 : w <= 4 ? 4 : 8; }
 
 }  // namespace gsc_api
 
@@ -118,7 +126,7 @@ struct gsc_batch {
     // Pinned staging of the instance table and the two work lists, so their
     // uploads do not wait for the set-up queued before them.
     InstanceDesc* hdesc_pin = nullptr;
-    uint32_t* hlist_pin = nullptr;   // [2][count + 4 * (count + 1)]
+    uint32_t* hlist_pin = nullptr;   // [2][work_list_words(count)]
     bool lists_uploaded = false;
     void* pin_early = nullptr;   // hplans, hrunning, hfc (from the context's pinned cache)
     void* pin_late = nullptr;    // hstats, hdesc_pin, hlist_pin (from the context's pinned cache)
@@ -129,14 +137,15 @@ struct gsc_batch {
     std::vector<std::vector<std::pair<void*, uint64_t>>> setup_tmp;
     uint32_t setup_base = 0, setup_count = gsc_context::kSetupStreams;
     cudaEvent_t stage1_ev[gsc_context::kSetupStreams] = {};
-    std::vector<uint32_t> small;     // indices of the instances the batched kernels run
+    std::vector<uint32_t> small;     // indices of the instances the batched kernels run, by row width
+    std::vector<BatchClass> classes; // their row widths
     std::vector<BigInstance> big;    // the instances the one-problem kernels run
     WorkTotals tot{}, tot_all{};
     WorkList wl{}, wl_all{};
     uint32_t step_launches = 0;      // kernel launches of one iteration step
     BatchShape shape{};
     uint32_t wmax = 1;
-    size_t smem = 0;
+    size_t smem = 0;                 // largest instance_smem of the small instances
     cudaGraphExec_t exec = nullptr;
     cudaGraph_t graph = nullptr;
     BatchShape graph_shape{};
@@ -167,6 +176,12 @@ struct ShapeKey {
 std::mutex g_tune_mu;
 std::map<ShapeKey, BatchShape> g_tuned;
 
+// Whether a launch shape takes instances of at most `smem` admission bytes a
+// task (one task per warp multiplies them).
+bool shape_admitted(const BatchShape& sh, size_t smem) {
+    return (sh.warp ? (sh.sat_threads / 32) * smem : smem) <= kFusedSmemMax;
+}
+
 uint32_t log2_ceil(uint64_t v) {
     uint32_t l = 0;
     while ((1ull << l) < v && l < 63) ++l;
@@ -183,6 +198,7 @@ int upload_list(gsc_batch* b, uint32_t chunk) {
         slots.push_back(i);
     }
     build_work_list(probs, slots, chunk, b->hlist, b->tot);
+    b->classes = batch_classes(probs);
     probs.clear();
     slots.clear();
     for (uint32_t i = 0; i < b->probs.size(); ++i) {
@@ -193,7 +209,7 @@ int upload_list(gsc_batch* b, uint32_t chunk) {
     // A new upload (autotuning) waits until the previous one has read the
     // pinned lists; the first does not wait.
     if (b->lists_uploaded) GSC_CU(b->ctx, cudaStreamSynchronize(b->ctx->stream));
-    const size_t words = b->probs.size() + 4 * (b->probs.size() + 1);
+    const size_t words = work_list_words(b->probs.size());
     uint32_t* pin_small = b->hlist_pin;
     uint32_t* pin_all = b->hlist_pin + words;
     std::memcpy(pin_small, b->hlist.data(), b->hlist.size() * 4);
@@ -208,8 +224,9 @@ int upload_list(gsc_batch* b, uint32_t chunk) {
 }
 
 cudaError_t enqueue_step(gsc_batch* b, cudaGraphConditionalHandle cond, int use_cond, uint32_t* launches) {
-    return launch_batch_step(b->ddesc, b->wl, b->tot, b->wl_all, b->big.data(), static_cast<uint32_t>(b->big.size()),
-                             b->shape, b->wmax, b->smem, sm_count(b->ctx), cond, use_cond, b->ctx->stream, launches);
+    return launch_batch_step(b->ddesc, b->wl, b->tot, b->classes.data(), static_cast<uint32_t>(b->classes.size()),
+                             b->wl_all, b->big.data(), static_cast<uint32_t>(b->big.size()), b->shape,
+                             sm_count(b->ctx), cond, use_cond, b->ctx->stream, launches);
 }
 
 int enqueue_iterations(gsc_batch* b, uint32_t count, uint32_t* launches) {
@@ -251,8 +268,9 @@ int autotune(gsc_batch* b) {
         if (e == cudaSuccess) e = cudaEventRecord(e0, ctx->stream);
         for (uint32_t done = 0; e == cudaSuccess && done < kTuneIterations; done += kTuneChunk) {
             for (uint32_t r = 0; e == cudaSuccess && r < kTuneChunk; ++r)
-                e = launch_batch_iteration(b->ddesc, b->wl, b->tot, b->shape, b->wmax, b->smem, sms, 0, 0,
-                                           ctx->stream, nullptr);
+                e = launch_batch_step(b->ddesc, b->wl, b->tot, b->classes.data(),
+                                      static_cast<uint32_t>(b->classes.size()), b->wl, nullptr, 0, b->shape, sms, 0, 0,
+                                      ctx->stream, nullptr);
             if (e == cudaSuccess) e = cudaMemcpyAsync(b->hrunning, b->drunning, 4, cudaMemcpyDeviceToHost, ctx->stream);
             if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
             if (e == cudaSuccess && *b->hrunning == 0) break;
@@ -269,7 +287,7 @@ int autotune(gsc_batch* b) {
         for (const Trial& tr : trials) {
             for (uint32_t ps : per_sm) {
                 const BatchShape cand{tr.threads, ps * static_cast<uint32_t>(sms), ch, tr.warp};
-                if (batch_sat_smem(cand, b->smem) > kFusedSmemMax) continue;
+                if (!shape_admitted(cand, b->smem)) continue;
                 float ms = 0.f;
                 status = time_shape(cand, &ms);
                 if (status != GSC_OK) break;
@@ -466,7 +484,7 @@ int batch_begin(gsc_batch* b, uint32_t count, const gsc_model_desc* models, cons
         std::string err;
         const int s = grid_from_model(&models[i], &a->g, &err);
         if (s != GSC_OK) return fail(ctx, s, "instance " + std::to_string(i) + ": " + err);
-        if (a->g.rows * a->g.W >= 0xFFFFFFFFull)
+        if (static_cast<uint64_t>(a->g.slices) * a->g.sw >= 0xFFFFFFFFull)
             return fail(ctx, GSC_ERR_UNSUPPORTED, "instance " + std::to_string(i) + ": grid too large for a batch");
         GSC_TRY(abstraction_enqueue(a.get(), ss.of(i), b->setup_tmp[i]));
         b->abs.push_back(std::move(a));
@@ -522,7 +540,7 @@ int batch_finish(gsc_batch* b, const gsc_batch_options* opt) {
         b->stats_off.push_back(stats_words);
         stats_words += static_cast<uint64_t>(kStatsCols) * b->probs[i]->stats_cap;
     }
-    const size_t list_bytes = 2 * 4ull * (count + 4ull * (count + 1));
+    const size_t list_bytes = 2 * 4ull * work_list_words(count);
     {
         const size_t bytes = ((sizeof(unsigned long long) * stats_words + 15) & ~size_t(15)) +
                              ((sizeof(InstanceDesc) * count + 15) & ~size_t(15)) + ((list_bytes + 15) & ~size_t(15));
@@ -551,15 +569,16 @@ int batch_finish(gsc_batch* b, const gsc_batch_options* opt) {
         smem = std::max(smem, instance_smem(p));
         nv_any |= p->need_valid ? 1u : 0u;
     }
-    b->wmax = wmax_of(wmax);
+    std::stable_sort(b->small.begin(), b->small.end(),
+                     [&](uint32_t x, uint32_t y) { return b->probs[x]->g.W < b->probs[y]->g.W; });
+    b->wmax = wmax;
     b->smem = smem;
-    b->step_launches = 3 * static_cast<uint32_t>(b->big.size()) + (b->small.empty() ? 0u : 3u) + 1u;
     void* q = nullptr;
     GSC_TRY(device_alloc(ctx, b->pool, b->own, b->own_bytes, &q, sizeof(InstanceDesc) * count));
     b->ddesc = static_cast<InstanceDesc*>(q);
-    GSC_TRY(device_alloc(ctx, b->pool, b->own, b->own_bytes, &q, 4ull * (count + 4ull * (count + 1))));
+    GSC_TRY(device_alloc(ctx, b->pool, b->own, b->own_bytes, &q, 4ull * work_list_words(count)));
     b->dlist = static_cast<uint32_t*>(q);
-    GSC_TRY(device_alloc(ctx, b->pool, b->own, b->own_bytes, &q, 4ull * (count + 4ull * (count + 1))));
+    GSC_TRY(device_alloc(ctx, b->pool, b->own, b->own_bytes, &q, 4ull * work_list_words(count)));
     b->dlist_all = static_cast<uint32_t*>(q);
     GSC_TRY(device_alloc(ctx, b->pool, b->own, b->own_bytes, &q, 4));
     b->drunning = static_cast<uint32_t*>(q);
@@ -575,9 +594,11 @@ int batch_finish(gsc_batch* b, const gsc_batch_options* opt) {
         return fail(ctx, GSC_ERR_INVALID_ARGUMENT, "sat_threads must be 64, 128 or 256");
     if (b->shape.chunk < 256 || b->shape.chunk % 256)
         return fail(ctx, GSC_ERR_INVALID_ARGUMENT, "chunk_words must be a positive multiple of 256");
-    if (batch_sat_smem(b->shape, smem) > kFusedSmemMax)
+    if (!shape_admitted(b->shape, smem))
         return fail(ctx, GSC_ERR_UNSUPPORTED, "batch: one task per warp needs more shared memory than a block has");
     GSC_TRY(upload_list(b, b->shape.chunk));
+    b->step_launches = static_cast<uint32_t>(b->classes.size()) + (b->tot.dil ? 1u : 0u) + 1u;
+    for (const BigInstance& x : b->big) b->step_launches += fused_launches(x.a.direct != 0);
     b->t.tuned = 0;
     if (opt && opt->autotune && !b->small.empty()) {
         uint64_t words = 0;

@@ -1,21 +1,18 @@
 // gsc_batch_kernels.cu -- the fused fixpoint over many instances at once.
 //
-// Each kernel is one launch over every listed instance: persistent blocks
-// walk a task list (instance k owns tasks off[k] .. off[k+1]-1, found by a
-// binary search) and run the same device bodies as the one-problem kernels
+// Each kernel is one launch over listed instances: blocks walk a task list
+// (instance k owns tasks off[k] .. off[k+1]-1, found by a binary search) and
+// run the same device bodies as the one-problem kernels
 // (gsc_fused_body.cuh), so an instance computes the same bits alone and in a
 // batch.  Instances that have stopped skip their tasks.  One iteration:
-//   k_batch_dilate    (theta, v)-dilated D' of every running instance;
-//   k_batch_sat       slice x omega-column tasks of every running instance;
-//   k_batch_finalize  word chunks; the last chunk of an instance (ticket)
-//                     applies its stop rules;
-//   k_batch_status    one block: a copy of every instance's control record,
-//                     the number still running, and the CUDA-graph loop
-//                     condition.
+//   k_batch_dilate  (theta, v)-dilated D' of the running instances that read it;
+//   k_batch_slice   one launch per row width, a task per slice of every running
+//                   instance of that width; an instance's last task (ticket)
+//                   applies its stop rules;
+//   k_batch_status  one block: a copy of every instance's control record, the
+//                   number still running, and the CUDA-graph loop condition.
 // Instances big enough to fill the GPU alone run the one-problem kernels in
 // the same step (launch_batch_step) and share only init and status.
-#include <atomic>
-
 #include "gsc_fused_body.cuh"
 
 namespace gsc_b200 {
@@ -55,38 +52,34 @@ __global__ void __launch_bounds__(256) k_batch_init(const InstanceDesc* __restri
 }
 
 __global__ void __launch_bounds__(256) k_batch_dilate(const InstanceDesc* __restrict__ descs, WorkList wl) {
+    extern __shared__ __align__(16) bword smem[];
     const uint32_t total = wl.dil_off[wl.n];
     for (uint32_t t = blockIdx.x; t < total; t += gridDim.x) {
+        // Instances that read D' itself have no task: the last of equal offsets.
         const uint32_t k = find_task(wl.dil_off, wl.n, t);
         const InstanceDesc& d = descs[wl.slot[k]];
         if (d.a.fc->stop) continue;
         const uint32_t c = d.a.fc->iter;
         const uint32_t* lost = c > 0 ? d.a.rowlost + (c & 1) * d.a.rl_words : nullptr;
-        uint32_t* next = d.a.rowlost + ((c + 1) & 1) * d.a.rl_words;
-        const uint32_t b = (t - wl.dil_off[k]) * wl.chunk;
-        const uint32_t end = min(b + wl.chunk, d.words);
-        // The last task also clears row-bit words beyond the positions.
-        const uint32_t span = end == d.words ? max(end, d.a.rl_words) : end;
-        for (uint32_t p = b + threadIdx.x; p < span; p += blockDim.x) {
-            if (p < d.a.rl_words) next[p] = 0;
-            if (p < end) dilate_position(d.g, d.a.dp, d.a.dzw, d.a.dil, p, lost);
-        }
+        dilate_tile(d.g, d.a.dp[c & 1], d.a.dzw, d.a.dil, d.a.tile, t - wl.dil_off[k], lost, smem);
+        __syncthreads();
     }
 }
 
+// The slices of the instances [kb, ke) of the list, whose rows have W words.
 // The instance of the current task is copied to shared memory when it
 // changes; the dynamic shared memory holds the largest instance's staging,
 // once per task group.  WARP: every warp of the block walks the task list
 // as its own group (tasks blockIdx.x * warps + warp, step gridDim.x *
 // warps), else the block is one group.
-template <int WMAX, bool WARP>
-__global__ void __launch_bounds__(256) k_batch_sat(const InstanceDesc* __restrict__ descs, WorkList wl,
-                                                   uint32_t task_words) {
+template <int W, bool WARP>
+__global__ void __launch_bounds__(256) k_batch_slice(const InstanceDesc* __restrict__ descs, WorkList wl, uint32_t kb,
+                                                     uint32_t ke, uint32_t task_words) {
     extern __shared__ __align__(16) bword smem[];
     constexpr uint32_t kGroups = WARP ? 8u : 1u;
     __shared__ __align__(16) InstanceDesc sd[kGroups];
-    __shared__ uint32_t s_meta[kGroups][4];
-    const uint32_t total = wl.sat_off[wl.n];
+    __shared__ uint32_t s_meta[kGroups][3];
+    const uint32_t first = wl.sat_off[kb], total = wl.sat_off[ke];
     const uint32_t grp = WARP ? (threadIdx.x >> 5) : 0u;
     const uint32_t ngrp = WARP ? (blockDim.x >> 5) : 1u;
     const uint32_t rank = WARP ? (threadIdx.x & 31u) : threadIdx.x;
@@ -94,8 +87,8 @@ __global__ void __launch_bounds__(256) k_batch_sat(const InstanceDesc* __restric
     bword* gsm = smem + grp * task_words;
     uint32_t cur = 0xFFFFFFFFu;
     bool stopped = false;
-    for (uint32_t t = blockIdx.x * ngrp + grp; t < total; t += gridDim.x * ngrp) {
-        const uint32_t k = find_task(wl.sat_off, wl.n, t);
+    for (uint32_t t = first + blockIdx.x * ngrp + grp; t < total; t += gridDim.x * ngrp) {
+        const uint32_t k = kb + find_task(wl.sat_off + kb, ke - kb, t);
         const uint32_t slot = wl.slot[k];
         if (slot != cur) {
             const uint32_t* src = reinterpret_cast<const uint32_t*>(descs + slot);
@@ -103,49 +96,26 @@ __global__ void __launch_bounds__(256) k_batch_sat(const InstanceDesc* __restric
             for (uint32_t i = rank; i < sizeof(InstanceDesc) / 4; i += gsize) dst[i] = src[i];
             group_sync<WARP>();
             cur = slot;
-            // An instance's stop flag changes only in the finalize kernel, so
-            // the tasks of a stopped instance are skipped without a look.
+            // An instance's stop flag changes only after its last task, so the
+            // tasks of a stopped instance are skipped without a look.
             stopped = __ldcg(&sd[grp].a.fc->stop) != 0;
         }
         if (stopped) continue;
-        sat_col_task<WMAX, false, 2, WARP>(sd[grp].g, sd[grp].a, t - wl.sat_off[k], gsm, s_meta[grp]);
+        const int done = slice_task<W, 2, 2, WARP, false>(sd[grp].g, sd[grp].a, t - wl.sat_off[k], gsm, s_meta[grp]);
+        // The counters are atomics; the barrier orders the group's before its
+        // first thread's fence (cumulative) and ticket.
         group_sync<WARP>();
-    }
-}
-
-__global__ void __launch_bounds__(256) k_batch_finalize(const InstanceDesc* __restrict__ descs, WorkList wl) {
-    __shared__ bool last;
-    const uint32_t total = wl.fin_off[wl.n];
-    for (uint32_t t = blockIdx.x; t < total; t += gridDim.x) {
-        const uint32_t k = find_task(wl.fin_off, wl.n, t);
-        const InstanceDesc& d = descs[wl.slot[k]];
-        FixControl* fc = d.a.fc;
-        // No chunk of this instance has taken its ticket yet, so its stop
-        // flag and iteration cannot change before this task's ticket.
-        if (fc->stop) continue;
-        const uint32_t it = fc->iter + 1;
-        const bword* rprev = (fc->iter & 1) ? d.a.reach1 : d.a.reach0;
-        bword* rnext = (fc->iter & 1) ? d.a.reach0 : d.a.reach1;
-        const uint64_t b = static_cast<uint64_t>(t - wl.fin_off[k]) * wl.chunk;
-        const uint64_t end = min(b + wl.chunk, static_cast<uint64_t>(d.words));
-        unsigned long long nr = 0, nc = 0;
-        for (uint64_t e = b + threadIdx.x; e < end; e += blockDim.x) finalize_word(d.g, d.a, rprev, rnext, e, it, nr, nc);
-        unsigned long long* row = d.a.stats + kStatsCols * it;
-        add_counters(row, nr, nc);
-        // The counters are atomics; the barrier orders them before the first
-        // thread's fence (cumulative) and ticket.
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            __threadfence();
-            last = atomicAdd(&fc->ticket, 1u) == wl.fin_off[k + 1] - wl.fin_off[k] - 1;
+        if (rank == 0 && done) {
+            FixControl* fc = sd[grp].a.fc;
+            if (done == 2) __threadfence();
+            if (atomicAdd(&fc->ticket, 1u) == wl.sat_off[k + 1] - wl.sat_off[k] - 1) {
+                __threadfence();
+                fc->ticket = 0;
+                const uint32_t it = __ldcg(&fc->iter) + 1;
+                control_step(fc, sd[grp].a.stats + kStatsCols * it, it);
+            }
         }
-        __syncthreads();
-        if (last && threadIdx.x == 0) {
-            __threadfence();
-            fc->ticket = 0;
-            control_step(fc, row, it);
-        }
-        __syncthreads();
+        group_sync<WARP>();
     }
 }
 
@@ -173,34 +143,26 @@ inline unsigned int grid_of(uint32_t tasks, uint32_t cap) {
     return b ? b : 1u;
 }
 
-template <int WMAX, bool WARP>
-cudaError_t launch_sat_t(const InstanceDesc* descs, const WorkList& wl, const WorkTotals& tot, const BatchShape& sh,
-                         size_t smem, cudaStream_t st) {
-    // Launches may come from several host threads (a server's loop and the
-    // caller's); setting the attribute twice is harmless.
-    static std::atomic<bool> configured[64];
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
+template <int W, bool WARP>
+cudaError_t launch_slice_t(const InstanceDesc* descs, const WorkList& wl, const BatchClass& c, const BatchShape& sh,
+                           cudaStream_t st) {
+    const cudaError_t e = allow_smem(k_batch_slice<W, WARP>);
     if (e != cudaSuccess) return e;
-    if (dev < 0 || dev >= 64 || !configured[dev].load()) {
-        e = cudaFuncSetAttribute(k_batch_sat<WMAX, WARP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(kFusedSmemMax));
-        if (e != cudaSuccess) return e;
-        if (dev >= 0 && dev < 64) configured[dev].store(true);
-    }
     const uint32_t per_block = WARP ? sh.sat_threads / 32 : 1u;
-    const uint32_t tasks = (tot.sat + per_block - 1) / per_block;
+    const uint32_t tasks = (c.tasks + per_block - 1) / per_block;
     const uint32_t blocks = sh.sat_blocks ? grid_of(tasks, sh.sat_blocks) : grid_of(tasks, 0xFFFFFFFFu);
-    k_batch_sat<WMAX, WARP><<<blocks, sh.sat_threads, batch_sat_smem(sh, smem), st>>>(
-        descs, wl, static_cast<uint32_t>(smem / sizeof(bword)));
+    k_batch_slice<W, WARP><<<blocks, sh.sat_threads, per_block * c.smem, st>>>(
+        descs, wl, c.begin, c.end, static_cast<uint32_t>(c.smem / sizeof(bword)));
     return cudaGetLastError();
 }
 
-template <int WMAX>
-cudaError_t launch_sat_w(const InstanceDesc* descs, const WorkList& wl, const WorkTotals& tot, const BatchShape& sh,
-                         size_t smem, cudaStream_t st) {
-    return sh.warp ? launch_sat_t<WMAX, true>(descs, wl, tot, sh, smem, st)
-                   : launch_sat_t<WMAX, false>(descs, wl, tot, sh, smem, st);
+template <int W>
+cudaError_t launch_slice_w(const InstanceDesc* descs, const WorkList& wl, const BatchClass& c, const BatchShape& sh,
+                           cudaStream_t st) {
+    // Warp tasks whose staging does not fit one block run one task per block.
+    return sh.warp && (sh.sat_threads / 32) * c.smem <= kFusedSmemOptIn
+               ? launch_slice_t<W, true>(descs, wl, c, sh, st)
+               : launch_slice_t<W, false>(descs, wl, c, sh, st);
 }
 
 }  // namespace
@@ -213,33 +175,33 @@ cudaError_t launch_batch_init(const InstanceDesc* descs, const WorkList& wl, con
 }
 
 cudaError_t launch_batch_step(const InstanceDesc* descs, const WorkList& small, const WorkTotals& tot_small,
-                              const WorkList& all, const BigInstance* big, uint32_t nbig, const BatchShape& sh,
-                              uint32_t wmax, size_t smem, int sms, cudaGraphConditionalHandle cond, int use_cond,
-                              cudaStream_t st, uint32_t* launches) {
-    if (sh.sat_threads < 32 || sh.sat_threads > 256 || sh.sat_threads % 32 || batch_sat_smem(sh, smem) > kFusedSmemMax)
-        return cudaErrorInvalidValue;
+                              const BatchClass* classes, uint32_t nclasses, const WorkList& all,
+                              const BigInstance* big, uint32_t nbig, const BatchShape& sh, int sms,
+                              cudaGraphConditionalHandle cond, int use_cond, cudaStream_t st, uint32_t* launches) {
+    if (sh.sat_threads < 32 || sh.sat_threads > 256 || sh.sat_threads % 32) return cudaErrorInvalidValue;
     uint32_t n = 0;
     cudaError_t e = cudaSuccess;
     // A stopped big instance's kernels return at once (they read its stop flag).
     for (uint32_t i = 0; e == cudaSuccess && i < nbig; ++i) e = launch_fused_iteration(big[i].g, big[i].a, st, &n);
     if (e == cudaSuccess && tot_small.dil) {
-        k_batch_dilate<<<grid_of(tot_small.dil, 16u * sms), 256, 0, st>>>(descs, small);
+        e = allow_smem(k_batch_dilate);
+        if (e != cudaSuccess) return e;
+        k_batch_dilate<<<grid_of(tot_small.dil, 16u * sms), 256, tot_small.dil_smem, st>>>(descs, small);
         e = cudaGetLastError();
         ++n;
     }
-    if (e == cudaSuccess && tot_small.sat) {
-        switch (wmax) {
-            case 1: e = launch_sat_w<1>(descs, small, tot_small, sh, smem, st); break;
-            case 2: e = launch_sat_w<2>(descs, small, tot_small, sh, smem, st); break;
-            case 3:
-            case 4: e = launch_sat_w<4>(descs, small, tot_small, sh, smem, st); break;
-            default: e = launch_sat_w<8>(descs, small, tot_small, sh, smem, st); break;
+    for (uint32_t i = 0; e == cudaSuccess && i < nclasses; ++i) {
+        const BatchClass& c = classes[i];
+        switch (c.W) {
+            case 1: e = launch_slice_w<1>(descs, small, c, sh, st); break;
+            case 2: e = launch_slice_w<2>(descs, small, c, sh, st); break;
+            case 3: e = launch_slice_w<3>(descs, small, c, sh, st); break;
+            case 4: e = launch_slice_w<4>(descs, small, c, sh, st); break;
+            case 5: e = launch_slice_w<5>(descs, small, c, sh, st); break;
+            case 6: e = launch_slice_w<6>(descs, small, c, sh, st); break;
+            case 7: e = launch_slice_w<7>(descs, small, c, sh, st); break;
+            default: e = launch_slice_w<8>(descs, small, c, sh, st); break;
         }
-        ++n;
-    }
-    if (e == cudaSuccess && tot_small.fin) {
-        k_batch_finalize<<<grid_of(tot_small.fin, 16u * sms), 256, 0, st>>>(descs, small);
-        e = cudaGetLastError();
         ++n;
     }
     if (e == cudaSuccess) {
@@ -249,13 +211,6 @@ cudaError_t launch_batch_step(const InstanceDesc* descs, const WorkList& small, 
     }
     if (launches) *launches += n;
     return e;
-}
-
-cudaError_t launch_batch_iteration(const InstanceDesc* descs, const WorkList& wl, const WorkTotals& tot,
-                                   const BatchShape& sh, uint32_t wmax, size_t smem, int sms,
-                                   cudaGraphConditionalHandle cond, int use_cond, cudaStream_t st,
-                                   uint32_t* launches) {
-    return launch_batch_step(descs, wl, tot, wl, nullptr, 0, sh, wmax, smem, sms, cond, use_cond, st, launches);
 }
 
 }  // namespace gsc_b200

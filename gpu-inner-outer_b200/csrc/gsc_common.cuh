@@ -39,6 +39,7 @@ struct GridInfo {
     uint32_t ma, mw, M;
     double T;
     uint32_t K;          // integration substeps
+    uint32_t xy_planes;  // x / y table planes per (theta, v) slice: see xy_plane
     double dt;           // T / K (model.hpp:33)
     uint64_t S;          // states
     uint32_t ps[4];      // padded prefix strides (grid.hpp:253-269)
@@ -46,13 +47,18 @@ struct GridInfo {
     uint32_t W;          // 32-bit words per x-row of a bit-sliced set
     uint64_t rows;       // n1 * n2 * n3 x-rows
     uint32_t slices;     // n2 * n3 (theta, v) slices
-    uint32_t magic_n1;   // fdiv(x, n1) / fdiv(x, n1 * W) multipliers (see fdiv)
-    uint32_t magic_nw;
+    uint32_t sw;         // words per slice of a bit-sliced set: n1 * W, up to a multiple of 4 (the rest 0)
+    uint32_t n1p;        // entries per plane of the y table: n1, up to a multiple of 4
+    uint32_t magic_n1;   // fdiv(x, n1) / fdiv(x, sw / 4) multipliers (see fdiv)
+    uint32_t magic_sw4;
 };
 
 // x / d for x * d < 2^32 with m = floor(2^32 / d) + 1 (m = 0 encodes d = 1).
 __host__ __device__ __forceinline__ uint32_t fdiv_magic(uint32_t d) {
     return d <= 1 ? 0u : static_cast<uint32_t>((1ull << 32) / d + 1);
+}
+__device__ __forceinline__ uint32_t fdiv_magic32(uint32_t d) {   // the same, d in 32 bits
+    return d <= 1 ? 0u : 0xFFFFFFFFu / d + 1u + (0xFFFFFFFFu % d == d - 1 ? 1u : 0u);
 }
 __device__ __forceinline__ uint32_t fdiv(uint32_t x, uint32_t m) { return m ? __umulhi(x, m) : x; }
 
@@ -77,6 +83,17 @@ struct QueryInfo {
     double cand[8];
     uint32_t max_iterations;
 };
+
+// Plane of the x / y tables (nominal successors, quantised boxes, shift
+// masks) of slice (i2, i3) and input j.  With one Euler substep x and y move
+// by dt * v * (cos, sin)(theta) of the source cell (model.hpp:34-41), the same
+// for every input, so a slice has one plane; with more substeps the input
+// acts on v and theta between them and every input has its own.  At
+__host__ __device__ __forceinline__ uint32_t xy_planes_of(uint32_t K, uint32_t M) { return K == 1 ? 1u : M; }
+__device__ __forceinline__ uint64_t xy_plane(const GridInfo& g, uint32_t i2, uint32_t i3, uint32_t j) {
+    const uint64_t q = static_cast<uint64_t>(i2) * g.n[3] + i3;
+    return g.xy_planes == 1 ? q : q * g.M + j;
+}
 
 __device__ __forceinline__ double dmul(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ double dadd(double a, double b) { return __dadd_rn(a, b); }
@@ -203,6 +220,12 @@ __host__ __device__ __forceinline__ uint32_t pack8(uint32_t a, uint32_t b, uint3
 __device__ __forceinline__ void cp_async4(void* smem_dst, const void* gmem_src) {
     const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst));
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(gmem_src) : "memory");
+}
+
+// The same for 16 bytes, both addresses 16-byte aligned (bypasses L1).
+__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src) {
+    const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst));
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(gmem_src) : "memory");
 }
 
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }

@@ -11,15 +11,13 @@
 // valid cell already reachable) and, when validity is more than safety, at
 // least one valid cell.
 //
-// One iteration = three launches:
-//   k_dilate         (theta, v)-dilated copies of D' for the box widths in use;
-//   k_sat_col        one block per (theta, v) slice x omega column: tests
-//                    every active state of the slice against every input of
-//                    the column and, per state, records the lowest satisfied
-//                    input with an atomicMin into best[] plus a hit bit;
-//   k_fused_finalize applies the hits (reachable, active, controller,
-//                    reach_step, counters), builds D' for the next iteration,
-//                    and its last block applies the stop rules.
+// One iteration is one launch: k_slice, one block per (theta, v) slice, tests
+// every active state of the slice against the slice's representative inputs
+// and updates the slice (slice_task); its last block applies the stop rules.
+// Where the boxes' (theta, v) windows are wide, k_dilate first brings the
+// dilated copies of D' up to date, and k_slice reads one word of those in
+// place of a window of D'.
+#include <algorithm>
 #include <atomic>
 
 #include "gsc_fused_body.cuh"
@@ -36,8 +34,13 @@ inline unsigned int blocks_for(uint64_t n, int threads) {
 
 using namespace fused;
 
+// Most threads of a satisfaction block: at most kSliceThreadsMax at 48
+// registers (40 warps an SM), or, where few slices share an SM,
+// kSliceThreadsWide at 64 (32 warps).
+constexpr uint32_t kSliceThreadsMax = 256, kSliceThreadsWide = 512;
+
 __global__ void k_fused_init(GridInfo g, FusedFixArgs a, const uint8_t* __restrict__ cand) {
-    const uint64_t words = g.rows * g.W;
+    const uint64_t words = static_cast<uint64_t>(g.slices) * g.sw;
     for (uint64_t e = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; e < words;
          e += static_cast<uint64_t>(gridDim.x) * blockDim.x)
         init_word(a, e);
@@ -46,24 +49,16 @@ __global__ void k_fused_init(GridInfo g, FusedFixArgs a, const uint8_t* __restri
         init_state(a, cand, s);
 }
 
-// (theta, v)-dilated copies of a bit-sliced set, one thread per word
-// position (dilate_position): after the first iteration, with the row-lost
-// records, only positions whose widest window holds a row that lost a D'
-// cell are recomputed.  The kernel also clears the row bits the next
-// finalize writes.
-__global__ void k_dilate(GridInfo g, const bword* __restrict__ src, bword* __restrict__ dst, DilateArgs d,
-                         const FixControl* fc, uint32_t* rowlost, uint32_t rl_words) {
+// Dilated copies of a bit-sliced set, one block per tile (dilate_tile).
+__global__ void __launch_bounds__(256) k_dilate(GridInfo g, const bword* src0, const bword* src1,
+                                                bword* __restrict__ dst, DilateArgs d, DilateTile t,
+                                                const FixControl* fc, const uint32_t* rowlost, uint32_t rl_words) {
+    extern __shared__ __align__(16) bword smem[];
     pdl_wait();
     if (fc && fc->stop) return;
     const uint32_t c = fc ? fc->iter : 0;
-    const uint32_t* lost = (rowlost && c > 0) ? rowlost + (c & 1) * rl_words : nullptr;
-    uint32_t* next = rowlost ? rowlost + ((c + 1) & 1) * rl_words : nullptr;
-    const uint32_t pos = static_cast<uint32_t>(g.rows * g.W);
-    const uint32_t span = next ? max(pos, rl_words) : pos;
-    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < span; p += gridDim.x * blockDim.x) {
-        if (next && p < rl_words) next[p] = 0;
-        if (p < pos) dilate_position(g, src, dst, d, p, lost);
-    }
+    const uint32_t* lost = (rowlost && c > 0) ? rowlost + static_cast<uint64_t>(c & 1) * rl_words : nullptr;
+    dilate_tile(g, (c & 1) ? src1 : src0, dst, d, t, blockIdx.x, lost, smem);
 }
 
 // The set-up plan (one block): which theta widths (wrapped lengths of the
@@ -80,12 +75,16 @@ __global__ void __launch_bounds__(256) k_plan(GridInfo g, const uint32_t* __rest
     const uint32_t tid = threadIdx.x;
     if (tid < 8) out->counts[tid] = counts[tid];
     if (tid == 0) {
-        out->flags = *flags;
+        out->flags = flags[0];
+        out->ylevels = flags[1];
         out->fused = xrep ? 1u : 0u;
     }
     if (!xrep) {
         if (tid == 0) {
             out->max_reps = 0;
+            out->ylevels = 0;
+            out->slice_reps = 0;
+            out->reps = out->rep_rows = 0;
             out->width_overflow = 0;
             out->dil = DilateArgs{};
         }
@@ -147,90 +146,176 @@ __global__ void __launch_bounds__(256) k_plan(GridInfo g, const uint32_t* __rest
     }
 }
 
-// The two parts of the word offset in dzw of a representative's dilated D'
-// row 0 (sat_col_task, phase B), (kslot * nl + lslot) * rows * W +
-// n1 * (lz + n2 * lw) * W in 32-bit arithmetic: per omega column and theta
-// cell the kslot and lz terms, per acceleration and v cell the lslot and lw
-// terms (0 for a rejected v box, which is never a representative).
-__global__ void k_sat_offsets(GridInfo g, const uint32_t* __restrict__ zt, const uint32_t* __restrict__ wt,
-                              const uint8_t* __restrict__ kidx, const uint8_t* __restrict__ lidx, uint32_t nl,
-                              uint32_t* __restrict__ offz, uint32_t* __restrict__ offv) {
-    const uint32_t n1 = g.n[1], n2 = g.n[2], W = g.W;
-    const uint32_t pos = static_cast<uint32_t>(g.rows * W);
-    const uint32_t nzt = n2 * g.mw, nwt = g.n[3] * g.ma;
-    for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < nzt + nwt; e += gridDim.x * blockDim.x) {
-        if (e < nzt) {
-            const uint32_t ze = zt[e];
-            const uint32_t lz = lo16(ze), hz = hi16(ze);
-            const uint32_t nz = (lz <= hz) ? hz - lz + 1 : n2 - lz + hz + 1;
-            offz[e] = kidx[nz] * nl * pos + n1 * lz * W;
-        } else {
-            const uint32_t we = wt[e - nzt];
-            uint32_t o = 0;
-            if (we != kReject && hi16(we) >= lo16(we)) {
-                const uint32_t lw = lo16(we), nwb = hi16(we) - lw + 1;
-                o = lidx[nwb] * pos + n1 * n2 * lw * W;
+// The boxes of one plane row in short: [i + a, i + b] alike for every cell
+// with one, those being cells [first, end).  By one warp.
+__device__ __forceinline__ bool short_boxes(const uint32_t* __restrict__ row, uint32_t n, uint32_t* ab, uint32_t* range) {
+    const uint32_t lane = threadIdx.x & 31;
+    int amin = 1 << 20, amax = -(1 << 20), bmin = 1 << 20, bmax = -(1 << 20);
+    uint32_t first = n, end = 0, cells = 0;
+    for (uint32_t i = lane; i < n; i += 32) {
+        const uint32_t e = row[i];
+        if (e == kReject) continue;
+        const int a = static_cast<int>(lo16(e)) - static_cast<int>(i), b = static_cast<int>(hi16(e)) - static_cast<int>(i);
+        amin = min(amin, a);
+        amax = max(amax, a);
+        bmin = min(bmin, b);
+        bmax = max(bmax, b);
+        first = min(first, i);
+        end = max(end, i + 1);
+        ++cells;
+    }
+    amin = __reduce_min_sync(0xFFFFFFFFu, amin);
+    amax = __reduce_max_sync(0xFFFFFFFFu, amax);
+    bmin = __reduce_min_sync(0xFFFFFFFFu, bmin);
+    bmax = __reduce_max_sync(0xFFFFFFFFu, bmax);
+    first = __reduce_min_sync(0xFFFFFFFFu, first);
+    end = __reduce_max_sync(0xFFFFFFFFu, end);
+    cells = __reduce_add_sync(0xFFFFFFFFu, cells);
+    if (!cells) {
+        *ab = *range = 0;   // no cell has a box
+        return true;
+    }
+    *ab = static_cast<uint32_t>(bmax - amin + 1) | (static_cast<uint32_t>(static_cast<uint8_t>(static_cast<int8_t>(amin))) << 8);
+    *range = pack16(first, end);
+    return amin == amax && bmin == bmax && cells == end - first && amin >= -31 && bmax <= 31 && bmax - amin < 32;
+}
+
+// SliceRep::off (kslot * nl + lslot) * slices * sw + (lz + n2 * lw) * sw and
+// the boxes in short, one warp per (slice, representative).  Offsets are sums
+// modulo 2^32 (below 2^32 with the row when the dilated copies are used).
+__global__ void __launch_bounds__(256) k_rep_boxes(const __grid_constant__ GridInfo g,
+                                                   const uint8_t* __restrict__ kidx,
+                                                   const uint8_t* __restrict__ lidx, uint32_t nl,
+                                                   const __grid_constant__ FusedFixArgs a, SliceRep* reps) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t total = static_cast<uint64_t>(g.slices) * g.M;
+    for (uint64_t t = (blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x) >> 5; t < total;
+         t += (static_cast<uint64_t>(gridDim.x) * blockDim.x) >> 5) {
+        const uint32_t s = static_cast<uint32_t>(t / g.M), k = static_cast<uint32_t>(t - static_cast<uint64_t>(s) * g.M);
+        if (k >= a.nreps[s]) continue;
+        SliceRep rp = reps[t];
+        const uint64_t pl = xy_plane(g, s % g.n[2], s / g.n[2], rp.j);
+        rp.off = (kidx[hi16(rp.zw)] * nl + lidx[hi16(rp.vw)]) * (g.slices * g.sw) +
+                 (lo16(rp.zw) + g.n[2] * lo16(rp.vw)) * g.sw;
+        const bool x = short_boxes(a.xt + pl * g.n[0], g.n[0], &rp.hx, &rp.xr);
+        const bool y = short_boxes(a.yt + pl * g.n1p, g.n[1], &rp.hy, &rp.yr);
+        rp.hx = (rp.hx & 0xFFFFu) | (x ? kBoxX : 0u) | (y ? kBoxY : 0u);
+        if (y) {
+            const uint32_t ny = rp.hy & 0xFFu, p = ny ? 31 - __clz(ny) : 0;
+            if (ny) {
+                rp.off += a.ylev[p] + static_cast<uint32_t>(static_cast<int>(static_cast<int8_t>(rp.hy >> 8)) * static_cast<int>(g.W));
+                rp.hy |= ((ny - (1u << p)) * g.W) << 16;
             }
-            offv[e - nzt] = o;
+            rp.yr = pack16(lo16(rp.yr), hi16(rp.yr) - lo16(rp.yr));
         }
+        if (lane == 0) reps[t] = rp;
     }
 }
 
-// One block per (theta, v) slice x omega column (sat_col_task); a sharded
-// solve launches the shard's slices only (task offset shard_begin * mw).
-template <int W, bool NV>
-__global__ void __launch_bounds__(kFusedWarps * 32) k_sat_col(GridInfo g, FusedFixArgs a) {
-    extern __shared__ __align__(16) bword smem[];
-    __shared__ uint32_t s_meta[4];
-    pdl_wait();
-    sat_col_task<W, true, NV ? 1 : 0, false, true>(g, a, blockIdx.x + a.shard_begin * g.mw, smem, s_meta);
+// Rows with a void (invalid yet safe) cell, one warp per 32 rows of a slice.
+__global__ void k_row_void(GridInfo g, const bword* __restrict__ validb, const bword* __restrict__ unsafeb,
+                           uint32_t* __restrict__ rowvoid) {
+    const uint32_t W1 = (g.n[1] + 31) / 32, lane = threadIdx.x & 31;
+    const uint64_t total = static_cast<uint64_t>(g.slices) * W1;
+    for (uint64_t t = (blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x) >> 5; t < total;
+         t += (static_cast<uint64_t>(gridDim.x) * blockDim.x) >> 5) {
+        const uint64_t slice = t / W1;
+        const uint32_t y = static_cast<uint32_t>(t - slice * W1) * 32 + lane;
+        bool any = false;
+        for (uint32_t w = 0; w < g.W && y < g.n[1]; ++w) {
+            const uint64_t e = slice * g.sw + y * g.W + w;
+            const uint32_t cells = min(32u, g.n[0] - w * kBits);
+            const bword in = cells == 32 ? ~0u : (1u << cells) - 1;
+            any |= (~validb[e] & ~unsafeb[e] & in) != 0;
+        }
+        const uint32_t m = __ballot_sync(0xFFFFFFFFu, any);
+        if (lane == 0) rowvoid[t] = m;
+    }
 }
 
-// Apply the iteration's hits, build next iteration's D', count, and let the
-// last block to finish apply the stop rules (reachability.hpp:133-144).  One
-// thread per word; the reachable set is updated in place.  A sharded solve
-// finalizes the shard's words only and leaves the stop rules to the host,
-// which applies them with every rank's counts.
-__global__ void __launch_bounds__(256) k_fused_finalize(GridInfo g, FusedFixArgs a) {
-    pdl_wait();
+// needv, one warp per (slice, representative), lanes over the rows.
+template <int W>
+__global__ void __launch_bounds__(256) k_need_valid(const __grid_constant__ GridInfo g,
+                                                    const __grid_constant__ FusedFixArgs a,
+                                                    const uint32_t* __restrict__ rowvoid, SliceRep* reps,
+                                                    uint32_t* __restrict__ needv) {
+    const uint32_t n1 = g.n[1], n2 = g.n[2], W1 = (n1 + 31) / 32, lane = threadIdx.x & 31;
+    const uint64_t total = static_cast<uint64_t>(g.slices) * g.M;
+    for (uint64_t t = (blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x) >> 5; t < total;
+         t += (static_cast<uint64_t>(gridDim.x) * blockDim.x) >> 5) {
+        const uint32_t s = static_cast<uint32_t>(t / g.M), k = static_cast<uint32_t>(t - static_cast<uint64_t>(s) * g.M);
+        if (k >= a.nreps[s]) continue;
+        const SliceRep rp = reps[t];
+        const uint64_t pl = xy_plane(g, s % n2, s / n2, rp.j);
+        auto void_word = [&](uint32_t q) {
+            uint32_t m = 0xFFFFFFFFu, z = lo16(rp.zw);
+            for (uint32_t i = 0; i < hi16(rp.zw) && m; ++i) {
+                for (uint32_t v = 0; v < hi16(rp.vw); ++v)
+                    m &= rowvoid[static_cast<uint64_t>(z + n2 * (lo16(rp.vw) + v)) * W1 + q];
+                z = (z + 1 == n2) ? 0 : z + 1;
+            }
+            return m;
+        };
+        bool some = false;
+        for (uint32_t q = 0; q < W1; ++q) {
+            const uint32_t y = q * 32 + lane;
+            const uint32_t ye = y < n1 ? a.yt[pl * g.n1p + y] : kReject;
+            bool need = false;
+            if (ye != kReject) {
+                const uint32_t ylo = lo16(ye), yhi = hi16(ye), wl = ylo >> 5, wh = yhi >> 5;
+                const uint32_t lo = void_word(wl), hi = wh != wl ? void_word(wh) : 0u;
+                if (!(~__funnelshift_r(lo, hi, ylo & 31) << (31u - (yhi - ylo)))) {
+                    bword V[W], m[W];
+                    valid_window<W>(g, a.validb, rp.zw, rp.vw, ye, V);
+                    const bword* src = a.srcb + static_cast<uint64_t>(s) * g.sw + y * W;
+                    const uint32_t* xrow = a.xt + pl * g.n[0];
+                    for (int w = 0; w < W; ++w) m[w] = src[w];
+                    without_cell<W>(xrow, V, m);
+                    for (int w = 0; w < W; ++w) {
+                        // without_cell also drops states that have no box.
+                        need |= m[w] != 0;
+                    }
+                }
+            }
+            const uint32_t bits = __ballot_sync(0xFFFFFFFFu, need);
+            if (lane == 0) needv[t * W1 + q] = bits;
+            some |= bits != 0;
+        }
+        if (some && lane == 0) reps[t].vw = rp.vw | 0x80000000u;
+    }
+}
+
+// One block per (theta, v) slice (slice_task); a sharded solve launches the
+// shard's slices only.  The last block to finish applies the stop rules
+// (reachability.hpp:133-144), except in a sharded solve.
+template <int W, int SHARED, int DIRECT, bool WIDE>
+__global__ void __launch_bounds__(WIDE ? kSliceThreadsWide : kSliceThreadsMax, WIDE ? 2 : 5)
+    k_slice(const __grid_constant__ GridInfo g, const __grid_constant__ FusedFixArgs a) {
+    extern __shared__ __align__(16) bword smem[];
+    __shared__ uint32_t s_meta[3];
     FixControl* fc = a.fc;
-    if (fc->stop) {
+    const int done = slice_task<W, SHARED, DIRECT, false, true>(g, a, blockIdx.x + a.shard_begin, smem, s_meta);
+    if (!done) {
         // Already stopped (e.g. max_iterations == 0): the graph loop must still end.
         if (a.use_cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(a.cond, 0u);
         if (a.mirror && blockIdx.x == 0 && threadIdx.x == 0) write_mirror(a.mirror, fc);
         return;
     }
-    const uint32_t it = fc->iter + 1;
-    const uint64_t nw = static_cast<uint64_t>(g.n[1]) * g.W;
-    const uint64_t first = static_cast<uint64_t>(a.shard_begin) * nw;
-    const uint64_t words = a.shard_slices ? a.shard_slices * nw : g.rows * g.W;
-    unsigned long long nr = 0, nc = 0;
-    for (uint64_t k = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; k < words;
-         k += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
-        finalize_word(g, a, a.reach0, a.reach0, first + k, it, nr, nc);
-    }
-    unsigned long long* row = a.stats + kStatsCols * it;
-    add_counters(row, nr, nc);
-    // Last block to finish: every block's counters are in.  The counters are
-    // device-scope atomics; the barrier orders a block's atomics before its
-    // first thread's fence (cumulative) and ticket.  Nothing else the last
-    // block reads was written by this kernel's other blocks.
-    __shared__ bool last;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        last = atomicAdd(&fc->ticket, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (!last) return;
-    if (threadIdx.x == 0) {
-        __threadfence();
-        fc->ticket = 0;
-        if (a.shard_slices) return;
-        control_step(fc, row, it);
-        if (a.use_cond) cudaGraphSetConditional(a.cond, fc->stop ? 0u : 1u);
-        if (a.mirror) write_mirror(a.mirror, fc);
-    }
+    if (a.shard_slices) return;
+    // The counters are device-scope atomics; the barrier orders a block's
+    // atomics before its first thread's fence (cumulative) and ticket, and a
+    // block without any has nothing to order.  Nothing else the last block
+    // reads was written by this kernel's others.
+    if (done == 2) __syncthreads();
+    if (threadIdx.x != 0) return;
+    if (done == 2) __threadfence();
+    if (atomicAdd(&fc->ticket, 1u) != gridDim.x - 1) return;
+    __threadfence();
+    fc->ticket = 0;
+    const uint32_t it = __ldcg(&fc->iter) + 1;
+    control_step(fc, a.stats + kStatsCols * it, it);
+    if (a.use_cond) cudaGraphSetConditional(a.cond, fc->stop ? 0u : 1u);
+    if (a.mirror) write_mirror(a.mirror, fc);
 }
 
 // Stop rules of a sharded iteration with the summed counts of every rank.
@@ -245,36 +330,77 @@ __global__ void k_shard_control(FixControl* fc, unsigned long long* stats, unsig
     fc->last_new = 0xFFFFFFFFu;   // every iteration of a sharded solve tests every pair
 }
 
-template <int W, bool NV>
-cudaError_t launch_sat_col_t(const GridInfo& g, const FusedFixArgs& a, size_t sm, cudaStream_t st) {
-    // Opting in above 48 KB of shared memory is a per-device function attribute.
-    // Launches may come from several host threads (a server's loop and the
-    // caller's); setting the attribute twice is harmless.
-    static std::atomic<bool> configured[64];
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
+template <int W, int SHARED, int DIRECT, bool WIDE>
+cudaError_t launch_slice_v(const GridInfo& g, const FusedFixArgs& a, cudaStream_t st) {
+    const cudaError_t e = allow_smem(k_slice<W, SHARED, DIRECT, WIDE>);
     if (e != cudaSuccess) return e;
-    if (dev < 0 || dev >= 64 || !configured[dev].load()) {
-        e = cudaFuncSetAttribute(k_sat_col<W, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(kFusedSmemMax));
-        if (e != cudaSuccess) return e;
-        if (dev >= 0 && dev < 64) configured[dev].store(true);
-    }
     const uint32_t slices = a.shard_slices ? a.shard_slices : g.slices;
-    return launch_pdl(k_sat_col<W, NV>, dim3(slices * g.mw), dim3(a.sat_threads), sm, st, g, a);
+    return launch_pdl(k_slice<W, SHARED, DIRECT, WIDE>, dim3(slices), dim3(a.sat_threads), fused_smem_bytes(g, a.pass),
+                      st, g, a);
+}
+
+template <int W, int SHARED, int DIRECT>
+cudaError_t launch_slice_t(const GridInfo& g, const FusedFixArgs& a, cudaStream_t st) {
+    return a.sat_threads > kSliceThreadsMax ? launch_slice_v<W, SHARED, DIRECT, true>(g, a, st)
+                                            : launch_slice_v<W, SHARED, DIRECT, false>(g, a, st);
+}
+
+template <int W>
+cudaError_t launch_slice_w(const GridInfo& g, const FusedFixArgs& a, cudaStream_t st) {
+    if (g.xy_planes == 1) return a.direct ? launch_slice_t<W, 1, 1>(g, a, st) : launch_slice_t<W, 1, 0>(g, a, st);
+    return a.direct ? launch_slice_t<W, 0, 1>(g, a, st) : launch_slice_t<W, 0, 0>(g, a, st);
 }
 
 }  // namespace
 
-uint32_t fused_sat_threads(const GridInfo& g, uint32_t max_reps) {
-    const uint64_t work = static_cast<uint64_t>(max_reps) * g.n[1] * g.W;
-    return work <= 2304 ? 128u : 256u;
+uint32_t fused_sat_threads(const GridInfo& g, uint32_t slice_reps) {
+    // A packed row of the slice per thread, for several representatives side
+    // by side.  As wide as lets every slice's block be resident at once (a
+    // second wave of a few blocks doubles an iteration), and at least 128.
+    const uint32_t per_sm = (g.slices + 147) / 148;
+    uint32_t most = per_sm <= 2 ? kSliceThreadsWide / per_sm * 2 : per_sm <= 10 ? 40 / per_sm * 32 : 128;
+    most = std::min(per_sm <= 2 ? kSliceThreadsWide : kSliceThreadsMax, std::max(128u, most));
+    const uint64_t items = static_cast<uint64_t>(g.n[1]) * std::max(1u, slice_reps);
+    return static_cast<uint32_t>(std::min<uint64_t>(most, (items + 31) & ~31ull));
 }
 
-size_t fused_smem_bytes(const GridInfo& g, uint32_t cls_words, int need_valid, uint32_t max_reps, bool bulk) {
-    const FusedSmemLayout L =
-        fused_smem_layout(g.n[1] * g.W, need_valid ? 2u : 1u, max_reps, cls_words, g.n[1], g.ma, bulk);
-    return sizeof(bword) * static_cast<size_t>(L.total);
+size_t fused_admission_bytes(const GridInfo& g, int need_valid, uint32_t max_reps) {
+    // Bulk-staged (16-byte slots three words longer) or word by word,
+    // whichever is more.
+    auto r4 = [](uint64_t x) { return (x + 3) & ~uint64_t(3); };
+    const uint64_t nw = static_cast<uint64_t>(g.n[1]) * g.W, nv = need_valid ? 2 : 1, mr = max_reps;
+    const uint64_t cw = 4 + (kShiftMax + 1) * g.W, n1 = g.n[1], w1 = (n1 + 31) / 32, ma = g.ma;
+    const uint64_t words = nw + mr * nv * nw + mr * nw + mr * cw + mr * n1 + 3 * ma + mr * w1;
+    uint64_t bulk = r4(r4(nw) + mr * nv * r4(nw + 3) + mr * nw) + mr * r4(cw + 3) + mr * r4(n1 + 3) + 3 * ma + mr * w1;
+    bulk = ((bulk + ma + 1) & ~uint64_t(1)) + 2;
+    return static_cast<size_t>(sizeof(bword) * std::max(words, bulk));
+}
+
+size_t fused_smem_bytes(const GridInfo& g, uint32_t pass) {
+    const uint64_t w1 = (g.n[1] + 31) / 32;
+    return sizeof(bword) * static_cast<size_t>(
+                               (8ull * pass + g.sw + pass * w1 + 2 * w1 + kHitNotes * (g.W + 1) + (g.n[1] <= kPackedRows ? (g.n[1] + 1) / 2 : 0) + 3) & ~3ull);
+}
+
+uint32_t fused_pass(const GridInfo& g, uint32_t slice_reps) {
+    // Up to 256 representatives, and 4 KB of changed rows.
+    const uint32_t w1 = (g.n[1] + 31) / 32;
+    return std::min(std::max(1u, slice_reps), std::max(1u, std::min(256u, 1024u / w1)));
+}
+
+DilateTile dilate_tile_of(const GridInfo& g, const DilateArgs& d, uint32_t levels) {
+    DilateTile t{};
+    t.levels = levels ? levels : 1u;
+    uint32_t halo = 0;
+    for (uint32_t p = 0; p < static_cast<uint32_t>(kYLevels); ++p)
+        if ((t.levels >> p) & 1u) halo = (1u << p) - 1;
+    // A tile's (theta, v) copies take at most 40 KB of shared memory.
+    const uint32_t row = d.nk * d.nl * g.W * 4;
+    const uint32_t fit = std::max<uint32_t>(1u, 40u * 1024u / row);
+    t.rows = std::min(g.n[1], fit > halo ? std::max<uint32_t>(fit - halo, 1u) : 1u);
+    t.tiles = (g.n[1] + t.rows - 1) / t.rows;
+    t.smem = std::min(g.n[1], t.rows + halo) * row;
+    return t;
 }
 
 cudaError_t launch_plan(const GridInfo& g, const uint32_t* zt, const uint32_t* wt, const uint8_t* xrep,
@@ -285,19 +411,43 @@ cudaError_t launch_plan(const GridInfo& g, const uint32_t* zt, const uint32_t* w
     return cudaGetLastError();
 }
 
-cudaError_t launch_dilate(const GridInfo& g, const bword* src, bword* dst, const DilateArgs& d, const FixControl* fc,
-                          uint32_t* rowlost, uint32_t rl_words, cudaStream_t st) {
-    const uint64_t pos = g.rows * g.W;
-    uint64_t b = (pos + 255) / 256;
-    if (b > 8192) b = 8192;
-    return launch_pdl(k_dilate, dim3(static_cast<unsigned int>(b ? b : 1)), dim3(256), 0, st, g, src, dst, d, fc,
-                      rowlost, rl_words);
+cudaError_t launch_dilate(const GridInfo& g, const bword* src0, const bword* src1, bword* dst, const DilateArgs& d,
+                          const DilateTile& t, const FixControl* fc, const uint32_t* rowlost, uint32_t rl_words,
+                          cudaStream_t st) {
+    cudaError_t e = allow_smem(k_dilate);
+    if (e != cudaSuccess) return e;
+    return launch_pdl(k_dilate, dim3(g.slices * t.tiles), dim3(256), t.smem, st, g, src0, src1, dst, d, t, fc, rowlost,
+                      rl_words);
 }
 
-cudaError_t launch_sat_offsets(const GridInfo& g, const uint32_t* zt, const uint32_t* wt, const uint8_t* kidx,
-                               const uint8_t* lidx, uint32_t nl, uint32_t* offz, uint32_t* offv, cudaStream_t st) {
-    const uint64_t n = static_cast<uint64_t>(g.n[2]) * g.mw + static_cast<uint64_t>(g.n[3]) * g.ma;
-    k_sat_offsets<<<blocks_for(n, 256), 256, 0, st>>>(g, zt, wt, kidx, lidx, nl, offz, offv);
+template <int W>
+cudaError_t launch_need_valid_t(const GridInfo& g, const FusedFixArgs& a, const uint32_t* rowvoid, SliceRep* reps,
+                                uint32_t* needv, cudaStream_t st) {
+    const uint64_t b = std::min<uint64_t>(148ull * 32, (static_cast<uint64_t>(g.slices) * g.M + 7) / 8);
+    k_need_valid<W><<<static_cast<unsigned int>(b), 256, 0, st>>>(g, a, rowvoid, reps, needv);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_need_valid(const GridInfo& g, const FusedFixArgs& a, uint32_t* rowvoid, SliceRep* reps,
+                              uint32_t* needv, cudaStream_t st) {
+    const uint64_t words = static_cast<uint64_t>(g.slices) * ((g.n[1] + 31) / 32);
+    k_row_void<<<blocks_for(words * 32, 256), 256, 0, st>>>(g, a.validb, a.unsafeb, rowvoid);
+    switch (g.W) {
+        case 1: return launch_need_valid_t<1>(g, a, rowvoid, reps, needv, st);
+        case 2: return launch_need_valid_t<2>(g, a, rowvoid, reps, needv, st);
+        case 3: return launch_need_valid_t<3>(g, a, rowvoid, reps, needv, st);
+        case 4: return launch_need_valid_t<4>(g, a, rowvoid, reps, needv, st);
+        case 5: return launch_need_valid_t<5>(g, a, rowvoid, reps, needv, st);
+        case 6: return launch_need_valid_t<6>(g, a, rowvoid, reps, needv, st);
+        case 7: return launch_need_valid_t<7>(g, a, rowvoid, reps, needv, st);
+        default: return launch_need_valid_t<8>(g, a, rowvoid, reps, needv, st);
+    }
+}
+
+cudaError_t launch_rep_boxes(const GridInfo& g, const uint8_t* kidx, const uint8_t* lidx, uint32_t nl,
+                             const FusedFixArgs& a, SliceRep* reps, cudaStream_t st) {
+    const uint64_t b = std::min<uint64_t>(148ull * 32, (static_cast<uint64_t>(g.slices) * g.M + 7) / 8);
+    k_rep_boxes<<<static_cast<unsigned int>(b), 256, 0, st>>>(g, kidx, lidx, nl, a, reps);
     return cudaGetLastError();
 }
 
@@ -307,7 +457,12 @@ cudaError_t launch_fused_init(const GridInfo& g, const FusedFixArgs& a, const ui
 }
 
 cudaError_t launch_shard_iteration(const GridInfo& g, const FusedFixArgs& a, cudaStream_t st) {
-    return launch_fused_iteration(g, a, st, nullptr, nullptr);
+    cudaError_t e = launch_fused_iteration(g, a, st, nullptr, nullptr);
+    if (e != cudaSuccess) return e;
+    // The ranks exchange dp[0]: the shard's new D' goes there.
+    const uint64_t sw = g.sw, first = a.shard_begin * sw;
+    return cudaMemcpyAsync(a.dp[0] + first, a.dp[1] + first, a.shard_slices * sw * sizeof(bword),
+                           cudaMemcpyDeviceToDevice, st);
 }
 
 cudaError_t launch_shard_control(FixControl* fc, unsigned long long* stats, unsigned long long new_reachable,
@@ -316,40 +471,34 @@ cudaError_t launch_shard_control(FixControl* fc, unsigned long long* stats, unsi
     return cudaGetLastError();
 }
 
+// Device time of an iteration (dilation + satisfaction + finalize launches
+// of one block per (slice, omega column), against this):
+//   65x65x38x25 x 100     38 -> 17 us       published demo   88 -> 54 us
+//   128x128x72x48 x 144  518 -> 135 us      47x83x29x17 x 63  24 -> 19 us
 cudaError_t launch_fused_iteration(const GridInfo& g, const FusedFixArgs& a, cudaStream_t st, uint32_t* launches,
                                    cudaEvent_t* ev) {
     if (ev) cudaEventRecord(ev[0], st);
-    // A sharded solve dilates the whole grid every iteration: the other
-    // ranks' D' slabs arrive without row-lost records.
-    cudaError_t derr = launch_dilate(g, a.dp, a.dzw, a.dil, a.fc, a.shard_slices ? nullptr : a.rowlost, a.rl_words, st);
-    if (derr != cudaSuccess) return derr;
-    if (ev) cudaEventRecord(ev[1], st);
-    const size_t sm = fused_smem_bytes(g, a.cls_words, a.need_valid, a.max_reps, true);
-    cudaError_t err;
-#define GSC_SAT_CASE(Wn)                                                                         \
-    case Wn:                                                                                     \
-        err = a.need_valid ? launch_sat_col_t<Wn, true>(g, a, sm, st) : launch_sat_col_t<Wn, false>(g, a, sm, st); \
-        break;
-    switch (g.W) {
-        GSC_SAT_CASE(1)
-        GSC_SAT_CASE(2)
-        GSC_SAT_CASE(3)
-        GSC_SAT_CASE(4)
-        GSC_SAT_CASE(5)
-        GSC_SAT_CASE(6)
-        GSC_SAT_CASE(7)
-        default:
-            err = a.need_valid ? launch_sat_col_t<8, true>(g, a, sm, st) : launch_sat_col_t<8, false>(g, a, sm, st);
-            break;
+    cudaError_t err = cudaSuccess;
+    if (!a.direct) {
+        // A sharded solve reads dp[0] and dilates the whole grid every
+        // iteration: the other ranks' D' slabs arrive without row-lost records.
+        err = launch_dilate(g, a.dp[0], a.shard_slices ? a.dp[0] : a.dp[1], a.dzw, a.dil, a.tile, a.fc,
+                            a.shard_slices ? nullptr : a.rowlost, a.rl_words, st);
+        if (err != cudaSuccess) return err;
     }
-#undef GSC_SAT_CASE
-    if (err != cudaSuccess) return err;
+    if (ev) cudaEventRecord(ev[1], st);
+    switch (g.W) {
+        case 1: err = launch_slice_w<1>(g, a, st); break;
+        case 2: err = launch_slice_w<2>(g, a, st); break;
+        case 3: err = launch_slice_w<3>(g, a, st); break;
+        case 4: err = launch_slice_w<4>(g, a, st); break;
+        case 5: err = launch_slice_w<5>(g, a, st); break;
+        case 6: err = launch_slice_w<6>(g, a, st); break;
+        case 7: err = launch_slice_w<7>(g, a, st); break;
+        default: err = launch_slice_w<8>(g, a, st); break;
+    }
+    if (launches) *launches += fused_launches(a.direct != 0);
     if (ev) cudaEventRecord(ev[5], st);
-    const uint64_t words = a.shard_slices ? static_cast<uint64_t>(a.shard_slices) * g.n[1] * g.W : g.rows * g.W;
-    uint64_t fb = (words + 255) / 256;
-    if (fb > 4096) fb = 4096;
-    if (launches) *launches += 3;
-    err = launch_pdl(k_fused_finalize, dim3(static_cast<unsigned int>(fb ? fb : 1)), dim3(256), 0, st, g, a);
     if (ev) cudaEventRecord(ev[6], st);
     return err;
 }

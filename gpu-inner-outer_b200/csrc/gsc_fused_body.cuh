@@ -37,20 +37,43 @@ __device__ __forceinline__ bword moved_word(const bword (&F)[WMAX], int w, int d
     return __funnelshift_r(up ? f0 : fm1, up ? fp1 : f0, static_cast<uint32_t>(d) & 31u);
 }
 
+// The bits of word w of a row at cell x and beyond (PTX shl gives 0 for a
+// shift of 32 or more).
+__device__ __forceinline__ bword bits_from(uint32_t x, int w) {
+    const int s = max(static_cast<int>(x) - w * kBits, 0);
+    bword m;
+    asm("shl.b32 %0, %1, %2;" : "=r"(m) : "r"(0xFFFFFFFFu), "r"(s));
+    return m;
+}
+
+// The states m of a row (from state srow on) satisfied by input j: a state is
+// satisfied in one iteration only, so its controller entry, still empty,
+// takes the lowest input by atomicMin.
+template <int W>
+__device__ __forceinline__ void take_hits(const FusedFixArgs& a, uint64_t srow, uint32_t j, bword* hits,
+                                          const bword (&m)[W]) {
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+        if (!m[w]) continue;
+        atomicOr(hits + w, m[w]);
+        for (bword t = m[w]; t; t &= t - 1) atomicMin(a.controller + srow + w * kBits + __ffs(t) - 1, j);
+    }
+}
+
 // Initial sets of word e: reachable = candidate, active = valid && safe
 // source, D' = (valid && !candidate) || unsafe.
 __device__ __forceinline__ void init_word(const FusedFixArgs& a, uint64_t e) {
     const bword c = a.candb[e];
     a.reach0[e] = c;
     a.active[e] = a.srcb[e];
-    a.hit[e] = 0;
-    a.dp[e] = (a.validb[e] & ~c) | a.unsafeb[e];
+    const bword d = (a.validb[e] & ~c) | a.unsafeb[e];
+    a.dp[0][e] = d;
+    a.dp[1][e] = d;
 }
 
 __device__ __forceinline__ void init_state(const FusedFixArgs& a, const uint8_t* cand, uint64_t s) {
     a.controller[s] = kInvalid32;
     a.reach_step[s] = cand[s] ? 0u : kInvalid32;
-    a.best[s] = kInvalid32;
 }
 
 // FixControl at the start of a solve (counts: [0] valid, [1] candidates).
@@ -70,71 +93,87 @@ __device__ __forceinline__ void init_control(FixControl* fc, uint32_t max_iterat
     fc->message = (max_iterations == 0) ? 3u : 0u;
 }
 
-// (theta, v)-dilated copies of a bit-sliced set at word position p: for
-// every theta width k in d.kval and v width l in d.lval, out[combo][y][z][v]
-// = OR of src over theta cells z .. z+k-1 (wrapped) and v cells v .. v+l-1
-// (entries whose v window leaves the grid are never read and are left 0).
-// The theta ORs are extended incrementally.
-// With `lost` (the rows that lost a D' cell since the last dilation) the
-// position is left as it is when no row of its widest window did.
-__device__ __forceinline__ void dilate_position(const GridInfo& g, const bword* __restrict__ src,
-                                                bword* __restrict__ dst, const DilateArgs& d, uint32_t p,
-                                                const uint32_t* __restrict__ lost) {
+// Dilated copies of one tile (rows [y0, y0 + t.rows) of one slice), by the
+// whole block: for every theta width k in d.kval and v width l in d.lval, the
+// OR of src over theta cells z .. z+k-1 (wrapped) and v cells v .. v+l-1
+// (copies whose v window leaves the grid are never read and are left 0), and
+// of that over the 2^p rows from each row on for every y level p in use.  The
+// theta ORs are extended incrementally, the y ORs read shared memory.
+// With `lost` (the rows that lost a D' cell since the last dilation) the tile
+// is left as it is when no row that it reads did.
+__device__ __forceinline__ void dilate_tile(const GridInfo& g, const bword* __restrict__ src, bword* __restrict__ dst,
+                                            const DilateArgs& d, const DilateTile& t, uint32_t task,
+                                            const uint32_t* __restrict__ lost, bword* smem) {
     const uint32_t n1 = g.n[1], n2 = g.n[2], n3 = g.n[3], W = g.W;
-    const uint32_t pos = static_cast<uint32_t>(g.rows * W);
-    const uint32_t kmax = d.kval[d.nk - 1];
-    const uint32_t lmax = d.lval[d.nl - 1];
-    const uint32_t r = p / W, wd = p - r * W;
-    const uint32_t y = r % n1, q = r / n1;
-    const uint32_t z = q % n2, v = q / n2;
+    const uint32_t pos = g.slices * g.sw;
+    const uint32_t kmax = d.kval[d.nk - 1], lmax = d.lval[d.nl - 1];
+    const uint32_t slice = task / t.tiles, y0 = (task - slice * t.tiles) * t.rows;
+    const uint32_t z = slice % n2, v = slice / n2;
     const uint32_t lfit = min(lmax, n3 - v);   // v windows that stay inside the grid
+    const uint32_t halo = (1u << (31 - __clz(t.levels))) - 1;
+    const uint32_t y1 = min(n1, y0 + t.rows), y2 = min(n1, y1 + halo);
     if (lost) {
-        // Every bit of the window is read (no early exit), so the loads of
-        // several theta cells are in flight together.  The row-lost words
-        // hold W1 = ceil(n1 / 32) words per (theta, v) slice, bit y % 32 of
-        // word y / 32 for row y.
-        const uint32_t W1 = (n1 + 31) / 32, yw = y >> 5, yb = y & 31;
-        uint32_t hit = 0, zz = z;
-#pragma unroll 4
+        // The row-lost words hold W1 = ceil(n1 / 32) words per (theta, v)
+        // slice, bit y % 32 of word y / 32 for row y.
+        const uint32_t W1 = (n1 + 31) / 32, w0 = y0 >> 5, nwin = kmax * lfit, ny = ((y2 - 1) >> 5) - w0 + 1;
+        uint32_t hit = 0;
+        for (uint32_t e = threadIdx.x; e < nwin * ny; e += blockDim.x) {
+            const uint32_t yw = w0 + e / nwin, q = e % nwin, j = q / kmax;
+            uint32_t zz = z + (q - j * kmax);
+            if (zz >= n2) zz -= n2;
+            uint32_t m = lost[(zz + n2 * (v + j)) * W1 + yw];
+            if (yw == w0) m &= 0xFFFFFFFFu << (y0 & 31);
+            if (yw == (y2 - 1) >> 5) m &= 0xFFFFFFFFu >> (31 - ((y2 - 1) & 31));
+            hit |= m;
+        }
+        if (!__syncthreads_or(hit != 0)) return;
+    }
+    const uint32_t words = (y2 - y0) * W, ncombo = d.nk * d.nl;
+    for (uint32_t e = threadIdx.x; e < words; e += blockDim.x) {
+        bword zor[kMaxDilate];
+#pragma unroll
+        for (uint32_t j = 0; j < kMaxDilate; ++j) zor[j] = 0;
+        uint32_t ki = 0, zz = z;
+#pragma unroll 2
         for (uint32_t i = 0; i < kmax; ++i) {
 #pragma unroll
-            for (uint32_t j = 0; j < kMaxDilate; ++j) {
-                if (j < lfit) {
-                    hit |= (lost[(zz + n2 * (v + j)) * W1 + yw] >> yb) & 1u;
-                }
-            }
+            for (uint32_t j = 0; j < kMaxDilate; ++j)
+                if (j < lfit) zor[j] |= __ldg(src + static_cast<uint64_t>(zz + n2 * (v + j)) * g.sw + y0 * W + e);
             zz = (zz + 1 == n2) ? 0 : zz + 1;
-        }
-        if (!hit) return;
-    }
-    bword zor[kMaxDilate];
+            if (i + 1 == d.kval[ki]) {
+                bword acc = 0;
+                uint32_t li = 0;
 #pragma unroll
-    for (uint32_t j = 0; j < kMaxDilate; ++j) zor[j] = 0;
-    uint32_t ki = 0, zz = z;
-#pragma unroll 2
-    for (uint32_t i = 0; i < kmax; ++i) {
-#pragma unroll
-        for (uint32_t j = 0; j < kMaxDilate; ++j)
-            if (j < lfit) zor[j] |= __ldg(src + (y + n1 * (zz + n2 * (v + j))) * W + wd);
-        zz = (zz + 1 == n2) ? 0 : zz + 1;
-        if (i + 1 == d.kval[ki]) {
-            bword acc = 0;
-            uint32_t li = 0;
-#pragma unroll
-            for (uint32_t j = 0; j < kMaxDilate; ++j) {
-                acc |= zor[j];
-                if (li < d.nl && j + 1 == d.lval[li]) {
-                    dst[static_cast<uint64_t>(ki * d.nl + li) * pos + p] = (j < lfit) ? acc : 0u;
-                    ++li;
+                for (uint32_t j = 0; j < kMaxDilate; ++j) {
+                    acc |= zor[j];
+                    if (li < d.nl && j + 1 == d.lval[li]) {
+                        smem[(ki * d.nl + li) * words + e] = (j < lfit) ? acc : 0u;
+                        ++li;
+                    }
                 }
+                ++ki;
             }
-            ++ki;
         }
+    }
+    __syncthreads();
+    const uint32_t out = (y1 - y0) * W;
+    bword* base = dst + static_cast<uint64_t>(slice) * g.sw + y0 * W;
+    for (uint32_t p = 0, rank = 0; p < kYLevels; ++p) {
+        if (!((t.levels >> p) & 1u)) continue;
+        for (uint32_t c = 0; c < ncombo; ++c) {
+            const bword* s = smem + c * words;
+            bword* o = base + static_cast<uint64_t>(rank * ncombo + c) * pos;
+            for (uint32_t e = threadIdx.x; e < out; e += blockDim.x) {
+                bword acc = s[e];
+                for (uint32_t i = 1, q = e + W; i < (1u << p) && q < words; ++i, q += W) acc |= s[q];
+                o[e] = acc;
+            }
+        }
+        ++rank;
     }
 }
 
-
-// The group that runs one satisfaction task: the whole block, or one warp
+// The group that runs one slice: the whole block, or one warp
 // (WARP), with its barrier and its barrier-with-OR.
 template <bool WARP>
 __device__ __forceinline__ void group_sync() {
@@ -153,435 +192,528 @@ __device__ __forceinline__ int group_sync_or(int p) {
     return __syncthreads_or(p);
 }
 
-// One (theta, v) slice x omega column jw (task = slice * mw + jw) of the
-// satisfaction test, by the whole block:
-//  B. per representative acceleration (the lowest of each group of inputs
-//     whose boxes coincide), E[y] = the (theta, v)-dilated D' row at the
-//     input's box corner: one load per word;
-//  C. each (representative, i1) item: F = OR of E over row i1's y range, then
-//     the x test 32 states per word: a state whose x box is [i0 + a, i0 + b]
-//     is blocked when F has a bit in it, i.e. bit i0 of OR_{d=a..b} (F >> d);
-//     with the plane's shift masks M_d (the states whose box holds i0 + d,
-//     launch_x_classes) that is bit i0 of OR_d ((F >> d) & M_d), one funnel
-//     shift per word and shift for the whole word of states; a plane with
-//     boxes of more than kShiftMax shifts is tested state by state;
-//  D. per state, the lowest satisfied input of the column goes to best[]
-//     (atomicMin, so the lowest over all columns wins) and the hit bit is set.
-// WMAX: register words per row; EXACTW: g.W == WMAX (else g.W <= WMAX at run
-// time).  NVMODE: 0 / 1 = validity test off / on, 2 = a.need_valid decides.
-// WARP: the task is one warp's (its own smem and s_meta), else the block's.
-// BULK (one task per block only): phase B stages each representative's rows,
-// class record and y table with three 1-D bulk copies (the TMA engine) that
-// complete on an mbarrier, instead of one cp.async per word.  A bulk copy
-// needs 16-byte aligned ends, so each copies the aligned span around its
-// words into a 16-byte aligned slot, and readers add the span's leading
-// offset (fused_smem_layout).
-// Every early return is taken by the whole group.
 // An iteration runs incrementally when the previous one added at most one
-// state per kIncrementalRows x-rows.  Measured at 128x128x72x48: 16 -> 4
-// took the fixpoint from 42.8 to 40.9 ms; 1 took it to 40.6 ms but slowed
-// the published demo by 0.5 %, and testing incrementally in every iteration
-// slowed it by 6 %.  A sharded solve sets last_new to 2^32 - 1, which no
-// threshold of 1 or more admits.
+// state per kIncrementalRows x-rows.  A sharded solve sets last_new to
+// 2^32 - 1, which no threshold of 1 or more admits.
 constexpr unsigned long long kIncrementalRows = 4;
 
-template <int WMAX, bool EXACTW, int NVMODE, bool WARP = false, bool BULK = false>
-__device__ __forceinline__ void sat_col_task(const GridInfo& g, const FusedFixArgs& a, uint32_t task,
-                                             bword* smem, uint32_t* s_meta) {
-    static_assert(!(BULK && WARP), "bulk staging is for one task per block");
-    const FixControl* fc = a.fc;
-    const uint32_t W = EXACTW ? static_cast<uint32_t>(WMAX) : g.W;
-    const bool NV = NVMODE == 2 ? (a.need_valid != 0) : (NVMODE == 1);
-    const uint32_t n0 = g.n[0], n1 = g.n[1], n2 = g.n[2], ma = g.ma, mw = g.mw;
-    const uint32_t nw = n1 * W;
-    const uint32_t slice = task / mw, jw = task - slice * mw;
-    const uint32_t i2 = slice % n2, i3 = slice / n2;
-    const uint64_t wbase = static_cast<uint64_t>(slice) * nw;
-    const uint32_t tid = WARP ? (threadIdx.x & 31u) : threadIdx.x;
-    const uint32_t bd = WARP ? 32u : blockDim.x;
-    const uint32_t lane = tid & 31;
-    const uint32_t nv = NV ? 2u : 1u;
-    const uint32_t cw = a.cls_words;
-    const uint32_t mr = a.max_reps;
-
-    const FusedSmemLayout L = fused_smem_layout(nw, nv, mr, cw, n1, ma, BULK);
-    bword* act = smem + L.act;
-    bword* Eall = smem + L.E;                             // max_reps * nv * L.e_stride
-    bword* sat = smem + L.sat;                            // max_reps * nw
-    bword* cls = smem + L.cls;                            // max_reps * L.c_stride
-    uint32_t* yts = smem + L.yts;                         // max_reps * L.y_stride
-    uint32_t* reps = smem + L.reps;                       // ma: acceleration of each representative slot
-    uint32_t* repw = reps + ma;                           // ma: its v window
-    uint32_t* repo = repw + ma;                           // ma: its part of the dilated rows' offset
-    uint32_t* rowchg = smem + L.rowchg;                   // max_reps * W1: y rows of a window that lost a cell
-    uint32_t* rsh = smem + L.rsh;                         // BULK, ma: leading offsets of a rep's three spans
-    uint64_t* mbar = reinterpret_cast<uint64_t*>(smem + L.mbar);
-    const uint32_t W1 = (n1 + 31) / 32;
-    if (BULK && tid == 0) mbar_init(mbar, 1);
-
-    const uint64_t pcol = (static_cast<uint64_t>(i2) * g.n[3] + i3) * g.M + static_cast<uint64_t>(ma) * jw;
-    // A. One round of loads that depend on the task alone: the active rows
-    // (two per thread before either is stored), the representatives in
-    // increasing acceleration order (warp ballot) with their v windows and
-    // offset parts, the omega column's theta window and offset part, and
-    // the control record (s_meta: [0] representatives, [1] theta window,
-    // [2] offset part, [3] iteration | incremental << 31, or all ones once
-    // stopped).
-    int any = 0;
-    for (uint32_t e0 = tid; e0 < nw; e0 += 2 * bd) {
-        const uint32_t e1 = e0 + bd;
-        const bword v0 = a.active[wbase + e0];
-        const bword v1 = e1 < nw ? a.active[wbase + e1] : 0u;
-        act[e0] = v0;
-        if (e1 < nw) act[e1] = v1;
-        any |= (v0 | v1) != 0;
-    }
-    if (tid < 32) {
-        uint32_t n = 0;
-        for (uint32_t base = 0; base < ma; base += 32) {
-            const uint32_t ja = base + lane;
-            uint32_t we = kReject, ov = 0;
-            bool is_rep = false;
-            if (ja < ma) {
-                we = a.wt[i3 * ma + ja];
-                ov = a.offv[i3 * ma + ja];
-                is_rep = a.xrep[pcol + ja] == ja && we != kReject;
-            }
-            const uint32_t m = __ballot_sync(0xFFFFFFFFu, is_rep);
-            if (is_rep) {
-                const uint32_t k = n + __popc(m & ((1u << lane) - 1));
-                reps[k] = ja;
-                repw[k] = we;
-                repo[k] = ov;
-            }
-            n += __popc(m);
+// The W words of a row (rows of 2 words are 8-byte and rows of 4 or 8 words
+// 16-byte aligned: one or two wide loads).
+template <int W>
+__device__ __forceinline__ void load_row(bword (&out)[W], const bword* row) {
+    if constexpr (W == 2) {
+        const uint2 v = *reinterpret_cast<const uint2*>(row);
+        out[0] = v.x;
+        out[1] = v.y;
+    } else if constexpr (W % 4 == 0) {
+#pragma unroll
+        for (int w = 0; w < W; w += 4) {
+            const uint4 v = *reinterpret_cast<const uint4*>(row + w);
+            out[w] = v.x;
+            out[w + 1] = v.y;
+            out[w + 2] = v.z;
+            out[w + 3] = v.w;
         }
-        if (lane == 0) s_meta[0] = n;
-    }
-    if (tid == (bd > 32 ? 32u : 0u)) {
-        // After the first iteration, every active state failed every input
-        // in the previous one, and D' only loses cells, so a state can newly
-        // pass only if its box holds a cell that left D' in the previous
-        // iteration.  When that iteration added few states (at most one per
-        // kIncrementalRows x-rows), the iteration runs incrementally (phase
-        // B).
-        const uint32_t stop = fc->stop, it = fc->iter, last = fc->last_new;
-        const bool inc = it > 0 && static_cast<unsigned long long>(last) * kIncrementalRows <= g.rows;
-        s_meta[1] = a.zt[i2 * mw + jw];
-        s_meta[2] = a.offz[i2 * mw + jw];
-        s_meta[3] = stop ? 0xFFFFFFFFu : (it | (inc ? 0x80000000u : 0u));
-    }
-    any = group_sync_or<WARP>(any);
-    const uint32_t nrep = s_meta[0], ctl = s_meta[3];
-    if (ctl == 0xFFFFFFFFu || !any || nrep == 0) return;
-    const uint32_t it = ctl & 0x7FFFFFFFu;
-    const bool incremental = (ctl >> 31) != 0;
-    const uint32_t ze = s_meta[1], offz = s_meta[2];
-    const uint32_t lz = lo16(ze), hz = hi16(ze);
-    const uint32_t nz = (lz <= hz) ? hz - lz + 1 : n2 - lz + hz + 1;
-
-    // B. The dilated D' (and valid) rows at each representative's (theta, v)
-    // box corner, its class records and y tables, copied asynchronously into
-    // shared memory, all in flight together.  In an incremental iteration
-    // the rows of each representative's (theta, v) window that lost a cell
-    // (rowlost, from the finalize kernel) are gathered first: a block with
-    // none stages nothing and skips, and a (representative, row) item whose
-    // y range has none is skipped; their states still fail.
-    auto stage = [&]() {
-        if constexpr (BULK) {
-            // Warp 0: lane r issues representative r's copies after lane 0
-            // has announced every copy's bytes on the barrier.
-            if (tid < 32) {
-                uint32_t bytes = 0;
-                for (uint32_t r = lane; r < nrep; r += 32) {
-                    const uint32_t offe = offz + repo[r];
-                    const uint64_t pl = pcol + reps[r];
-                    const uint32_t she = offe & 3u, shc = static_cast<uint32_t>(pl * cw) & 3u,
-                                   shy = static_cast<uint32_t>(pl * n1) & 3u;
-                    bytes += 4u * (nv * ((nw + she + 3u) & ~3u) + ((cw + shc + 3u) & ~3u) + ((n1 + shy + 3u) & ~3u));
-                }
-                for (int off = 16; off > 0; off >>= 1) bytes += __shfl_down_sync(0xFFFFFFFFu, bytes, off);
-                if (lane == 0) mbar_arrive_expect_tx(mbar, bytes);
-                __syncwarp();
-                for (uint32_t r = lane; r < nrep; r += 32) {
-                    const uint32_t offe = offz + repo[r];
-                    const uint64_t pl = pcol + reps[r];
-                    const uint32_t she = offe & 3u;
-                    const uint64_t offc = pl * cw, offy = pl * n1;
-                    const uint32_t shc = static_cast<uint32_t>(offc) & 3u, shy = static_cast<uint32_t>(offy) & 3u;
-                    bword* e0 = Eall + r * nv * L.e_stride;
-                    const uint32_t ne = 4u * ((nw + she + 3u) & ~3u);
-                    bulk_copy_g2s(e0, a.dzw + (offe - she), ne, mbar);
-                    if (NV) bulk_copy_g2s(e0 + L.e_stride, a.vzw + (offe - she), ne, mbar);
-                    bulk_copy_g2s(cls + r * L.c_stride, a.xcls + (offc - shc), 4u * ((cw + shc + 3u) & ~3u), mbar);
-                    bulk_copy_g2s(yts + r * L.y_stride, a.yt + (offy - shy), 4u * ((n1 + shy + 3u) & ~3u), mbar);
-                    rsh[r] = she | (shc << 8) | (shy << 16);
-                }
-            }
-        } else {
-            for (uint32_t e = tid; e < nrep * nw; e += bd) {
-                const uint32_t r = fdiv(e, g.magic_nw), rem = e - r * nw;
-                const uint32_t off = offz + repo[r] + rem;
-                cp_async4(Eall + r * nw * nv + rem, a.dzw + off);
-                if (NV) cp_async4(Eall + r * nw * nv + nw + rem, a.vzw + off);
-            }
-            for (uint32_t r = tid >> 5; r < nrep; r += bd >> 5) {
-                const uint64_t pl = pcol + reps[r];
-                for (uint32_t e = lane; e < cw; e += 32) cp_async4(cls + r * cw + e, a.xcls + pl * cw + e);
-                for (uint32_t e = lane; e < n1; e += 32) cp_async4(yts + r * n1 + e, a.yt + pl * n1 + e);
-            }
-        }
-    };
-    if (!incremental) stage();
-    int lost = 0;
-    if (incremental) {
-        const uint32_t* rl = a.rowlost + (it & 1) * a.rl_words;
-        for (uint32_t e = tid; e < nrep * W1; e += bd) {
-            const uint32_t r = e / W1, yw = e - r * W1;
-            const uint32_t we = repw[r];
-            const uint32_t v0 = lo16(we), v1 = hi16(we);
-            // The window's (theta, v) slices' row-lost words (W1 per slice),
-            // the next slice's load issued before the current one is used.
-            uint32_t z = lz, v = v0;
-            uint32_t c0 = __ldg(rl + (z + n2 * v) * W1 + yw);
-            uint32_t m = 0;
-            for (uint32_t q = 1; q < nz * (v1 - v0 + 1); ++q) {
-                if (v == v1) {
-                    v = v0;
-                    z = (z + 1 == n2) ? 0 : z + 1;
-                } else {
-                    ++v;
-                }
-                const uint32_t d0 = __ldg(rl + (z + n2 * v) * W1 + yw);
-                m |= c0;
-                c0 = d0;
-            }
-            m |= c0;
-            rowchg[r * W1 + yw] = m;
-            lost |= m != 0;
-        }
-    }
-    if (incremental) {
-        if (!group_sync_or<WARP>(lost)) return;
-        stage();
-    }
-    if constexpr (BULK) {
-        // Bounded wait for the copies.  A wait that gives up (it cannot in a
-        // working device: the copies are a few KB) stops the solve with
-        // kMsgDeviceTimeout, which the host reports as GSC_ERR_TIMEOUT, and
-        // waits once more, again bounded, before the block leaves.
-        bool done = false;
-        for (uint32_t k = 0; k < kBulkWaitProbes && !done; ++k) done = mbar_try_wait(mbar, 0);
-        if (!done) {
-            FixControl* wfc = a.fc;
-            wfc->message = kMsgDeviceTimeout;
-            atomicExch(&wfc->stop, 1u);
-            for (uint32_t k = 0; k < kBulkWaitProbes && !done; ++k) done = mbar_try_wait(mbar, 0);
-        }
-        if (group_sync_or<WARP>(done ? 0 : 1)) return;
     } else {
-        cp_async_wait_all();
-        group_sync<WARP>();
+#pragma unroll
+        for (int w = 0; w < W; ++w) out[w] = row[w];
     }
-    if (tid == 0) atomicAdd(a.stats + kStatsCols * (it + 1) + 3, static_cast<unsigned long long>(nrep));
-    // C. the (representative, row) items.
-    unsigned long long ntest = 0;
-    for (uint32_t e = tid; e < nrep * n1; e += bd) {
-        const uint32_t r = fdiv(e, g.magic_n1), i1 = e - r * n1;
-        const uint32_t ja = reps[r];
-        bword cm[WMAX], sw[WMAX];
-        bword anyc = 0;
+}
+
+// Y = X | X >> s over a row of W words (s < 32).
+template <int W>
+__device__ __forceinline__ void or_shifted(const bword (&X)[W], bword (&Y)[W], uint32_t s) {
 #pragma unroll
-        for (int w = 0; w < WMAX; ++w) {
-            cm[w] = (EXACTW || static_cast<uint32_t>(w) < W) ? act[i1 * W + w] : 0u;
-            sw[w] = 0;
-            anyc |= cm[w];
+    for (int w = 0; w < W; ++w) Y[w] = X[w] | __funnelshift_r(X[w], w + 1 < W ? X[w + 1] : 0u, s);
+}
+
+// T = the OR of X >> 0 .. nd - 1 (nd <= 32; X itself for nd = 0).
+template <int W>
+__device__ __forceinline__ void or_range(const bword (&X)[W], bword (&T)[W], uint32_t nd) {
+    or_shifted<W>(X, T, nd > 1 ? 1u : 0u);
+    if (nd <= 2) return;
+    if (nd > 4) {
+        // By twos up to nd - 1 or nd - 2, then the rest at once.
+        for (uint32_t i = 2; i + 2 < nd; i += 2) {
+            bword u[W];
+            or_shifted<W>(T, u, 2u);
+#pragma unroll
+            for (int w = 0; w < W; ++w) T[w] = u[w];
         }
-        const uint32_t rs = BULK ? rsh[r] : 0u;
-        const uint32_t ye = BULK ? yts[r * L.y_stride + (rs >> 16) + i1] : yts[r * n1 + i1];
-        if (anyc && ye != kReject && incremental) {
-            // Bits [lo, hi] of the representative's changed-row mask (fused
-            // boxes span at most 32 rows): one funnel shift.
-            const uint32_t lo = lo16(ye), hi = hi16(ye);
-            const uint32_t* rc = rowchg + r * W1;
-            const uint32_t wl = lo >> 5, wh = hi >> 5;
-            const uint32_t bits = __funnelshift_r(rc[wl], wh != wl ? rc[wh] : 0u, lo & 31);
-            const uint32_t len = hi - lo + 1;
-            if (!(len >= 32 ? bits : (bits & ((1u << len) - 1)))) anyc = 0;
+    }
+    bword u[W];
+    or_shifted<W>(T, u, nd <= 4 ? nd - 2 : (nd & 1u) ? 1u : 2u);
+#pragma unroll
+    for (int w = 0; w < W; ++w) T[w] = u[w];
+}
+
+// Any bits of X in each state's x box: U = OR_d ((X >> d) & M_d) over the
+// plane's shifts (launch_x_classes; masks at rec, W words each), without the
+// masks where every state with a box has all the shifts.  G is X moved by
+// dmin, one word longer, so every shift is a right funnel shift by d - dmin
+// in [0, kShiftMax).
+template <int W>
+__device__ __forceinline__ void in_x_box(const bword (&X)[W], bword (&U)[W], bword hdr, const bword* rec) {
+    const int dmin = static_cast<int8_t>((hdr >> 8) & 0xFFu);
+    const uint32_t nd = hdr & 0xFFu;
+    bword G[W + 1];
+#pragma unroll
+    for (int w = 0; w <= W; ++w) G[w] = moved_word<W>(X, w, dmin);
+    if (hdr & 0x10000u) {
+#pragma unroll
+        for (int w = 0; w < W; ++w) U[w] = nd ? G[w] : 0u;
+        for (uint32_t i = 1; i < nd; ++i) {
+#pragma unroll
+            for (int w = 0; w < W; ++w) U[w] |= __funnelshift_r(G[w], G[w + 1], i);
         }
-        if (anyc && ye != kReject) {
+    } else {
 #pragma unroll
-            for (int w = 0; w < WMAX; ++w) ntest += __popc(cm[w]);
-            const bword* E = BULK ? Eall + r * nv * L.e_stride + (rs & 0xFFu) : Eall + r * nw * nv;
-            const uint32_t ev = BULK ? L.e_stride : nw;   // the valid rows follow the D' rows
-            bword F[WMAX], FV[WMAX];
+        for (int w = 0; w < W; ++w) U[w] = 0;
+        for (uint32_t i = 0; i < nd; ++i) {
 #pragma unroll
-            for (int w = 0; w < WMAX; ++w) F[w] = FV[w] = 0;
+            for (int w = 0; w < W; ++w) U[w] |= __funnelshift_r(G[w], G[w + 1], i) & __ldg(rec + i * W + w);
+        }
+    }
+}
+
+// Of the states m of a row, those whose x box (xrow: the row's box per cell)
+// is there and holds no cell of X.
+template <int W>
+__device__ __noinline__ void without_cell(const uint32_t* xrow, const bword (&X)[W], bword (&m)[W]) {
+    for (int w = 0; w < W; ++w) {
+        for (bword t = m[w]; t; t &= t - 1) {
+            const uint32_t bit = __ffs(t) - 1;
+            const uint32_t xe = __ldg(xrow + w * kBits + bit);
+            if (xe == kReject || extract_bits<W>(X, lo16(xe), hi16(xe)) != 0) m[w] &= ~(bword(1) << bit);
+        }
+    }
+}
+
+// The valid cells of row i1's (y, theta, v) box ranges under a representative, ORed along x.
+template <int W>
+__device__ __forceinline__ void valid_window(const GridInfo& g, const bword* validb, uint32_t zw, uint32_t vw,
+                                             uint32_t ye, bword (&V)[W]) {
+    const uint32_t n2 = g.n[2], nz = hi16(zw), v0 = lo16(vw), nv = hi16(vw) & 0x7FFFu;
+#pragma unroll
+    for (int w = 0; w < W; ++w) V[w] = 0;
+    uint32_t z = lo16(zw);
+    for (uint32_t i = 0; i < nz; ++i) {
+        for (uint32_t v = v0; v < v0 + nv; ++v) {
+            const bword* vr = validb + static_cast<uint64_t>(z + n2 * v) * g.sw;
             for (uint32_t y = lo16(ye); y <= hi16(ye); ++y) {
 #pragma unroll
-                for (int w = 0; w < WMAX; ++w) {
-                    if (!EXACTW && static_cast<uint32_t>(w) >= W) continue;
-                    F[w] |= E[y * W + w];
-                    if (NV) FV[w] |= E[ev + y * W + w];
-                }
-            }
-            const bword* rec = BULK ? cls + r * L.c_stride + ((rs >> 8) & 0xFFu) : cls + r * cw;
-            const bword hdr = rec[0];
-            const uint32_t nd = hdr & 0xFFu;
-            if (nd != 0xFFu) {
-                // U = OR_d ((F >> d) & M_d) over the plane's shifts (and VA
-                // likewise over the valid rows): G is F moved by dmin, one
-                // word longer, so every shift is a right funnel shift by
-                // d - dmin in [0, kShiftMax).
-                const int dmin = static_cast<int8_t>((hdr >> 8) & 0xFFu);
-                bword G[WMAX + 1], GV[WMAX + 1];
-#pragma unroll
-                for (int w = 0; w <= WMAX; ++w) {
-                    G[w] = moved_word<WMAX>(F, w, dmin);
-                    GV[w] = NV ? moved_word<WMAX>(FV, w, dmin) : 0u;
-                }
-                bword U[WMAX], VA[WMAX];
-#pragma unroll
-                for (int w = 0; w < WMAX; ++w) U[w] = VA[w] = 0;
-                for (uint32_t i = 0; i < nd; ++i) {
-#pragma unroll
-                    for (int w = 0; w < WMAX; ++w) {
-                        if (!EXACTW && static_cast<uint32_t>(w) >= W) continue;
-                        const bword m = rec[4 + i * W + w];
-                        U[w] |= __funnelshift_r(G[w], G[w + 1], i) & m;
-                        if (NV) VA[w] |= __funnelshift_r(GV[w], GV[w + 1], i) & m;
-                    }
-                }
-#pragma unroll
-                for (int w = 0; w < WMAX; ++w) {
-                    const bword ok = (EXACTW || static_cast<uint32_t>(w) < W) ? rec[4 + kShiftMax * W + w] : 0u;
-                    sw[w] = cm[w] & ok & ~U[w] & (NV ? VA[w] : ~0u);
-                }
-            } else {
-                const uint32_t* xrow = a.xt + (pcol + ja) * n0;
-#pragma unroll
-                for (int w = 0; w < WMAX; ++w) {
-                    bword m = cm[w];
-                    while (m) {
-                        const uint32_t b = __ffs(m) - 1;
-                        m &= m - 1;
-                        const uint32_t xe = __ldg(xrow + w * kBits + b);
-                        if (xe == kReject) continue;
-                        const uint32_t lx = lo16(xe), hx = hi16(xe);
-                        bool ok = extract_bits<WMAX>(F, lx, hx) == 0;
-                        if (NV) ok = ok && extract_bits<WMAX>(FV, lx, hx) != 0;
-                        if (ok) sw[w] |= bword(1) << b;
-                    }
-                }
+                for (int w = 0; w < W; ++w) V[w] |= __ldg(vr + y * W + w);
             }
         }
-#pragma unroll
-        for (int w = 0; w < WMAX; ++w)
-            if (EXACTW || static_cast<uint32_t>(w) < W) sat[r * nw + i1 * W + w] = sw[w];
+        z = (z + 1 == n2) ? 0 : z + 1;
     }
+}
+
+// The OR of two rows `d` words apart.
+template <int W>
+__device__ __forceinline__ void two_rows(const bword* row, uint32_t d, bword (&F)[W]) {
+    bword t[W];
+    load_row<W>(F, row);
+    load_row<W>(t, row + d);
+#pragma unroll
+    for (int w = 0; w < W; ++w) F[w] |= t[w];
+}
+
+// Of the states m of row i1 of a slice, those whose box under the slice's
+// representative number `index` holds a valid cell: the x test on the valid
+// set's dilated copies.  Only rows marked in needv (launch_need_valid) have a
+// state whose box does not.
+template <int W>
+__device__ __noinline__ void keep_valid(const GridInfo& g, const FusedFixArgs& a, uint4 rp, uint4 bx, uint32_t slice,
+                                        uint32_t index, uint32_t i1, bword (&m)[W]) {
+    const uint32_t W1 = (g.n[1] + 31) / 32;
+    if (!((__ldg(a.needv + (static_cast<uint64_t>(slice) * g.M + index) * W1 + (i1 >> 5)) >> (i1 & 31)) & 1u)) return;
+    const uint64_t pl = xy_plane(g, slice % g.n[2], slice / g.n[2], rp.x);
+    bword V[W], none[W];
+    if (bx.x & kBoxY) {
+        two_rows<W>(a.vzw + (rp.w + i1 * W), bx.y >> 16, V);
+    } else {
+        const uint32_t ye = __ldg(a.yt + pl * g.n1p + i1), ylo = lo16(ye), ny = hi16(ye) - ylo + 1, p = 31 - __clz(ny);
+        two_rows<W>(a.vzw + (a.ylev[p] + rp.w + ylo * W), (ny - (1u << p)) * W, V);
+    }
+    if (bx.x & kBoxX) {
+        bword T[W];
+        or_range<W>(V, T, bx.x & 0xFFu);
+        const int dmin = static_cast<int8_t>(bx.x >> 8);
+#pragma unroll
+        for (int w = 0; w < W; ++w) m[w] &= moved_word<W>(T, w, dmin);
+        return;
+    }
+#pragma unroll
+    for (int w = 0; w < W; ++w) none[w] = m[w];
+    without_cell<W>(a.xt + pl * g.n[0], V, none);
+#pragma unroll
+    for (int w = 0; w < W; ++w) m[w] &= ~none[w];
+}
+
+// D' cells of rows [ylo, ylo + ny) in a representative's (theta, v) window,
+// ORed, from D' itself.
+template <int W>
+__device__ __forceinline__ void window_rows(const GridInfo& g, const bword* cur, uint4 rp, uint32_t ylo, uint32_t ny,
+                                            bword (&F)[W]) {
+    const uint32_t n2 = g.n[2], z0 = lo16(rp.y), nz = hi16(rp.y), v0 = lo16(rp.z), nv = hi16(rp.z) & 0x7FFFu;
+#pragma unroll
+    for (int w = 0; w < W; ++w) F[w] = 0;
+    for (uint32_t v = v0; v < v0 + nv; ++v) {
+        for (uint32_t i = 0; i < nz; i += 2) {
+            // Two theta cells at a time (the last one twice when there is no second).
+            uint32_t za = z0 + i, zb = za + (i + 1 < nz ? 1u : 0u);
+            if (za >= n2) za -= n2;
+            if (zb >= n2) zb -= n2;
+            const bword* A = cur + static_cast<uint64_t>(za + n2 * v) * g.sw + ylo * W;
+            const bword* B = cur + static_cast<uint64_t>(zb + n2 * v) * g.sw + ylo * W;
+#pragma unroll 2
+            for (uint32_t y = 0; y < ny; ++y) {
+                bword s[W], t[W];
+                load_row<W>(s, A + y * W);
+                load_row<W>(t, B + y * W);
+#pragma unroll
+                for (int w = 0; w < W; ++w) F[w] |= s[w] | t[w];
+            }
+        }
+    }
+}
+
+// One (theta, v) slice of one iteration, by one group: the satisfaction test
+// of every active state against every representative input, the lowest
+// satisfied input, and the state update.  A slice's states are updated by
+// its own group alone and D' is double-buffered (this iteration reads
+// dp[iter & 1] and writes its slice of the other), so the update needs no
+// further kernel, and an iteration is one launch (two with the dilation).
+//
+// A thread takes a row of the slice and every kpar-th of its representatives
+// (launch_slice_reps).  For each, F = D' ORed over the box's y, theta and v
+// ranges (from a y level of the dilated copies two rows, which cover the y
+// range; from D' itself, direct, every row of the window), then the x test, 32 states per word: a state whose x box
+// is [i0 + a, i0 + b] is blocked when F has a bit in it, i.e. bit i0 of
+// OR_{d=a..b} (F >> d); with the plane's shift masks M_d (launch_x_classes)
+// that is bit i0 of OR_d ((F >> d) & M_d); a plane whose boxes are alike needs
+// no masks (SliceRep::hx), one with boxes of more than kShiftMax shifts is
+// tested state by state.  When validity is more than
+// safety, the box must also hold a valid cell (keep_valid; few rows have a box
+// that may not).
+// In incremental iterations a representative's rows that lost a D' cell in
+// the last iteration are gathered first, and a (representative, row) item
+// with none in its y range is left out: its states failed, and nothing they
+// wait for changed.
+// Then the words with a hit: D' loses the hit bits (a hit state is valid and
+// safe, so its bit is 1 exactly while it is not reachable: the newly reachable
+// are hit & D', the newly certified candidates hit & ~D'), and the rows that
+// lost one are recorded for the next iteration.
+//
+// Bound: latency and issue, with every slice's block resident at once
+// (fused_sat_threads).  Rows are read from L2 straight into registers: staged
+// in shared memory in chunks of representatives (bulk copies on an mbarrier,
+// double-buffered, or OR-ed there), three block barriers a chunk and 45 M warp
+// instructions took 85 us an iteration on the published demo; so, 16 M take
+// 51 us, where one block per (slice, omega column) with a finalize kernel of
+// its own took 88.  Hits are noted and taken after the loop: taken in it, by
+// one lane while its warp waits, the same iteration took 76 us.  Loading two
+// or four representatives ahead costs registers (resident warps) and was no
+// faster (55 to 58 us).
+//
+// Returns 0 once the solve has stopped, 2 when the group counted a hit, else 1.  Every early return is taken by
+// the whole group.  s_meta: [0] iteration | incremental << 31, or all ones once
+// stopped, [1] rows packed, [2] hits noted.  SHARED: the slice has one x / y plane (xy_plane); DIRECT: as
+// a.direct; 2 = decided at run time.
+template <int W, int SHARED, int DIRECT, bool WARP, bool PDL>
+__device__ __forceinline__ int slice_task(const GridInfo& g, const FusedFixArgs& a, uint32_t slice, bword* smem,
+                                           uint32_t* s_meta) {
+    const uint32_t n0 = g.n[0], n1 = g.n[1], n2 = g.n[2];
+    const uint32_t sw = g.sw, W1 = (n1 + 31) / 32;
+    const uint32_t i2 = slice % n2, i3 = slice / n2;
+    const uint64_t wbase = static_cast<uint64_t>(slice) * sw;
+    const uint32_t tid = WARP ? (threadIdx.x & 31u) : threadIdx.x;
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t bd = WARP ? 32u : blockDim.x;
+    const bool shared_xy = SHARED == 2 ? g.xy_planes == 1 : SHARED == 1;
+    const bool direct = DIRECT == 2 ? a.direct != 0 : DIRECT == 1;
+    const uint32_t pass = a.pass;
+    uint4* reps = reinterpret_cast<uint4*>(smem);            // [pass][2] SliceRep
+    bword* hits = smem + 8 * pass;                           // [sw] states satisfied now
+    uint32_t* rowchg = hits + sw;                            // [pass][W1]
+    uint32_t* lostown = rowchg + pass * W1;                  // [W1] rows of this slice that lost a cell
+    uint32_t* lostnew = lostown + W1;                        // [W1] that lose one now
+    uint32_t* notes = lostnew + W1;                          // [kHitNotes][W + 1] hits: row | representative << 16, states
+    uint16_t* rows = reinterpret_cast<uint16_t*>(notes + kHitNotes * (W + 1));   // [n1] rows with an active state, up to kPackedRows
+
+    // Tables that no iteration changes, before waiting for the last one.
+    const uint32_t nrep = a.nreps[slice];
+    const uint4* list = reinterpret_cast<const uint4*>(a.reps) + static_cast<uint64_t>(slice) * g.M * 2;
+    for (uint32_t r = tid; r < 2 * min(pass, nrep); r += bd) reps[r] = list[r];
+    for (uint32_t e = tid; e < sw; e += bd) hits[e] = 0;
+    if (tid == 0) s_meta[1] = s_meta[2] = 0;
     group_sync<WARP>();
-    // D. lowest satisfied input of the column per state -> best[] and hit
-    // bits.  Representatives are in increasing order and each is the lowest
-    // input of its group, so the first representative that satisfies a state
-    // gives its lowest satisfied input of the column.
-    for (uint32_t e = tid; e < nw; e += bd) {
-        bword open = act[e], got = 0;
-        const uint32_t y = e / W;
-        const uint64_t srow = (static_cast<uint64_t>(slice) * n1 + y) * n0 + (e - y * W) * kBits;
-        for (uint32_t r = 0; r < nrep && open; ++r) {
-            const bword nb = sat[r * nw + e] & open;
-            if (!nb) continue;
-            open &= ~nb;
-            got |= nb;
-            const uint32_t j = reps[r] + ma * jw;
-            bword m = nb;
-            while (m) {
-                const uint32_t b = __ffs(m) - 1;
-                m &= m - 1;
-                atomicMin(a.best + srow + b, j);
+    if (PDL) pdl_wait();
+
+    const FixControl* fc = a.fc;
+    const uint32_t it = fc->iter;
+    if (tid == 0) {
+        const bool inc = it > 0 && static_cast<unsigned long long>(fc->last_new) * kIncrementalRows <= g.rows;
+        s_meta[0] = fc->stop ? 0xFFFFFFFFu : (it | (inc ? 0x80000000u : 0u));
+    }
+    // The rows with an active state, packed (in no particular order), so that
+    // every thread of the group has as many items.
+    const bool packed = n1 <= kPackedRows;
+    int any = 0;
+    for (uint32_t y0 = tid & ~31u; y0 < n1; y0 += bd) {
+        const uint32_t y = y0 + lane;
+        bword v[W], o = 0;
+        if (y < n1) {
+            load_row<W>(v, a.active + wbase + y * W);
+#pragma unroll
+            for (int w = 0; w < W; ++w) o |= v[w];
+        }
+        const uint32_t m = __ballot_sync(0xFFFFFFFFu, o != 0);
+        any |= m != 0;
+        if (packed && m) {
+            uint32_t at = 0;
+            if (lane == 0) at = atomicAdd(s_meta + 1, __popc(m));
+            at = __shfl_sync(0xFFFFFFFFu, at, 0);
+            if (o) rows[at + __popc(m & ((1u << lane) - 1))] = static_cast<uint16_t>(y);
+        }
+    }
+    const uint32_t* rl = a.rowlost + static_cast<uint64_t>(it & 1u) * a.rl_words;
+    uint32_t* rlnext = a.rowlost + static_cast<uint64_t>((it + 1) & 1u) * a.rl_words;
+    const bool odd = !a.shard_slices && (it & 1u);
+    const bword* cur = odd ? a.dp[1] : a.dp[0];
+    // Changed rows of `n` staged representatives' windows (unless this is the
+    // first iteration, which has no record of any).
+    auto changed_rows = [&](uint32_t n) {
+        for (uint32_t e = tid; e < n * W1; e += bd) {
+            const uint32_t r = e / W1, yw = e - r * W1;
+            const uint4 rp = reps[2 * r];
+            const uint32_t z0 = lo16(rp.y), nz = hi16(rp.y), v0 = lo16(rp.z), nv = hi16(rp.z) & 0x7FFFu;
+            const auto at = [&](uint32_t z, uint32_t v) { return rl[static_cast<uint64_t>(z + n2 * v) * W1 + yw]; };
+            uint32_t m = 0;
+            if (nz <= 2 && nv <= 2) {
+                const uint32_t z1 = nz < 2 ? z0 : (z0 + 1 == n2 ? 0 : z0 + 1), v1 = v0 + nv - 1;
+                m = at(z0, v0) | at(z0, v1) | at(z1, v0) | at(z1, v1);
+            } else {
+                uint32_t z = z0;
+                for (uint32_t i = 0; i < nz; ++i) {
+#pragma unroll 4
+                    for (uint32_t v = v0; v < v0 + nv; ++v) m |= at(z, v);
+                    z = (z + 1 == n2) ? 0 : z + 1;
+                }
+            }
+            rowchg[e] = m;
+        }
+    };
+    if (it) changed_rows(min(pass, nrep));
+    for (uint32_t e = tid; e < W1; e += bd) {
+        lostown[e] = it ? rl[static_cast<uint64_t>(slice) * W1 + e] : 0u;
+        lostnew[e] = 0;
+    }
+    any = group_sync_or<WARP>(any);
+    const uint32_t ctl = s_meta[0];
+    if (ctl == 0xFFFFFFFFu) return 0;
+    const bool incremental = (ctl >> 31) != 0;
+    // Threads = rows x kpar; a group smaller than the rows strides over them.
+    const uint32_t nrows = packed ? s_meta[1] : n1;
+    const uint32_t kpar = any && nrows < bd ? bd / nrows : 1u;
+    const uint32_t kk = any && nrows < bd ? tid / nrows : 0u;
+    unsigned long long ntest = 0;
+    int hit_any = 0;   // of the group, once a pass is through
+    for (uint32_t p0 = 0; any && p0 < nrep; p0 += pass) {
+        const uint32_t np = min(pass, nrep - p0);
+        if (p0) {
+            group_sync<WARP>();
+            for (uint32_t r = tid; r < 2 * np; r += bd) reps[r] = list[2 * p0 + r];
+            group_sync<WARP>();
+            if (incremental) {
+                changed_rows(np);
+                group_sync<WARP>();
             }
         }
-        if (got) atomicOr(a.hit + wbase + e, got);
-    }
-    for (int off = 16; off > 0; off >>= 1) ntest += __shfl_down_sync(0xFFFFFFFFu, ntest, off);
-    if ((tid & 31) == 0 && ntest) atomicAdd(a.stats + kStatsCols * (it + 1) + 2, ntest);
-}
-
-// Apply the iteration's hits to word e and build next iteration's D';
-// nr / nc collect newly reachable states and newly certified candidates.
-// The reachable set is updated in place (rprev and rnext name one buffer),
-// and D' = (valid & ~reachable) | unsafe holds for every word between
-// iterations, so a word without a hit keeps all of its bits: its thread
-// reads the hit word and stops.
-__device__ __forceinline__ void finalize_word(const GridInfo& g, const FusedFixArgs& a, const bword* rprev,
-                                              bword* rnext, uint64_t e, uint32_t it, unsigned long long& nr,
-                                              unsigned long long& nc) {
-    const bword h = a.hit[e];
-    if (!h) return;
-    // Every load the word needs, issued before any of its stores (one round
-    // trip): its sets and the best[] entries of its first four new states.
-    const bword rp = rprev[e];
-    const bword vb = a.validb[e], ub = a.unsafeb[e], dpo = a.dp[e], c = a.candb[e], act = a.active[e];
-    const uint64_t r = e / g.W;
-    const uint64_t sbase = r * g.n[0] + (e - r * g.W) * kBits;
-    bword m = h;
-    uint32_t b[4], j[4];
-    // Four states at a time: their best[] loads in flight together.
-    auto load4 = [&]() {
+        for (uint32_t row = tid - kk * nrows; row < nrows && kk < kpar; row += bd) {
+            const uint32_t i1 = packed ? rows[row] : row;
+            bword open[W], anyo = 0;
+            load_row<W>(open, a.active + wbase + i1 * W);
+            if (p0) {
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            b[k] = m ? static_cast<uint32_t>(__ffs(m) - 1) : kBits;
-            m &= m - 1;
+                for (int w = 0; w < W; ++w) open[w] &= ~hits[i1 * W + w];
+            }
+            uint32_t states = 0;
+#pragma unroll
+            for (int w = 0; w < W; ++w) {
+                anyo |= open[w];
+                states += __popc(open[w]);
+            }
+            if (!anyo) continue;
+            const uint64_t base_pl = xy_plane(g, i2, i3, 0);
+            uint32_t tested = 0;
+            for (uint32_t k = kk; k < np; k += kpar) {
+                const uint4 rp = reps[2 * k], bx = reps[2 * k + 1];
+                uint32_t ye = 0;
+                if (bx.x & kBoxY) {
+                    if (i1 - lo16(bx.z) >= hi16(bx.z)) continue;
+                } else {
+                    ye = __ldg(a.yt + (shared_xy ? base_pl : base_pl + rp.x) * g.n1p + i1);
+                    if (ye == kReject) continue;
+                }
+                bword F[W];
+                if (incremental || direct || !(bx.x & kBoxY)) {
+                    const uint32_t ylo = bx.x & kBoxY ? i1 + static_cast<int8_t>(bx.y >> 8) : lo16(ye);
+                    const uint32_t ny = bx.x & kBoxY ? bx.y & 0xFFu : hi16(ye) - lo16(ye) + 1;
+                    if (incremental) {
+                        // Bits [ylo, ylo + ny) of the representative's changed-row
+                        // mask (fused boxes span at most 32 rows): one funnel shift.
+                        const uint32_t* rc = rowchg + k * W1;
+                        const uint32_t wl = ylo >> 5, wh = (ylo + ny - 1) >> 5;
+                        const uint32_t bits = __funnelshift_r(rc[wl], wh != wl ? rc[wh] : 0u, ylo & 31);
+                        if (!(bits << (32u - ny))) continue;
+                    }
+                    if (direct) {
+                        window_rows<W>(g, cur, rp, ylo, ny, F);
+                    } else if (!(bx.x & kBoxY)) {
+                        const uint32_t p = 31 - __clz(ny);
+                        two_rows<W>(a.dzw + (a.ylev[p] + rp.w + ylo * W), (ny - (1u << p)) * W, F);
+                    }
+                }
+                if (!direct && (bx.x & kBoxY)) two_rows<W>(a.dzw + (rp.w + i1 * W), bx.y >> 16, F);
+                tested += states;
+                bword sm[W], anys = 0;
+                if (bx.x & kBoxX) {
+                    // T = the OR of F >> 0 .. b - a (bits that come in from
+                    // beyond the row belong to no state with a box), moved by a.
+                    bword T[W];
+                    or_range<W>(F, T, bx.x & 0xFFu);
+                    const int dmin = static_cast<int8_t>(bx.x >> 8);
+                    const uint32_t x0 = lo16(bx.w), x1 = hi16(bx.w);
+#pragma unroll
+                    for (int w = 0; w < W; ++w) {
+                        sm[w] = open[w] & ~moved_word<W>(T, w, dmin) & bits_from(x0, w) & ~bits_from(x1, w);
+                        anys |= sm[w];
+                    }
+                } else {
+                    const uint64_t pl = shared_xy ? base_pl : base_pl + rp.x;
+                    const bword* rec = a.xcls + pl * a.cls_words;
+                    const bword hdr = __ldg(rec);
+                    if ((hdr & 0xFFu) != 0xFFu) {
+                        bword U[W];
+                        in_x_box<W>(F, U, hdr, rec + 4);
+#pragma unroll
+                        for (int w = 0; w < W; ++w) sm[w] = open[w] & __ldg(rec + 4 + kShiftMax * W + w) & ~U[w];
+                    } else {
+                        bword x[W], y[W];
+#pragma unroll
+                        for (int w = 0; w < W; ++w) {
+                            x[w] = F[w];
+                            y[w] = open[w];
+                        }
+                        without_cell<W>(a.xt + pl * n0, x, y);
+#pragma unroll
+                        for (int w = 0; w < W; ++w) sm[w] = y[w];
+                    }
+#pragma unroll
+                    for (int w = 0; w < W; ++w) anys |= sm[w];
+                }
+                if (!anys) continue;
+                if (rp.z >> 31) {
+                    bword x[W];
+#pragma unroll
+                    for (int w = 0; w < W; ++w) x[w] = sm[w];
+                    keep_valid<W>(g, a, rp, bx, slice, p0 + k, i1, x);
+#pragma unroll
+                    for (int w = 0; w < W; ++w) sm[w] = x[w];
+                }
+                // Noted for later, so that a warp does not stop for each of its
+                // lanes' hits (at once when the list is full).
+                hit_any = 1;
+                const uint32_t at = atomicAdd(s_meta + 2, 1u);
+                if (at < kHitNotes) {
+                    uint32_t* note = notes + at * (W + 1);
+                    note[0] = i1 | (k << 16);
+#pragma unroll
+                    for (int w = 0; w < W; ++w) note[1 + w] = sm[w];
+                } else {
+                    take_hits<W>(a, (static_cast<uint64_t>(slice) * n1 + i1) * n0, rp.x, hits + i1 * W, sm);
+                }
+                anyo = 0;
+                states = 0;
+#pragma unroll
+                for (int w = 0; w < W; ++w) {
+                    open[w] &= ~sm[w];
+                    anyo |= open[w];
+                    states += __popc(open[w]);
+                }
+                if (!anyo) break;
+            }
+            ntest += tested;
         }
+        // The noted hits (of this pass: its representatives are still staged).
+        hit_any = group_sync_or<WARP>(hit_any);
+        if (hit_any) {
+            const uint32_t n = min(s_meta[2], kHitNotes);
+            for (uint32_t e = tid; e < n; e += bd) {
+                const uint32_t* note = notes + e * (W + 1);
+                const uint32_t i1 = note[0] & 0xFFFFu;
+                bword sm[W];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) j[k] = b[k] < kBits ? a.best[sbase + b[k]] : kInvalid32;
-    };
-    load4();
-    const bword rn = rp | h;
-    rnext[e] = rn;
-    const bword dn = (vb & ~rn) | ub;
-    if (dpo & ~dn) {   // the row lost a D' cell in iteration `it`: word y / 32 of its slice
-        const uint32_t row = static_cast<uint32_t>(r), n1 = g.n[1];
-        const uint32_t sl = row / n1, y = row - sl * n1;
-        atomicOr(a.rowlost + (it & 1) * a.rl_words + sl * ((n1 + 31) / 32) + (y >> 5), 1u << (y & 31));
-    }
-    a.dp[e] = dn;
-    a.hit[e] = 0;
-    a.active[e] = act & ~h;
-    nr += __popc(h & ~rp);
-    nc += __popc(h & c);
-    for (;;) {
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            if (b[k] >= kBits) continue;
-            const uint64_t s = sbase + b[k];
-            a.controller[s] = j[k];
-            a.best[s] = kInvalid32;
-            if (!((c >> b[k]) & 1u)) a.reach_step[s] = it;
+                for (int w = 0; w < W; ++w) sm[w] = note[1 + w];
+                take_hits<W>(a, (static_cast<uint64_t>(slice) * n1 + i1) * n0, reps[2 * (note[0] >> 16)].x, hits + i1 * W,
+                             sm);
+            }
+            group_sync<WARP>();
+            if (tid == 0) s_meta[2] = 0;
         }
-        if (!m) break;
-        load4();
     }
-}
-
-// Block-wide: add the block's counters to the iteration's stats row.
-__device__ __forceinline__ void add_counters(unsigned long long* row, unsigned long long nr, unsigned long long nc) {
-    for (int off = 16; off > 0; off >>= 1) {
-        nr += __shfl_down_sync(0xFFFFFFFFu, nr, off);
-        nc += __shfl_down_sync(0xFFFFFFFFu, nc, off);
+    // The update: words with a hit, and D' rows whose other buffer is behind.
+    bword* next = odd ? a.dp[0] : a.dp[1];
+    unsigned long long nr = 0, nc = 0;
+    const uint32_t step = it + 1;
+    for (uint32_t e = tid; e < n1 * W; e += bd) {
+        const uint32_t y = e / W, yb = 1u << (y & 31);
+        const bword h = hit_any ? hits[e] : 0u;
+        if (!h && !(lostown[y >> 5] & yb)) continue;
+        const bword d = cur[wbase + e];
+        next[wbase + e] = d & ~h;
+        if (!h) continue;
+        a.active[wbase + e] &= ~h;
+        a.reach0[wbase + e] |= h;
+        const bword fresh = h & d;
+        nr += __popc(fresh);
+        nc += __popc(h & ~d);
+        if (fresh) {
+            atomicOr(lostnew + (y >> 5), yb);
+            const uint64_t srow = (static_cast<uint64_t>(slice) * n1 + y) * n0 + (e - y * W) * kBits;
+            for (bword m = fresh; m; m &= m - 1) a.reach_step[srow + __ffs(m) - 1] = step;
+        }
     }
-    if ((threadIdx.x & 31) == 0) {
-        if (nr) atomicAdd(row, nr);
-        if (nc) atomicAdd(row + 1, nc);
+    if (hit_any) group_sync<WARP>();
+    for (uint32_t e = tid; e < W1; e += bd) rlnext[static_cast<uint64_t>(slice) * W1 + e] = lostnew[e];
+    if (any) {   // else nothing was tested
+        unsigned long long* row = a.stats + kStatsCols * step;
+        for (int off = 16; off > 0; off >>= 1) ntest += __shfl_down_sync(0xFFFFFFFFu, ntest, off);
+        if (lane == 0 && ntest) atomicAdd(row + 2, ntest);
+        if (tid == 0) atomicAdd(row + 3, static_cast<unsigned long long>(nrep));
+        if (hit_any) {
+            for (int off = 16; off > 0; off >>= 1) {
+                nr += __shfl_down_sync(0xFFFFFFFFu, nr, off);
+                nc += __shfl_down_sync(0xFFFFFFFFu, nc, off);
+            }
+            if (lane == 0) {
+                if (nr) atomicAdd(row, nr);
+                if (nc) atomicAdd(row + 1, nc);
+            }
+        }
     }
+    return hit_any ? 2 : 1;
 }
 
 // iter | stop << 32 of the control record into the host's mirror word, for
-// a host loop that polls it instead of copying the record back.
+// a host loop that polls it instead of copying the record back.  One 8-byte
+// store, with no fence after it: the host needs nothing else from the word's
+// iteration, and a system fence held the iteration's end for 2 us.
 __device__ __forceinline__ void write_mirror(unsigned long long* mirror, const FixControl* fc) {
     *reinterpret_cast<volatile unsigned long long*>(mirror) =
         fc->iter | (static_cast<unsigned long long>(fc->stop ? 1u : 0u) << 32);
-    __threadfence_system();
 }
 
 // The stop rules after iteration `it` (reachability.hpp:133-144), by one

@@ -131,20 +131,25 @@ struct gsc_problem {
     int32_t* pd = nullptr;
     uint8_t* reach8 = nullptr;
     // fused
-    gsc_b200::bword *validb = nullptr, *unsafeb = nullptr, *srcb = nullptr, *candb = nullptr, *dp = nullptr;
-    gsc_b200::bword *reach0 = nullptr, *reach1 = nullptr, *active = nullptr, *hit = nullptr;
-    uint32_t* best = nullptr;
+    gsc_b200::bword *validb = nullptr, *unsafeb = nullptr, *srcb = nullptr, *candb = nullptr;
+    gsc_b200::bword* dp[2] = {nullptr, nullptr};
+    gsc_b200::bword *reach0 = nullptr, *reach1 = nullptr, *active = nullptr;
     gsc_b200::bword* xcls = nullptr;
     uint8_t* xrep = nullptr;
-    uint32_t max_reps = 0;
+    uint32_t max_reps = 0;      // most representative accelerations of one omega column
+    gsc_b200::SliceRep* reps = nullptr;
+    uint32_t* nreps = nullptr;
+    uint32_t pass = 1, sat_threads = 128;   // of the satisfaction kernel (FusedFixArgs)
+    uint32_t* needv = nullptr;
+    bool direct = false;        // D' windows are read from D' itself
+    gsc_b200::DilateTile tile{};          // else from dilated copies
+    uint32_t ylev[gsc_b200::kYLevels] = {};
     gsc_b200::bword *dzw = nullptr, *vzw = nullptr;
     uint32_t* rowlost = nullptr;
     // sharded solve (gsc_problem_shard_*): this rank's slices and iterations done
     uint32_t shard_begin = 0, shard_slices = 0, shard_iter = 0;
     bool shard_stopped = false;
     uint32_t rl_words = 0;
-    uint32_t* offz = nullptr;   // per omega column and theta cell: part of a dilated row's offset
-    uint32_t* offv = nullptr;   // per acceleration and v cell: the other part
     uint8_t *kidx = nullptr, *lidx = nullptr;
     gsc_b200::DilateArgs dil{};
     int need_valid = 0;
@@ -251,14 +256,17 @@ bool stored_fits(const gsc_b200::GridInfo& g);
 
 // Batched execution of fused problems (gsc_batch.cu).
 gsc_b200::InstanceDesc make_instance(const gsc_problem* p);
+// Shared memory of one task of a problem under the rule that admits launch
+// shapes (fused_admission_bytes).
 size_t instance_smem(const gsc_problem* p);
-// Host work list [slot | sat_off | dil_off | fin_off | ini_off] of probs[k]
-// placed at slots[k].
+// Host work list [slot | sat_off | dil_off | ini_off] of probs[k] placed at
+// slots[k].
 void build_work_list(const std::vector<const gsc_problem*>& probs, const std::vector<uint32_t>& slots,
                      uint32_t chunk, std::vector<uint32_t>& buf, gsc_b200::WorkTotals& tot);
 gsc_b200::WorkList device_work_list(const uint32_t* dbuf, uint32_t n, uint32_t chunk, gsc_b200::FixControl* status,
                                     uint32_t* running);
-// Register words of the batched satisfaction kernel for rows of w words.
-uint32_t wmax_of(uint32_t w);
+constexpr size_t work_list_words(size_t n) { return n + 3 * (n + 1); }
+// The classes of a work list whose problems are sorted by row width.
+std::vector<gsc_b200::BatchClass> batch_classes(const std::vector<const gsc_problem*>& probs);
 
 }  // namespace gsc_api

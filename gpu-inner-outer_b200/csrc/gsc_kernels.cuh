@@ -2,6 +2,10 @@
 #pragma once
 
 #include <cstdint>
+#include <mutex>
+#include <set>
+#include <utility>
+
 #include <cuda_runtime.h>
 
 #include "gsc_common.cuh"
@@ -26,8 +30,26 @@ cudaError_t launch_pdl(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, 
     return cudaLaunchKernelEx(&cfg, k, static_cast<KArgs>(args)...);
 }
 
+// Opts `k` in to kFusedSmemOptIn bytes of dynamic shared memory on the current
+// device, once per device.  Launches may come from several host threads (a
+// server's loop and the caller's); setting the attribute twice is harmless.
+constexpr size_t kFusedSmemOptIn = 220 * 1024;
+template <typename... KArgs>
+cudaError_t allow_smem(void (*k)(KArgs...)) {
+    static std::mutex mu;
+    static std::set<std::pair<int, const void*>> done;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lk(mu);
+    if (done.count({dev, reinterpret_cast<const void*>(k)})) return cudaSuccess;
+    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kFusedSmemOptIn));
+    if (e == cudaSuccess) done.insert({dev, reinterpret_cast<const void*>(k)});
+    return e;
+}
+
 // ---- abstraction (resident nominal successors) ------------------------------------------
-// xn[((i2*n3 + i3)*M + j)*n0 + i0] = nominal x after K Euler substeps (model.hpp:26-46),
+// xn[xy_plane(i2, i3, j)*n0 + i0] = nominal x after K Euler substeps (model.hpp:26-46),
 // yn likewise over i1.  cosT/sinT[(i2*mw + jw)*K + k], vseq[(i3*ma + ja)*K + k].
 cudaError_t launch_nominal_xy(const GridInfo& g, const double* cosT, const double* sinT, const double* vseq,
                               double* xn, double* yn, cudaStream_t st);
@@ -48,14 +70,16 @@ struct MaskArgs {
 cudaError_t launch_masks(const GridInfo& g, const QueryInfo& q, const MaskArgs& a, cudaStream_t st);
 cudaError_t launch_safe2(const GridInfo& g, const QueryInfo& q, uint8_t* safe2, cudaStream_t st);
 
-// Per-axis quantised boxes.  xt/yt: [n2][n3][M][n0|n1], zt: [n2][mw], wt: [n3][ma], packed
+// Per-axis quantised boxes.  xt/yt: [xy_plane][n0|n1], zt: [n2][mw], wt: [n3][ma], packed
 // lo | hi << 16 or kReject.  flags |= 1 if an accepted non-wrap interval is empty (hi < lo),
-// |= 2 if one is wider than 64 cells.
+// |= 2 if one is wider than 32 cells.  flags[1] |= 1 << p for every accepted y interval of
+// 2^p .. 2^(p+1) - 1 cells.
 cudaError_t launch_axis_tables(const GridInfo& g, const QueryInfo& q, const double* xn, const double* yn,
                                const double* thf, const double* vf, uint32_t* xt, uint32_t* yt, uint32_t* zt,
                                uint32_t* wt, unsigned int* flags, cudaStream_t st);
 
-// Bit-sliced sets: bit b of word w of x-row r is state r*n0 + 32*w + b.
+// Bit-sliced sets: g.sw words per (theta, v) slice, of which word y*W + w
+// holds cells 32*w .. 32*w + 31 of row y.
 // mode 0: bit = src[s] != 0; 1: bit = src[s] == 0; 2: bit = src2d[i1*n0 + i0] == 0;
 // 3: bit = src[s] != 0 && src2d[i1*n0+i0] != 0; 4: bit = src[s] != 0 && src[s] (4-D second) != 0
 cudaError_t launch_pack_bits(const GridInfo& g, int mode, const uint8_t* src, const uint8_t* src2, bword* out,
@@ -156,6 +180,16 @@ struct DilateArgs {
     uint32_t kval[kMaxDilate];
     uint32_t lval[kMaxDilate];
 };
+// y levels: a copy of level p ORs the 2^p rows from each row on, so that any
+// y interval of 2^p .. 2^(p+1) - 1 rows is the OR of two rows of it.
+constexpr int kYLevels = 6;   // fused boxes span at most 32 rows
+// How one launch brings the dilated copies up to date: the y levels in use
+// (bit mask; copy (level, k, l) at ((level's rank * nk + k) * nl + l) * slices * sw)
+// and the rows of a slice that one block takes, plus the rows its highest
+// level reads beyond them.
+struct DilateTile {
+    uint32_t levels, rows, tiles, smem;
+};
 
 // Set-up plan of a problem, written by k_plan and copied to the host once:
 // the mask counts and axis-table flags, the largest number of representative
@@ -164,51 +198,69 @@ struct PlanRecord {
     unsigned long long counts[8];
     uint32_t flags;
     uint32_t max_reps;
+    uint32_t ylevels;          // y levels in use (bit mask)
     uint32_t width_overflow;   // more widths than kMaxDilate, or a v width above kMaxDilate
     uint32_t fused;            // 1 when the fused tables were planned
     DilateArgs dil;
+    uint32_t slice_reps;            // most representatives of one slice
+    unsigned long long reps;        // representatives of all slices
+    unsigned long long rep_rows;    // (theta, v) cells of their windows, summed
 };
 
+// A representative input of a (theta, v) slice: the lowest of the inputs
+// whose boxes coincide for every state of the slice (all x and y rows, the
+// theta box and the v box).
+struct __align__(16) SliceRep {
+    uint32_t j;     // the input
+    uint32_t zw;    // theta window: first cell | cells << 16 (wraps)
+    uint32_t vw;    // v window: first cell | cells << 16 (at most kMaxDilate) | 1 << 31 when some row is
+                    // marked in needv
+    uint32_t off;   // word offset of the window's copy in dzw: with kBoxY of the box's first row for row 0,
+                    // in the y level in use, else of row 0 in level 0's place
+    // Its plane's x and y boxes in short (launch_rep_boxes), so that a plane
+    // whose boxes are all [i + a, i + b] over a range of cells needs no table:
+    uint32_t hx;    // x: b - a + 1 | a << 8 (int8), kBoxX where the boxes are like that, kBoxY likewise for y
+    uint32_t hy;    // y: b - a + 1 | a << 8 (int8) | words from the first to the second row of the level << 16
+    uint32_t yr;    // rows with a y box: first | number << 16
+    uint32_t xr;    // x cells with a box: first | end << 16
+};
+constexpr uint32_t kBoxX = 1u << 16, kBoxY = 1u << 17;
+
 struct FusedFixArgs {
-    const uint32_t *xt, *yt, *zt, *wt;
+    const uint32_t *xt, *yt;
     const bword* validb;
     const bword* unsafeb;
     const bword* srcb;         // valid && source-safe
     const bword* candb;
-    bword* dp;
-    bword* reach0;
-    bword* reach1;             // the same buffer as reach0: the reachable set is updated in place
+    bword* dp[2];              // D': iteration k (from 0) reads dp[k & 1] and writes the other
+    bword* reach0;             // updated in place
     bword* active;
-    bword* hit;                // states satisfied this iteration (cleared by the finalize kernel)
-    uint32_t* best;            // lowest satisfied input per state this iteration (else 0xFFFFFFFF)
     uint32_t* controller;
     uint32_t* reach_step;
     FixControl* fc;
     unsigned long long* stats;
     int need_valid;
     const bword* xcls;         // per-plane x-box classes (launch_x_classes)
-    const uint8_t* xrep;       // per plane: the first acceleration of its omega column with identical boxes
     uint32_t cls_words;        // 32-bit words per class record
-    uint32_t max_reps;         // max representative accelerations of one omega column
-    uint32_t sat_threads;      // threads per satisfaction block (64, 128 or 256)
-    bword* dzw;                // (theta, v)-dilated D' [combo][rows * W], brought up to date each iteration
-    uint32_t* rowlost;         // [2][rl_words] bit per x-row: the row lost a D' cell in the iteration
-                               // (W1 = ceil(n1 / 32) words per (theta, v) slice, bit y % 32 of word y / 32)
-                               // (iter & 1) just finalised
-    uint32_t rl_words;         // rows / 32 + 2
-    const bword* vzw;          // (theta, v)-dilated valid set (when validity is more than safety)
-    const uint8_t* kidx;       // [n2 + 1]: theta width -> its slot in dil.kval
-    const uint8_t* lidx;       // [n3 + 1]: v width -> its slot in dil.lval
-    uint32_t nl;
+    const SliceRep* reps;      // [slices][M]: each slice's representatives, in input order
+    const uint32_t* nreps;     // [slices]
+    uint32_t pass;             // representatives whose records and changed rows are in shared memory at a time
+    uint32_t sat_threads;      // threads per block
+    uint32_t direct;           // 1: D' windows are read from D' itself, 0: from dzw
+    bword* dzw;                // (y, theta, v)-dilated copies of D' (DilateTile), brought up to date each iteration
+    uint32_t ylev[kYLevels];   // word offset of each y level in dzw
+    DilateTile tile;
+    uint32_t* rowlost;         // [2][rl_words] bit per x-row: the row lost a D' cell in the iteration before
+                               // (W1 = ceil(n1 / 32) words per (theta, v) slice, bit y % 32 of word y / 32):
+                               // iteration k reads [k & 1] and writes the other
+    uint32_t rl_words;         // slices * W1 + 1
+    const bword* vzw;          // the dilated copies of the valid set, and
+    const uint32_t* needv;     // [slices][M][W1] bit per representative and row: some state's box may hold no
+                               // valid cell (both when validity is more than safety)
     DilateArgs dil;
-    // Word offset of a representative's dilated D' row 0 in dzw, split into
-    // a part per omega column and theta cell and a part per acceleration and
-    // v cell (sums modulo 2^32, as dzw offsets are 32-bit):
-    const uint32_t* offz;      // [n2 * mw]: kslot * nl * rows * W + n1 * lz * W
-    const uint32_t* offv;      // [n3 * ma]: lslot * rows * W + n1 * n2 * lw * W
-    // Sharded solve (one rank of several): the satisfaction launch covers
-    // slices [shard_begin, shard_begin + shard_slices) only, and the stop
-    // rules are left to the host, which applies them with the counts of
+    // Sharded solve (one rank of several): the launch covers slices
+    // [shard_begin, shard_begin + shard_slices) only, reads dp[0], and the
+    // stop rules are left to the host, which applies them with the counts of
     // every rank (gsc_problem_shard_control).  shard_slices == 0: not sharded.
     uint32_t shard_begin;
     uint32_t shard_slices;
@@ -216,54 +268,28 @@ struct FusedFixArgs {
     int use_cond;
     unsigned long long* mirror;   // as StoredFixArgs::mirror
 };
-constexpr int kFusedWarps = 8;   // most warps of a satisfaction block
 
-// Shared-memory layout of one satisfaction task, in 32-bit words: the
-// active rows, the representatives' dilated D' (and valid) rows, their
-// satisfied masks, class records and y tables, the representatives' index,
-// v window and offset part, the changed-row masks, and with bulk staging
-// the spans' leading offsets and the mbarrier.  Bulk staging gives every
-// staged span a 16-byte aligned slot three words longer than its data.
-struct FusedSmemLayout {
-    uint32_t act, E, sat, cls, yts, reps, rowchg, rsh, mbar, total;
-    uint32_t e_stride, c_stride, y_stride;
-};
-__host__ __device__ inline FusedSmemLayout fused_smem_layout(uint32_t nw, uint32_t nv, uint32_t mr, uint32_t cw,
-                                                             uint32_t n1, uint32_t ma, bool bulk) {
-    auto r4 = [](uint32_t x) { return (x + 3u) & ~3u; };
-    const uint32_t w1 = (n1 + 31) / 32;
-    FusedSmemLayout L;
-    L.act = 0;
-    L.e_stride = bulk ? r4(nw + 3) : nw;
-    L.c_stride = bulk ? r4(cw + 3) : cw;
-    L.y_stride = bulk ? r4(n1 + 3) : n1;
-    L.E = bulk ? r4(nw) : nw;
-    L.sat = L.E + mr * nv * L.e_stride;
-    L.cls = bulk ? r4(L.sat + mr * nw) : L.sat + mr * nw;
-    L.yts = L.cls + mr * L.c_stride;
-    L.reps = L.yts + mr * L.y_stride;
-    L.rowchg = L.reps + 3 * ma;
-    L.rsh = L.rowchg + mr * w1;
-    L.mbar = bulk ? ((L.rsh + ma + 1) & ~1u) : L.rsh;
-    L.total = bulk ? L.mbar + 2 : L.rsh;
-    return L;
-}
 constexpr int kShiftMax = 8;   // most shifts d of a plane's shift-mask record
+// Which problems the fused method takes is a rule on the staging of one
+// (slice, omega column) task with max_reps representative accelerations
+// (fused_admission_bytes at most kFusedSmemMax); a slice's task needs less.
 constexpr size_t kFusedSmemMax = 200 * 1024;
-// Dynamic shared memory of one fused satisfaction task (bulk: the
-// one-problem kernel's bulk-staged layout; else the batched kernels').
-size_t fused_smem_bytes(const GridInfo& g, uint32_t cls_words, int need_valid, uint32_t max_reps, bool bulk);
-// Threads per satisfaction block for a problem: 128, or 256 when a block has
-// more representative rows to stage and test (max_reps * n1 * W words above
-// 2304).  128 measured 1 % faster than 64 at 65x65x38x25 and equal on the
-// published demo.
-uint32_t fused_sat_threads(const GridInfo& g, uint32_t max_reps);
+size_t fused_admission_bytes(const GridInfo& g, int need_valid, uint32_t max_reps);
+// Representatives kept in shared memory at a time, and the shared memory of a
+// slice's task (k_slice, k_batch_slice).
+constexpr uint32_t kPackedRows = 8192;   // more rows a slice than this are all tested
+constexpr uint32_t kHitNotes = 384;      // (row, representative) hits noted at a time
+uint32_t fused_pass(const GridInfo& g, uint32_t slice_reps);
+size_t fused_smem_bytes(const GridInfo& g, uint32_t pass);
+DilateTile dilate_tile_of(const GridInfo& g, const DilateArgs& d, uint32_t levels);
+// Threads per block for a problem.
+uint32_t fused_sat_threads(const GridInfo& g, uint32_t slice_reps);
 // Dilated copies of src into dst.  With fc and rowlost (during a fixpoint,
-// after its first iteration) only positions whose window holds a row that
-// lost a D' cell are recomputed; it also clears the row bits the next
-// finalize writes.
-cudaError_t launch_dilate(const GridInfo& g, const bword* src, bword* dst, const DilateArgs& d, const FixControl* fc,
-                          uint32_t* rowlost, uint32_t rl_words, cudaStream_t st);
+// after its first iteration) only tiles whose windows hold a row that lost a
+// D' cell are recomputed, and src is src0 or src1 by the iteration's parity.
+cudaError_t launch_dilate(const GridInfo& g, const bword* src0, const bword* src1, bword* dst, const DilateArgs& d,
+                          const DilateTile& t, const FixControl* fc, const uint32_t* rowlost, uint32_t rl_words,
+                          cudaStream_t st);
 // Fills a PlanRecord from the counts, flags and (when xrep is set) the
 // theta / v tables and plane representatives; writes kidx / lidx.
 cudaError_t launch_plan(const GridInfo& g, const uint32_t* zt, const uint32_t* wt, const uint8_t* xrep,
@@ -278,24 +304,31 @@ struct InstanceDesc {
     const unsigned long long* counts;
     uint32_t max_iterations;
     uint32_t stats_cap;
-    uint32_t sat_tasks;   // slices * mw
     uint32_t words;       // rows * W
 };
 
 // The instances one launch works on: slot[k] and, per task kind, the prefix
-// offsets of their tasks (off[0] = 0, off[n] = total).  A dilate / finalize
-// task covers `chunk` word positions; an init task `chunk` words, states and
+// offsets of their tasks (off[0] = 0, off[n] = total).  A satisfaction task
+// is a slice; a dilate task is a tile (none for an instance that reads D'
+// itself); an init task `chunk` words, states and
 // stats entries.
 struct WorkList {
     const uint32_t* slot;
     const uint32_t* sat_off;
     const uint32_t* dil_off;
-    const uint32_t* fin_off;
     const uint32_t* ini_off;
     uint32_t n;
     uint32_t chunk;
     FixControl* status;   // [n]: copy of each instance's FixControl after the iteration (optional)
     uint32_t* running;    // instances still running after the iteration (optional)
+};
+
+// Consecutive instances [begin, end) of a work list whose rows have W words:
+// one launch of the satisfaction kernel compiled for W.  smem: the largest
+// instance's task.
+struct BatchClass {
+    uint32_t W, begin, end, tasks;
+    size_t smem;
 };
 
 // Launch shapes of the batched kernels.
@@ -308,7 +341,8 @@ struct BatchShape {
 
 // Host-side task counts of one list (matching WorkList's offsets).
 struct WorkTotals {
-    uint32_t sat, dil, fin, ini;
+    uint32_t sat, dil, ini;
+    uint32_t dil_smem;   // shared memory of the largest dilate task
 };
 
 // An instance of a batch that keeps the GPU busy on its own (at least
@@ -328,32 +362,26 @@ struct BigInstance {
 
 cudaError_t launch_batch_init(const InstanceDesc* descs, const WorkList& wl, const WorkTotals& tot, int sms,
                               cudaStream_t st);
-// One fixpoint iteration of every listed instance: dilate, satisfaction,
-// finalize and status (which also sets the graph condition when use_cond).
-cudaError_t launch_batch_iteration(const InstanceDesc* descs, const WorkList& wl, const WorkTotals& tot,
-                                   const BatchShape& sh, uint32_t wmax, size_t smem, int sms,
-                                   cudaGraphConditionalHandle cond, int use_cond, cudaStream_t st,
-                                   uint32_t* launches);
-// One fixpoint iteration of a mixed batch: each of the nbig big instances
-// with the one-problem kernels, the instances of `small` with the batched
-// kernels (wmax and smem are theirs), then the status kernel over `all`
-// (every instance, big and small, in the order its status records use).
+// One fixpoint iteration of a batch: each of the nbig big instances with the
+// one-problem kernels, the instances of `small` with the batched kernels (a
+// dilation where one needs it, then one satisfaction launch per row width:
+// `classes`), then the status kernel over `all` (every instance, big and
+// small, in the order its status records use), which also sets the graph
+// condition when use_cond.
 cudaError_t launch_batch_step(const InstanceDesc* descs, const WorkList& small, const WorkTotals& tot_small,
-                              const WorkList& all, const BigInstance* big, uint32_t nbig, const BatchShape& sh,
-                              uint32_t wmax, size_t smem, int sms, cudaGraphConditionalHandle cond, int use_cond,
-                              cudaStream_t st, uint32_t* launches);
-// Dynamic shared memory of one satisfaction block for a shape, given one
-// task's staging (smem).
-inline size_t batch_sat_smem(const BatchShape& sh, size_t smem) { return sh.warp ? (sh.sat_threads / 32) * smem : smem; }
-
-// Shift-mask record words per plane: a 16-byte header + (kShiftMax + 1) * W masks.
-__host__ __device__ inline uint32_t class_words(const GridInfo& g) { return 4 + (kShiftMax + 1) * g.W; }
+                              const BatchClass* classes, uint32_t nclasses, const WorkList& all,
+                              const BigInstance* big, uint32_t nbig, const BatchShape& sh, int sms,
+                              cudaGraphConditionalHandle cond, int use_cond, cudaStream_t st, uint32_t* launches);
+// Shift-mask record words per plane: a 16-byte header + (kShiftMax + 1) * W
+// masks, up to a multiple of 4.
+__host__ __device__ inline uint32_t class_words(const GridInfo& g) { return (4 + (kShiftMax + 1) * g.W + 3) & ~3u; }
 // Per (slice, input) plane, the x boxes [i0 + a, i0 + b] of its states as
 // shift masks: M_d = the states whose box holds i0 + d, for the nd shifts
 // d = dmin .. dmin + nd - 1 (nd <= kShiftMax), and OK = the states with a
 // box.  A state is blocked by a row F exactly when bit i0 of
 // OR_d ((F >> d) & M_d) is set.  Header word 0: byte 0 = nd (0xFF: the plane
-// is irregular and tested state by state), byte 1 = dmin (int8); then M_d
+// is irregular and tested state by state), byte 1 = dmin (int8), byte 2 = 1
+// when every state with a box has all nd shifts (M_d = OK); then M_d
 // for each d (W words each) at word 4 + (d - dmin) * W, and OK at word
 // 4 + kShiftMax * W.  |a|, |b| < 32.
 cudaError_t launch_x_classes(const GridInfo& g, const uint32_t* xt, bword* xcls, cudaStream_t st);
@@ -364,19 +392,36 @@ cudaError_t launch_x_classes(const GridInfo& g, const uint32_t* xt, bword* xcls,
 // Also raises *max_reps to the most representatives of one omega column.
 cudaError_t launch_plane_reps(const GridInfo& g, const uint32_t* xt, const uint32_t* yt, const uint32_t* wt,
                               uint8_t* xrep, uint32_t* max_reps, cudaStream_t st);
+// Each slice's representatives: of the accelerations that launch_plane_reps
+// keeps, in input order, those whose theta box, v box and rows equal no
+// earlier one's of the slice.  Raises plan->slice_reps, reps and rep_rows.
+cudaError_t launch_slice_reps(const GridInfo& g, const uint32_t* xt, const uint32_t* yt, const uint32_t* zt,
+                              const uint32_t* wt, const uint8_t* xrep, SliceRep* reps, uint32_t* nreps,
+                              PlanRecord* plan, cudaStream_t st);
+// The offsets and boxes in short of every representative (after the plan:
+// kidx, lidx, nl).
+cudaError_t launch_rep_boxes(const GridInfo& g, const uint8_t* kidx, const uint8_t* lidx, uint32_t nl,
+                             const FusedFixArgs& a, SliceRep* reps, cudaStream_t st);
+// When validity is more than safety: the rows (needv) with a state whose box
+// under a representative holds no valid cell, marked in the representative
+// when there are any; rowvoid: [slices * W1] scratch.  A box with no D' cell
+// and a row without a void cell (invalid yet safe) in its y, theta and v
+// ranges holds a valid one, since none of that row's cells is unsafe; only
+// the others are looked at cell by cell.
+cudaError_t launch_need_valid(const GridInfo& g, const FusedFixArgs& a, uint32_t* rowvoid, SliceRep* reps,
+                              uint32_t* needv, cudaStream_t st);
 cudaError_t launch_fused_init(const GridInfo& g, const FusedFixArgs& a, const uint8_t* cand, cudaStream_t st);
-// The offz / offv tables of a problem (after its plan: kidx, lidx, nl).
-cudaError_t launch_sat_offsets(const GridInfo& g, const uint32_t* zt, const uint32_t* wt, const uint8_t* kidx,
-                               const uint8_t* lidx, uint32_t nl, uint32_t* offz, uint32_t* offv, cudaStream_t st);
-// One iteration is three launches: the dilation, the satisfaction kernel
-// and the finalize kernel (whose last block applies the stop rules).
-// ev (optional, kProfileEvents events): [0] before the dilation, [1..4] after
-// it, [5] after the satisfaction kernel, [6] after the finalize kernel.
+// One iteration is one launch (k_slice, whose last block applies the stop
+// rules), after the dilation unless a.direct.
+// ev (optional, kProfileEvents events): [0] before the dilation, [1] after
+// it, [5] and [6] after the satisfaction kernel.
 cudaError_t launch_fused_iteration(const GridInfo& g, const FusedFixArgs& a, cudaStream_t st, uint32_t* launches,
                                    cudaEvent_t* ev = nullptr);
 
-// Sharded solve: the iteration's dilation (of the whole grid) and
-// satisfaction (of the shard's slices) without the stop rules.
+inline uint32_t fused_launches(bool direct) { return direct ? 1u : 2u; }
+
+// Sharded solve: one iteration of the shard's slices without the stop rules;
+// dp[0] then holds the shard's new D'.
 cudaError_t launch_shard_iteration(const GridInfo& g, const FusedFixArgs& a, cudaStream_t st);
 // Stop rules of a sharded solve's iteration fc->iter + 1 with the counts of
 // every rank; the next iteration is never incremental.

@@ -340,10 +340,11 @@ void loop(gsc_server* s) {
     bool list_dirty = true;
     std::vector<const gsc_problem*> probs, sprobs;
     std::vector<uint32_t> slots, sslots, hl, hls;
+    std::vector<Req*> small;
     std::vector<BigInstance> big;
     WorkTotals tot{}, tot_small{};
     WorkList wl{}, wl_small{};
-    uint32_t wmax = 1;
+    std::vector<BatchClass> classes;
     size_t smem = 0;
     const uint32_t K = s->opt.iterations_per_step;
     while (true) {
@@ -367,8 +368,8 @@ void loop(gsc_server* s) {
             slots.clear();
             sprobs.clear();
             sslots.clear();
+            small.clear();
             big.clear();
-            uint32_t w = 1;
             smem = 0;
             for (Req* r : s->running) {
                 probs.push_back(r->p.get());
@@ -377,12 +378,16 @@ void loop(gsc_server* s) {
                     big.push_back(BigInstance{r->p->g, s->hdesc[r->slot].a});
                     continue;
                 }
-                sprobs.push_back(r->p.get());
-                sslots.push_back(r->slot);
-                w = std::max(w, r->p->g.W);
+                small.push_back(r);
                 smem = std::max(smem, instance_smem(r->p.get()));
             }
-            wmax = wmax_of(w);
+            std::stable_sort(small.begin(), small.end(),
+                             [](const Req* x, const Req* y) { return x->p->g.W < y->p->g.W; });
+            for (Req* r : small) {
+                sprobs.push_back(r->p.get());
+                sslots.push_back(r->slot);
+            }
+            classes = batch_classes(sprobs);
             build_work_list(probs, slots, s->shape.chunk, hl, tot);
             build_work_list(sprobs, sslots, s->shape.chunk, hls, tot_small);
             std::memcpy(s->hlist, hl.data(), hl.size() * 4);
@@ -398,10 +403,11 @@ void loop(gsc_server* s) {
         const uint32_t n = static_cast<uint32_t>(s->running.size());
         cudaError_t e = cudaSuccess;
         BatchShape shape = s->shape;
-        if (batch_sat_smem(shape, smem) > kFusedSmemMax) shape.warp = 0;
+        if (shape.warp && (shape.sat_threads / 32) * smem > kFusedSmemMax) shape.warp = 0;
         for (uint32_t i = 0; e == cudaSuccess && i < K; ++i)
-            e = launch_batch_step(s->ddesc, wl_small, tot_small, wl, big.data(), static_cast<uint32_t>(big.size()),
-                                  shape, wmax, smem, sms, 0, 0, s->s_main, nullptr);
+            e = launch_batch_step(s->ddesc, wl_small, tot_small, classes.data(), static_cast<uint32_t>(classes.size()),
+                                  wl, big.data(), static_cast<uint32_t>(big.size()), shape, sms, 0, 0, s->s_main,
+                                  nullptr);
         if (e == cudaSuccess) e = cudaEventRecord(s->ev_step, s->s_main);
         {
             std::lock_guard<std::mutex> lk(s->mu);
@@ -517,7 +523,7 @@ int gsc_server_create(gsc_context* ctx, const gsc_server_options* options, gsc_s
     s->ictx.stream = s->s_prep;
     GSC_CU(ctx, cudaEventCreateWithFlags(&s->ev_step, cudaEventDisableTiming));
     const uint32_t n = o.max_slots;
-    const size_t list_words = n + 4ull * (n + 1);
+    const size_t list_words = work_list_words(n);
     const size_t dbytes = sizeof(InstanceDesc) * n + 2 * 4 * list_words + 256 * 3;
     GSC_CU(ctx, cudaMalloc(&s->dmem, dbytes));
     char* d = static_cast<char*>(s->dmem);

@@ -50,8 +50,8 @@ __device__ __forceinline__ bool in_rect(const double* lb, const double* ub, cons
 
 // ---- nominal successors -----------------------------------------------------------------
 
-// One warp per plane (i2, i3, j), plane = (i2*n3 + i3)*M + j; lanes over
-// the x then the y cells.  The plane's trajectory terms dt * (v * cos theta)
+// One warp per plane (xy_plane: (i2*n3 + i3)*M + j, or i2*n3 + i3 with one
+// substep, whose terms input 0 stands for); lanes over the x then the y cells.  The plane's trajectory terms dt * (v * cos theta)
 // and dt * (v * sin theta) do not depend on the cell, so each is computed once
 // (staged in shared memory for up to kTermsMax substeps) and added to the
 // cell centre in the reference's order (model.hpp:34-45).
@@ -64,14 +64,14 @@ __global__ void __launch_bounds__(kPlaneThreads) k_nominal_xy(GridInfo g, const 
                                                              double* __restrict__ xn, double* __restrict__ yn) {
     __shared__ double terms[kPlaneThreads / 32][2][kTermsMax];
     const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const uint64_t planes = static_cast<uint64_t>(g.slices) * g.M;
+    const uint64_t planes = static_cast<uint64_t>(g.slices) * g.xy_planes;
     const uint64_t wstride = static_cast<uint64_t>(gridDim.x) * (blockDim.x >> 5);
     const uint32_t K = g.K;
     const bool staged = K <= kTermsMax;
     for (uint64_t plane = blockIdx.x * static_cast<uint64_t>(blockDim.x >> 5) + wib; plane < planes;
          plane += wstride) {
-        const uint32_t j = static_cast<uint32_t>(plane % g.M);
-        const uint64_t q = plane / g.M;
+        const uint32_t j = static_cast<uint32_t>(plane % g.xy_planes);
+        const uint64_t q = plane / g.xy_planes;
         const uint32_t i3 = static_cast<uint32_t>(q % g.n[3]);
         const uint32_t i2 = static_cast<uint32_t>(q / g.n[3]);
         const uint32_t ja = j % g.ma, jw = j / g.ma;
@@ -232,25 +232,26 @@ __global__ void __launch_bounds__(kPlaneThreads) k_axis_tables(GridInfo g, Query
                                                               const double* __restrict__ vf, uint32_t* xt,
                                                               uint32_t* yt, uint32_t* zt, uint32_t* wt,
                                                               unsigned int* flags) {
-    const uint64_t planes = static_cast<uint64_t>(g.slices) * g.M;
+    const uint64_t planes = static_cast<uint64_t>(g.slices) * g.xy_planes;
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t wstride = static_cast<uint64_t>(gridDim.x) * (blockDim.x >> 5);
-    unsigned int fl = 0;
+    unsigned int fl = 0, levels = 0;
     for (uint64_t plane = blockIdx.x * static_cast<uint64_t>(blockDim.x >> 5) + (threadIdx.x >> 5);
          plane < planes; plane += wstride) {
-        const uint32_t i3 = static_cast<uint32_t>((plane / g.M) % g.n[3]);
+        const uint32_t i3 = static_cast<uint32_t>((plane / g.xy_planes) % g.n[3]);
         const double vc = centre(g, 3, i3);
         for (int d = 0; d < 2; ++d) {
             const uint32_t n = g.n[d];
             const double r = box_radius(g, q, d, vc);
             const double* nom = (d ? yn : xn) + plane * n;
-            uint32_t* out = (d ? yt : xt) + plane * n;
+            uint32_t* out = d ? yt + plane * g.n1p : xt + plane * n;
             for (uint32_t i = lane; i < n; i += 32) {
                 uint32_t lo, hi;
                 const bool ok = axis_box(g, d, nom[i], r, &lo, &hi);
                 out[i] = ok ? pack16(lo, hi) : kReject;
                 if (ok && hi < lo) fl |= 1u;
                 if (ok && hi >= lo && hi - lo >= kBits) fl |= 2u;
+                if (d && ok && hi >= lo) levels |= 1u << (31 - __clz(hi - lo + 1));
             }
         }
     }
@@ -274,6 +275,8 @@ __global__ void __launch_bounds__(kPlaneThreads) k_axis_tables(GridInfo g, Query
         }
     }
     if (fl) atomicOr(flags, fl);
+    levels = __reduce_or_sync(0xFFFFFFFFu, levels);
+    if (lane == 0 && levels) atomicOr(flags + 1, levels);
 }
 
 // ---- bit-sliced sets --------------------------------------------------------------------
@@ -281,15 +284,15 @@ __global__ void __launch_bounds__(kPlaneThreads) k_axis_tables(GridInfo g, Query
 // One thread per word: the 32 cells of word w of x-row r.
 __global__ void k_pack_bits(GridInfo g, int mode, const uint8_t* __restrict__ src, const uint8_t* __restrict__ src2,
                             bword* __restrict__ out) {
-    const uint64_t words = g.rows * g.W;
+    const uint64_t words = static_cast<uint64_t>(g.slices) * g.sw;
     for (uint64_t e = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; e < words;
          e += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
-        const uint64_t r = e / g.W;
-        const uint32_t w = static_cast<uint32_t>(e - r * g.W);
-        const uint32_t i1 = static_cast<uint32_t>(r % g.n[1]);
-        const uint64_t base = r * g.n[0];
+        const uint64_t slice = e / g.sw;
+        const uint32_t rem = static_cast<uint32_t>(e - slice * g.sw);
+        const uint32_t i1 = rem / g.W, w = rem - i1 * g.W;
+        const uint64_t base = (slice * g.n[1] + i1) * g.n[0];
         bword word = 0;
-        for (uint32_t b = 0; b < kBits; ++b) {
+        if (i1 < g.n[1]) for (uint32_t b = 0; b < kBits; ++b) {
             const uint32_t i0 = w * kBits + b;
             if (i0 >= g.n[0]) break;
             bool bit;
@@ -320,7 +323,8 @@ __global__ void __launch_bounds__(kPlaneThreads) k_unpack_bits(GridInfo g, const
     const uint64_t wstride = static_cast<uint64_t>(gridDim.x) * (blockDim.x >> 5);
     for (uint64_t r = blockIdx.x * static_cast<uint64_t>(blockDim.x >> 5) + (threadIdx.x >> 5); r < g.rows;
          r += wstride) {
-        const bword* row = bits + r * g.W;
+        const uint64_t slice = r / g.n[1];
+        const bword* row = bits + slice * g.sw + (r - slice * g.n[1]) * g.W;
         uint8_t* o = out + r * g.n[0];
         for (uint32_t i0 = lane; i0 < g.n[0]; i0 += 32) o[i0] = static_cast<uint8_t>((row[i0 / kBits] >> (i0 % kBits)) & 1u);
     }
@@ -386,9 +390,9 @@ __device__ __forceinline__ PairBox pair_box(const GridInfo& g, const uint32_t* _
     uint32_t idx[4];
     unflatten(g, s, idx);
     const uint32_t ja = j % g.ma, jw = j / g.ma;
-    const uint64_t plane = (static_cast<uint64_t>(idx[2]) * g.n[3] + idx[3]) * g.M + j;
+    const uint64_t plane = xy_plane(g, idx[2], idx[3], j);
     const uint32_t xe = __ldg(xt + plane * g.n[0] + idx[0]);
-    const uint32_t ye = __ldg(yt + plane * g.n[1] + idx[1]);
+    const uint32_t ye = __ldg(yt + plane * g.n1p + idx[1]);
     const uint32_t ze = __ldg(zt + idx[2] * g.mw + jw);
     const uint32_t we = __ldg(wt + idx[3] * g.ma + ja);
     bool src = true;
@@ -473,7 +477,7 @@ __global__ void k_x_classes(GridInfo g, const uint32_t* __restrict__ xt, bword* 
     extern __shared__ uint32_t s_xrows[];
     const uint32_t cw = class_words(g);
     const uint32_t n0 = g.n[0];
-    const uint64_t planes = static_cast<uint64_t>(g.slices) * g.M;
+    const uint64_t planes = static_cast<uint64_t>(g.slices) * g.xy_planes;
     for (uint64_t first = blockIdx.x * static_cast<uint64_t>(blockDim.x); first < planes;
          first += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
         const uint32_t np = static_cast<uint32_t>(min(static_cast<uint64_t>(blockDim.x), planes - first));
@@ -484,7 +488,7 @@ __global__ void k_x_classes(GridInfo g, const uint32_t* __restrict__ xt, bword* 
         if (threadIdx.x >= np) continue;
         const uint64_t plane = first + threadIdx.x;
         const uint32_t* row = s_xrows + threadIdx.x * n0;
-        int dmin = 32, dmax = -32;
+        int dmin = 32, dmax = -32, amax = -32, bmin = 32;
         bool irregular = false;
         for (uint32_t i0 = 0; i0 < n0; ++i0) {
             const uint32_t xe = row[i0];
@@ -496,6 +500,8 @@ __global__ void k_x_classes(GridInfo g, const uint32_t* __restrict__ xt, bword* 
                 break;
             }
             dmin = min(dmin, a);
+            amax = max(amax, a);
+            bmin = min(bmin, b);
             dmax = max(dmax, b);
         }
         const int nd = (dmax >= dmin) ? dmax - dmin + 1 : 0;
@@ -503,7 +509,8 @@ __global__ void k_x_classes(GridInfo g, const uint32_t* __restrict__ xt, bword* 
         bword* o = out + plane * cw;
         o[0] = irregular ? 0xFFu
                          : static_cast<bword>(nd) |
-                               (static_cast<bword>(static_cast<uint8_t>(static_cast<int8_t>(nd ? dmin : 0))) << 8);
+                               (static_cast<bword>(static_cast<uint8_t>(static_cast<int8_t>(nd ? dmin : 0))) << 8) |
+                               (amax <= dmin && bmin >= dmax ? 0x10000u : 0u);
         o[1] = o[2] = o[3] = 0;
         // One x word at a time, its masks in registers.
         for (uint32_t w = 0; w < g.W; ++w) {
@@ -535,7 +542,7 @@ __global__ void k_plane_reps(GridInfo g, const uint32_t* __restrict__ xt, const 
     // One warp per column; the lanes compare a pair of planes' x and y rows
     // together.  Representatives are kept in increasing order, so an input
     // maps to the lowest earlier input with the same rows and v box.  With
-    // stage_words (= ma * (n0 + n1)), the column's x rows and then its y rows
+    // stage_words (= ma * (n0 + n1p)), the column's x rows and then its y rows
     // are first copied into the warp's shared memory in one round and
     // compared there; else they are compared in global memory.
     extern __shared__ uint32_t s_rows[];
@@ -543,7 +550,8 @@ __global__ void k_plane_reps(GridInfo g, const uint32_t* __restrict__ xt, const 
     const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     uint8_t* reps = s_reps[wib];
     uint32_t* rows = s_rows + static_cast<uint64_t>(wib) * stage_words;
-    const uint32_t n0 = g.n[0], n1 = g.n[1], ma = g.ma;
+    const uint32_t n0 = g.n[0], n1 = g.n[1], n1p = g.n1p, ma = g.ma;
+    const bool shared_xy = g.xy_planes == 1;   // one x / y plane per slice: every row pair is equal
     const uint32_t nx = ma * n0;
     const uint64_t columns = static_cast<uint64_t>(g.slices) * g.mw;
     const uint64_t wstride = static_cast<uint64_t>(gridDim.x) * (blockDim.x >> 5);
@@ -554,10 +562,10 @@ __global__ void k_plane_reps(GridInfo g, const uint32_t* __restrict__ xt, const 
         const uint32_t i3 = static_cast<uint32_t>((col / g.mw) % g.n[3]);
         const uint64_t p0 = col * ma;
         const uint32_t* X = xt + p0 * n0;
-        const uint32_t* Y = yt + p0 * n1;
+        const uint32_t* Y = yt + p0 * n1p;
         if (stage_words) {
             for (uint32_t i = lane; i < nx; i += 32) cp_async4(rows + i, X + i);
-            for (uint32_t i = lane; i < ma * n1; i += 32) cp_async4(rows + nx + i, Y + i);
+            for (uint32_t i = lane; i < ma * n1p; i += 32) cp_async4(rows + nx + i, Y + i);
             cp_async_wait_all();
             __syncwarp();
             X = rows;
@@ -571,8 +579,8 @@ __global__ void k_plane_reps(GridInfo g, const uint32_t* __restrict__ xt, const 
                 const uint32_t jb = reps[k];
                 if (wt[i3 * ma + jb] != we) continue;
                 bool same = true;
-                for (uint32_t i = lane; i < n0; i += 32) same = same && X[jb * n0 + i] == X[ja * n0 + i];
-                for (uint32_t i = lane; i < n1; i += 32) same = same && Y[jb * n1 + i] == Y[ja * n1 + i];
+                for (uint32_t i = lane; !shared_xy && i < n0; i += 32) same = same && X[jb * n0 + i] == X[ja * n0 + i];
+                for (uint32_t i = lane; !shared_xy && i < n1; i += 32) same = same && Y[jb * n1p + i] == Y[ja * n1p + i];
                 if (__all_sync(0xFFFFFFFFu, same)) {
                     r = jb;
                     break;
@@ -588,6 +596,101 @@ __global__ void k_plane_reps(GridInfo g, const uint32_t* __restrict__ xt, const 
         most = max(most, nrep);
     }
     if (lane == 0 && most) atomicMax(max_reps, most);
+}
+
+// One warp per slice (theta i2, v i3): the column representatives of
+// k_plane_reps in input order; one whose theta box, v box and x and y rows
+// equal an earlier representative's of the slice is dropped.  The list's
+// (theta, v) boxes are compared 32 at a time, rows only where those agree.
+constexpr int kSliceRepsCache = 64;   // list entries whose boxes are also kept in shared memory
+
+__global__ void __launch_bounds__(kThreadsReps) k_slice_reps(GridInfo g, const uint32_t* __restrict__ xt,
+                                                             const uint32_t* __restrict__ yt,
+                                                             const uint32_t* __restrict__ zt,
+                                                             const uint32_t* __restrict__ wt,
+                                                             const uint8_t* __restrict__ xrep, SliceRep* reps,
+                                                             uint32_t* nreps, PlanRecord* plan) {
+    __shared__ uint2 s_zw[kThreadsReps / 32][kSliceRepsCache];
+    const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    uint2* cache = s_zw[wib];
+    const uint32_t n0 = g.n[0], n1 = g.n[1], n2 = g.n[2], ma = g.ma, mw = g.mw;
+    uint32_t most = 0;
+    unsigned long long total = 0, rows = 0;
+    for (uint32_t s = blockIdx.x * (blockDim.x >> 5) + wib; s < g.slices; s += gridDim.x * (blockDim.x >> 5)) {
+        const uint32_t i2 = s % n2, i3 = s / n2;
+        SliceRep* list = reps + static_cast<uint64_t>(s) * g.M;
+        const uint8_t* col = xrep + (static_cast<uint64_t>(i2) * g.n[3] + i3) * g.M;
+        uint32_t n = 0;
+        // The first 32 accelerations' v boxes stay in registers, and a column's
+        // loads go out one column ahead.
+        const uint32_t we0 = lane < ma ? wt[i3 * ma + lane] : kReject;
+        uint32_t znext = zt[i2 * mw], cnext = lane < ma ? col[lane] : 0xFFFFu;
+        for (uint32_t jw = 0; jw < mw; ++jw) {
+            const uint32_t ze = znext, c0 = cnext;
+            if (jw + 1 < mw) {
+                znext = zt[i2 * mw + jw + 1];
+                cnext = lane < ma ? col[(jw + 1) * ma + lane] : 0xFFFFu;
+            }
+            for (uint32_t base = 0; base < ma; base += 32) {
+                const uint32_t ja = base + lane;
+                const uint32_t we = base == 0 ? we0 : ja < ma ? wt[i3 * ma + ja] : kReject;
+                const uint32_t rep = base == 0 ? c0 : ja < ma ? col[jw * ma + ja] : 0xFFFFu;
+                uint32_t todo = __ballot_sync(0xFFFFFFFFu, we != kReject && rep == ja);
+                for (; todo; todo &= todo - 1) {
+                    const uint32_t src = __ffs(todo) - 1;
+                    const uint32_t w = __shfl_sync(0xFFFFFFFFu, we, src);
+                    const uint32_t j = base + src + ma * jw;
+                    bool dup = false;
+                    for (uint32_t k0 = 0; k0 < n && !dup; k0 += 32) {
+                        const uint32_t k = k0 + lane;
+                        bool same = false;
+                        if (k < n) {
+                            uint2 box;
+                            if (k < kSliceRepsCache) {
+                                box = cache[k];
+                            } else {
+                                const uint32_t jb = list[k].j;
+                                box = make_uint2(zt[i2 * mw + jb / ma], wt[i3 * ma + jb % ma]);
+                            }
+                            same = box.x == ze && box.y == w;
+                        }
+                        uint32_t m = __ballot_sync(0xFFFFFFFFu, same);
+                        if (g.xy_planes == 1) {
+                            dup = m != 0;
+                            continue;
+                        }
+                        for (; m && !dup; m &= m - 1) {
+                            const uint64_t pa = xy_plane(g, i2, i3, j), pb = xy_plane(g, i2, i3, list[k0 + __ffs(m) - 1].j);
+                            bool eq = true;
+                            for (uint32_t i = lane; i < n0; i += 32) eq = eq && xt[pa * n0 + i] == xt[pb * n0 + i];
+                            for (uint32_t i = lane; i < n1; i += 32) eq = eq && yt[pa * g.n1p + i] == yt[pb * g.n1p + i];
+                            dup = __all_sync(0xFFFFFFFFu, eq);
+                        }
+                    }
+                    if (dup) continue;
+                    const uint32_t lz = lo16(ze), hz = hi16(ze), lw = lo16(w);
+                    const uint32_t nz = (lz <= hz) ? hz - lz + 1 : n2 - lz + hz + 1;
+                    const uint32_t nv = hi16(w) >= lw ? hi16(w) - lw + 1 : 0;   // an empty box: no fused solve
+                    if (lane == 0) {
+                        list[n] = SliceRep{j, pack16(lz, nz), pack16(lw, nv), 0u, 0u, 0u, 0u, 0u};
+                        if (n < kSliceRepsCache) cache[n] = make_uint2(ze, w);
+                    }
+                    __syncwarp();
+                    ++n;
+                    rows += static_cast<unsigned long long>(nz) * nv;
+                }
+            }
+        }
+        if (lane == 0) nreps[s] = n;
+        most = max(most, n);
+        total += n;
+        __syncwarp();
+    }
+    if (lane == 0 && total) {
+        atomicMax(&plan->slice_reps, most);
+        atomicAdd(&plan->reps, total);
+        atomicAdd(&plan->rep_rows, rows);
+    }
 }
 
 // 2-D prefix of unsafe (x, y) centres; one block: rows, then columns.
@@ -615,8 +718,8 @@ __global__ void k_prefix2(GridInfo g, const uint8_t* __restrict__ safe2, int32_t
 
 cudaError_t launch_nominal_xy(const GridInfo& g, const double* cosT, const double* sinT, const double* vseq,
                               double* xn, double* yn, cudaStream_t st) {
-    k_nominal_xy<<<warp_blocks(static_cast<uint64_t>(g.slices) * g.M), kPlaneThreads, 0, st>>>(g, cosT, sinT, vseq,
-                                                                                            xn, yn);
+    k_nominal_xy<<<warp_blocks(static_cast<uint64_t>(g.slices) * g.xy_planes), kPlaneThreads, 0, st>>>(
+        g, cosT, sinT, vseq, xn, yn);
     return cudaGetLastError();
 }
 
@@ -633,15 +736,14 @@ cudaError_t launch_safe2(const GridInfo& g, const QueryInfo& q, uint8_t* safe2, 
 cudaError_t launch_axis_tables(const GridInfo& g, const QueryInfo& q, const double* xn, const double* yn,
                                const double* thf, const double* vf, uint32_t* xt, uint32_t* yt, uint32_t* zt,
                                uint32_t* wt, unsigned int* flags, cudaStream_t st) {
-    k_axis_tables<<<warp_blocks(static_cast<uint64_t>(g.slices) * g.M), kPlaneThreads, 0, st>>>(g, q, xn, yn, thf,
-                                                                                             vf, xt, yt, zt, wt,
-                                                                                             flags);
+    k_axis_tables<<<warp_blocks(static_cast<uint64_t>(g.slices) * g.xy_planes), kPlaneThreads, 0, st>>>(
+        g, q, xn, yn, thf, vf, xt, yt, zt, wt, flags);
     return cudaGetLastError();
 }
 
 cudaError_t launch_pack_bits(const GridInfo& g, int mode, const uint8_t* src, const uint8_t* src2, bword* out,
                              cudaStream_t st) {
-    k_pack_bits<<<blocks_for(g.rows * g.W), kThreads, 0, st>>>(g, mode, src, src2, out);
+    k_pack_bits<<<blocks_for(static_cast<uint64_t>(g.slices) * g.sw), kThreads, 0, st>>>(g, mode, src, src2, out);
     return cudaGetLastError();
 }
 
@@ -676,7 +778,7 @@ cudaError_t launch_x_classes(const GridInfo& g, const uint32_t* xt, bword* xcls,
     uint32_t tpb = static_cast<uint32_t>((44u * 1024u) / (4u * std::max<uint32_t>(g.n[0], 1u)));
     tpb = std::min<uint32_t>(128u, std::max<uint32_t>(32u, tpb & ~31u));
     if (4ull * tpb * g.n[0] > 48 * 1024) return cudaErrorInvalidValue;
-    k_x_classes<<<blocks_for(static_cast<uint64_t>(g.slices) * g.M, tpb), tpb, 4ull * tpb * g.n[0], st>>>(g, xt, xcls);
+    k_x_classes<<<blocks_for(static_cast<uint64_t>(g.slices) * g.xy_planes, tpb), tpb, 4ull * tpb * g.n[0], st>>>(g, xt, xcls);
     return cudaGetLastError();
 }
 
@@ -687,10 +789,20 @@ cudaError_t launch_plane_reps(const GridInfo& g, const uint32_t* xt, const uint3
     if (b > 8192) b = 8192;
     // Stage a column's rows in shared memory when they fit 44 KB a block (the
     // default 48 KB less the representatives' static arrays).
-    const uint64_t words = static_cast<uint64_t>(g.ma) * (g.n[0] + g.n[1]);
-    const uint32_t stage = words * 4 * (kThreadsReps / 32) <= 44 * 1024 ? static_cast<uint32_t>(words) : 0u;
+    const uint64_t words = static_cast<uint64_t>(g.ma) * (g.n[0] + g.n1p);
+    const uint32_t stage =
+        g.xy_planes != 1 && words * 4 * (kThreadsReps / 32) <= 44 * 1024 ? static_cast<uint32_t>(words) : 0u;
     k_plane_reps<<<static_cast<unsigned int>(b), kThreadsReps, 4ull * stage * (kThreadsReps / 32), st>>>(
         g, xt, yt, wt, xrep, max_reps, stage);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_slice_reps(const GridInfo& g, const uint32_t* xt, const uint32_t* yt, const uint32_t* zt,
+                              const uint32_t* wt, const uint8_t* xrep, SliceRep* reps, uint32_t* nreps,
+                              PlanRecord* plan, cudaStream_t st) {
+    uint64_t b = (g.slices + kThreadsReps / 32 - 1) / (kThreadsReps / 32);
+    if (b > 8192) b = 8192;
+    k_slice_reps<<<static_cast<unsigned int>(b), kThreadsReps, 0, st>>>(g, xt, yt, zt, wt, xrep, reps, nreps, plan);
     return cudaGetLastError();
 }
 
