@@ -672,6 +672,17 @@ int problem_stage1(gsc_problem* p, const gsc_query_desc* qd) {
     ma.build_cand = qd->candidate_mask ? 0 : 1;
     ma.safe = qd->safe_mask ? p->safe : nullptr;
     ma.safe_rank = p->safe_rank;
+    if (p->fused_candidate) {
+        const uint64_t words = static_cast<uint64_t>(g.slices) * g.sw;
+        GSC_TRY(palloc(p, &p->validb, words));
+        GSC_TRY(palloc(p, &p->unsafeb, words));
+        GSC_TRY(palloc(p, &p->srcb, words));
+        GSC_TRY(palloc(p, &p->candb, words));
+        ma.validb = p->validb;
+        ma.unsafeb = p->unsafeb;
+        ma.srcb = p->srcb;
+        ma.candb = p->candb;
+    }
     ma.cmp_safe = p->safe;
     ma.cmp_rank = p->safe_rank;
     ma.counts = p->counts;
@@ -681,22 +692,23 @@ int problem_stage1(gsc_problem* p, const gsc_query_desc* qd) {
     const uint64_t planes = table_planes(g);
     GSC_TRY(palloc(p, &p->xt, planes * g.n[0]));
     GSC_TRY(palloc(p, &p->yt, planes * g.n1p));
+    GSC_TRY(palloc(p, &p->shorts, static_cast<uint64_t>(g.slices) * g.xy_planes));
     GSC_TRY(palloc(p, &p->zt, static_cast<uint64_t>(g.n[2]) * g.mw));
     GSC_TRY(palloc(p, &p->wt, static_cast<uint64_t>(g.n[3]) * g.ma));
     GSC_CU(ctx, launch_axis_tables(g, q, p->abs->xn, p->abs->yn, p->abs->thf, p->abs->vf, p->xt, p->yt, p->zt, p->wt,
-                                   p->flags, st));
+                                   p->shorts, p->flags, st));
 
     // Fused tables that do not depend on the sets, and the plan.
     GSC_TRY(palloc(p, &p->dplan, 1));
     GSC_CU(ctx, cudaMemsetAsync(p->dplan, 0, sizeof(PlanRecord), st));
     if (p->fused_candidate) {
         GSC_TRY(palloc(p, &p->xcls, planes * class_words(g)));
-        GSC_CU(ctx, launch_x_classes(g, p->xt, p->xcls, st));
+        GSC_CU(ctx, launch_x_classes(g, p->xt, p->shorts, p->xcls, st));
         GSC_TRY(palloc(p, &p->xrep, planes));
-        GSC_CU(ctx, launch_plane_reps(g, p->xt, p->yt, p->wt, p->xrep, &p->dplan->max_reps, st));
+        GSC_CU(ctx, launch_plane_reps(g, p->xt, p->yt, p->wt, p->shorts, p->xrep, &p->dplan->max_reps, st));
         GSC_TRY(palloc(p, &p->reps, planes));
         GSC_TRY(palloc(p, &p->nreps, g.slices));
-        GSC_CU(ctx, launch_slice_reps(g, p->xt, p->yt, p->zt, p->wt, p->xrep, p->reps, p->nreps, p->dplan, st));
+        GSC_CU(ctx, launch_slice_reps(g, p->xt, p->yt, p->zt, p->wt, p->shorts, p->xrep, p->reps, p->nreps, p->dplan, st));
         GSC_TRY(palloc(p, &p->kidx, static_cast<uint64_t>(g.n[2]) + 1));
         GSC_TRY(palloc(p, &p->lidx, static_cast<uint64_t>(g.n[3]) + 1));
     }
@@ -804,10 +816,6 @@ int problem_stage2(gsc_problem* p) {
         return GSC_OK;
     }
     const uint64_t words = static_cast<uint64_t>(g.slices) * g.sw;
-    GSC_TRY(palloc(p, &p->validb, words));
-    GSC_TRY(palloc(p, &p->unsafeb, words));
-    GSC_TRY(palloc(p, &p->srcb, words));
-    GSC_TRY(palloc(p, &p->candb, words));
     GSC_TRY(palloc(p, &p->dp[0], words));
     GSC_TRY(palloc(p, &p->dp[1], words));
     GSC_TRY(palloc(p, &p->reach0, words));
@@ -820,19 +828,7 @@ int problem_stage2(gsc_problem* p) {
     if (!p->direct) GSC_TRY(palloc(p, &p->dzw, copies * words));
     p->rl_words = g.slices * ((g.n[1] + 31) / 32) + 1;
     GSC_TRY(palloc(p, &p->rowlost, 2ull * p->rl_words));
-    GSC_CU(ctx, launch_rep_boxes(g, p->kidx, p->lidx, p->dil.nl, fused_args(p, 0, 0), p->reps, st));
-    GSC_CU(ctx, launch_pack_bits(g, 0, p->valid, nullptr, p->validb, st));
-    GSC_CU(ctx, launch_pack_bits(g, 0, p->cand, nullptr, p->candb, st));
-    if (!p->safe) {
-        GSC_CU(ctx, cudaMemsetAsync(p->unsafeb, 0, words * sizeof(bword), st));
-        GSC_CU(ctx, cudaMemcpyAsync(p->srcb, p->validb, words * sizeof(bword), cudaMemcpyDeviceToDevice, st));
-    } else if (p->safe_rank == 2) {
-        GSC_CU(ctx, launch_pack_bits(g, 2, nullptr, p->safe, p->unsafeb, st));
-        GSC_CU(ctx, launch_pack_bits(g, 3, p->valid, p->safe, p->srcb, st));
-    } else {
-        GSC_CU(ctx, launch_pack_bits(g, 1, p->safe, nullptr, p->unsafeb, st));
-        GSC_CU(ctx, launch_pack_bits(g, 4, p->valid, p->safe, p->srcb, st));
-    }
+    GSC_CU(ctx, launch_rep_offsets(g, p->kidx, p->lidx, p->dil.nl, fused_args(p, 0, 0), p->reps, st));
     if (p->need_valid) {
         GSC_TRY(palloc(p, &p->vzw, copies * words));
         GSC_CU(ctx, launch_dilate(g, p->validb, p->validb, p->vzw, p->dil, p->tile, nullptr, nullptr, 0, st));
@@ -1380,7 +1376,7 @@ int gsc_problem_phase_timings(const gsc_problem* p, gsc_phase_timings* out) {
     for (const void* q : {static_cast<const void*>(p->xt), static_cast<const void*>(p->yt),
                           static_cast<const void*>(p->zt), static_cast<const void*>(p->wt),
                           static_cast<const void*>(p->boxes), static_cast<const void*>(p->boxes16),
-                          static_cast<const void*>(p->xcls),
+                          static_cast<const void*>(p->xcls), static_cast<const void*>(p->shorts),
                           static_cast<const void*>(p->xrep), static_cast<const void*>(p->reps),
                           static_cast<const void*>(p->nreps), static_cast<const void*>(p->kidx),
                           static_cast<const void*>(p->lidx), static_cast<const void*>(p->unsafe2),

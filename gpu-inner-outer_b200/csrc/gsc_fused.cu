@@ -146,69 +146,33 @@ __global__ void __launch_bounds__(256) k_plan(GridInfo g, const uint32_t* __rest
     }
 }
 
-// The boxes of one plane row in short: [i + a, i + b] alike for every cell
-// with one, those being cells [first, end).  By one warp.
-__device__ __forceinline__ bool short_boxes(const uint32_t* __restrict__ row, uint32_t n, uint32_t* ab, uint32_t* range) {
+// SliceRep::off (kslot * nl + lslot) * slices * sw + (lz + n2 * lw) * sw and,
+// where its y boxes are alike, the level's rows; one warp per slice.  Offsets
+// are sums modulo 2^32 (below it with a row's when the dilated copies are used).
+__global__ void __launch_bounds__(256) k_rep_offsets(const __grid_constant__ GridInfo g,
+                                                     const uint8_t* __restrict__ kidx,
+                                                     const uint8_t* __restrict__ lidx, uint32_t nl,
+                                                     const __grid_constant__ FusedFixArgs a, SliceRep* reps) {
     const uint32_t lane = threadIdx.x & 31;
-    int amin = 1 << 20, amax = -(1 << 20), bmin = 1 << 20, bmax = -(1 << 20);
-    uint32_t first = n, end = 0, cells = 0;
-    for (uint32_t i = lane; i < n; i += 32) {
-        const uint32_t e = row[i];
-        if (e == kReject) continue;
-        const int a = static_cast<int>(lo16(e)) - static_cast<int>(i), b = static_cast<int>(hi16(e)) - static_cast<int>(i);
-        amin = min(amin, a);
-        amax = max(amax, a);
-        bmin = min(bmin, b);
-        bmax = max(bmax, b);
-        first = min(first, i);
-        end = max(end, i + 1);
-        ++cells;
-    }
-    amin = __reduce_min_sync(0xFFFFFFFFu, amin);
-    amax = __reduce_max_sync(0xFFFFFFFFu, amax);
-    bmin = __reduce_min_sync(0xFFFFFFFFu, bmin);
-    bmax = __reduce_max_sync(0xFFFFFFFFu, bmax);
-    first = __reduce_min_sync(0xFFFFFFFFu, first);
-    end = __reduce_max_sync(0xFFFFFFFFu, end);
-    cells = __reduce_add_sync(0xFFFFFFFFu, cells);
-    if (!cells) {
-        *ab = *range = 0;   // no cell has a box
-        return true;
-    }
-    *ab = static_cast<uint32_t>(bmax - amin + 1) | (static_cast<uint32_t>(static_cast<uint8_t>(static_cast<int8_t>(amin))) << 8);
-    *range = pack16(first, end);
-    return amin == amax && bmin == bmax && cells == end - first && amin >= -31 && bmax <= 31 && bmax - amin < 32;
-}
-
-// SliceRep::off (kslot * nl + lslot) * slices * sw + (lz + n2 * lw) * sw and
-// the boxes in short, one warp per (slice, representative).  Offsets are sums
-// modulo 2^32 (below 2^32 with the row when the dilated copies are used).
-__global__ void __launch_bounds__(256) k_rep_boxes(const __grid_constant__ GridInfo g,
-                                                   const uint8_t* __restrict__ kidx,
-                                                   const uint8_t* __restrict__ lidx, uint32_t nl,
-                                                   const __grid_constant__ FusedFixArgs a, SliceRep* reps) {
-    const uint32_t lane = threadIdx.x & 31;
-    const uint64_t total = static_cast<uint64_t>(g.slices) * g.M;
-    for (uint64_t t = (blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x) >> 5; t < total;
-         t += (static_cast<uint64_t>(gridDim.x) * blockDim.x) >> 5) {
-        const uint32_t s = static_cast<uint32_t>(t / g.M), k = static_cast<uint32_t>(t - static_cast<uint64_t>(s) * g.M);
-        if (k >= a.nreps[s]) continue;
-        SliceRep rp = reps[t];
-        const uint64_t pl = xy_plane(g, s % g.n[2], s / g.n[2], rp.j);
-        rp.off = (kidx[hi16(rp.zw)] * nl + lidx[hi16(rp.vw)]) * (g.slices * g.sw) +
-                 (lo16(rp.zw) + g.n[2] * lo16(rp.vw)) * g.sw;
-        const bool x = short_boxes(a.xt + pl * g.n[0], g.n[0], &rp.hx, &rp.xr);
-        const bool y = short_boxes(a.yt + pl * g.n1p, g.n[1], &rp.hy, &rp.yr);
-        rp.hx = (rp.hx & 0xFFFFu) | (x ? kBoxX : 0u) | (y ? kBoxY : 0u);
-        if (y) {
-            const uint32_t ny = rp.hy & 0xFFu, p = ny ? 31 - __clz(ny) : 0;
-            if (ny) {
-                rp.off += a.ylev[p] + static_cast<uint32_t>(static_cast<int>(static_cast<int8_t>(rp.hy >> 8)) * static_cast<int>(g.W));
-                rp.hy |= ((ny - (1u << p)) * g.W) << 16;
+    for (uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < g.slices; s += (gridDim.x * blockDim.x) >> 5) {
+        SliceRep* list = reps + static_cast<uint64_t>(s) * g.M;
+        const uint32_t n = a.nreps[s];
+        for (uint32_t k = lane; k < n; k += 32) {
+            SliceRep rp = list[k];
+            rp.off = (kidx[hi16(rp.zw)] * nl + lidx[hi16(rp.vw)]) * (g.slices * g.sw) +
+                     (lo16(rp.zw) + g.n[2] * lo16(rp.vw)) * g.sw;
+            if (rp.hx & kBoxY) {
+                const uint32_t ny = rp.hy & 0xFFu;
+                if (ny) {
+                    const uint32_t p = 31 - __clz(ny);
+                    const int first = static_cast<int8_t>(rp.hy >> 8);
+                    rp.off += a.ylev[p] + static_cast<uint32_t>(first * static_cast<int>(g.W));
+                    rp.hy |= ((ny - (1u << p)) * g.W) << 16;
+                }
+                rp.yr = pack16(lo16(rp.yr), hi16(rp.yr) - lo16(rp.yr));
             }
-            rp.yr = pack16(lo16(rp.yr), hi16(rp.yr) - lo16(rp.yr));
+            list[k] = rp;
         }
-        if (lane == 0) reps[t] = rp;
     }
 }
 
@@ -256,7 +220,15 @@ __global__ void __launch_bounds__(256) k_need_valid(const __grid_constant__ Grid
             }
             return m;
         };
+        // Void rows of the window, a word a lane; usually there are none.
         bool some = false;
+        uint32_t mine = 0;
+        for (uint32_t q = lane; q < W1; q += 32) {
+            mine |= void_word(q);
+            needv[t * W1 + q] = 0;
+        }
+        if (!__any_sync(0xFFFFFFFFu, mine != 0)) continue;
+        __syncwarp();
         for (uint32_t q = 0; q < W1; ++q) {
             const uint32_t y = q * 32 + lane;
             const uint32_t ye = y < n1 ? a.yt[pl * g.n1p + y] : kReject;
@@ -266,19 +238,26 @@ __global__ void __launch_bounds__(256) k_need_valid(const __grid_constant__ Grid
                 const uint32_t lo = void_word(wl), hi = wh != wl ? void_word(wh) : 0u;
                 if (!(~__funnelshift_r(lo, hi, ylo & 31) << (31u - (yhi - ylo)))) {
                     bword V[W], m[W];
-                    valid_window<W>(g, a.validb, rp.zw, rp.vw, ye, V);
+                    box_rows<W>(a, a.vzw, rp.off, rp.hx, rp.hy, y, ye, V);
                     const bword* src = a.srcb + static_cast<uint64_t>(s) * g.sw + y * W;
-                    const uint32_t* xrow = a.xt + pl * g.n[0];
+#pragma unroll
                     for (int w = 0; w < W; ++w) m[w] = src[w];
-                    without_cell<W>(xrow, V, m);
-                    for (int w = 0; w < W; ++w) {
-                        // without_cell also drops states that have no box.
-                        need |= m[w] != 0;
+                    if (rp.hx & kBoxX) {
+                        bword T[W];
+                        or_range<W>(V, T, rp.hx & 0xFFu);
+                        const int dmin = static_cast<int8_t>(rp.hx >> 8);
+#pragma unroll
+                        for (int w = 0; w < W; ++w)
+                            m[w] &= ~moved_word<W>(T, w, dmin) & bits_from(lo16(rp.xr), w) & ~bits_from(hi16(rp.xr), w);
+                    } else {
+                        without_cell<W>(a.xt + pl * g.n[0], V, m);   // drops states without a box too
                     }
+#pragma unroll
+                    for (int w = 0; w < W; ++w) need |= m[w] != 0;
                 }
             }
             const uint32_t bits = __ballot_sync(0xFFFFFFFFu, need);
-            if (lane == 0) needv[t * W1 + q] = bits;
+            if (lane == 0 && bits) needv[t * W1 + q] = bits;
             some |= bits != 0;
         }
         if (some && lane == 0) reps[t].vw = rp.vw | 0x80000000u;
@@ -444,10 +423,9 @@ cudaError_t launch_need_valid(const GridInfo& g, const FusedFixArgs& a, uint32_t
     }
 }
 
-cudaError_t launch_rep_boxes(const GridInfo& g, const uint8_t* kidx, const uint8_t* lidx, uint32_t nl,
-                             const FusedFixArgs& a, SliceRep* reps, cudaStream_t st) {
-    const uint64_t b = std::min<uint64_t>(148ull * 32, (static_cast<uint64_t>(g.slices) * g.M + 7) / 8);
-    k_rep_boxes<<<static_cast<unsigned int>(b), 256, 0, st>>>(g, kidx, lidx, nl, a, reps);
+cudaError_t launch_rep_offsets(const GridInfo& g, const uint8_t* kidx, const uint8_t* lidx, uint32_t nl,
+                               const FusedFixArgs& a, SliceRep* reps, cudaStream_t st) {
+    k_rep_offsets<<<blocks_for(static_cast<uint64_t>(g.slices) * 32, 256), 256, 0, st>>>(g, kidx, lidx, nl, a, reps);
     return cudaGetLastError();
 }
 

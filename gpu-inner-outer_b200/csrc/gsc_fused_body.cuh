@@ -289,26 +289,6 @@ __device__ __noinline__ void without_cell(const uint32_t* xrow, const bword (&X)
     }
 }
 
-// The valid cells of row i1's (y, theta, v) box ranges under a representative, ORed along x.
-template <int W>
-__device__ __forceinline__ void valid_window(const GridInfo& g, const bword* validb, uint32_t zw, uint32_t vw,
-                                             uint32_t ye, bword (&V)[W]) {
-    const uint32_t n2 = g.n[2], nz = hi16(zw), v0 = lo16(vw), nv = hi16(vw) & 0x7FFFu;
-#pragma unroll
-    for (int w = 0; w < W; ++w) V[w] = 0;
-    uint32_t z = lo16(zw);
-    for (uint32_t i = 0; i < nz; ++i) {
-        for (uint32_t v = v0; v < v0 + nv; ++v) {
-            const bword* vr = validb + static_cast<uint64_t>(z + n2 * v) * g.sw;
-            for (uint32_t y = lo16(ye); y <= hi16(ye); ++y) {
-#pragma unroll
-                for (int w = 0; w < W; ++w) V[w] |= __ldg(vr + y * W + w);
-            }
-        }
-        z = (z + 1 == n2) ? 0 : z + 1;
-    }
-}
-
 // The OR of two rows `d` words apart.
 template <int W>
 __device__ __forceinline__ void two_rows(const bword* row, uint32_t d, bword (&F)[W]) {
@@ -317,6 +297,19 @@ __device__ __forceinline__ void two_rows(const bword* row, uint32_t d, bword (&F
     load_row<W>(t, row + d);
 #pragma unroll
     for (int w = 0; w < W; ++w) F[w] |= t[w];
+}
+
+// Row i1's box rows of the dilated copies Z under a representative (offset
+// off, boxes in short hx, hy; ye: its y box where those are not alike).
+template <int W>
+__device__ __forceinline__ void box_rows(const FusedFixArgs& a, const bword* Z, uint32_t off, uint32_t hx, uint32_t hy,
+                                         uint32_t i1, uint32_t ye, bword (&F)[W]) {
+    if (hx & kBoxY) {
+        two_rows<W>(Z + (off + i1 * W), hy >> 16, F);
+    } else {
+        const uint32_t ylo = lo16(ye), ny = hi16(ye) - ylo + 1, p = 31 - __clz(ny);
+        two_rows<W>(Z + (a.ylev[p] + off + ylo * W), (ny - (1u << p)) * W, F);
+    }
 }
 
 // Of the states m of row i1 of a slice, those whose box under the slice's
@@ -330,12 +323,7 @@ __device__ __noinline__ void keep_valid(const GridInfo& g, const FusedFixArgs& a
     if (!((__ldg(a.needv + (static_cast<uint64_t>(slice) * g.M + index) * W1 + (i1 >> 5)) >> (i1 & 31)) & 1u)) return;
     const uint64_t pl = xy_plane(g, slice % g.n[2], slice / g.n[2], rp.x);
     bword V[W], none[W];
-    if (bx.x & kBoxY) {
-        two_rows<W>(a.vzw + (rp.w + i1 * W), bx.y >> 16, V);
-    } else {
-        const uint32_t ye = __ldg(a.yt + pl * g.n1p + i1), ylo = lo16(ye), ny = hi16(ye) - ylo + 1, p = 31 - __clz(ny);
-        two_rows<W>(a.vzw + (a.ylev[p] + rp.w + ylo * W), (ny - (1u << p)) * W, V);
-    }
+    box_rows<W>(a, a.vzw, rp.w, bx.x, bx.y, i1, bx.x & kBoxY ? 0u : __ldg(a.yt + pl * g.n1p + i1), V);
     if (bx.x & kBoxX) {
         bword T[W];
         or_range<W>(V, T, bx.x & 0xFFu);
@@ -569,14 +557,9 @@ __device__ __forceinline__ int slice_task(const GridInfo& g, const FusedFixArgs&
                         const uint32_t bits = __funnelshift_r(rc[wl], wh != wl ? rc[wh] : 0u, ylo & 31);
                         if (!(bits << (32u - ny))) continue;
                     }
-                    if (direct) {
-                        window_rows<W>(g, cur, rp, ylo, ny, F);
-                    } else if (!(bx.x & kBoxY)) {
-                        const uint32_t p = 31 - __clz(ny);
-                        two_rows<W>(a.dzw + (a.ylev[p] + rp.w + ylo * W), (ny - (1u << p)) * W, F);
-                    }
+                    if (direct) window_rows<W>(g, cur, rp, ylo, ny, F);
                 }
-                if (!direct && (bx.x & kBoxY)) two_rows<W>(a.dzw + (rp.w + i1 * W), bx.y >> 16, F);
+                if (!direct) box_rows<W>(a, a.dzw, rp.w, bx.x, bx.y, i1, ye, F);
                 tested += states;
                 bword sm[W], anys = 0;
                 if (bx.x & kBoxX) {

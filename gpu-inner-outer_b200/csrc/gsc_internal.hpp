@@ -111,6 +111,7 @@ struct gsc_problem {
     unsigned long long* counts = nullptr;   // [0] valid [1] cand [2] cand-not-valid [3] valid pairs [4] valid!=safe
     unsigned int* flags = nullptr;
     uint32_t *xt = nullptr, *yt = nullptr, *zt = nullptr, *wt = nullptr;
+    uint4* shorts = nullptr;   // the x / y tables' boxes in short (launch_axis_tables)
     int32_t* unsafe2 = nullptr;
     int32_t* unsafe4 = nullptr;
     int32_t* pvalid = nullptr;

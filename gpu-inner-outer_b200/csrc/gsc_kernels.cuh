@@ -63,6 +63,9 @@ struct MaskArgs {
     int build_cand;
     const uint8_t* safe;      // caller's constraint mask (rank 2 or 4), or null: use the constraint kind
     int safe_rank;
+    // Bit-sliced sets to fill too (or null): valid, candidate, unsafe (by
+    // cmp_safe; none where that is null), valid and safe.
+    bword *validb, *candb, *unsafeb, *srcb;
     const uint8_t* cmp_safe;  // safety at the centres (rank cmp_rank), to count cells whose validity differs
     int cmp_rank;
     unsigned long long* counts;  // [0] valid, [1] candidate, [2] candidate-not-valid, [4] valid != safe
@@ -74,16 +77,16 @@ cudaError_t launch_safe2(const GridInfo& g, const QueryInfo& q, uint8_t* safe2, 
 // lo | hi << 16 or kReject.  flags |= 1 if an accepted non-wrap interval is empty (hi < lo),
 // |= 2 if one is wider than 32 cells.  flags[1] |= 1 << p for every accepted y interval of
 // 2^p .. 2^(p+1) - 1 cells.
+// shorts: per plane its x and y boxes in short, {hx, hy, yr, xr}: hx = b - a + 1 | a << 8 of the x boxes
+// [i + a, i + b], with kBoxX where they are alike, |a|, |b| < 32, and the cells with one (xr: first |
+// end << 16) are in a row, and kBoxY likewise for the y boxes (hy, yr).
+constexpr uint32_t kBoxX = 1u << 16, kBoxY = 1u << 17;
 cudaError_t launch_axis_tables(const GridInfo& g, const QueryInfo& q, const double* xn, const double* yn,
                                const double* thf, const double* vf, uint32_t* xt, uint32_t* yt, uint32_t* zt,
-                               uint32_t* wt, unsigned int* flags, cudaStream_t st);
+                               uint32_t* wt, uint4* shorts, unsigned int* flags, cudaStream_t st);
 
 // Bit-sliced sets: g.sw words per (theta, v) slice, of which word y*W + w
 // holds cells 32*w .. 32*w + 31 of row y.
-// mode 0: bit = src[s] != 0; 1: bit = src[s] == 0; 2: bit = src2d[i1*n0 + i0] == 0;
-// 3: bit = src[s] != 0 && src2d[i1*n0+i0] != 0; 4: bit = src[s] != 0 && src[s] (4-D second) != 0
-cudaError_t launch_pack_bits(const GridInfo& g, int mode, const uint8_t* src, const uint8_t* src2, bword* out,
-                             cudaStream_t st);
 cudaError_t launch_unpack_bits(const GridInfo& g, const bword* bits, uint8_t* out, cudaStream_t st);
 // n words from src to dst by one small kernel (dst may be pinned host memory
 // mapped into the device's address space).
@@ -217,14 +220,12 @@ struct __align__(16) SliceRep {
                     // marked in needv
     uint32_t off;   // word offset of the window's copy in dzw: with kBoxY of the box's first row for row 0,
                     // in the y level in use, else of row 0 in level 0's place
-    // Its plane's x and y boxes in short (launch_rep_boxes), so that a plane
-    // whose boxes are all [i + a, i + b] over a range of cells needs no table:
-    uint32_t hx;    // x: b - a + 1 | a << 8 (int8), kBoxX where the boxes are like that, kBoxY likewise for y
-    uint32_t hy;    // y: b - a + 1 | a << 8 (int8) | words from the first to the second row of the level << 16
-    uint32_t yr;    // rows with a y box: first | number << 16
-    uint32_t xr;    // x cells with a box: first | end << 16
+    // Its plane's x and y boxes in short (launch_axis_tables), so that a plane
+    // whose boxes are all alike needs no table; with kBoxY (launch_rep_offsets)
+    // hy also has the words from the first to the second row of the level << 16,
+    // and yr the number of rows in place of their end:
+    uint32_t hx, hy, yr, xr;
 };
-constexpr uint32_t kBoxX = 1u << 16, kBoxY = 1u << 17;
 
 struct FusedFixArgs {
     const uint32_t *xt, *yt;
@@ -384,24 +385,25 @@ __host__ __device__ inline uint32_t class_words(const GridInfo& g) { return (4 +
 // when every state with a box has all nd shifts (M_d = OK); then M_d
 // for each d (W words each) at word 4 + (d - dmin) * W, and OK at word
 // 4 + kShiftMax * W.  |a|, |b| < 32.
-cudaError_t launch_x_classes(const GridInfo& g, const uint32_t* xt, bword* xcls, cudaStream_t st);
+cudaError_t launch_x_classes(const GridInfo& g, const uint32_t* xt, const uint4* shorts, bword* xcls,
+                             cudaStream_t st);
 // Per plane (slice, j = ja + ma * jw): the lowest ja' of the same omega column
 // whose x row, y row and v box equal those of ja, so the two inputs test every
 // state alike (with one Euler substep the x and y successors do not depend on
 // the acceleration at all).
 // Also raises *max_reps to the most representatives of one omega column.
 cudaError_t launch_plane_reps(const GridInfo& g, const uint32_t* xt, const uint32_t* yt, const uint32_t* wt,
-                              uint8_t* xrep, uint32_t* max_reps, cudaStream_t st);
+                              const uint4* shorts, uint8_t* xrep, uint32_t* max_reps, cudaStream_t st);
 // Each slice's representatives: of the accelerations that launch_plane_reps
 // keeps, in input order, those whose theta box, v box and rows equal no
 // earlier one's of the slice.  Raises plan->slice_reps, reps and rep_rows.
 cudaError_t launch_slice_reps(const GridInfo& g, const uint32_t* xt, const uint32_t* yt, const uint32_t* zt,
-                              const uint32_t* wt, const uint8_t* xrep, SliceRep* reps, uint32_t* nreps,
-                              PlanRecord* plan, cudaStream_t st);
-// The offsets and boxes in short of every representative (after the plan:
-// kidx, lidx, nl).
-cudaError_t launch_rep_boxes(const GridInfo& g, const uint8_t* kidx, const uint8_t* lidx, uint32_t nl,
-                             const FusedFixArgs& a, SliceRep* reps, cudaStream_t st);
+                              const uint32_t* wt, const uint4* shorts, const uint8_t* xrep, SliceRep* reps,
+                              uint32_t* nreps, PlanRecord* plan, cudaStream_t st);
+// The offset and the level's rows of every representative (after the plan:
+// kidx, lidx, nl, a.ylev).
+cudaError_t launch_rep_offsets(const GridInfo& g, const uint8_t* kidx, const uint8_t* lidx, uint32_t nl,
+                               const FusedFixArgs& a, SliceRep* reps, cudaStream_t st);
 // When validity is more than safety: the rows (needv) with a state whose box
 // under a representative holds no valid cell, marked in the representative
 // when there are any; rowvoid: [slices * W1] scratch.  A box with no D' cell

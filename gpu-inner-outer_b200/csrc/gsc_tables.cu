@@ -140,11 +140,16 @@ __global__ void __launch_bounds__(kPlaneThreads) k_masks(GridInfo g, QueryInfo q
         const double dy = dsub(x[1], q.cand[1]);
         const double ty = dmul(dmul(dy, dy), q.cand[3]);
         const uint64_t base = r * g.n[0];
-        for (uint32_t i0 = lane; i0 < g.n[0]; i0 += 32) {
-            const uint64_t s = base + i0;
+        const uint64_t word0 = r2 * g.sw + i1 * g.W;
+        for (uint32_t w0 = 0; w0 < g.n[0]; w0 += 32) {
+            const uint32_t i0 = w0 + lane;
+            const bool in = i0 < g.n[0];
+            const uint64_t s = base + (in ? i0 : 0u);
             x[0] = centre(g, 0, i0);
             bool v;
-            if (a.build_valid) {
+            if (!in) {
+                v = false;
+            } else if (a.build_valid) {
                 v = map_row && !(x[0] < q.map_lb[0] || x[0] > q.map_ub[0]);
                 if (v) {
                     if (few_obstacles) {
@@ -175,7 +180,9 @@ __global__ void __launch_bounds__(kPlaneThreads) k_masks(GridInfo g, QueryInfo q
                 v = a.valid[s] != 0;
             }
             bool k;
-            if (a.build_cand) {
+            if (!in) {
+                k = false;
+            } else if (a.build_cand) {
                 if (q.cand_kind == 0) {
                     k = cand_rect_row && !(x[0] < q.cand[0] || x[0] > q.cand[4]);
                 } else {
@@ -186,14 +193,33 @@ __global__ void __launch_bounds__(kPlaneThreads) k_masks(GridInfo g, QueryInfo q
             } else {
                 k = a.cand[s] != 0;
             }
-            if (a.cmp_safe) {
-                const uint8_t sf =
-                    a.cmp_rank == 4 ? a.cmp_safe[s] : a.cmp_safe[static_cast<uint64_t>(i1) * g.n[0] + i0];
-                ndiff += (v != (sf != 0));
+            bool sf = true;
+            if (a.cmp_safe && in) {
+                sf = (a.cmp_rank == 4 ? a.cmp_safe[s] : a.cmp_safe[static_cast<uint64_t>(i1) * g.n[0] + i0]) != 0;
+                ndiff += v != sf;
             }
             nv += v;
             nc += k;
             nbad += (k && !v);
+            if (a.validb) {
+                // The bit-sliced sets' words, one ballot each.
+                const uint32_t vb = __ballot_sync(0xFFFFFFFFu, v), kb = __ballot_sync(0xFFFFFFFFu, k);
+                const uint32_t ub = __ballot_sync(0xFFFFFFFFu, in && !sf);
+                if (lane == 0) {
+                    const uint64_t e = word0 + w0 / 32;
+                    a.validb[e] = vb;
+                    a.candb[e] = kb;
+                    a.unsafeb[e] = ub;
+                    a.srcb[e] = vb & ~ub;
+                }
+            }
+        }
+        // A slice's padding words are 0.
+        if (a.validb && i1 + 1 == g.n[1]) {
+            for (uint32_t e = g.n[1] * g.W + lane; e < g.sw; e += 32) {
+                const uint64_t at = r2 * g.sw + e;
+                a.validb[at] = a.candb[at] = a.unsafeb[at] = a.srcb[at] = 0;
+            }
         }
     }
     for (int off = 16; off > 0; off >>= 1) {
@@ -231,7 +257,7 @@ __global__ void __launch_bounds__(kPlaneThreads) k_axis_tables(GridInfo g, Query
                                                               const double* __restrict__ thf,
                                                               const double* __restrict__ vf, uint32_t* xt,
                                                               uint32_t* yt, uint32_t* zt, uint32_t* wt,
-                                                              unsigned int* flags) {
+                                                              uint4* __restrict__ shorts, unsigned int* flags) {
     const uint64_t planes = static_cast<uint64_t>(g.slices) * g.xy_planes;
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t wstride = static_cast<uint64_t>(gridDim.x) * (blockDim.x >> 5);
@@ -240,20 +266,43 @@ __global__ void __launch_bounds__(kPlaneThreads) k_axis_tables(GridInfo g, Query
          plane < planes; plane += wstride) {
         const uint32_t i3 = static_cast<uint32_t>((plane / g.xy_planes) % g.n[3]);
         const double vc = centre(g, 3, i3);
+        // The plane's boxes in short (ShortBox): one ballot, shuffle and vote a 32 cells.
+        uint32_t ab[2] = {0, 0}, range[2] = {0, 0};
+        bool alike[2];
         for (int d = 0; d < 2; ++d) {
             const uint32_t n = g.n[d];
             const double r = box_radius(g, q, d, vc);
             const double* nom = (d ? yn : xn) + plane * n;
             uint32_t* out = d ? yt + plane * g.n1p : xt + plane * n;
-            for (uint32_t i = lane; i < n; i += 32) {
-                uint32_t lo, hi;
-                const bool ok = axis_box(g, d, nom[i], r, &lo, &hi);
-                out[i] = ok ? pack16(lo, hi) : kReject;
+            uint32_t ref = 0, first = 0, end = 0, cells = 0;
+            bool same = true;
+            for (uint32_t base = 0; base < n; base += 32) {
+                const uint32_t i = base + lane;
+                uint32_t lo = 0, hi = 0;
+                const bool ok = i < n && axis_box(g, d, nom[i], r, &lo, &hi);
+                if (i < n) out[i] = ok ? pack16(lo, hi) : kReject;
                 if (ok && hi < lo) fl |= 1u;
                 if (ok && hi >= lo && hi - lo >= kBits) fl |= 2u;
                 if (d && ok && hi >= lo) levels |= 1u << (31 - __clz(hi - lo + 1));
+                const uint32_t m = __ballot_sync(0xFFFFFFFFu, ok);
+                if (!m) continue;
+                const uint32_t mine = pack16((lo - i) & 0xFFFFu, (hi - i) & 0xFFFFu);
+                if (!cells) {
+                    first = base + __ffs(m) - 1;
+                    ref = __shfl_sync(0xFFFFFFFFu, mine, __ffs(m) - 1);
+                }
+                same = same && __all_sync(0xFFFFFFFFu, !ok || mine == ref);
+                end = base + 32 - __clz(m);
+                cells += __popc(m);
             }
+            const int a = static_cast<int16_t>(lo16(ref)), b = static_cast<int16_t>(hi16(ref));
+            alike[d] = same && cells == end - first && a >= -31 && b <= 31 && a <= b && b - a < 32;
+            if (cells) ab[d] = (static_cast<uint32_t>(b - a + 1) & 0xFFu) | ((static_cast<uint32_t>(a) & 0xFFu) << 8);
+            range[d] = pack16(first, end);
+            if (!cells) alike[d] = true;
         }
+        if (lane == 0)
+            shorts[plane] = make_uint4(ab[0] | (alike[0] ? kBoxX : 0u) | (alike[1] ? kBoxY : 0u), ab[1], range[1], range[0]);
     }
     const uint64_t nz = static_cast<uint64_t>(g.n[2]) * g.mw;
     const uint64_t nw = static_cast<uint64_t>(g.n[3]) * g.ma;
@@ -280,34 +329,6 @@ __global__ void __launch_bounds__(kPlaneThreads) k_axis_tables(GridInfo g, Query
 }
 
 // ---- bit-sliced sets --------------------------------------------------------------------
-
-// One thread per word: the 32 cells of word w of x-row r.
-__global__ void k_pack_bits(GridInfo g, int mode, const uint8_t* __restrict__ src, const uint8_t* __restrict__ src2,
-                            bword* __restrict__ out) {
-    const uint64_t words = static_cast<uint64_t>(g.slices) * g.sw;
-    for (uint64_t e = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; e < words;
-         e += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
-        const uint64_t slice = e / g.sw;
-        const uint32_t rem = static_cast<uint32_t>(e - slice * g.sw);
-        const uint32_t i1 = rem / g.W, w = rem - i1 * g.W;
-        const uint64_t base = (slice * g.n[1] + i1) * g.n[0];
-        bword word = 0;
-        if (i1 < g.n[1]) for (uint32_t b = 0; b < kBits; ++b) {
-            const uint32_t i0 = w * kBits + b;
-            if (i0 >= g.n[0]) break;
-            bool bit;
-            switch (mode) {
-                case 0: bit = src[base + i0] != 0; break;
-                case 1: bit = src[base + i0] == 0; break;
-                case 2: bit = src2[i1 * g.n[0] + i0] == 0; break;
-                case 3: bit = src[base + i0] != 0 && src2[i1 * g.n[0] + i0] != 0; break;
-                default: bit = src[base + i0] != 0 && src2[base + i0] != 0; break;
-            }
-            word |= static_cast<bword>(bit) << b;
-        }
-        out[e] = word;
-    }
-}
 
 __global__ void k_store_words(const uint32_t* __restrict__ src, uint32_t* __restrict__ dst, uint32_t n) {
     for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) dst[i] = src[i];
@@ -473,7 +494,9 @@ __global__ void k_export(GridInfo g, ExportArgs a) {
 // One thread per plane; a block first copies its planes' x rows (contiguous)
 // into shared memory in one coalesced round, then each thread scans its row
 // there twice (a row stride of n0 words): the shift range, then the masks.
-__global__ void k_x_classes(GridInfo g, const uint32_t* __restrict__ xt, bword* __restrict__ out) {
+// Planes whose boxes are alike need no record (ShortBox) and get none.
+__global__ void k_x_classes(GridInfo g, const uint32_t* __restrict__ xt, const uint4* __restrict__ shorts,
+                            bword* __restrict__ out) {
     extern __shared__ uint32_t s_xrows[];
     const uint32_t cw = class_words(g);
     const uint32_t n0 = g.n[0];
@@ -481,11 +504,12 @@ __global__ void k_x_classes(GridInfo g, const uint32_t* __restrict__ xt, bword* 
     for (uint64_t first = blockIdx.x * static_cast<uint64_t>(blockDim.x); first < planes;
          first += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
         const uint32_t np = static_cast<uint32_t>(min(static_cast<uint64_t>(blockDim.x), planes - first));
-        __syncthreads();   // the previous round's rows are read
+        const bool need = threadIdx.x < np && !(shorts[first + threadIdx.x].x & kBoxX);
+        if (!__syncthreads_or(need)) continue;   // (the previous round's rows are read)
         for (uint32_t i = threadIdx.x; i < np * n0; i += blockDim.x) cp_async4(s_xrows + i, xt + first * n0 + i);
         cp_async_wait_all();
         __syncthreads();
-        if (threadIdx.x >= np) continue;
+        if (!need) continue;
         const uint64_t plane = first + threadIdx.x;
         const uint32_t* row = s_xrows + threadIdx.x * n0;
         int dmin = 32, dmax = -32, amax = -32, bmin = 32;
@@ -536,61 +560,66 @@ __global__ void k_x_classes(GridInfo g, const uint32_t* __restrict__ xt, bword* 
 
 constexpr int kThreadsReps = 128;
 
-__global__ void k_plane_reps(GridInfo g, const uint32_t* __restrict__ xt, const uint32_t* __restrict__ yt,
-                             const uint32_t* __restrict__ wt, uint8_t* __restrict__ rep, uint32_t* max_reps,
-                             uint32_t stage_words) {
-    // One warp per column; the lanes compare a pair of planes' x and y rows
-    // together.  Representatives are kept in increasing order, so an input
-    // maps to the lowest earlier input with the same rows and v box.  With
-    // stage_words (= ma * (n0 + n1p)), the column's x rows and then its y rows
-    // are first copied into the warp's shared memory in one round and
-    // compared there; else they are compared in global memory.
-    extern __shared__ uint32_t s_rows[];
+// Whether planes pa and pb have the same x and y rows: from their boxes in
+// short where those say all, else cell by cell (by one warp, or by one thread
+// where lanes = 1).
+__device__ __forceinline__ bool same_rows(const GridInfo& g, const uint32_t* __restrict__ xt,
+                                          const uint32_t* __restrict__ yt, const uint4* __restrict__ shorts, uint64_t pa,
+                                          uint64_t pb, uint32_t lane, uint32_t lanes) {
+    if (pa == pb) return true;
+    const uint4 a = shorts[pa], b = shorts[pb];
+    if ((a.x ^ b.x) & (kBoxX | kBoxY)) return false;
+    const bool xs = a.x & kBoxX, ys = a.x & kBoxY;
+    if (xs && (((a.x ^ b.x) & 0xFFFFu) || a.w != b.w)) return false;
+    if (ys && (a.y != b.y || a.z != b.z)) return false;
+    bool eq = true;
+    for (uint32_t i = lane; !xs && i < g.n[0]; i += lanes) eq = eq && xt[pa * g.n[0] + i] == xt[pb * g.n[0] + i];
+    for (uint32_t i = lane; !ys && i < g.n[1]; i += lanes) eq = eq && yt[pa * g.n1p + i] == yt[pb * g.n1p + i];
+    return lanes == 1 ? eq : __all_sync(0xFFFFFFFFu, eq) != 0;
+}
+
+// One warp per column: representatives are kept in increasing order, so an
+// input maps to the lowest earlier input with the same rows and v box.
+__global__ void __launch_bounds__(kThreadsReps) k_plane_reps(GridInfo g, const uint32_t* __restrict__ xt,
+                                                             const uint32_t* __restrict__ yt,
+                                                             const uint32_t* __restrict__ wt,
+                                                             const uint4* __restrict__ shorts, uint8_t* __restrict__ rep,
+                                                             uint32_t* max_reps) {
+    __shared__ uint32_t s_wt[kThreadsReps / 32][256];
     __shared__ uint8_t s_reps[kThreadsReps / 32][256];
     const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     uint8_t* reps = s_reps[wib];
-    uint32_t* rows = s_rows + static_cast<uint64_t>(wib) * stage_words;
-    const uint32_t n0 = g.n[0], n1 = g.n[1], n1p = g.n1p, ma = g.ma;
-    const bool shared_xy = g.xy_planes == 1;   // one x / y plane per slice: every row pair is equal
-    const uint32_t nx = ma * n0;
+    uint32_t* ws = s_wt[wib];
+    const uint32_t ma = g.ma;
     const uint64_t columns = static_cast<uint64_t>(g.slices) * g.mw;
     const uint64_t wstride = static_cast<uint64_t>(gridDim.x) * (blockDim.x >> 5);
     uint32_t most = 0;
     for (uint64_t col = blockIdx.x * static_cast<uint64_t>(blockDim.x >> 5) + wib; col < columns; col += wstride) {
-        // Planes are ((i2 * n3 + i3) * M + j) with j = ja + ma * jw, so column
-        // col = (i2 * n3 + i3) * mw + jw starts at plane col * ma.
-        const uint32_t i3 = static_cast<uint32_t>((col / g.mw) % g.n[3]);
-        const uint64_t p0 = col * ma;
-        const uint32_t* X = xt + p0 * n0;
-        const uint32_t* Y = yt + p0 * n1p;
-        if (stage_words) {
-            for (uint32_t i = lane; i < nx; i += 32) cp_async4(rows + i, X + i);
-            for (uint32_t i = lane; i < ma * n1p; i += 32) cp_async4(rows + nx + i, Y + i);
-            cp_async_wait_all();
-            __syncwarp();
-            X = rows;
-            Y = rows + nx;
-        }
+        // Column col = (i2 * n3 + i3) * mw + jw holds inputs ja + ma * jw.
+        const uint32_t jw = static_cast<uint32_t>(col % g.mw);
+        const uint32_t i3 = static_cast<uint32_t>((col / g.mw) % g.n[3]), i2 = static_cast<uint32_t>(col / g.mw / g.n[3]);
+        __syncwarp();
+        for (uint32_t ja = lane; ja < ma; ja += 32) ws[ja] = wt[i3 * ma + ja];
+        __syncwarp();
         uint32_t nrep = 0;
         for (uint32_t ja = 0; ja < ma; ++ja) {
-            const uint32_t we = wt[i3 * ma + ja];
+            const uint32_t we = ws[ja];
             uint32_t r = ja;
-            for (uint32_t k = 0; k < nrep; ++k) {
-                const uint32_t jb = reps[k];
-                if (wt[i3 * ma + jb] != we) continue;
-                bool same = true;
-                for (uint32_t i = lane; !shared_xy && i < n0; i += 32) same = same && X[jb * n0 + i] == X[ja * n0 + i];
-                for (uint32_t i = lane; !shared_xy && i < n1; i += 32) same = same && Y[jb * n1p + i] == Y[ja * n1p + i];
-                if (__all_sync(0xFFFFFFFFu, same)) {
-                    r = jb;
-                    break;
+            for (uint32_t k0 = 0; k0 < nrep && r == ja; k0 += 32) {
+                const uint32_t k = k0 + lane;
+                uint32_t m = __ballot_sync(0xFFFFFFFFu, k < nrep && ws[reps[k < nrep ? k : 0]] == we);
+                for (; m && r == ja; m &= m - 1) {
+                    const uint32_t jb = reps[k0 + __ffs(m) - 1];
+                    if (same_rows(g, xt, yt, shorts, xy_plane(g, i2, i3, ja + ma * jw), xy_plane(g, i2, i3, jb + ma * jw),
+                                  lane, 32))
+                        r = jb;
                 }
             }
             if (r == ja) {
                 if (lane == 0) reps[nrep] = static_cast<uint8_t>(ja);
                 ++nrep;
             }
-            if (lane == 0) rep[p0 + ja] = static_cast<uint8_t>(r);
+            if (lane == 0) rep[col * ma + ja] = static_cast<uint8_t>(r);
             __syncwarp();
         }
         most = max(most, nrep);
@@ -598,93 +627,70 @@ __global__ void k_plane_reps(GridInfo g, const uint32_t* __restrict__ xt, const 
     if (lane == 0 && most) atomicMax(max_reps, most);
 }
 
-// One warp per slice (theta i2, v i3): the column representatives of
-// k_plane_reps in input order; one whose theta box, v box and x and y rows
-// equal an earlier representative's of the slice is dropped.  The list's
-// (theta, v) boxes are compared 32 at a time, rows only where those agree.
-constexpr int kSliceRepsCache = 64;   // list entries whose boxes are also kept in shared memory
-
+// One block per slice (theta i2, v i3), one thread per input: a column
+// representative of k_plane_reps is one of the slice unless one of an earlier
+// column has the same theta box, v box and rows; the list is in input order.
 __global__ void __launch_bounds__(kThreadsReps) k_slice_reps(GridInfo g, const uint32_t* __restrict__ xt,
                                                              const uint32_t* __restrict__ yt,
                                                              const uint32_t* __restrict__ zt,
                                                              const uint32_t* __restrict__ wt,
+                                                             const uint4* __restrict__ shorts,
                                                              const uint8_t* __restrict__ xrep, SliceRep* reps,
                                                              uint32_t* nreps, PlanRecord* plan) {
-    __shared__ uint2 s_zw[kThreadsReps / 32][kSliceRepsCache];
-    const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    uint2* cache = s_zw[wib];
-    const uint32_t n0 = g.n[0], n1 = g.n[1], n2 = g.n[2], ma = g.ma, mw = g.mw;
+    __shared__ uint32_t s_count[kThreadsReps / 32];
+    const uint32_t tid = threadIdx.x, lane = tid & 31, wib = tid >> 5;
+    const uint32_t n2 = g.n[2], ma = g.ma, mw = g.mw;
     uint32_t most = 0;
     unsigned long long total = 0, rows = 0;
-    for (uint32_t s = blockIdx.x * (blockDim.x >> 5) + wib; s < g.slices; s += gridDim.x * (blockDim.x >> 5)) {
+    for (uint32_t s = blockIdx.x; s < g.slices; s += gridDim.x) {
         const uint32_t i2 = s % n2, i3 = s / n2;
         SliceRep* list = reps + static_cast<uint64_t>(s) * g.M;
         const uint8_t* col = xrep + (static_cast<uint64_t>(i2) * g.n[3] + i3) * g.M;
+        const uint32_t *zs = zt + i2 * mw, *ws = wt + i3 * ma;
         uint32_t n = 0;
-        // The first 32 accelerations' v boxes stay in registers, and a column's
-        // loads go out one column ahead.
-        const uint32_t we0 = lane < ma ? wt[i3 * ma + lane] : kReject;
-        uint32_t znext = zt[i2 * mw], cnext = lane < ma ? col[lane] : 0xFFFFu;
-        for (uint32_t jw = 0; jw < mw; ++jw) {
-            const uint32_t ze = znext, c0 = cnext;
-            if (jw + 1 < mw) {
-                znext = zt[i2 * mw + jw + 1];
-                cnext = lane < ma ? col[(jw + 1) * ma + lane] : 0xFFFFu;
+        for (uint32_t j0 = 0; j0 < g.M; j0 += kThreadsReps) {
+            const uint32_t j = j0 + tid, jw = j / ma, ja = j - jw * ma;
+            bool keep = false;
+            uint32_t ze = 0, w = 0;
+            if (j < g.M) {
+                ze = zs[jw];
+                w = ws[ja];
+                keep = w != kReject && col[j] == ja;
             }
-            for (uint32_t base = 0; base < ma; base += 32) {
-                const uint32_t ja = base + lane;
-                const uint32_t we = base == 0 ? we0 : ja < ma ? wt[i3 * ma + ja] : kReject;
-                const uint32_t rep = base == 0 ? c0 : ja < ma ? col[jw * ma + ja] : 0xFFFFu;
-                uint32_t todo = __ballot_sync(0xFFFFFFFFu, we != kReject && rep == ja);
-                for (; todo; todo &= todo - 1) {
-                    const uint32_t src = __ffs(todo) - 1;
-                    const uint32_t w = __shfl_sync(0xFFFFFFFFu, we, src);
-                    const uint32_t j = base + src + ma * jw;
-                    bool dup = false;
-                    for (uint32_t k0 = 0; k0 < n && !dup; k0 += 32) {
-                        const uint32_t k = k0 + lane;
-                        bool same = false;
-                        if (k < n) {
-                            uint2 box;
-                            if (k < kSliceRepsCache) {
-                                box = cache[k];
-                            } else {
-                                const uint32_t jb = list[k].j;
-                                box = make_uint2(zt[i2 * mw + jb / ma], wt[i3 * ma + jb % ma]);
-                            }
-                            same = box.x == ze && box.y == w;
-                        }
-                        uint32_t m = __ballot_sync(0xFFFFFFFFu, same);
-                        if (g.xy_planes == 1) {
-                            dup = m != 0;
-                            continue;
-                        }
-                        for (; m && !dup; m &= m - 1) {
-                            const uint64_t pa = xy_plane(g, i2, i3, j), pb = xy_plane(g, i2, i3, list[k0 + __ffs(m) - 1].j);
-                            bool eq = true;
-                            for (uint32_t i = lane; i < n0; i += 32) eq = eq && xt[pa * n0 + i] == xt[pb * n0 + i];
-                            for (uint32_t i = lane; i < n1; i += 32) eq = eq && yt[pa * g.n1p + i] == yt[pb * g.n1p + i];
-                            dup = __all_sync(0xFFFFFFFFu, eq);
-                        }
-                    }
-                    if (dup) continue;
-                    const uint32_t lz = lo16(ze), hz = hi16(ze), lw = lo16(w);
-                    const uint32_t nz = (lz <= hz) ? hz - lz + 1 : n2 - lz + hz + 1;
-                    const uint32_t nv = hi16(w) >= lw ? hi16(w) - lw + 1 : 0;   // an empty box: no fused solve
-                    if (lane == 0) {
-                        list[n] = SliceRep{j, pack16(lz, nz), pack16(lw, nv), 0u, 0u, 0u, 0u, 0u};
-                        if (n < kSliceRepsCache) cache[n] = make_uint2(ze, w);
-                    }
-                    __syncwarp();
-                    ++n;
-                    rows += static_cast<unsigned long long>(nz) * nv;
-                }
+            for (uint32_t kw = 0; keep && kw < jw; ++kw) {
+                if (zs[kw] != ze) continue;
+                for (uint32_t ka = 0; keep && ka < ma; ++ka)
+                    if (ws[ka] == w && col[kw * ma + ka] == ka &&
+                        same_rows(g, xt, yt, shorts, xy_plane(g, i2, i3, j), xy_plane(g, i2, i3, ka + ma * kw), 0, 1))
+                        keep = false;
             }
+            const uint32_t m = __ballot_sync(0xFFFFFFFFu, keep);
+            if (lane == 0) s_count[wib] = __popc(m);
+            __syncthreads();
+            uint32_t before = n, all = 0;
+            for (uint32_t k = 0; k < kThreadsReps / 32; ++k) {
+                if (k < wib) before += s_count[k];
+                all += s_count[k];
+            }
+            if (keep) {
+                const uint32_t lz = lo16(ze), hz = hi16(ze), lw = lo16(w);
+                const uint32_t nz = (lz <= hz) ? hz - lz + 1 : n2 - lz + hz + 1;
+                const uint32_t nv = hi16(w) >= lw ? hi16(w) - lw + 1 : 0;   // an empty box: no fused solve
+                const uint4 b = shorts[xy_plane(g, i2, i3, j)];
+                list[before + __popc(m & ((1u << lane) - 1))] =
+                    SliceRep{j, pack16(lz, nz), pack16(lw, nv), 0u, b.x, b.y, b.z, b.w};
+                rows += static_cast<unsigned long long>(nz) * nv;
+                ++total;
+            }
+            n += all;
+            __syncthreads();
         }
-        if (lane == 0) nreps[s] = n;
+        if (tid == 0) nreps[s] = n;
         most = max(most, n);
-        total += n;
-        __syncwarp();
+    }
+    for (int off = 16; off > 0; off >>= 1) {
+        total += __shfl_down_sync(0xFFFFFFFFu, total, off);
+        rows += __shfl_down_sync(0xFFFFFFFFu, rows, off);
     }
     if (lane == 0 && total) {
         atomicMax(&plan->slice_reps, most);
@@ -735,15 +741,9 @@ cudaError_t launch_safe2(const GridInfo& g, const QueryInfo& q, uint8_t* safe2, 
 
 cudaError_t launch_axis_tables(const GridInfo& g, const QueryInfo& q, const double* xn, const double* yn,
                                const double* thf, const double* vf, uint32_t* xt, uint32_t* yt, uint32_t* zt,
-                               uint32_t* wt, unsigned int* flags, cudaStream_t st) {
+                               uint32_t* wt, uint4* shorts, unsigned int* flags, cudaStream_t st) {
     k_axis_tables<<<warp_blocks(static_cast<uint64_t>(g.slices) * g.xy_planes), kPlaneThreads, 0, st>>>(
-        g, q, xn, yn, thf, vf, xt, yt, zt, wt, flags);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_pack_bits(const GridInfo& g, int mode, const uint8_t* src, const uint8_t* src2, bword* out,
-                             cudaStream_t st) {
-    k_pack_bits<<<blocks_for(static_cast<uint64_t>(g.slices) * g.sw), kThreads, 0, st>>>(g, mode, src, src2, out);
+        g, q, xn, yn, thf, vf, xt, yt, zt, wt, shorts, flags);
     return cudaGetLastError();
 }
 
@@ -773,36 +773,31 @@ cudaError_t launch_stored_build(const GridInfo& g, const StoredBuildArgs& a, cud
     return cudaGetLastError();
 }
 
-cudaError_t launch_x_classes(const GridInfo& g, const uint32_t* xt, bword* xcls, cudaStream_t st) {
+cudaError_t launch_x_classes(const GridInfo& g, const uint32_t* xt, const uint4* shorts, bword* xcls,
+                             cudaStream_t st) {
     // Threads (planes) a block: as many rows as fit 44 KB of shared memory, 32 to 128.
     uint32_t tpb = static_cast<uint32_t>((44u * 1024u) / (4u * std::max<uint32_t>(g.n[0], 1u)));
     tpb = std::min<uint32_t>(128u, std::max<uint32_t>(32u, tpb & ~31u));
     if (4ull * tpb * g.n[0] > 48 * 1024) return cudaErrorInvalidValue;
-    k_x_classes<<<blocks_for(static_cast<uint64_t>(g.slices) * g.xy_planes, tpb), tpb, 4ull * tpb * g.n[0], st>>>(g, xt, xcls);
+    const uint64_t planes = static_cast<uint64_t>(g.slices) * g.xy_planes;
+    k_x_classes<<<blocks_for(planes, tpb), tpb, 4ull * tpb * g.n[0], st>>>(g, xt, shorts, xcls);
     return cudaGetLastError();
 }
 
 cudaError_t launch_plane_reps(const GridInfo& g, const uint32_t* xt, const uint32_t* yt, const uint32_t* wt,
-                              uint8_t* xrep, uint32_t* max_reps, cudaStream_t st) {
+                              const uint4* shorts, uint8_t* xrep, uint32_t* max_reps, cudaStream_t st) {
     const uint64_t warps = static_cast<uint64_t>(g.slices) * g.mw;
     uint64_t b = (warps + kThreadsReps / 32 - 1) / (kThreadsReps / 32);
     if (b > 8192) b = 8192;
-    // Stage a column's rows in shared memory when they fit 44 KB a block (the
-    // default 48 KB less the representatives' static arrays).
-    const uint64_t words = static_cast<uint64_t>(g.ma) * (g.n[0] + g.n1p);
-    const uint32_t stage =
-        g.xy_planes != 1 && words * 4 * (kThreadsReps / 32) <= 44 * 1024 ? static_cast<uint32_t>(words) : 0u;
-    k_plane_reps<<<static_cast<unsigned int>(b), kThreadsReps, 4ull * stage * (kThreadsReps / 32), st>>>(
-        g, xt, yt, wt, xrep, max_reps, stage);
+    k_plane_reps<<<static_cast<unsigned int>(b), kThreadsReps, 0, st>>>(g, xt, yt, wt, shorts, xrep, max_reps);
     return cudaGetLastError();
 }
 
 cudaError_t launch_slice_reps(const GridInfo& g, const uint32_t* xt, const uint32_t* yt, const uint32_t* zt,
-                              const uint32_t* wt, const uint8_t* xrep, SliceRep* reps, uint32_t* nreps,
-                              PlanRecord* plan, cudaStream_t st) {
-    uint64_t b = (g.slices + kThreadsReps / 32 - 1) / (kThreadsReps / 32);
-    if (b > 8192) b = 8192;
-    k_slice_reps<<<static_cast<unsigned int>(b), kThreadsReps, 0, st>>>(g, xt, yt, zt, wt, xrep, reps, nreps, plan);
+                              const uint32_t* wt, const uint4* shorts, const uint8_t* xrep, SliceRep* reps,
+                              uint32_t* nreps, PlanRecord* plan, cudaStream_t st) {
+    k_slice_reps<<<std::min(g.slices, 148u * 16u), kThreadsReps, 0, st>>>(g, xt, yt, zt, wt, shorts, xrep, reps, nreps,
+                                                                      plan);
     return cudaGetLastError();
 }
 
