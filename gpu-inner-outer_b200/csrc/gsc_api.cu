@@ -642,9 +642,9 @@ int problem_stage1(gsc_problem* p, const gsc_query_desc* qd) {
     GSC_TRY(palloc(p, &p->valid, g.S));
     GSC_TRY(palloc(p, &p->cand, g.S));
     GSC_TRY(palloc(p, &p->counts, 8));
-    GSC_TRY(palloc(p, &p->flags, 2));
+    GSC_TRY(palloc(p, &p->flags, 3));
     GSC_CU(ctx, cudaMemsetAsync(p->counts, 0, 8 * sizeof(unsigned long long), st));
-    GSC_CU(ctx, cudaMemsetAsync(p->flags, 0, 2 * sizeof(unsigned int), st));
+    GSC_CU(ctx, cudaMemsetAsync(p->flags, 0, 3 * sizeof(unsigned int), st));
     if (p->time_h2d) GSC_CU(ctx, cudaEventRecord(ctx->pev[0], st));
     if (qd->obstacle_count) {
         GSC_TRY(palloc(p, &p->obstacles, 8ull * qd->obstacle_count));
@@ -672,17 +672,33 @@ int problem_stage1(gsc_problem* p, const gsc_query_desc* qd) {
     ma.build_cand = qd->candidate_mask ? 0 : 1;
     ma.safe = qd->safe_mask ? p->safe : nullptr;
     ma.safe_rank = p->safe_rank;
+    const uint64_t words = static_cast<uint64_t>(g.slices) * g.sw;
     if (p->fused_candidate) {
-        const uint64_t words = static_cast<uint64_t>(g.slices) * g.sw;
         GSC_TRY(palloc(p, &p->validb, words));
         GSC_TRY(palloc(p, &p->unsafeb, words));
         GSC_TRY(palloc(p, &p->srcb, words));
         GSC_TRY(palloc(p, &p->candb, words));
-        ma.validb = p->validb;
-        ma.unsafeb = p->unsafeb;
-        ma.srcb = p->srcb;
-        ma.candb = p->candb;
+        GSC_TRY(palloc(p, &p->kidx, static_cast<uint64_t>(g.n[2]) + 1));
+        GSC_TRY(palloc(p, &p->lidx, static_cast<uint64_t>(g.n[3]) + 1));
+    } else if (stored_ok) {
+        // The bit-sliced sets and width ranks of the box table take the place of
+        // the valid set's prefix counts, which it makes needless.
+        GSC_TRY(palloc(p, &p->pvalid, g.tsize));
+        if (5 * words + (g.n[2] + g.n[3] + 2ull + 3) / 4 <= g.tsize) {
+            uint32_t* at = reinterpret_cast<uint32_t*>(p->pvalid);
+            p->validb = at;
+            p->unsafeb = at + words;
+            p->srcb = at + 2 * words;
+            p->candb = at + 3 * words;
+            p->dbits = at + 4 * words;
+            p->kidx = reinterpret_cast<uint8_t*>(at + 5 * words);
+            p->lidx = p->kidx + g.n[2] + 1;
+        }
     }
+    ma.validb = p->validb;
+    ma.unsafeb = p->unsafeb;
+    ma.srcb = p->srcb;
+    ma.candb = p->candb;
     ma.cmp_safe = p->safe;
     ma.cmp_rank = p->safe_rank;
     ma.counts = p->counts;
@@ -709,10 +725,8 @@ int problem_stage1(gsc_problem* p, const gsc_query_desc* qd) {
         GSC_TRY(palloc(p, &p->reps, planes));
         GSC_TRY(palloc(p, &p->nreps, g.slices));
         GSC_CU(ctx, launch_slice_reps(g, p->xt, p->yt, p->zt, p->wt, p->shorts, p->xrep, p->reps, p->nreps, p->dplan, st));
-        GSC_TRY(palloc(p, &p->kidx, static_cast<uint64_t>(g.n[2]) + 1));
-        GSC_TRY(palloc(p, &p->lidx, static_cast<uint64_t>(g.n[3]) + 1));
     }
-    GSC_CU(ctx, launch_plan(g, p->zt, p->wt, p->fused_candidate ? p->xrep : nullptr, p->counts, p->flags, p->kidx,
+    GSC_CU(ctx, launch_plan(g, p->zt, p->wt, p->fused_candidate, p->counts, p->flags, p->kidx,
                             p->lidx, p->dplan, st));
     if (!p->hplan) p->hplan = &p->hplan_own;
     if (p->hplan_dev)
@@ -735,7 +749,7 @@ int problem_plan(gsc_problem* p) {
     const bool stored_ok = stored_fits(g);
     // An empty or over-wide interval, or too many box widths: only the
     // stored count is exact.
-    bool fused_ok = p->fused_candidate && pl.fused && pl.flags == 0 && !pl.width_overflow;
+    bool fused_ok = p->fused_candidate && pl.fused && !(pl.flags & 3u) && !pl.width_overflow;
     if (fused_ok) {
         p->max_reps = pl.max_reps;
         p->dil = pl.dil;
@@ -757,6 +771,13 @@ int problem_plan(gsc_problem* p) {
         return fail(ctx, GSC_ERR_UNSUPPORTED,
                     "fused method: an interval is empty or wider than 32 cells, or too many box widths");
     p->method = method;
+    // The stored method looks boxes up in bit tables where those are exact: no
+    // empty interval, none wider than a lookup's word, not too many widths.
+    if (method == GSC_METHOD_STORED && pl.flags == 0 && !pl.width_overflow &&
+        (p->dbits || static_cast<uint64_t>(g.slices) * g.sw <= g.tsize)) {
+        p->dil = pl.dil;
+        p->sbits = stored_bits_of(g, pl.dil, pl.ywidths);
+    }
     const uint64_t iter_bound = std::min<uint64_t>(p->q.max_iterations, g.S + 1);
     if (iter_bound + 2 > kStatsCapMax)
         return fail(ctx, GSC_ERR_UNSUPPORTED, "more than 2^20 fixpoint iterations requested");
@@ -778,9 +799,14 @@ int problem_stage2(gsc_problem* p) {
     GSC_CU(ctx, cudaMemsetAsync(p->fc, 0, sizeof(FixControl), st));
 
     if (p->method == GSC_METHOD_STORED) {
-        GSC_TRY(palloc(p, &p->pvalid, g.tsize));
-        GSC_CU(ctx, cudaMemsetAsync(p->pvalid, 0, g.tsize * 4, st));
-        GSC_CU(ctx, launch_prefix4(g, 0, p->valid, nullptr, p->pvalid, nullptr, st));
+        const bool bits = p->sbits.copies != 0;
+        if (!p->pvalid) GSC_TRY(palloc(p, &p->pvalid, g.tsize));
+        if (!bits) {
+            GSC_CU(ctx, cudaMemsetAsync(p->pvalid, 0, g.tsize * 4, st));
+            GSC_CU(ctx, launch_prefix4(g, 0, p->valid, nullptr, p->pvalid, nullptr, st));
+        } else if (!p->dbits) {
+            p->dbits = reinterpret_cast<uint32_t*>(p->pvalid);   // (the sets have buffers of their own)
+        }
         if (p->safe && p->safe_rank == 2) {
             GSC_TRY(palloc(p, &p->unsafe2, static_cast<uint64_t>(g.n[0] + 1) * (g.n[1] + 1)));
             GSC_CU(ctx, launch_prefix2_unsafe(g, p->safe, p->unsafe2, st));
@@ -805,14 +831,24 @@ int problem_stage2(gsc_problem* p) {
         sb.unsafe2 = p->unsafe2;
         sb.unsafe4 = p->unsafe4;
         sb.pvalid = p->pvalid;
-        sb.boxes = p->boxes;
+        GSC_TRY(palloc(p, &p->pd, g.tsize));
+        if (bits) {
+            // The valid set's box table first, in the place of D's.
+            uint32_t* table = reinterpret_cast<uint32_t*>(p->pd);
+            GSC_CU(ctx, launch_box_table(g, p->validb, table, p->sbits, p->dil, nullptr, st));
+            sb.bits = p->sbits;
+            sb.vbits = table;
+            sb.kidx = p->kidx;
+            sb.lidx = p->lidx;
+        } else {
+            GSC_CU(ctx, cudaMemsetAsync(p->pd, 0, g.tsize * 4, st));
+        }
+        sb.boxes = p->wide ? reinterpret_cast<uint2*>(p->boxes16) : p->boxes;   // (box table: 8 bytes a pair)
         sb.S_pad = p->S_pad;
         sb.boxes16 = p->boxes16;
         sb.wide = p->wide ? 1 : 0;
         sb.valid_pairs = p->counts + 3;
         GSC_CU(ctx, launch_stored_build(g, sb, st));
-        GSC_TRY(palloc(p, &p->pd, g.tsize));
-        GSC_CU(ctx, cudaMemsetAsync(p->pd, 0, g.tsize * 4, st));
         return GSC_OK;
     }
     const uint64_t words = static_cast<uint64_t>(g.slices) * g.sw;
@@ -846,7 +882,13 @@ namespace {
 
 StoredFixArgs stored_args(const gsc_problem* p, cudaGraphConditionalHandle cond, int use_cond) {
     StoredFixArgs a{};
-    a.boxes = p->boxes;
+    a.bits = p->sbits;
+    a.dil = p->dil;
+    a.dbits = p->dbits;
+    a.validb = p->validb;
+    a.candb = p->candb;
+    a.table = reinterpret_cast<uint32_t*>(p->pd);
+    a.boxes = p->wide ? reinterpret_cast<const uint2*>(p->boxes16) : p->boxes;
     a.S_pad = p->S_pad;
     a.boxes16 = p->boxes16;
     a.wide = p->wide ? 1 : 0;
@@ -1031,13 +1073,13 @@ int gsc_problem_solve(gsc_problem* p, uint32_t flags) {
     uint32_t launches = 0;
     double sat_ms = 0.0, scan_ms = 0.0;
     uint32_t sat_launches = 0;
-    const uint32_t per_iter = (p->method == GSC_METHOD_STORED) ? prefix4_launches(p->g) + 2 : fused_launches(p->direct);
+    const uint32_t per_iter = (p->method == GSC_METHOD_STORED) ? stored_launches(p->g, p->sbits) : fused_launches(p->direct);
     if (flags & GSC_SOLVE_PROFILE) {
         GSC_CU(ctx, enqueue_init(p));
         launches += 2;
         cudaEvent_t* ev = nullptr;
         GSC_CU(ctx, profile_events(ctx, &ev));
-        const int npass = p->method == GSC_METHOD_STORED ? static_cast<int>(prefix4_launches(p->g)) : 1;
+        const int npass = p->method == GSC_METHOD_STORED ? static_cast<int>(stored_passes(p->g, p->sbits)) : 1;
         for (double& v : p->pass_ms) v = 0.0;
         p->prof_sat_ms = p->prof_reduce_ms = p->prof_memcpy_ms = 0.0;
         p->iter_prof.clear();

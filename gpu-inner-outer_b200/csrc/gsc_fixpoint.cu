@@ -18,9 +18,10 @@
 // Every iteration's kernels first read the control block and return at once
 // when a stop rule has fired, so extra queued iterations are no-ops and the
 // loop can run as a CUDA graph whose while-condition the control kernel sets.
+#include <algorithm>
 #include <atomic>
 
-#include "gsc_kernels.cuh"
+#include "gsc_fused_body.cuh"
 
 namespace gsc_b200 {
 
@@ -265,7 +266,51 @@ __device__ __forceinline__ uint32_t dcount16(const int32_t* __restrict__ P, cons
     return q16(P, g, l0, l1, l2, l3, r0, r1, g.n[2], r3) + q16(P, g, l0, l1, 0, l3, r0, r1, h2 + 1, r3);
 }
 
+// The box table of a bit-sliced set (StoredBits), one block per tile of rows
+// of a slice: the (theta, v) ORs of every width into shared memory, the y ORs
+// and the overlapping words from there.
+// Measured: 10.3 us at 48x40x31x12, 12.9 us at 300x24x20x8.
+__global__ void __launch_bounds__(256) k_box_table(GridInfo g, const bword* set, uint32_t* __restrict__ table,
+                                                   StoredBits b, DilateArgs d, const FixControl* fc) {
+    extern __shared__ __align__(16) bword smem[];
+    pdl_wait();
+    if (fc && fc->stop) return;
+    const uint32_t n1 = g.n[1], n2 = g.n[2], n3 = g.n[3], W = g.W;
+    const uint32_t kmax = d.kval[d.nk - 1], lmax = d.lval[d.nl - 1], ncombo = d.nk * d.nl;
+    const uint32_t slice = blockIdx.x / b.tiles, y0 = (blockIdx.x - slice * b.tiles) * b.rows;
+    const uint32_t z = slice % n2, v = slice / n2, lfit = min(lmax, n3 - v);
+    const uint32_t halo = 31 - __clz(b.ywidths);
+    const uint32_t y1 = min(n1, y0 + b.rows), y2 = min(n1, y1 + halo), words = (y2 - y0) * W;
+    if (blockIdx.x == 0 && threadIdx.x < kBoxTableHead) table[threadIdx.x] = 0xFFFFFFFFu;
+    fused::window_copies(g, set, d, z, v, kmax, lfit, y0 * W, words, smem);
+    __syncthreads();
+    const uint32_t out = (y1 - y0) * b.hw;
+    for (uint32_t m = b.ywidths, iy = 0; m; m &= m - 1, ++iy) {
+        const uint32_t ny = __ffs(m);
+        for (uint32_t e = threadIdx.x; e < out * ncombo; e += blockDim.x) {
+            const uint32_t c = e / out, q = e - c * out, y = q / b.hw, h = q - y * b.hw, w = h >> 1;
+            const bword* row = smem + c * words + y * W + w;
+            const uint32_t last = min(ny, y2 - y0 - y);
+            bword lo = 0, hi = 0;
+            const bool two = (h & 1u) && w + 1 < W;
+            for (uint32_t i = 0; i < last; ++i, row += W) {
+                lo |= row[0];
+                if (two) hi |= row[1];
+            }
+            const uint64_t at = ((static_cast<uint64_t>(iy * ncombo + c) * g.slices + slice) * n1 + y0) * b.hw + q;
+            table[kBoxTableHead + at] = (h & 1u) ? __funnelshift_r(lo, hi, 16) : lo;
+        }
+    }
+}
+
 __global__ void k_stored_init(GridInfo g, StoredFixArgs a) {
+    if (a.bits.copies) {
+        // D = valid && !candidate, by the word.
+        const uint64_t words = static_cast<uint64_t>(g.slices) * g.sw;
+        for (uint64_t e = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; e < words;
+             e += static_cast<uint64_t>(gridDim.x) * blockDim.x)
+            a.dbits[e] = a.validb[e] & ~a.candb[e];
+    }
     for (uint64_t s = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; s < g.S;
          s += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
         const uint8_t c = a.cand[s];
@@ -356,6 +401,93 @@ __global__ void __launch_bounds__(256) k_sat_stored(GridInfo g, StoredFixArgs a)
         if (nload) atomicAdd(row + 2, nload);
         if (ncount) atomicAdd(row + 3, ncount);
     }
+}
+
+// The same with the box table: a pair is one streamed {word, mask} and one
+// lookup instead of 16 or 32 gathers.  One state a thread, four inputs at a
+// time, their loads in flight before the first is looked at.  The last block
+// applies the stop rules.
+// Bound: DRAM sectors that the open states of a warp (about half its lanes)
+// use in part; a profile of the two-state form read 3.4 TB/s at 42 % occupancy.
+// Measured, an iteration of a graph solve with its table: 48x40x31x12 x 64
+// inputs 191 -> 70 us, 300x24x20x8 x 25 94 -> 49 us.  Two states a thread: 75
+// and 53; the next four boxes fetched ahead as well: 85 and 59 (fetched in vain
+// by the states that hit); two inputs at a time, one state: 87 and 55; blocks
+// of 64 or 128 threads, or more blocks an SM: no better on both grids.
+__global__ void __launch_bounds__(256) k_sat_bits(GridInfo g, StoredFixArgs a) {
+    pdl_wait();
+    FixControl* fc = a.fc;
+    if (fc->stop) {
+        if (a.use_cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(a.cond, 0u);
+        if (a.mirror && blockIdx.x == 0 && threadIdx.x == 0) fused::write_mirror(a.mirror, fc);
+        return;
+    }
+    const uint32_t it = fc->iter + 1;
+    const uint64_t s = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
+    uint32_t nr = 0, nc = 0, nload = 0, ncount = 0;
+    if (s < g.S && a.valid[s] != 0) {
+        const bool isc = a.cand[s] != 0, rch = a.reach[s] != 0;
+        bool open = isc ? a.controller[s] == kInvalid32 : !rch;
+        uint32_t chosen = kInvalid32;
+        for (uint32_t j = 0; j < g.M && open; j += 4) {
+            uint2 b[4];
+            uint32_t w[4];
+#pragma unroll
+            for (uint32_t q = 0; q < 4; ++q)
+                b[q] = j + q < g.M ? __ldcs(a.boxes + (j + q) * a.S_pad + s) : make_uint2(0u, 0xFFFFFFFFu);
+#pragma unroll
+            for (uint32_t q = 0; q < 4; ++q) w[q] = a.table[b[q].x];
+#pragma unroll
+            for (uint32_t q = 0; q < 4; ++q) {
+                if (open && j + q < g.M) {
+                    ++nload;
+                    ncount += b[q].x != 0;
+                    if (!(w[q] & b[q].y)) {
+                        open = false;
+                        chosen = j + q;
+                    }
+                }
+            }
+        }
+        if (chosen != kInvalid32) {
+            a.controller[s] = chosen;
+            if (!rch) {
+                a.reach[s] = 1;
+                ++nr;
+                const uint64_t row = s / g.n[0], slice = row / g.n[1];
+                const uint32_t x = static_cast<uint32_t>(s - row * g.n[0]);
+                atomicAnd(a.dbits + slice * g.sw + (row - slice * g.n[1]) * g.W + x / kBits, ~(1u << (x % kBits)));
+            }
+            if (isc)
+                ++nc;
+            else
+                a.reach_step[s] = it;
+        }
+    }
+    // Boxes read: of states taken in pairs both are, until both are done.
+    if (!a.wide) nload = max(nload, __shfl_xor_sync(0xFFFFFFFFu, nload, 1));
+    unsigned long long* row = a.stats + kStatsCols * it;
+    nr = __reduce_add_sync(0xFFFFFFFFu, nr);
+    nc = __reduce_add_sync(0xFFFFFFFFu, nc);
+    nload = __reduce_add_sync(0xFFFFFFFFu, nload);
+    ncount = __reduce_add_sync(0xFFFFFFFFu, ncount);
+    if ((threadIdx.x & 31) == 0) {
+        if (nr) atomicAdd(row, static_cast<unsigned long long>(nr));
+        if (nc) atomicAdd(row + 1, static_cast<unsigned long long>(nc));
+        if (nload) atomicAdd(row + 2, static_cast<unsigned long long>(nload));
+        if (ncount) atomicAdd(row + 3, static_cast<unsigned long long>(ncount));
+    }
+    // The last block applies the stop rules: the barrier orders a block's
+    // counter atomics before its first thread's fence (cumulative) and ticket.
+    const int counted = __syncthreads_or(nr | nc);
+    if (threadIdx.x != 0) return;
+    if (counted) __threadfence();
+    if (atomicAdd(&fc->ticket, 1u) != gridDim.x - 1) return;
+    __threadfence();
+    fc->ticket = 0;
+    fused::control_step(fc, row, it);
+    if (a.use_cond) cudaGraphSetConditional(a.cond, fc->stop ? 0u : 1u);
+    if (a.mirror) fused::write_mirror(a.mirror, fc);
 }
 
 // The same test on a wide grid (a dimension of more than 255 cells): one
@@ -542,6 +674,16 @@ cudaError_t launch_stored_init(const GridInfo& g, const StoredFixArgs& a, cudaSt
 cudaError_t launch_stored_iteration(const GridInfo& g, const StoredFixArgs& a, cudaStream_t st, uint32_t* launches,
                                     cudaEvent_t* ev) {
     if (ev) cudaEventRecord(ev[0], st);
+    if (a.bits.copies) {
+        cudaError_t e = launch_box_table(g, a.dbits, a.table, a.bits, a.dil, a.fc, st);
+        if (e != cudaSuccess) return e;
+        if (ev) cudaEventRecord(ev[1], st);
+        e = launch_pdl(k_sat_bits, dim3(blocks_for(g.S, 256)), dim3(256), 0, st, g, a);
+        if (ev) cudaEventRecord(ev[5], st);
+        if (ev) cudaEventRecord(ev[6], st);
+        if (launches) *launches += stored_launches(g, a.bits);
+        return e;
+    }
     cudaError_t e = launch_prefix4(g, 1, a.valid, a.reach, a.pd, a.fc, st, ev ? ev + 1 : nullptr);
     if (e != cudaSuccess) return e;
     if (a.wide)
@@ -553,6 +695,36 @@ cudaError_t launch_stored_iteration(const GridInfo& g, const StoredFixArgs& a, c
     if (ev) cudaEventRecord(ev[6], st);
     if (launches) *launches += prefix4_launches(g) + 2;
     return cudaGetLastError();
+}
+
+uint32_t stored_passes(const GridInfo& g, const StoredBits& b) { return b.copies ? 1u : prefix4_launches(g); }
+
+StoredBits stored_bits_of(const GridInfo& g, const DilateArgs& d, uint32_t ywidths) {
+    StoredBits b{};
+    uint32_t nyw = 0;
+    for (uint32_t m = ywidths; m; m &= m - 1) ++nyw;
+    if (!nyw || !d.nk || !d.nl) return b;
+    b.ywidths = ywidths;
+    b.nk = d.nk;
+    b.nl = d.nl;
+    b.hw = (g.n[0] + 15) / 16;
+    const uint32_t halo = 31 - __builtin_clz(ywidths), row = d.nk * d.nl * g.W * 4;
+    const uint32_t fit = 40u * 1024u / row;
+    if (fit <= halo) return b;
+    b.rows = std::min(g.n[1], fit - halo);
+    b.tiles = (g.n[1] + b.rows - 1) / b.rows;
+    b.smem = std::min(g.n[1], b.rows + halo) * row;
+    // The table takes the place of D's prefix counts, so it is no larger (which
+    // also keeps its indexes within 32 bits); inputs are a grid dimension of the build.
+    const uint64_t copies = static_cast<uint64_t>(nyw) * d.nk * d.nl;
+    if (kBoxTableHead + copies * g.slices * g.n[1] * b.hw > g.tsize || g.M > 65535) return b;
+    b.copies = static_cast<uint32_t>(copies);
+    return b;
+}
+
+cudaError_t launch_box_table(const GridInfo& g, const bword* set, uint32_t* table, const StoredBits& b,
+                             const DilateArgs& d, const FixControl* fc, cudaStream_t st) {
+    return launch_pdl(k_box_table, dim3(g.slices * b.tiles), dim3(256), b.smem, st, g, set, table, b, d, fc);
 }
 
 uint32_t prefix4_launches(const GridInfo& g) {

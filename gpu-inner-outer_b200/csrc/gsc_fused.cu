@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(256) k_dilate(GridInfo g, const bword* src0, c
 // occur, numbered in increasing order.  out->max_reps (zeroed before, then
 // raised by k_plane_reps) becomes at least 1.
 __global__ void __launch_bounds__(256) k_plan(GridInfo g, const uint32_t* __restrict__ zt,
-                                              const uint32_t* __restrict__ wt, const uint8_t* __restrict__ xrep,
+                                              const uint32_t* __restrict__ wt, uint32_t fused,
                                               const unsigned long long* __restrict__ counts,
                                               const unsigned int* __restrict__ flags, uint8_t* __restrict__ kidx,
                                               uint8_t* __restrict__ lidx, PlanRecord* __restrict__ out) {
@@ -77,17 +77,11 @@ __global__ void __launch_bounds__(256) k_plan(GridInfo g, const uint32_t* __rest
     if (tid == 0) {
         out->flags = flags[0];
         out->ylevels = flags[1];
-        out->fused = xrep ? 1u : 0u;
+        out->ywidths = flags[2];
+        out->fused = fused;
     }
-    if (!xrep) {
-        if (tid == 0) {
-            out->max_reps = 0;
-            out->ylevels = 0;
-            out->slice_reps = 0;
-            out->reps = out->rep_rows = 0;
-            out->width_overflow = 0;
-            out->dil = DilateArgs{};
-        }
+    if (!kidx) {
+        if (tid == 0) out->width_overflow = 1;
         return;
     }
     const uint32_t n2 = g.n[2], n3 = g.n[3];
@@ -382,11 +376,11 @@ DilateTile dilate_tile_of(const GridInfo& g, const DilateArgs& d, uint32_t level
     return t;
 }
 
-cudaError_t launch_plan(const GridInfo& g, const uint32_t* zt, const uint32_t* wt, const uint8_t* xrep,
+cudaError_t launch_plan(const GridInfo& g, const uint32_t* zt, const uint32_t* wt, bool fused,
                         const unsigned long long* counts, const unsigned int* flags, uint8_t* kidx, uint8_t* lidx,
                         PlanRecord* out, cudaStream_t st) {
-    if (xrep && (g.n[2] > 65535 || g.n[3] > 65535)) return cudaErrorInvalidValue;
-    k_plan<<<1, 256, 0, st>>>(g, zt, wt, xrep, counts, flags, kidx, lidx, out);
+    if (kidx && (g.n[2] > 65535 || g.n[3] > 65535)) return cudaErrorInvalidValue;
+    k_plan<<<1, 256, 0, st>>>(g, zt, wt, fused ? 1u : 0u, counts, flags, kidx, lidx, out);
     return cudaGetLastError();
 }
 

@@ -93,12 +93,49 @@ __device__ __forceinline__ void init_control(FixControl* fc, uint32_t max_iterat
     fc->message = (max_iterations == 0) ? 3u : 0u;
 }
 
+// Words [first, first + words) of slice (z, v) of src ORed over theta cells
+// z .. z+k-1 (wrapped) and v cells v .. v+l-1 for every width k and l, into
+// smem [(ki * nl + li) * words]; 0 where the v window leaves the grid (lfit: v
+// cells that stay inside it).  By the whole block; the theta ORs are extended
+// incrementally.
+__device__ __forceinline__ void window_copies(const GridInfo& g, const bword* src, const DilateArgs& d, uint32_t z,
+                                              uint32_t v, uint32_t kmax, uint32_t lfit, uint32_t first, uint32_t words,
+                                              bword* smem) {
+    const uint32_t n2 = g.n[2];
+    for (uint32_t e = threadIdx.x; e < words; e += blockDim.x) {
+        bword zor[kMaxDilate];
+#pragma unroll
+        for (uint32_t j = 0; j < kMaxDilate; ++j) zor[j] = 0;
+        uint32_t ki = 0, zz = z;
+#pragma unroll 2
+        for (uint32_t i = 0; i < kmax; ++i) {
+#pragma unroll
+            for (uint32_t j = 0; j < kMaxDilate; ++j)
+                if (j < lfit) zor[j] |= __ldg(src + static_cast<uint64_t>(zz + n2 * (v + j)) * g.sw + first + e);
+            zz = (zz + 1 == n2) ? 0 : zz + 1;
+            if (i + 1 == d.kval[ki]) {
+                bword acc = 0;
+                uint32_t li = 0;
+#pragma unroll
+                for (uint32_t j = 0; j < kMaxDilate; ++j) {
+                    acc |= zor[j];
+                    if (li < d.nl && j + 1 == d.lval[li]) {
+                        smem[(ki * d.nl + li) * words + e] = (j < lfit) ? acc : 0u;
+                        ++li;
+                    }
+                }
+                ++ki;
+            }
+        }
+    }
+}
+
 // Dilated copies of one tile (rows [y0, y0 + t.rows) of one slice), by the
 // whole block: for every theta width k in d.kval and v width l in d.lval, the
 // OR of src over theta cells z .. z+k-1 (wrapped) and v cells v .. v+l-1
 // (copies whose v window leaves the grid are never read and are left 0), and
 // of that over the 2^p rows from each row on for every y level p in use.  The
-// theta ORs are extended incrementally, the y ORs read shared memory.
+// y ORs read shared memory.
 // With `lost` (the rows that lost a D' cell since the last dilation) the tile
 // is left as it is when no row that it reads did.
 __device__ __forceinline__ void dilate_tile(const GridInfo& g, const bword* __restrict__ src, bword* __restrict__ dst,
@@ -129,32 +166,7 @@ __device__ __forceinline__ void dilate_tile(const GridInfo& g, const bword* __re
         if (!__syncthreads_or(hit != 0)) return;
     }
     const uint32_t words = (y2 - y0) * W, ncombo = d.nk * d.nl;
-    for (uint32_t e = threadIdx.x; e < words; e += blockDim.x) {
-        bword zor[kMaxDilate];
-#pragma unroll
-        for (uint32_t j = 0; j < kMaxDilate; ++j) zor[j] = 0;
-        uint32_t ki = 0, zz = z;
-#pragma unroll 2
-        for (uint32_t i = 0; i < kmax; ++i) {
-#pragma unroll
-            for (uint32_t j = 0; j < kMaxDilate; ++j)
-                if (j < lfit) zor[j] |= __ldg(src + static_cast<uint64_t>(zz + n2 * (v + j)) * g.sw + y0 * W + e);
-            zz = (zz + 1 == n2) ? 0 : zz + 1;
-            if (i + 1 == d.kval[ki]) {
-                bword acc = 0;
-                uint32_t li = 0;
-#pragma unroll
-                for (uint32_t j = 0; j < kMaxDilate; ++j) {
-                    acc |= zor[j];
-                    if (li < d.nl && j + 1 == d.lval[li]) {
-                        smem[(ki * d.nl + li) * words + e] = (j < lfit) ? acc : 0u;
-                        ++li;
-                    }
-                }
-                ++ki;
-            }
-        }
-    }
+    window_copies(g, src, d, z, v, kmax, lfit, y0 * W, words, smem);
     __syncthreads();
     const uint32_t out = (y1 - y0) * W;
     bword* base = dst + static_cast<uint64_t>(slice) * g.sw + y0 * W;

@@ -129,6 +129,8 @@ struct gsc_problem {
     uint64_t S_pad = 0;
     uint4* boxes16 = nullptr;     // wide grids (a dimension of more than 255 cells)
     bool wide = false;
+    gsc_b200::StoredBits sbits{};   // boxes looked up in a bit table (in pd), else counted (pd)
+    uint32_t* dbits = nullptr;      // the bit-sliced D (in pvalid)
     int32_t* pd = nullptr;
     uint8_t* reach8 = nullptr;
     // fused

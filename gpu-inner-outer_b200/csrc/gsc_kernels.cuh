@@ -76,7 +76,8 @@ cudaError_t launch_safe2(const GridInfo& g, const QueryInfo& q, uint8_t* safe2, 
 // Per-axis quantised boxes.  xt/yt: [xy_plane][n0|n1], zt: [n2][mw], wt: [n3][ma], packed
 // lo | hi << 16 or kReject.  flags |= 1 if an accepted non-wrap interval is empty (hi < lo),
 // |= 2 if one is wider than 32 cells.  flags[1] |= 1 << p for every accepted y interval of
-// 2^p .. 2^(p+1) - 1 cells.
+// 2^p .. 2^(p+1) - 1 cells, flags[2] |= 1 << (ny - 1) for one of ny; flags |= 4 if an x interval is wider
+// than 17 cells.
 // shorts: per plane its x and y boxes in short, {hx, hy, yr, xr}: hx = b - a + 1 | a << 8 of the x boxes
 // [i + a, i + b], with kBoxX where they are alike, |a|, |b| < 32, and the cells with one (xr: first |
 // end << 16) are in a row, and kBoxY likewise for the y boxes (hy, yr).
@@ -110,6 +111,27 @@ uint32_t prefix4_launches(const GridInfo& g);
 cudaError_t launch_prefix2_unsafe(const GridInfo& g, const uint8_t* safe2, int32_t* table, cudaStream_t st);
 
 // ---- stored per-pair boxes --------------------------------------------------------------
+// Box widths present in a problem: theta widths kval[0..nk) and v widths
+// lval[0..nl), ascending; combo (ki, li) indexes the dilated copies.
+constexpr int kMaxDilate = 8;
+struct DilateArgs {
+    uint32_t nk, nl;
+    uint32_t kval[kMaxDilate];
+    uint32_t lval[kMaxDilate];
+};
+// Box table of the stored method: a set ORed over every (y, theta, v) box
+// width in use, as overlapping 32-bit words (word h of a row covers x cells
+// 16 h .. 16 h + 31), so that any box of at most 17 x cells is one word and a
+// mask of it.  Copy c = (y width's rank * nk + k) * nl + l, words
+// kBoxTableHead + ((c * slices + slice) * n1 + y) * hw + h; the head is all ones.
+constexpr uint32_t kBoxTableHead = 4, kBoxBits = 17;
+struct StoredBits {
+    uint32_t copies;    // 0: prefix counts instead
+    uint32_t ywidths;   // bit ny - 1 for every y width ny
+    uint32_t nk, nl;
+    uint32_t hw;        // words a row
+    uint32_t rows, tiles, smem;   // rows a block, blocks a slice, and its shared memory
+};
 struct StoredBuildArgs {
     const uint32_t *xt, *yt, *zt, *wt;
     const uint8_t* safe;      // rank 2 or 4
@@ -117,6 +139,9 @@ struct StoredBuildArgs {
     const int32_t* unsafe2;   // rank 2 prefix
     const int32_t* unsafe4;   // rank 4 prefix
     const int32_t* pvalid;    // 4-D valid prefix
+    StoredBits bits;          // with copies: boxes hold {word, mask} of the box table, vbits the valid set's
+    const uint32_t* vbits;
+    const uint8_t *kidx, *lidx;
     uint2* boxes;             // [M][S_pad]: one byte per bound (every dimension <= 255 cells)
     uint64_t S_pad;
     uint4* boxes16;           // [M][S]: 16 bits per bound, when a dimension has more than 255 cells
@@ -141,6 +166,11 @@ cudaError_t launch_export(const GridInfo& g, const ExportArgs& a, cudaStream_t s
 
 // ---- fixpoint ---------------------------------------------------------------------------
 struct StoredFixArgs {
+    StoredBits bits;          // with copies: boxes, dbits and table in place of pd
+    DilateArgs dil;
+    bword* dbits;             // D = valid && !reachable, bit-sliced
+    const bword *validb, *candb;
+    uint32_t* table;          // its box table, rebuilt every iteration
     const uint2* boxes;
     uint64_t S_pad;
     const uint4* boxes16;     // wide grids: {lo0 | lo1 << 16, lo2 | lo3 << 16, hi0 | hi1 << 16, hi2 | hi3 << 16}
@@ -160,10 +190,20 @@ struct StoredFixArgs {
     // rules (write_mirror), or nullptr.
     unsigned long long* mirror;
 };
+// The box table of a bit-sliced set, and its sizes for the widths in use
+// (copies 0 where they are too many).
+cudaError_t launch_box_table(const GridInfo& g, const bword* set, uint32_t* table, const StoredBits& b,
+                             const DilateArgs& d, const FixControl* fc, cudaStream_t st);
+StoredBits stored_bits_of(const GridInfo& g, const DilateArgs& d, uint32_t ywidths);
+inline uint64_t box_table_words(const GridInfo& g, const StoredBits& b) {
+    return kBoxTableHead + static_cast<uint64_t>(b.copies) * g.slices * g.n[1] * b.hw;
+}
+// Kernels of one iteration, and those of them that rebuild the table.
+uint32_t stored_passes(const GridInfo& g, const StoredBits& b);
+inline uint32_t stored_launches(const GridInfo& g, const StoredBits& b) { return stored_passes(g, b) + (b.copies ? 1u : 2u); }
 cudaError_t launch_stored_init(const GridInfo& g, const StoredFixArgs& a, cudaStream_t st);
 // ev (optional, kProfileEvents events): [0] before the prefix rebuild,
-// [1..n] after its n passes (launch_prefix4: n = prefix4_launches(g); events
-// n+1 .. 4 are not recorded), [5] after the satisfaction kernel, [6] after
+// [1..n] after its n passes (stored_passes; events n+1 .. 4 are not recorded), [5] after the satisfaction kernel, [6] after
 // the control kernel.  The fused iteration records [0], [1] after the
 // dilation, [5] and [6] alike.
 constexpr int kProfileEvents = 8;
@@ -175,14 +215,6 @@ cudaError_t launch_stored_iteration(const GridInfo& g, const StoredFixArgs& a, c
 // kernels rather than the host's enqueueing.
 cudaError_t launch_hold(cudaStream_t st, uint64_t ns);
 
-// Box widths present in a problem: theta widths kval[0..nk) and v widths
-// lval[0..nl), ascending; combo (ki, li) indexes the dilated copies.
-constexpr int kMaxDilate = 8;
-struct DilateArgs {
-    uint32_t nk, nl;
-    uint32_t kval[kMaxDilate];
-    uint32_t lval[kMaxDilate];
-};
 // y levels: a copy of level p ORs the 2^p rows from each row on, so that any
 // y interval of 2^p .. 2^(p+1) - 1 rows is the OR of two rows of it.
 constexpr int kYLevels = 6;   // fused boxes span at most 32 rows
@@ -202,6 +234,7 @@ struct PlanRecord {
     uint32_t flags;
     uint32_t max_reps;
     uint32_t ylevels;          // y levels in use (bit mask)
+    uint32_t ywidths;          // y widths in use: bit ny - 1 (up to 32 cells)
     uint32_t width_overflow;   // more widths than kMaxDilate, or a v width above kMaxDilate
     uint32_t fused;            // 1 when the fused tables were planned
     DilateArgs dil;
@@ -293,7 +326,7 @@ cudaError_t launch_dilate(const GridInfo& g, const bword* src0, const bword* src
                           cudaStream_t st);
 // Fills a PlanRecord from the counts, flags and (when xrep is set) the
 // theta / v tables and plane representatives; writes kidx / lidx.
-cudaError_t launch_plan(const GridInfo& g, const uint32_t* zt, const uint32_t* wt, const uint8_t* xrep,
+cudaError_t launch_plan(const GridInfo& g, const uint32_t* zt, const uint32_t* wt, bool fused,
                         const unsigned long long* counts, const unsigned int* flags, uint8_t* kidx, uint8_t* lidx,
                         PlanRecord* out, cudaStream_t st);
 // One instance of a batched solve (or of the serving loop), resident in

@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(kPlaneThreads) k_axis_tables(GridInfo g, Query
     const uint64_t planes = static_cast<uint64_t>(g.slices) * g.xy_planes;
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t wstride = static_cast<uint64_t>(gridDim.x) * (blockDim.x >> 5);
-    unsigned int fl = 0, levels = 0;
+    unsigned int fl = 0, levels = 0, widths = 0;
     for (uint64_t plane = blockIdx.x * static_cast<uint64_t>(blockDim.x >> 5) + (threadIdx.x >> 5);
          plane < planes; plane += wstride) {
         const uint32_t i3 = static_cast<uint32_t>((plane / g.xy_planes) % g.n[3]);
@@ -283,7 +283,11 @@ __global__ void __launch_bounds__(kPlaneThreads) k_axis_tables(GridInfo g, Query
                 if (i < n) out[i] = ok ? pack16(lo, hi) : kReject;
                 if (ok && hi < lo) fl |= 1u;
                 if (ok && hi >= lo && hi - lo >= kBits) fl |= 2u;
-                if (d && ok && hi >= lo) levels |= 1u << (31 - __clz(hi - lo + 1));
+                if (d && ok && hi >= lo) {
+                    levels |= 1u << (31 - __clz(hi - lo + 1));
+                    widths |= 1u << ((hi - lo) & 31);
+                }
+                if (!d && ok && hi >= lo && hi - lo >= kBoxBits) fl |= 4u;
                 const uint32_t m = __ballot_sync(0xFFFFFFFFu, ok);
                 if (!m) continue;
                 const uint32_t mine = pack16((lo - i) & 0xFFFFu, (hi - i) & 0xFFFFu);
@@ -325,7 +329,11 @@ __global__ void __launch_bounds__(kPlaneThreads) k_axis_tables(GridInfo g, Query
     }
     if (fl) atomicOr(flags, fl);
     levels = __reduce_or_sync(0xFFFFFFFFu, levels);
-    if (lane == 0 && levels) atomicOr(flags + 1, levels);
+    widths = __reduce_or_sync(0xFFFFFFFFu, widths);
+    if (lane == 0 && levels) {
+        atomicOr(flags + 1, levels);
+        atomicOr(flags + 2, widths);
+    }
 }
 
 // ---- bit-sliced sets --------------------------------------------------------------------
@@ -462,6 +470,37 @@ __global__ void k_stored_build(GridInfo g, StoredBuildArgs a) {
                                            pack8(b.hi[0], b.hi[1], b.hi[2], b.hi[3]))
                               : make_uint2(kBoxSentinel, kBoxSentinel);
         }
+    }
+    for (int off = 16; off > 0; off >>= 1) nvp += __shfl_down_sync(0xFFFFFFFFu, nvp, off);
+    if ((threadIdx.x & 31) == 0 && nvp) atomicAdd(a.valid_pairs, nvp);
+}
+
+// The same pairs as a word of the box table and a mask of it (StoredBits):
+// the pair is satisfied when the word has no D bit under the mask.  V(box) > 0
+// is one lookup in the valid set's table.  Pairs that can never satisfy get
+// word 0, which is all ones, and a full mask.  One thread per (state, input),
+// inputs in the grid's y dimension.
+__global__ void __launch_bounds__(256) k_stored_bits(GridInfo g, StoredBuildArgs a) {
+    const uint32_t j = blockIdx.y;
+    unsigned long long nvp = 0;
+    for (uint64_t s = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; s < a.S_pad;
+         s += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
+        uint2 e = make_uint2(0u, 0xFFFFFFFFu);
+        if (s < g.S) {
+            const PairBox b = pair_box(g, a.xt, a.yt, a.zt, a.wt, a.safe, a.safe_rank, s, j);
+            if (b.ok && box_safe(g, a.safe, a.safe_rank, a.unsafe2, a.unsafe4, b.lo, b.hi)) {
+                ++nvp;
+                const uint32_t nz = b.lo[2] <= b.hi[2] ? b.hi[2] - b.lo[2] + 1 : g.n[2] - b.lo[2] + b.hi[2] + 1;
+                const uint32_t nv = b.hi[3] - b.lo[3] + 1, ny = b.hi[1] - b.lo[1] + 1, nx = b.hi[0] - b.lo[0] + 1;
+                const uint32_t iy = __popc(a.bits.ywidths & ((1u << (ny - 1)) - 1));
+                const uint32_t c = (iy * a.bits.nk + a.kidx[nz]) * a.bits.nl + a.lidx[nv];
+                const uint32_t slice = b.lo[2] + g.n[2] * b.lo[3];
+                const uint32_t off = kBoxTableHead + ((c * g.slices + slice) * g.n[1] + b.lo[1]) * a.bits.hw + (b.lo[0] >> 4);
+                const uint32_t mask = ((1u << nx) - 1) << (b.lo[0] & 15u);
+                if (__ldg(a.vbits + off) & mask) e = make_uint2(off, mask);
+            }
+        }
+        a.boxes[j * a.S_pad + s] = e;
     }
     for (int off = 16; off > 0; off >>= 1) nvp += __shfl_down_sync(0xFFFFFFFFu, nvp, off);
     if ((threadIdx.x & 31) == 0 && nvp) atomicAdd(a.valid_pairs, nvp);
@@ -769,6 +808,11 @@ cudaError_t launch_prefix2_unsafe(const GridInfo& g, const uint8_t* safe2, int32
 }
 
 cudaError_t launch_stored_build(const GridInfo& g, const StoredBuildArgs& a, cudaStream_t st) {
+    if (a.bits.copies) {
+        const unsigned int b = std::min<unsigned int>(blocks_for(a.S_pad), 148u * 64u);
+        k_stored_bits<<<dim3(b, g.M), kThreads, 0, st>>>(g, a);
+        return cudaGetLastError();
+    }
     k_stored_build<<<blocks_for((a.wide ? g.S : a.S_pad) * g.M), kThreads, 0, st>>>(g, a);
     return cudaGetLastError();
 }
