@@ -31,7 +31,7 @@
 #include <mutex>
 
 #include "../../include/gsc_b200.h"
-#include "gsc_kernels.cuh"
+#include "gsc_fused_body.cuh"
 
 namespace gsc_b200 {
 namespace {
@@ -47,7 +47,7 @@ constexpr size_t kStatsBytes = sizeof(unsigned long long) * kStatsCols * (kNoAll
 constexpr size_t kStatsOffset = kCtlBytes;
 constexpr size_t kTableOffset = (kStatsOffset + kStatsBytes + 255) / 256 * 256;
 constexpr size_t kTableBytes = kNoAllocTableEntries * sizeof(int32_t);
-constexpr size_t kNextOffset = kTableOffset + 2 * kTableBytes;      // next reachable mask (states < entries)
+constexpr size_t kNextOffset = kTableOffset + 2 * kTableBytes;      // D: valid && !reachable (states < entries)
 constexpr size_t kScratchBytes = kNextOffset + kNoAllocTableEntries;   // about 40.5 MiB
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
@@ -82,14 +82,15 @@ int scratch_for_current_device(unsigned char** out) {
 
 __global__ void k_noalloc_init(GridInfo g, const uint8_t* __restrict__ valid, const uint8_t* __restrict__ cand,
                                uint8_t* __restrict__ reach, uint32_t* __restrict__ controller,
-                               uint32_t* __restrict__ reach_step, NoAllocCtl* ctl, unsigned long long* stats,
-                               uint32_t stats_words) {
+                               uint32_t* __restrict__ reach_step, uint8_t* __restrict__ open, NoAllocCtl* ctl,
+                               unsigned long long* stats, uint32_t stats_words) {
     unsigned long long nv = 0, nc = 0, nbad = 0;
     for (uint64_t s = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; s < g.S;
          s += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
         const uint8_t c = cand[s] ? 1 : 0;
         const bool v = valid[s] != 0;
         reach[s] = c;
+        open[s] = (v && !c) ? 1 : 0;
         controller[s] = kInvalid32;
         reach_step[s] = c ? 0u : kInvalid32;
         nv += v;
@@ -142,106 +143,99 @@ __device__ __forceinline__ uint32_t nq16(const int32_t* __restrict__ P, const Gr
     return t;
 }
 
-// Box count of a (min_flat, max_flat) pair in the reference's flat layout
-// (prefix_sum.hpp:87-105): unflatten both corners, split a theta-wrapped box.
-__device__ __forceinline__ uint32_t flat_count(const int32_t* __restrict__ P, const GridInfo& g, uint32_t mn,
-                                               uint32_t mx) {
-    uint32_t lo[4], hi[4];
-    uint32_t v = mn, w = mx;
+// The corners of a (min_flat, max_flat) pair in the reference's flat layout
+// (prefix_sum.hpp:87-105).  Division by a grid extent n is the high half of a
+// product with floor(2^64 / n) + 1, which is exact for 32-bit numerators
+// (Lemire, Kaser and Kurz, "Faster remainder by direct computation", 2019).
+struct FlatDiv {
+    unsigned long long m[3];
+};
+__device__ __forceinline__ uint32_t flat_div(uint32_t v, uint32_t n, unsigned long long m) {
+    return n == 1 ? v : static_cast<uint32_t>(__umul64hi(m, v));
+}
+__device__ __forceinline__ void flat_corner(const GridInfo& g, const FlatDiv& f, uint32_t v, uint32_t c[4]) {
+#pragma unroll
     for (int d = 0; d < 3; ++d) {
-        lo[d] = v % g.n[d];
-        v /= g.n[d];
-        hi[d] = w % g.n[d];
-        w /= g.n[d];
+        const uint32_t q = flat_div(v, g.n[d], f.m[d]);
+        c[d] = v - q * g.n[d];
+        v = q;
     }
-    lo[3] = v;
-    hi[3] = w;
+    c[3] = v;
+}
+// A box's count, a theta-wrapped box in two parts.
+__device__ __forceinline__ uint32_t flat_count(const int32_t* __restrict__ P, const GridInfo& g, const uint32_t lo[4],
+                                               const uint32_t hi[4]) {
     if (lo[2] <= hi[2]) return nq16(P, g, lo[0], lo[1], lo[2], lo[3], hi[0] + 1, hi[1] + 1, hi[2] + 1, hi[3] + 1);
     return nq16(P, g, lo[0], lo[1], lo[2], lo[3], hi[0] + 1, hi[1] + 1, g.n[2], hi[3] + 1) +
            nq16(P, g, lo[0], lo[1], 0, lo[3], hi[0] + 1, hi[1] + 1, hi[2] + 1, hi[3] + 1);
 }
 
 // One Jacobi iteration over the caller's abstraction (reachability.hpp:53-109):
-// per state, the lowest input whose box has valid_count > 0 and
-// reachable_count == valid_count.
-__global__ void k_noalloc_iteration(GridInfo g, const uint32_t* __restrict__ min_flat,
-                                    const uint32_t* __restrict__ max_flat, const uint8_t* __restrict__ pair_valid,
-                                    const uint8_t* __restrict__ valid, const uint8_t* __restrict__ cand,
-                                    uint8_t* reach, uint8_t* reach_next, uint32_t* controller, uint32_t* reach_step,
-                                    const int32_t* __restrict__ pvalid, const int32_t* __restrict__ preach,
-                                    NoAllocCtl* ctl, unsigned long long* stats) {
-    const FixControl* fc = &ctl->fc;
-    if (fc->stop) return;
-    const uint32_t it = fc->iter + 1;
-    unsigned long long nr = 0, nc = 0;
-    for (uint64_t s = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; s < g.S;
-         s += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
-        if (!valid[s]) continue;
-        const bool is_cand = cand[s] != 0;
-        const bool reached = reach[s] != 0;
-        const bool certified = controller[s] != kInvalid32;
-        if ((!is_cand && reached) || (is_cand && certified)) continue;
-        const uint64_t base = s * g.M;
-        for (uint32_t j = 0; j < g.M; ++j) {
-            if (!pair_valid[base + j]) continue;
-            const uint32_t vc = flat_count(pvalid, g, min_flat[base + j], max_flat[base + j]);
-            if (vc == 0) continue;
-            const uint32_t rc = flat_count(preach, g, min_flat[base + j], max_flat[base + j]);
-            if (rc != vc) continue;
-            if (!reached) {
-                reach_next[s] = 1;
-                ++nr;
-            }
-            if (!certified) {
-                controller[s] = j;
-                if (is_cand)
-                    ++nc;
-                else
-                    reach_step[s] = it;
-            }
-            break;
-        }
-    }
-    for (int off = 16; off > 0; off >>= 1) {
-        nr += __shfl_down_sync(0xFFFFFFFFu, nr, off);
-        nc += __shfl_down_sync(0xFFFFFFFFu, nc, off);
-    }
-    if ((threadIdx.x & 31) == 0) {
-        if (nr) atomicAdd(&stats[kStatsCols * it], nr);
-        if (nc) atomicAdd(&stats[kStatsCols * it + 1], nc);
-    }
-}
-
-// reach <- reach_next (the Jacobi swap), then the stop rules
-// (reachability.hpp:133-144).
-__global__ void k_noalloc_commit(GridInfo g, uint8_t* reach, const uint8_t* __restrict__ reach_next, NoAllocCtl* ctl,
-                                 const unsigned long long* stats) {
-    if (ctl->fc.stop) return;
-    for (uint64_t s = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; s < g.S;
-         s += static_cast<uint64_t>(gridDim.x) * blockDim.x)
-        if (reach_next[s]) reach[s] = 1;
-}
-
-__global__ void k_noalloc_control(NoAllocCtl* ctl, const unsigned long long* stats) {
+// per state, the lowest input whose box has valid cells and none of them
+// unreached (D).  A pair's two corner cells are looked at before its box is counted: D only shrinks while the
+// iteration runs, so a corner still in it decides the pair, at one or two
+// loads instead of up to 64; which is why the sets can be updated in place.
+// (A box of no cells along x, y or v has no such corner, and is counted.)
+// The last block applies the stop rules (reachability.hpp:133-144).
+// Bound, by reading: the 9 bytes of an open pair, each thread in a row of its own,
+// M pairs apart.  41x39x33x8 x 25 inputs: a launch 72 -> 41 us, a whole call 2852
+// -> 1640 us.  1, 4, 8, 16 or 32 lanes a state with a vote an input: 2.1, 2.7,
+// 3.4, 4.5, 6.6 ms against 1.74 for this loop; four inputs' loads at a time: no gain.
+__global__ void __launch_bounds__(256) k_noalloc_iteration(GridInfo g, FlatDiv f, const uint32_t* __restrict__ min_flat,
+                                                           const uint32_t* __restrict__ max_flat,
+                                                           const uint8_t* __restrict__ pair_valid,
+                                                           const uint8_t* __restrict__ valid,
+                                                           const uint8_t* __restrict__ cand, uint8_t* reach,
+                                                           uint8_t* unreached, uint32_t* controller,
+                                                           uint32_t* reach_step, const int32_t* __restrict__ pvalid,
+                                                           const int32_t* pd, NoAllocCtl* ctl,
+                                                           unsigned long long* stats) {
     FixControl* fc = &ctl->fc;
     if (fc->stop) return;
     const uint32_t it = fc->iter + 1;
-    const unsigned long long nr = stats[kStatsCols * it];
-    const unsigned long long nc = stats[kStatsCols * it + 1];
-    fc->certified += nc;
-    fc->reachable += nr;
-    fc->iter = it;
-    if (fc->certified == fc->candidate_count) {
-        fc->converged = 1;
-        fc->message = 1;
-        fc->stop = 1;
-    } else if (nr == 0 && nc == 0) {
-        fc->message = 2;
-        fc->stop = 1;
-    } else if (it >= fc->max_iterations || it + 1 >= fc->stats_cap) {
-        fc->message = 3;
-        fc->stop = 1;
+    uint32_t nr = 0, nc = 0;
+    for (uint64_t s = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; s < g.S;
+         s += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
+        if (!valid[s]) continue;
+        const bool isc = cand[s] != 0, rch = reach[s] != 0;
+        if (isc ? controller[s] != kInvalid32 : rch) continue;
+        const uint64_t base = s * g.M;
+        for (uint32_t j = 0; j < g.M; ++j) {
+            if (!pair_valid[base + j]) continue;
+            const uint32_t mn = min_flat[base + j], mx = max_flat[base + j];
+            uint32_t lo[4], hi[4];
+            flat_corner(g, f, mn, lo);
+            flat_corner(g, f, mx, hi);
+            const bool cells = lo[0] <= hi[0] && lo[1] <= hi[1] && lo[3] <= hi[3];
+            if (cells && (unreached[mn] | unreached[mx])) continue;
+            if (flat_count(pd, g, lo, hi) != 0 || flat_count(pvalid, g, lo, hi) == 0) continue;
+            controller[s] = j;
+            if (!rch) {
+                reach[s] = 1;
+                unreached[s] = 0;
+                ++nr;
+            }
+            if (isc)
+                ++nc;
+            else
+                reach_step[s] = it;
+            break;
+        }
     }
+    unsigned long long* row = stats + kStatsCols * it;
+    nr = __reduce_add_sync(0xFFFFFFFFu, nr);
+    nc = __reduce_add_sync(0xFFFFFFFFu, nc);
+    if ((threadIdx.x & 31) == 0) {
+        if (nr) atomicAdd(row, static_cast<unsigned long long>(nr));
+        if (nc) atomicAdd(row + 1, static_cast<unsigned long long>(nc));
+    }
+    const int counted = __syncthreads_or(nr | nc);
+    if (threadIdx.x != 0) return;
+    if (counted) __threadfence();
+    if (atomicAdd(&fc->ticket, 1u) != gridDim.x - 1) return;
+    __threadfence();
+    fc->ticket = 0;
+    fused::control_step(fc, row, it);
 }
 
 unsigned int nblocks(uint64_t n) {
@@ -292,8 +286,8 @@ extern "C" int gsc_fixpoint_noalloc(const uint32_t shape[4], uint32_t inputs, in
     NoAllocCtl* ctl = reinterpret_cast<NoAllocCtl*>(base);
     unsigned long long* stats = reinterpret_cast<unsigned long long*>(base + kStatsOffset);
     int32_t* pvalid = reinterpret_cast<int32_t*>(base + kTableOffset);
-    int32_t* preach = reinterpret_cast<int32_t*>(base + kTableOffset + kTableBytes);
-    uint8_t* reachable_next = base + kNextOffset;
+    int32_t* pd = reinterpret_cast<int32_t*>(base + kTableOffset + kTableBytes);
+    uint8_t* unreached = base + kNextOffset;
     const uint32_t stats_cap = static_cast<uint32_t>(iter_bound + 2);
     const uint32_t stats_words = kStatsCols * stats_cap;
     cudaStream_t st = static_cast<cudaStream_t>(cuda_stream);
@@ -315,25 +309,24 @@ extern "C" int gsc_fixpoint_noalloc(const uint32_t shape[4], uint32_t inputs, in
     // the counters and the control block.
     NA_CU(cudaMemsetAsync(ctl, 0, sizeof(NoAllocCtl), st));
     NA_CU(cudaMemsetAsync(pvalid, 0, T * sizeof(int32_t), st));
-    NA_CU(cudaMemsetAsync(preach, 0, T * sizeof(int32_t), st));
+    NA_CU(cudaMemsetAsync(pd, 0, T * sizeof(int32_t), st));
     k_noalloc_init<<<nblocks(S), 256, 0, st>>>(g, valid_mask, candidate_mask, reachable_mask, controller, reach_step,
-                                                ctl, stats, stats_words);
+                                                unreached, ctl, stats, stats_words);
     NA_CU(cudaGetLastError());
     k_noalloc_start<<<1, 1, 0, st>>>(ctl, max_iterations, stats_cap);
     NA_CU(cudaGetLastError());
     NA_CU(launch_prefix4(g, 0, valid_mask, nullptr, pvalid, nullptr, st));
-    NA_CU(cudaMemcpyAsync(reachable_next, reachable_mask, S, cudaMemcpyDeviceToDevice, st));
+    FlatDiv f;
+    for (int d = 0; d < 3; ++d) f.m[d] = ~0ull / g.n[d] + 1;
 
     NoAllocCtl hc;
     FixControl& h = hc.fc;
     for (;;) {
         for (int k = 0; k < 8; ++k) {
-            NA_CU(launch_prefix4(g, 0, reachable_mask, nullptr, preach, &ctl->fc, st));
-            k_noalloc_iteration<<<nblocks(S), 256, 0, st>>>(g, min_flat, max_flat, pair_valid, valid_mask,
-                                                             candidate_mask, reachable_mask, reachable_next,
-                                                             controller, reach_step, pvalid, preach, ctl, stats);
-            k_noalloc_commit<<<nblocks(S), 256, 0, st>>>(g, reachable_mask, reachable_next, ctl, stats);
-            k_noalloc_control<<<1, 1, 0, st>>>(ctl, stats);
+            NA_CU(launch_prefix4(g, 0, unreached, nullptr, pd, &ctl->fc, st));
+            k_noalloc_iteration<<<nblocks(S), 256, 0, st>>>(
+                g, f, min_flat, max_flat, pair_valid, valid_mask, candidate_mask, reachable_mask, unreached, controller,
+                reach_step, pvalid, pd, ctl, stats);
             NA_CU(cudaGetLastError());
         }
         NA_CU(cudaMemcpyAsync(&hc, ctl, sizeof(hc), cudaMemcpyDeviceToHost, st));

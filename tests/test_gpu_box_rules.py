@@ -3,6 +3,9 @@ x boxes about 16, 17 (the widest one lookup holds) and 32 cells (the widest a
 fused row takes), tall y boxes, rows that end inside a word, obstacles (the
 valid-cell test), several rows of representatives.  Bit-exact against the
 oracle, both methods, both loops."""
+import ctypes
+
+import numpy as np
 import pytest
 
 import gsc_b200 as G
@@ -66,3 +69,32 @@ def test_box_lookups_against_oracle(ctx, shape, cells, inputs, obstacle):
         p.close()
         absn.close()
     assert solved >= 4
+
+
+@pytest.mark.parametrize("shape", [(33, 9, 5, 3), (1, 9, 8, 3), (9, 1, 8, 3), (33, 5, 1, 3), (17, 6, 8, 1),
+                                   (64, 20, 6, 4)])
+def test_noalloc_corner_tests_against_oracle(ctx, shape):
+    """Corner cells before counts over the caller's pairs, and extents of one
+    cell (whose division is none)."""
+    import torch
+    case = box_case(shape, (1.5, 1.0, 1.0, 0.0), (5, 5), False)
+    want = O.solve(case)
+    absn = G.Abstraction(ctx, case)
+    p = G.Problem(ctx, absn, case, G.METHOD_AUTO)
+    pairs = [np.ascontiguousarray(a) for a in p.export_abstraction()]
+    p.close()
+    absn.close()
+    dev = [torch.from_numpy(a.view(np.int32) if a.dtype == np.uint32 else a.view(np.uint8)).cuda() for a in
+           pairs + [np.asarray(want["valid_mask"]), np.asarray(want["candidate_mask"])]]
+    S = int(np.prod(shape))
+    out = [torch.empty(S, dtype=torch.uint8, device="cuda"), torch.empty(S, dtype=torch.int32, device="cuda"),
+           torch.empty(S, dtype=torch.int32, device="cuda")]
+    st = G.lib().gsc_fixpoint_noalloc((ctypes.c_uint32 * 4)(*shape), pairs[0].size // S, 2,
+                                      *[ctypes.c_void_p(t.data_ptr()) for t in dev], case["max_iterations"],
+                                      *[ctypes.c_void_p(t.data_ptr()) for t in out], None,
+                                      ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert st == 0
+    torch.cuda.synchronize()
+    for got, name in zip(out, ("reachable_mask", "controller", "reach_step")):
+        w = np.asarray(want[name])
+        assert np.array_equal(got.cpu().numpy().view(w.dtype), w), name
