@@ -942,7 +942,7 @@ def main():
               "note": "per iteration of one host-loop solve, its launches queued behind a short hold so that they "
                       "run back to back, with CUDA events between the phases (each event adds about 2.5 us)"}
     used = tp["method"]
-    kname = "k_sat_stored" if used == G.METHOD_STORED else "k_sat_col"
+    kname = "k_sat_bits" if used == G.METHOD_STORED else "k_slice"
     per_launch_ms = tp["sat_kernel_ms"] / max(tp["sat_launches"], 1)
     alg = algorithmic_bytes(used, {"shape": shape}, tp)
     peak, peak_kind = measured_peak()

@@ -119,10 +119,8 @@ int grid_from_model(const gsc_model_desc* m, GridInfo* g, std::string* err) {
     g->W = (g->n[0] + kBits - 1) / kBits;
     g->rows = static_cast<uint64_t>(g->n[1]) * g->n[2] * g->n[3];
     g->slices = g->n[2] * g->n[3];
-    g->magic_n1 = fdiv_magic(g->n[1]);
     g->sw = (g->n[1] * g->W + 3) & ~3u;
     g->n1p = (g->n[1] + 3) & ~3u;
-    g->magic_sw4 = fdiv_magic(g->sw / 4);
     return GSC_OK;
 }
 
@@ -1192,8 +1190,6 @@ int gsc_problem_solve(gsc_problem* p, uint32_t flags) {
         tests += hs[kStatsCols * i + 2];
         aux += hs[kStatsCols * i + 3];
     }
-    if (hfc.message == kMsgDeviceTimeout)
-        return fail(ctx, GSC_ERR_TIMEOUT, "a bounded device wait for staged tables gave up; the solve stopped");
     p->timings.iterations = hfc.iter;
     p->timings.pair_tests = tests;
     p->timings.aux_count = aux;
@@ -1288,8 +1284,6 @@ int gsc_problem_read(gsc_problem* p, gsc_result* r) {
     r->states = g.S;
     r->inputs = g.M;
     r->pairs = g.S * g.M;
-    if (fc.message == kMsgDeviceTimeout)
-        return fail(ctx, GSC_ERR_TIMEOUT, "the last solve stopped at a bounded device wait that gave up");
     r->iterations = fc.iter;
     r->converged = static_cast<int32_t>(fc.converged);
     r->message = static_cast<int32_t>(fc.message ? fc.message : GSC_MSG_MAX_ITERATIONS);

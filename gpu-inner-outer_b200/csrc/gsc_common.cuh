@@ -49,18 +49,7 @@ struct GridInfo {
     uint32_t slices;     // n2 * n3 (theta, v) slices
     uint32_t sw;         // words per slice of a bit-sliced set: n1 * W, up to a multiple of 4 (the rest 0)
     uint32_t n1p;        // entries per plane of the y table: n1, up to a multiple of 4
-    uint32_t magic_n1;   // fdiv(x, n1) / fdiv(x, sw / 4) multipliers (see fdiv)
-    uint32_t magic_sw4;
 };
-
-// x / d for x * d < 2^32 with m = floor(2^32 / d) + 1 (m = 0 encodes d = 1).
-__host__ __device__ __forceinline__ uint32_t fdiv_magic(uint32_t d) {
-    return d <= 1 ? 0u : static_cast<uint32_t>((1ull << 32) / d + 1);
-}
-__device__ __forceinline__ uint32_t fdiv_magic32(uint32_t d) {   // the same, d in 32 bits
-    return d <= 1 ? 0u : 0xFFFFFFFFu / d + 1u + (0xFFFFFFFFu % d == d - 1 ? 1u : 0u);
-}
-__device__ __forceinline__ uint32_t fdiv(uint32_t x, uint32_t m) { return m ? __umulhi(x, m) : x; }
 
 // Programmatic dependent launch (PTX griddepcontrol, sm_90 and later): wait
 // until the kernel this one was launched after has completed and its writes
@@ -214,7 +203,6 @@ __host__ __device__ __forceinline__ uint32_t pack8(uint32_t a, uint32_t b, uint3
     return a | (b << 8) | (c << 16) | (d << 24);
 }
 
-// Fixpoint control block of one instance (device memory).
 // 4-byte asynchronous copy global -> shared (cp.async), complete after
 // cp_async_wait_all and the group's next barrier.
 __device__ __forceinline__ void cp_async4(void* smem_dst, const void* gmem_src) {
@@ -222,56 +210,9 @@ __device__ __forceinline__ void cp_async4(void* smem_dst, const void* gmem_src) 
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(gmem_src) : "memory");
 }
 
-// The same for 16 bytes, both addresses 16-byte aligned (bypasses L1).
-__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src) {
-    const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst));
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(gmem_src) : "memory");
-}
-
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
-// ---- 1-D bulk copies global -> shared (the TMA engine, no tensor map, no
-// multicast) completing on an mbarrier.  Source and destination 16-byte
-// aligned, size a multiple of 16 bytes.
-__device__ __forceinline__ uint32_t smem_addr(const void* p) {
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
-__device__ __forceinline__ void mbar_init(uint64_t* mbar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(mbar)), "r"(count) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-
-// One arrival that also announces `bytes` of copies completing on the barrier.
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* mbar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(mbar)), "r"(bytes)
-                 : "memory");
-}
-
-__device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* mbar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smem_addr(dst)),
-                 "l"(src), "r"(bytes), "r"(smem_addr(mbar))
-                 : "memory");
-}
-
-// One bounded probe of the barrier's phase `parity` (the hardware may
-// suspend the thread for a while inside the probe).
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* mbar, uint32_t parity) {
-    uint32_t ok = 0;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(smem_addr(mbar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-
-// Probes of a bulk-copy wait before it is given up as failed.
-constexpr uint32_t kBulkWaitProbes = 1u << 20;
-// FixControl::message of a solve stopped by a device wait that gave up.
-constexpr uint32_t kMsgDeviceTimeout = 4;
-
+// Fixpoint control block of one instance (device memory).
 struct FixControl {
     uint32_t iter;            // iterations completed
     uint32_t stop;            // 1 once a stop rule fired
