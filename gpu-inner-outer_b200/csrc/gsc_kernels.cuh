@@ -338,7 +338,7 @@ struct InstanceDesc {
     const unsigned long long* counts;
     uint32_t max_iterations;
     uint32_t stats_cap;
-    uint32_t words;       // rows * W
+    uint32_t words;       // slices * sw
 };
 
 // The instances one launch works on: slot[k] and, per task kind, the prefix

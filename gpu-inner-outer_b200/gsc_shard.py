@@ -9,9 +9,8 @@ of the bit-sliced D' = (valid and not reachable) or unsafe.
 
 One iteration on every rank (the Jacobi update of reachability.hpp:53-109):
 
-1. ``engine.step()``: the (theta, v) dilation of D' over the whole grid, then
-   the satisfaction test, the exists-input reduction and the finalize of the
-   rank's own slices; returns its newly reachable and newly certified counts.
+1. ``engine.step()``: the (theta, v) dilation of D' over the whole grid where
+   it is used, then the test and the update of the rank's own slices; returns its newly reachable and newly certified counts.
 2. ``comm.exchange_dprime``: an all-gather of the ranks' D' slabs, so every
    rank holds the whole next D' (S / 8 bytes in all: 0.5 MB at 65x65x38x25).
 3. ``comm.sum``: an all-reduce of the two counts.

@@ -274,7 +274,7 @@ typedef struct {
                                          dilation of D'                                                */
     double prefix_build_total_ms;     /* sum of scan_axis_ms                                           */
     double pair_satisfaction_ms;      /* satisfaction kernels (exists-input reduction fused in)        */
-    double reduce_inputs_ms;          /* stored: control kernel; fused: finalize kernel                */
+    double reduce_inputs_ms;          /* stored by prefix counts: control kernel; else event gap */
     double iteration_memcpy_ms;       /* the host loop's reads of the stop record                      */
     double result_memcpy_d2h_ms;      /* last gsc_problem_read                                         */
     double total_kernel_ms;           /* abstraction + prefix + satisfaction + reduction (kernels.cu:841-845) */
@@ -352,9 +352,8 @@ int gsc_fixpoint_noalloc(const uint32_t shape[4], uint32_t inputs, int32_t wrap_
  * (theta, v) slices [slice_begin, slice_end).  States are x-fastest, so a
  * slice range is one contiguous slab of every state array, and of the
  * bit-sliced D' words (words_per_slice words per slice).  Per iteration each
- * rank calls gsc_problem_shard_step (the dilation of D' over the whole grid,
- * then the satisfaction test, the exists-input reduction and the finalize of
- * its own slices; counts[] = its newly reachable and newly certified
+ * rank calls gsc_problem_shard_step (the dilation of D' over the whole grid
+ * where it is used, then the test and the update of its own slices; counts[] = its newly reachable and newly certified
  * states), the ranks all-gather their slabs of D' in place
  * (gsc_problem_shard_words: device memory, slab k at word
  * slice_begin_k * words_per_slice) and sum their counts, and every rank
