@@ -38,12 +38,16 @@ __device__ __forceinline__ bword moved_word(const bword (&F)[WMAX], int w, int d
 }
 
 // The bits of word w of a row at cell x and beyond (PTX shl gives 0 for a
-// shift of 32 or more).
+// shift of 32 or more; C++ leaves that open).
 __device__ __forceinline__ bword bits_from(uint32_t x, int w) {
     const int s = max(static_cast<int>(x) - w * kBits, 0);
+#ifdef __CUDA_ARCH__
     bword m;
     asm("shl.b32 %0, %1, %2;" : "=r"(m) : "r"(0xFFFFFFFFu), "r"(s));
     return m;
+#else
+    return s < kBits ? 0xFFFFFFFFu << s : 0u;   // (a test on the CPU)
+#endif
 }
 
 // The states m of a row (from state srow on) satisfied by input j: a state is
@@ -535,10 +539,6 @@ __device__ __forceinline__ int slice_task(const GridInfo& g, const FusedFixArgs&
             const uint32_t i1 = packed ? rows[row] : row;
             bword open[W], anyo = 0;
             load_row<W>(open, a.active + wbase + i1 * W);
-            if (p0) {
-#pragma unroll
-                for (int w = 0; w < W; ++w) open[w] &= ~hits[i1 * W + w];
-            }
             uint32_t states = 0;
 #pragma unroll
             for (int w = 0; w < W; ++w) {
@@ -657,6 +657,13 @@ __device__ __forceinline__ int slice_task(const GridInfo& g, const FusedFixArgs&
             }
             group_sync<WARP>();
             if (tid == 0) s_meta[2] = 0;
+            // The next pass tests the states that this one left, which it reads
+            // from the active set: `hits` may be written at once by a thread of
+            // a pass while another, with a lower input, begins the same row.
+            if (p0 + pass < nrep) {
+                for (uint32_t e = tid; e < n1 * W; e += bd)
+                    if (hits[e]) a.active[wbase + e] &= ~hits[e];
+            }
         }
     }
     // The update: words with a hit, and D' rows whose other buffer is behind.
