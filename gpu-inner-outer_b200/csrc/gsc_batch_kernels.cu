@@ -21,19 +21,6 @@ using namespace fused;
 
 namespace {
 
-// Largest k in [0, n) with off[k] <= t, given off[0] <= t < off[n].
-__device__ __forceinline__ uint32_t find_task(const uint32_t* __restrict__ off, uint32_t n, uint32_t t) {
-    uint32_t lo = 0, hi = n;
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (off[mid] <= t)
-            lo = mid;
-        else
-            hi = mid;
-    }
-    return lo;
-}
-
 __global__ void __launch_bounds__(256) k_batch_init(const InstanceDesc* __restrict__ descs, WorkList wl) {
     const uint32_t total = wl.ini_off[wl.n];
     for (uint32_t t = blockIdx.x; t < total; t += gridDim.x) {
@@ -66,12 +53,10 @@ __global__ void __launch_bounds__(256) k_batch_dilate(const InstanceDesc* __rest
     }
 }
 
-// The slices of the instances [kb, ke) of the list, whose rows have W words.
-// The instance of the current task is copied to shared memory when it
-// changes; the dynamic shared memory holds the largest instance's staging,
-// once per task group.  WARP: every warp of the block walks the task list
-// as its own group (tasks blockIdx.x * warps + warp, step gridDim.x *
-// warps), else the block is one group.
+// One launch per row width: the slices of the instances [kb, ke) of the list,
+// whose rows have W words (batch_slices).  The dynamic shared memory holds the
+// largest instance's staging, once per task group: every warp of the block
+// (WARP) or the block.
 template <int W, bool WARP>
 __global__ void __launch_bounds__(256) k_batch_slice(const InstanceDesc* __restrict__ descs, WorkList wl, uint32_t kb,
                                                      uint32_t ke, uint32_t task_words) {
@@ -79,44 +64,10 @@ __global__ void __launch_bounds__(256) k_batch_slice(const InstanceDesc* __restr
     constexpr uint32_t kGroups = WARP ? 8u : 1u;
     __shared__ __align__(16) InstanceDesc sd[kGroups];
     __shared__ uint32_t s_meta[kGroups][3];
-    const uint32_t first = wl.sat_off[kb], total = wl.sat_off[ke];
     const uint32_t grp = WARP ? (threadIdx.x >> 5) : 0u;
     const uint32_t ngrp = WARP ? (blockDim.x >> 5) : 1u;
-    const uint32_t rank = WARP ? (threadIdx.x & 31u) : threadIdx.x;
-    const uint32_t gsize = WARP ? 32u : blockDim.x;
-    bword* gsm = smem + grp * task_words;
-    uint32_t cur = 0xFFFFFFFFu;
-    bool stopped = false;
-    for (uint32_t t = first + blockIdx.x * ngrp + grp; t < total; t += gridDim.x * ngrp) {
-        const uint32_t k = kb + find_task(wl.sat_off + kb, ke - kb, t);
-        const uint32_t slot = wl.slot[k];
-        if (slot != cur) {
-            const uint32_t* src = reinterpret_cast<const uint32_t*>(descs + slot);
-            uint32_t* dst = reinterpret_cast<uint32_t*>(&sd[grp]);
-            for (uint32_t i = rank; i < sizeof(InstanceDesc) / 4; i += gsize) dst[i] = src[i];
-            group_sync<WARP>();
-            cur = slot;
-            // An instance's stop flag changes only after its last task, so the
-            // tasks of a stopped instance are skipped without a look.
-            stopped = __ldcg(&sd[grp].a.fc->stop) != 0;
-        }
-        if (stopped) continue;
-        const int done = slice_task<W, 2, 2, WARP, false>(sd[grp].g, sd[grp].a, t - wl.sat_off[k], gsm, s_meta[grp]);
-        // The counters are atomics; the barrier orders the group's before its
-        // first thread's fence (cumulative) and ticket.
-        group_sync<WARP>();
-        if (rank == 0 && done) {
-            FixControl* fc = sd[grp].a.fc;
-            if (done == 2) __threadfence();
-            if (atomicAdd(&fc->ticket, 1u) == wl.sat_off[k + 1] - wl.sat_off[k] - 1) {
-                __threadfence();
-                fc->ticket = 0;
-                const uint32_t it = __ldcg(&fc->iter) + 1;
-                control_step(fc, sd[grp].a.stats + kStatsCols * it, it);
-            }
-        }
-        group_sync<WARP>();
-    }
+    batch_slices<W, WARP>(descs, wl, kb, ke, blockIdx.x * ngrp + grp, gridDim.x * ngrp, smem + grp * task_words, sd[grp],
+                          s_meta[grp]);
 }
 
 __global__ void __launch_bounds__(256) k_batch_status(const InstanceDesc* __restrict__ descs, WorkList wl,

@@ -747,5 +747,64 @@ __device__ __forceinline__ void control_step(FixControl* fc, unsigned long long*
     }
 }
 
+// Largest k in [0, n) with off[k] <= t, given off[0] <= t < off[n].
+__device__ __forceinline__ uint32_t find_task(const uint32_t* __restrict__ off, uint32_t n, uint32_t t) {
+    uint32_t lo = 0, hi = n;
+    while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (off[mid] <= t)
+            lo = mid;
+        else
+            hi = mid;
+    }
+    return lo;
+}
+
+// Every task t = first, first + step, ... of the slices of the instances
+// [kb, ke) of a list, by one group.  The instance of the current task is
+// copied to shared memory (sd) when it changes.
+template <int W, bool WARP>
+__device__ __forceinline__ void batch_slices(const InstanceDesc* __restrict__ descs, const WorkList& wl, uint32_t kb,
+                                             uint32_t ke, uint32_t first, uint32_t step, bword* smem, InstanceDesc& sd,
+                                             uint32_t* s_meta) {
+    const uint32_t total = wl.sat_off[ke];
+    const uint32_t rank = WARP ? (threadIdx.x & 31u) : threadIdx.x;
+    const uint32_t gsize = WARP ? 32u : blockDim.x;
+    uint32_t cur = 0xFFFFFFFFu;
+    bool stopped = false;
+    for (uint32_t t = wl.sat_off[kb] + first; t < total; t += step) {
+        const uint32_t k = kb + find_task(wl.sat_off + kb, ke - kb, t);
+        const uint32_t slot = wl.slot[k];
+        if (slot != cur) {
+            // (A thread may still read the last record's stop flag.)
+            group_sync<WARP>();
+            const uint32_t* src = reinterpret_cast<const uint32_t*>(descs + slot);
+            uint32_t* dst = reinterpret_cast<uint32_t*>(&sd);
+            for (uint32_t i = rank; i < sizeof(InstanceDesc) / 4; i += gsize) dst[i] = src[i];
+            group_sync<WARP>();
+            cur = slot;
+            // An instance's stop flag changes only after its last task, so the
+            // tasks of a stopped instance are skipped without a look.
+            stopped = __ldcg(&sd.a.fc->stop) != 0;
+        }
+        if (stopped) continue;
+        const int done = slice_task<W, 2, 2, WARP, false>(sd.g, sd.a, t - wl.sat_off[k], smem, s_meta);
+        // The counters are atomics; the barrier orders the group's before its
+        // first thread's fence (cumulative) and ticket.
+        group_sync<WARP>();
+        if (rank == 0 && done) {
+            FixControl* fc = sd.a.fc;
+            if (done == 2) __threadfence();
+            if (atomicAdd(&fc->ticket, 1u) == wl.sat_off[k + 1] - wl.sat_off[k] - 1) {
+                __threadfence();
+                fc->ticket = 0;
+                const uint32_t it = __ldcg(&fc->iter) + 1;
+                control_step(fc, sd.a.stats + kStatsCols * it, it);
+            }
+        }
+        group_sync<WARP>();
+    }
+}
+
 }  // namespace fused
 }  // namespace gsc_b200

@@ -91,7 +91,7 @@ def test_solves_against_oracle(ctx, solved, name):
 @pytest.mark.parametrize("warp", [False, True], ids=["block", "warp"])
 def test_batch_against_oracle(ctx, solved, warp):
     names = sorted(CASES)
-    b = G.Batch(ctx, [solved[n][0] for n in names], sat_threads=128, sat_warp_tasks=warp)
+    b = G.Batch(ctx, [solved[n][0] for n in names], sat_threads=64, sat_warp_tasks=warp)
     b.solve(graph=True)
     for i, n in enumerate(names):
         check(b.read(i), solved[n][1], f"batch/{n}")

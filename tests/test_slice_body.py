@@ -54,3 +54,16 @@ def test_lowest_input_over_passes(slice_check, order, rows, cells, inputs, per_p
 ])
 def test_random_boxes(slice_check, order, seed, rows, cells, inputs, per_pass, threads):
     assert run(slice_check, order, seed, rows, cells, inputs, per_pass, threads) > 0
+
+
+@pytest.fixture(scope="module")
+def batch_check(tmp_path_factory):
+    return compiled(tmp_path_factory, "batch_check")
+
+
+@pytest.mark.parametrize("order", range(5))
+@pytest.mark.parametrize("threads,warp", [(64, 0), (256, 0), (32, 1), (128, 1)])
+def test_stopped_instances_beside_running_ones(batch_check, order, threads, warp):
+    """A group that skips a stopped instance's tasks goes on to the next
+    instance's record while some of its threads still read the stop flag."""
+    assert run(batch_check, order, threads, warp) == 3 * 512
