@@ -588,17 +588,6 @@ namespace {
 
 namespace gsc_api {
 
-// Whether the satisfaction test reads a representative's (theta, v) window
-// of D' itself (nz * nv words per staged word) rather than one word of a
-// dilated copy that a kernel of its own brings up to date every iteration.
-static bool reads_windows_directly(const GridInfo& g, const PlanRecord& pl) {
-    // Offsets into the dilated copies are 32-bit.
-    if (static_cast<uint64_t>(pl.dil.nk) * pl.dil.nl * __builtin_popcount(pl.ylevels | 1u) * g.slices * g.sw >=
-        0xFFFFFFFFull)
-        return true;
-    return pl.rep_rows <= 4 * pl.reps && (pl.rep_rows - pl.reps) * g.sw * 4ull <= 32ull << 20;
-}
-
 int problem_stage1(gsc_problem* p, const gsc_query_desc* qd) {
     gsc_context* ctx = p->ctx;
     const GridInfo& g = p->g;
@@ -864,8 +853,10 @@ int problem_stage2(gsc_problem* p) {
     GSC_TRY(palloc(p, &p->rowlost, 2ull * p->rl_words));
     GSC_CU(ctx, launch_rep_offsets(g, p->kidx, p->lidx, p->dil.nl, fused_args(p, 0, 0), p->reps, st));
     if (p->need_valid) {
-        GSC_TRY(palloc(p, &p->vzw, copies * words));
-        GSC_CU(ctx, launch_dilate(g, p->validb, p->validb, p->vzw, p->dil, p->tile, nullptr, nullptr, 0, st));
+        if (!p->direct) {
+            GSC_TRY(palloc(p, &p->vzw, copies * words));
+            GSC_CU(ctx, launch_dilate(g, p->validb, p->validb, p->vzw, p->dil, p->tile, nullptr, nullptr, 0, st));
+        }
         uint32_t* rowvoid = nullptr;
         GSC_TRY(palloc(p, &rowvoid, static_cast<uint64_t>(p->rl_words)));
         GSC_TRY(palloc(p, &p->needv, static_cast<uint64_t>(g.slices) * g.M * ((g.n[1] + 31) / 32)));

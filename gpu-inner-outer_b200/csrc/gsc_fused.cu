@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(256) k_need_valid(const __grid_constant__ Grid
                 const uint32_t lo = void_word(wl), hi = wh != wl ? void_word(wh) : 0u;
                 if (!(~__funnelshift_r(lo, hi, ylo & 31) << (31u - (yhi - ylo)))) {
                     bword V[W], m[W];
-                    box_rows<W>(a, a.vzw, rp.off, rp.hx, rp.hy, y, ye, V);
+                    valid_rows<W, 2>(g, a, make_uint4(rp.j, rp.zw, rp.vw, rp.off), rp.hx, rp.hy, y, ye, V);
                     const bword* src = a.srcb + static_cast<uint64_t>(s) * g.sw + y * W;
 #pragma unroll
                     for (int w = 0; w < W; ++w) m[w] = src[w];

@@ -328,18 +328,49 @@ __device__ __forceinline__ void box_rows(const FusedFixArgs& a, const bword* Z, 
     }
 }
 
+// Row i1's box rows of the valid set under a representative (as box_rows): from
+// its dilated copies where D' has such copies too, else from the set itself
+// (DIRECT: as a.direct; 2 = decided at run time).
+template <int W, int DIRECT>
+__device__ __forceinline__ void valid_rows(const GridInfo& g, const FusedFixArgs& a, uint4 rp, uint32_t hx, uint32_t hy,
+                                           uint32_t i1, uint32_t ye, bword (&V)[W]) {
+    if (DIRECT == 2 ? !a.direct : !DIRECT) {
+        box_rows<W>(a, a.vzw, rp.w, hx, hy, i1, ye, V);
+        return;
+    }
+    // Row by row, in few registers: few states come here.
+    const uint32_t ylo = hx & kBoxY ? i1 + static_cast<int8_t>(hy >> 8) : lo16(ye);
+    const uint32_t words = (hx & kBoxY ? hy & 0xFFu : hi16(ye) - ylo + 1) * W;
+#pragma unroll
+    for (int w = 0; w < W; ++w) V[w] = 0;
+    uint32_t z = lo16(rp.y);
+#pragma unroll 1
+    for (uint32_t i = 0; i < hi16(rp.y); ++i) {
+#pragma unroll 1
+        for (uint32_t v = 0; v < (hi16(rp.z) & 0x7FFFu); ++v) {
+            const bword* row = a.validb + static_cast<uint64_t>(z + g.n[2] * (lo16(rp.z) + v)) * g.sw + ylo * W;
+#pragma unroll 1
+            for (uint32_t e = 0; e < words; e += W) {
+#pragma unroll
+                for (int w = 0; w < W; ++w) V[w] |= row[e + w];
+            }
+        }
+        z = (z + 1 == g.n[2]) ? 0 : z + 1;
+    }
+}
+
 // Of the states m of row i1 of a slice, those whose box under the slice's
 // representative number `index` holds a valid cell: the x test on the valid
-// set's dilated copies.  Only rows marked in needv (launch_need_valid) have a
-// state whose box does not.
-template <int W>
+// set (valid_rows).  Only rows marked in needv (launch_need_valid) have a state
+// whose box does not.
+template <int W, int DIRECT>
 __device__ __noinline__ void keep_valid(const GridInfo& g, const FusedFixArgs& a, uint4 rp, uint4 bx, uint32_t slice,
                                         uint32_t index, uint32_t i1, bword (&m)[W]) {
     const uint32_t W1 = (g.n[1] + 31) / 32;
     if (!((__ldg(a.needv + (static_cast<uint64_t>(slice) * g.M + index) * W1 + (i1 >> 5)) >> (i1 & 31)) & 1u)) return;
     const uint64_t pl = xy_plane(g, slice % g.n[2], slice / g.n[2], rp.x);
     bword V[W], none[W];
-    box_rows<W>(a, a.vzw, rp.w, bx.x, bx.y, i1, bx.x & kBoxY ? 0u : __ldg(a.yt + pl * g.n1p + i1), V);
+    valid_rows<W, DIRECT>(g, a, rp, bx.x, bx.y, i1, bx.x & kBoxY ? 0u : __ldg(a.yt + pl * g.n1p + i1), V);
     if (bx.x & kBoxX) {
         bword T[W];
         or_range<W>(V, T, bx.x & 0xFFu);
@@ -614,7 +645,7 @@ __device__ __forceinline__ int slice_task(const GridInfo& g, const FusedFixArgs&
                     bword x[W];
 #pragma unroll
                     for (int w = 0; w < W; ++w) x[w] = sm[w];
-                    keep_valid<W>(g, a, rp, bx, slice, p0 + k, i1, x);
+                    keep_valid<W, DIRECT>(g, a, rp, bx, slice, p0 + k, i1, x);
 #pragma unroll
                     for (int w = 0; w < W; ++w) sm[w] = x[w];
                 }

@@ -243,6 +243,20 @@ struct PlanRecord {
     unsigned long long rep_rows;    // (theta, v) cells of their windows, summed
 };
 
+// Words of the dilated copies of a set for these widths and y levels.
+inline uint64_t dilated_words(const GridInfo& g, const DilateArgs& d, uint32_t levels) {
+    return static_cast<uint64_t>(d.nk) * d.nl * __builtin_popcount(levels | 1u) * g.slices * g.sw;
+}
+// Whether the satisfaction test reads a representative's (theta, v) window
+// of D' itself (nz * nv words per staged word), and of the valid set, rather
+// than one word of a dilated copy that a kernel of its own brings up to date
+// every iteration.
+inline bool reads_windows_directly(const GridInfo& g, const PlanRecord& pl) {
+    // Offsets into the dilated copies (SliceRep::off, ylev) are 32-bit.
+    if (dilated_words(g, pl.dil, pl.ylevels) >= 0xFFFFFFFFull) return true;
+    return pl.rep_rows <= 4 * pl.reps && (pl.rep_rows - pl.reps) * g.sw * 4ull <= 32ull << 20;
+}
+
 // A representative input of a (theta, v) slice: the lowest of the inputs
 // whose boxes coincide for every state of the slice (all x and y rows, the
 // theta box and the v box).
@@ -280,7 +294,7 @@ struct FusedFixArgs {
     const uint32_t* nreps;     // [slices]
     uint32_t pass;             // representatives whose records and changed rows are in shared memory at a time
     uint32_t sat_threads;      // threads per block
-    uint32_t direct;           // 1: D' windows are read from D' itself, 0: from dzw
+    uint32_t direct;           // 1: windows are read from D' and the valid set themselves, 0: from dzw and vzw
     bword* dzw;                // (y, theta, v)-dilated copies of D' (DilateTile), brought up to date each iteration
     uint32_t ylev[kYLevels];   // word offset of each y level in dzw
     DilateTile tile;
@@ -288,9 +302,10 @@ struct FusedFixArgs {
                                // (W1 = ceil(n1 / 32) words per (theta, v) slice, bit y % 32 of word y / 32):
                                // iteration k reads [k & 1] and writes the other
     uint32_t rl_words;         // slices * W1 + 1
-    const bword* vzw;          // the dilated copies of the valid set, and
+    // When validity is more than safety:
+    const bword* vzw;          // the dilated copies of the valid set (not with direct, which reads validb)
     const uint32_t* needv;     // [slices][M][W1] bit per representative and row: some state's box may hold no
-                               // valid cell (both when validity is more than safety)
+                               // valid cell
     DilateArgs dil;
     // Sharded solve (one rank of several): the launch covers slices
     // [shard_begin, shard_begin + shard_slices) only, reads dp[0], and the

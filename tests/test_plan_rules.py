@@ -1,0 +1,28 @@
+"""Host rules of the fused method's plan, on the CPU."""
+import subprocess
+
+import pytest
+
+from test_slice_body import compiled
+
+
+@pytest.fixture(scope="module")
+def plan_check(tmp_path_factory):
+    return compiled(tmp_path_factory, "plan_check")
+
+
+@pytest.mark.parametrize("shape,nk,nl,levels,windows,direct", [
+    ((4, 1000, 360, 900), 2, 2, 0b1111, 9, True),    # 2 * 2 * 4 copies of 324 M words: above 32-bit offsets
+    ((4, 1000, 360, 900), 2, 2, 0b0111, 9, False),   # three levels: below
+    ((4, 1000, 360, 900), 2, 2, 0b0111, 1, True),    # no wider than the set itself
+    ((1, 1, 20000, 26000), 2, 1, 0b1, 9, False),     # slices of one word are held as four
+    ((1, 1, 20000, 27000), 2, 1, 0b1, 9, True),
+])
+def test_dilated_copies_stay_within_their_offsets(plan_check, shape, nk, nl, levels, windows, direct):
+    """Where a set has dilated copies, every word of them has a 32-bit offset."""
+    out = subprocess.run([plan_check] + [str(v) for v in (*shape, nk, nl, levels, windows)], capture_output=True,
+                         text=True, check=True).stdout.split()
+    assert bool(int(out[0])) == direct
+    words = nk * nl * bin(levels).count("1") * shape[2] * shape[3] * ((shape[1] * ((shape[0] + 31) // 32) + 3) // 4 * 4)
+    assert int(out[1]) == words
+    assert direct or words < 2**32

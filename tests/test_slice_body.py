@@ -56,6 +56,15 @@ def test_random_boxes(slice_check, order, seed, rows, cells, inputs, per_pass, t
     assert run(slice_check, order, seed, rows, cells, inputs, per_pass, threads) > 0
 
 
+@pytest.mark.parametrize("seed", range(1, 4))
+@pytest.mark.parametrize("rows,cells,inputs,per_pass,threads", [(64, 40, 24, 8, 512), (70, 33, 24, 24, 128),
+                                                                (17, 20, 24, 8, 32)])
+def test_valid_cells_of_windows_read_directly(slice_check, seed, rows, cells, inputs, per_pass, threads):
+    """Where D' is read without dilated copies the valid set has none either,
+    and its cells are looked up in the set itself."""
+    assert run(slice_check, seed, seed, rows, cells, inputs, per_pass, threads, 0, 1) > 0
+
+
 @pytest.fixture(scope="module")
 def batch_check(tmp_path_factory):
     return compiled(tmp_path_factory, "batch_check")
