@@ -588,6 +588,56 @@ namespace {
 
 namespace gsc_api {
 
+// Gives back one buffer of a problem that no queued work uses.
+template <typename T>
+static void give_back(gsc_problem* p, T** ptr) {
+    const auto it = std::find_if(p->allocs.begin(), p->allocs.end(), [&](const auto& a) { return a.first == *ptr; });
+    if (*ptr && it != p->allocs.end()) {
+        std::vector<std::pair<void*, uint64_t>> one{*it};
+        uint64_t bytes = it->second;
+        p->bytes -= bytes;
+        p->allocs.erase(it);
+        device_release_all(p->ctx, p->pool, one, bytes);
+    }
+    *ptr = nullptr;
+}
+
+// The bit-sliced sets and, for the fused method, its tables of
+// representatives.  Takes all of them or none.
+static int method_tables(gsc_problem* p, bool stored_ok) {
+    const GridInfo& g = p->g;
+    const uint64_t words = static_cast<uint64_t>(g.slices) * g.sw;
+    int s = GSC_OK;
+    if (p->fused_candidate) {
+        for (bword** set : {&p->validb, &p->unsafeb, &p->srcb, &p->candb})
+            if (s == GSC_OK) s = palloc(p, set, words);
+        if (s == GSC_OK) s = palloc(p, &p->shorts, static_cast<uint64_t>(g.slices) * g.xy_planes);
+        if (s == GSC_OK) s = palloc(p, &p->reps, table_planes(g));
+        if (s == GSC_OK) s = palloc(p, &p->nreps, g.slices);
+        if (s == GSC_OK) return s;
+        for (bword** set : {&p->validb, &p->unsafeb, &p->srcb, &p->candb}) give_back(p, set);
+        give_back(p, &p->shorts);
+        give_back(p, &p->reps);
+        give_back(p, &p->nreps);
+        return s;
+    }
+    if (!stored_ok) return s;
+    // The bit-sliced sets and width ranks of the box table take the place of
+    // the valid set's prefix counts, which it makes needless.
+    GSC_TRY(palloc(p, &p->pvalid, g.tsize));
+    if (5 * words + (g.n[2] + g.n[3] + 2ull + 3) / 4 <= g.tsize) {
+        uint32_t* at = reinterpret_cast<uint32_t*>(p->pvalid);
+        p->validb = at;
+        p->unsafeb = at + words;
+        p->srcb = at + 2 * words;
+        p->candb = at + 3 * words;
+        p->dbits = at + 4 * words;
+        p->kidx = reinterpret_cast<uint8_t*>(at + 5 * words);
+        p->lidx = p->kidx + g.n[2] + 1;
+    }
+    return s;
+}
+
 int problem_stage1(gsc_problem* p, const gsc_query_desc* qd) {
     gsc_context* ctx = p->ctx;
     const GridInfo& g = p->g;
@@ -651,6 +701,25 @@ int problem_stage1(gsc_problem* p, const gsc_query_desc* qd) {
         GSC_TRY(palloc(p, &p->safe, static_cast<uint64_t>(g.n[0]) * g.n[1]));
         GSC_CU(ctx, launch_safe2(g, q, p->safe, st));
     }
+    // What judges the query (candidate set, intervals, widths) before what the
+    // method works on, so that a query is refused for itself, not for memory,
+    // wherever the former fits.
+    const uint64_t planes = table_planes(g);
+    GSC_TRY(palloc(p, &p->xt, planes * g.n[0]));
+    GSC_TRY(palloc(p, &p->yt, planes * g.n1p));
+    GSC_TRY(palloc(p, &p->zt, static_cast<uint64_t>(g.n[2]) * g.mw));
+    GSC_TRY(palloc(p, &p->wt, static_cast<uint64_t>(g.n[3]) * g.ma));
+    GSC_TRY(palloc(p, &p->dplan, 1));
+    if (p->fused_candidate) {
+        GSC_TRY(palloc(p, &p->xcls, planes * class_words(g)));
+        GSC_TRY(palloc(p, &p->xrep, planes));
+        GSC_TRY(palloc(p, &p->kidx, static_cast<uint64_t>(g.n[2]) + 1));
+        GSC_TRY(palloc(p, &p->lidx, static_cast<uint64_t>(g.n[3]) + 1));
+    }
+    const int room = method_tables(p, stored_ok);
+    if (room != GSC_OK && room != GSC_ERR_OUT_OF_MEMORY) return room;
+    p->no_room = room != GSC_OK;
+
     MaskArgs ma{};
     ma.obstacles = p->obstacles;
     ma.valid = p->valid;
@@ -659,29 +728,6 @@ int problem_stage1(gsc_problem* p, const gsc_query_desc* qd) {
     ma.build_cand = qd->candidate_mask ? 0 : 1;
     ma.safe = qd->safe_mask ? p->safe : nullptr;
     ma.safe_rank = p->safe_rank;
-    const uint64_t words = static_cast<uint64_t>(g.slices) * g.sw;
-    if (p->fused_candidate) {
-        GSC_TRY(palloc(p, &p->validb, words));
-        GSC_TRY(palloc(p, &p->unsafeb, words));
-        GSC_TRY(palloc(p, &p->srcb, words));
-        GSC_TRY(palloc(p, &p->candb, words));
-        GSC_TRY(palloc(p, &p->kidx, static_cast<uint64_t>(g.n[2]) + 1));
-        GSC_TRY(palloc(p, &p->lidx, static_cast<uint64_t>(g.n[3]) + 1));
-    } else if (stored_ok) {
-        // The bit-sliced sets and width ranks of the box table take the place of
-        // the valid set's prefix counts, which it makes needless.
-        GSC_TRY(palloc(p, &p->pvalid, g.tsize));
-        if (5 * words + (g.n[2] + g.n[3] + 2ull + 3) / 4 <= g.tsize) {
-            uint32_t* at = reinterpret_cast<uint32_t*>(p->pvalid);
-            p->validb = at;
-            p->unsafeb = at + words;
-            p->srcb = at + 2 * words;
-            p->candb = at + 3 * words;
-            p->dbits = at + 4 * words;
-            p->kidx = reinterpret_cast<uint8_t*>(at + 5 * words);
-            p->lidx = p->kidx + g.n[2] + 1;
-        }
-    }
     ma.validb = p->validb;
     ma.unsafeb = p->unsafeb;
     ma.srcb = p->srcb;
@@ -692,25 +738,14 @@ int problem_stage1(gsc_problem* p, const gsc_query_desc* qd) {
     GSC_CU(ctx, launch_masks(g, q, ma, st));
 
     // Per-axis boxes.
-    const uint64_t planes = table_planes(g);
-    GSC_TRY(palloc(p, &p->xt, planes * g.n[0]));
-    GSC_TRY(palloc(p, &p->yt, planes * g.n1p));
-    GSC_TRY(palloc(p, &p->shorts, static_cast<uint64_t>(g.slices) * g.xy_planes));
-    GSC_TRY(palloc(p, &p->zt, static_cast<uint64_t>(g.n[2]) * g.mw));
-    GSC_TRY(palloc(p, &p->wt, static_cast<uint64_t>(g.n[3]) * g.ma));
     GSC_CU(ctx, launch_axis_tables(g, q, p->abs->xn, p->abs->yn, p->abs->thf, p->abs->vf, p->xt, p->yt, p->zt, p->wt,
                                    p->shorts, p->flags, st));
 
     // Fused tables that do not depend on the sets, and the plan.
-    GSC_TRY(palloc(p, &p->dplan, 1));
     GSC_CU(ctx, cudaMemsetAsync(p->dplan, 0, sizeof(PlanRecord), st));
-    if (p->fused_candidate) {
-        GSC_TRY(palloc(p, &p->xcls, planes * class_words(g)));
+    if (p->fused_candidate && !p->no_room) {
         GSC_CU(ctx, launch_x_classes(g, p->xt, p->shorts, p->xcls, st));
-        GSC_TRY(palloc(p, &p->xrep, planes));
         GSC_CU(ctx, launch_plane_reps(g, p->xt, p->yt, p->wt, p->shorts, p->xrep, &p->dplan->max_reps, st));
-        GSC_TRY(palloc(p, &p->reps, planes));
-        GSC_TRY(palloc(p, &p->nreps, g.slices));
         GSC_CU(ctx, launch_slice_reps(g, p->xt, p->yt, p->zt, p->wt, p->shorts, p->xrep, p->reps, p->nreps, p->dplan, st));
     }
     GSC_CU(ctx, launch_plan(g, p->zt, p->wt, p->fused_candidate, p->counts, p->flags, p->kidx,
@@ -760,7 +795,7 @@ int problem_plan(gsc_problem* p) {
     p->method = method;
     // The stored method looks boxes up in bit tables where those are exact: no
     // empty interval, none wider than a lookup's word, not too many widths.
-    if (method == GSC_METHOD_STORED && pl.flags == 0 && !pl.width_overflow &&
+    if (method == GSC_METHOD_STORED && pl.flags == 0 && !pl.width_overflow && p->validb &&
         (p->dbits || static_cast<uint64_t>(g.slices) * g.sw <= g.tsize)) {
         p->dil = pl.dil;
         p->sbits = stored_bits_of(g, pl.dil, pl.ywidths);
@@ -769,6 +804,8 @@ int problem_plan(gsc_problem* p) {
     if (iter_bound + 2 > kStatsCapMax)
         return fail(ctx, GSC_ERR_UNSUPPORTED, "more than 2^20 fixpoint iterations requested");
     p->stats_cap = static_cast<uint32_t>(iter_bound + 2);
+    if (p->no_room && method == GSC_METHOD_FUSED)
+        return fail(ctx, GSC_ERR_OUT_OF_MEMORY, "no device memory for the fused method's tables");
     return GSC_OK;
 }
 

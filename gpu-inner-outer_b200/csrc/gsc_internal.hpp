@@ -124,6 +124,7 @@ struct gsc_problem {
     // hold large result copies).
     gsc_b200::PlanRecord* hplan_dev = nullptr;
     bool fused_candidate = false;
+    bool no_room = false;   // stage 1 had no memory for the method's tables: the query is judged without them
     // stored
     uint2* boxes = nullptr;
     uint64_t S_pad = 0;
@@ -245,9 +246,12 @@ int abstraction_enqueue(gsc_abstraction* a, cudaStream_t st, std::vector<std::pa
 // Problem set-up in three steps:
 //   stage1  masks, per-axis boxes and (for the fused method) the x classes,
 //           plane representatives and the set-up plan, ending with the copy
-//           of the plan record to p->hplan -- no host wait;
+//           of the plan record to p->hplan -- no host wait.  Where memory
+//           lasts for the masks and boxes alone it goes on with those
+//           (no_room), so that plan can say whether the query is at fault;
 //   plan    (after the stream has passed stage1) chooses the method from the
-//           plan record and checks the candidate set;
+//           plan record and checks the candidate set, then reports a lack of
+//           memory in stage1;
 //   stage2  fixpoint buffers and the method's tables -- no host wait.
 int problem_stage1(gsc_problem* p, const gsc_query_desc* qd);
 int problem_plan(gsc_problem* p);

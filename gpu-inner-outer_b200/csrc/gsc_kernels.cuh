@@ -78,7 +78,7 @@ cudaError_t launch_safe2(const GridInfo& g, const QueryInfo& q, uint8_t* safe2, 
 // |= 2 if one is wider than 32 cells.  flags[1] |= 1 << p for every accepted y interval of
 // 2^p .. 2^(p+1) - 1 cells, flags[2] |= 1 << (ny - 1) for one of ny; flags |= 4 if an x interval is wider
 // than 17 cells.
-// shorts: per plane its x and y boxes in short, {hx, hy, yr, xr}: hx = b - a + 1 | a << 8 of the x boxes
+// shorts (or null): per plane its x and y boxes in short, {hx, hy, yr, xr}: hx = b - a + 1 | a << 8 of the x boxes
 // [i + a, i + b], with kBoxX where they are alike, |a|, |b| < 32, and the cells with one (xr: first |
 // end << 16) are in a row, and kBoxY likewise for the y boxes (hy, yr).
 constexpr uint32_t kBoxX = 1u << 16, kBoxY = 1u << 17;

@@ -151,6 +151,7 @@ bool admit(gsc_server* s) {
         p->hplan = s->hplans + r->slot;
         p->hplan_dev = s->hplans_dev + r->slot;
         int status = problem_stage1(p, &r->q);
+        if (status == GSC_OK && p->no_room && !nothing_in_flight(s)) status = GSC_ERR_OUT_OF_MEMORY;
         if (status == GSC_OK && cudaEventRecord(r->ev, s->s_prep) != cudaSuccess) status = GSC_ERR_CUDA;
         if (status == GSC_ERR_OUT_OF_MEMORY && !nothing_in_flight(s)) {
             // Wait for memory: back to the head of the queue.

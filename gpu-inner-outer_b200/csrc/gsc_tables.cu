@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(kPlaneThreads) k_axis_tables(GridInfo g, Query
             range[d] = pack16(first, end);
             if (!cells) alike[d] = true;
         }
-        if (lane == 0)
+        if (lane == 0 && shorts)
             shorts[plane] = make_uint4(ab[0] | (alike[0] ? kBoxX : 0u) | (alike[1] ? kBoxY : 0u), ab[1], range[1], range[0]);
     }
     const uint64_t nz = static_cast<uint64_t>(g.n[2]) * g.mw;
