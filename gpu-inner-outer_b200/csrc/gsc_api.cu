@@ -120,7 +120,6 @@ int grid_from_model(const gsc_model_desc* m, GridInfo* g, std::string* err) {
     g->rows = static_cast<uint64_t>(g->n[1]) * g->n[2] * g->n[3];
     g->slices = g->n[2] * g->n[3];
     g->sw = (g->n[1] * g->W + 3) & ~3u;
-    g->n1p = (g->n[1] + 3) & ~3u;
     return GSC_OK;
 }
 
@@ -602,6 +601,20 @@ static void give_back(gsc_problem* p, T** ptr) {
     *ptr = nullptr;
 }
 
+// `count` elements in the part of the class records that no plane uses (a
+// slice with a single plane has its share for every input: table_planes), or
+// null where they do not fit.  So a one-substep query's lists take no memory of
+// their own.
+template <typename T>
+static T* spare_records(gsc_problem* p, uint64_t count) {
+    const uint64_t record = class_words(p->g) * sizeof(bword);
+    const uint64_t at = std::max(p->xcls_used, static_cast<uint64_t>(p->g.slices) * p->g.xy_planes * record);
+    const uint64_t end = at + (count * sizeof(T) + 15) / 16 * 16;
+    if (end > table_planes(p->g) * record) return nullptr;
+    p->xcls_used = end;
+    return reinterpret_cast<T*>(reinterpret_cast<char*>(p->xcls) + at);
+}
+
 // The bit-sliced sets and, for the fused method, its tables of
 // representatives.  Takes all of them or none.
 static int method_tables(gsc_problem* p, bool stored_ok) {
@@ -612,7 +625,7 @@ static int method_tables(gsc_problem* p, bool stored_ok) {
         for (bword** set : {&p->validb, &p->unsafeb, &p->srcb, &p->candb})
             if (s == GSC_OK) s = palloc(p, set, words);
         if (s == GSC_OK) s = palloc(p, &p->shorts, static_cast<uint64_t>(g.slices) * g.xy_planes);
-        if (s == GSC_OK) s = palloc(p, &p->reps, table_planes(g));
+        if (s == GSC_OK && !(p->reps = spare_records<SliceRep>(p, table_planes(g)))) s = palloc(p, &p->reps, table_planes(g));
         if (s == GSC_OK) s = palloc(p, &p->nreps, g.slices);
         if (s == GSC_OK) return s;
         for (bword** set : {&p->validb, &p->unsafeb, &p->srcb, &p->candb}) give_back(p, set);
@@ -706,7 +719,7 @@ int problem_stage1(gsc_problem* p, const gsc_query_desc* qd) {
     // wherever the former fits.
     const uint64_t planes = table_planes(g);
     GSC_TRY(palloc(p, &p->xt, planes * g.n[0]));
-    GSC_TRY(palloc(p, &p->yt, planes * g.n1p));
+    GSC_TRY(palloc(p, &p->yt, planes * g.n[1]));
     GSC_TRY(palloc(p, &p->zt, static_cast<uint64_t>(g.n[2]) * g.mw));
     GSC_TRY(palloc(p, &p->wt, static_cast<uint64_t>(g.n[3]) * g.ma));
     GSC_TRY(palloc(p, &p->dplan, 1));
@@ -822,7 +835,13 @@ int problem_stage2(gsc_problem* p) {
     // control record (no iterations), not a previous owner's bytes.
     GSC_CU(ctx, cudaMemsetAsync(p->fc, 0, sizeof(FixControl), st));
 
+    // What only stage 1 used (it is over by now).
+    give_back(p, &p->xrep);
     if (p->method == GSC_METHOD_STORED) {
+        give_back(p, &p->shorts);
+        give_back(p, &p->reps);
+        give_back(p, &p->nreps);
+        give_back(p, &p->xcls);
         const bool bits = p->sbits.copies != 0;
         if (!p->pvalid) GSC_TRY(palloc(p, &p->pvalid, g.tsize));
         if (!bits) {
@@ -884,19 +903,38 @@ int problem_stage2(gsc_problem* p) {
     // the same buffer and every parity choice picks it.
     p->reach1 = p->reach0;
     GSC_TRY(palloc(p, &p->active, words));
-    const uint64_t copies = static_cast<uint64_t>(p->dil.nk) * p->dil.nl * __builtin_popcount(p->tile.levels);
-    if (!p->direct) GSC_TRY(palloc(p, &p->dzw, copies * words));
-    p->rl_words = g.slices * ((g.n[1] + 31) / 32) + 1;
+    const uint64_t w1 = (g.n[1] + 31) / 32;
+    p->rl_words = static_cast<uint32_t>(g.slices * w1 + 1);
     GSC_TRY(palloc(p, &p->rowlost, 2ull * p->rl_words));
+    uint32_t* rowvoid = nullptr;
+    if (p->need_valid) {
+        GSC_TRY(palloc(p, &rowvoid, static_cast<uint64_t>(p->rl_words)));
+        // needv in the class records' spare part, or in the place of the boxes
+        // in short (16 bytes a plane), or on its own.
+        const uint64_t words_v = static_cast<uint64_t>(g.slices) * g.M * w1;
+        p->needv = spare_records<uint32_t>(p, words_v);
+        if (!p->needv && g.xy_planes == g.M && w1 <= 4) {
+            p->needv = reinterpret_cast<uint32_t*>(p->shorts);
+            p->shorts = nullptr;
+        }
+        if (!p->needv) GSC_TRY(palloc(p, &p->needv, words_v));
+    }
+    give_back(p, &p->shorts);
+    // The dilated copies last: without room for them, D' is read directly.
+    if (!p->direct) {
+        const uint64_t copies = dilated_words(g, p->dil, p->tile.levels);
+        int s = palloc(p, &p->dzw, copies);
+        if (s == GSC_OK && p->need_valid) s = palloc(p, &p->vzw, copies);
+        if (s != GSC_OK) {
+            give_back(p, &p->dzw);
+            if (s != GSC_ERR_OUT_OF_MEMORY || !p->copies_optional) return s;
+            ctx->last_error.clear();
+            p->direct = true;
+        }
+    }
     GSC_CU(ctx, launch_rep_offsets(g, p->kidx, p->lidx, p->dil.nl, fused_args(p, 0, 0), p->reps, st));
     if (p->need_valid) {
-        if (!p->direct) {
-            GSC_TRY(palloc(p, &p->vzw, copies * words));
-            GSC_CU(ctx, launch_dilate(g, p->validb, p->validb, p->vzw, p->dil, p->tile, nullptr, nullptr, 0, st));
-        }
-        uint32_t* rowvoid = nullptr;
-        GSC_TRY(palloc(p, &rowvoid, static_cast<uint64_t>(p->rl_words)));
-        GSC_TRY(palloc(p, &p->needv, static_cast<uint64_t>(g.slices) * g.M * ((g.n[1] + 31) / 32)));
+        if (!p->direct) GSC_CU(ctx, launch_dilate(g, p->validb, p->validb, p->vzw, p->dil, p->tile, nullptr, nullptr, 0, st));
         GSC_CU(ctx, launch_need_valid(g, fused_args(p, 0, 0), rowvoid, p->reps, p->needv, st));
     }
     return GSC_OK;

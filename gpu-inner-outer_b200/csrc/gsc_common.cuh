@@ -48,7 +48,6 @@ struct GridInfo {
     uint64_t rows;       // n1 * n2 * n3 x-rows
     uint32_t slices;     // n2 * n3 (theta, v) slices
     uint32_t sw;         // words per slice of a bit-sliced set: n1 * W, up to a multiple of 4 (the rest 0)
-    uint32_t n1p;        // entries per plane of the y table: n1, up to a multiple of 4
 };
 
 // Programmatic dependent launch (PTX griddepcontrol, sm_90 and later): wait

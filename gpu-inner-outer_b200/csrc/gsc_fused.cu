@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(256) k_need_valid(const __grid_constant__ Grid
         __syncwarp();
         for (uint32_t q = 0; q < W1; ++q) {
             const uint32_t y = q * 32 + lane;
-            const uint32_t ye = y < n1 ? a.yt[pl * g.n1p + y] : kReject;
+            const uint32_t ye = y < n1 ? a.yt[pl * g.n[1] + y] : kReject;
             bool need = false;
             if (ye != kReject) {
                 const uint32_t ylo = lo16(ye), yhi = hi16(ye), wl = ylo >> 5, wh = yhi >> 5;

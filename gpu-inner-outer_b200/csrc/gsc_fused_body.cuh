@@ -370,7 +370,7 @@ __device__ __noinline__ void keep_valid(const GridInfo& g, const FusedFixArgs& a
     if (!((__ldg(a.needv + (static_cast<uint64_t>(slice) * g.M + index) * W1 + (i1 >> 5)) >> (i1 & 31)) & 1u)) return;
     const uint64_t pl = xy_plane(g, slice % g.n[2], slice / g.n[2], rp.x);
     bword V[W], none[W];
-    valid_rows<W, DIRECT>(g, a, rp, bx.x, bx.y, i1, bx.x & kBoxY ? 0u : __ldg(a.yt + pl * g.n1p + i1), V);
+    valid_rows<W, DIRECT>(g, a, rp, bx.x, bx.y, i1, bx.x & kBoxY ? 0u : __ldg(a.yt + pl * g.n[1] + i1), V);
     if (bx.x & kBoxX) {
         bword T[W];
         or_range<W>(V, T, bx.x & 0xFFu);
@@ -585,7 +585,7 @@ __device__ __forceinline__ int slice_task(const GridInfo& g, const FusedFixArgs&
                 if (bx.x & kBoxY) {
                     if (i1 - lo16(bx.z) >= hi16(bx.z)) continue;
                 } else {
-                    ye = __ldg(a.yt + (shared_xy ? base_pl : base_pl + rp.x) * g.n1p + i1);
+                    ye = __ldg(a.yt + (shared_xy ? base_pl : base_pl + rp.x) * g.n[1] + i1);
                     if (ye == kReject) continue;
                 }
                 bword F[W];

@@ -139,6 +139,7 @@ struct gsc_problem {
     gsc_b200::bword* dp[2] = {nullptr, nullptr};
     gsc_b200::bword *reach0 = nullptr, *reach1 = nullptr, *active = nullptr;
     gsc_b200::bword* xcls = nullptr;
+    uint64_t xcls_used = 0;     // bytes of it up to the last list placed behind its records
     uint8_t* xrep = nullptr;
     uint32_t max_reps = 0;      // most representative accelerations of one omega column
     gsc_b200::SliceRep* reps = nullptr;
@@ -146,6 +147,7 @@ struct gsc_problem {
     uint32_t pass = 1, sat_threads = 128;   // of the satisfaction kernel (FusedFixArgs)
     uint32_t* needv = nullptr;
     bool direct = false;        // windows are read from D' and the valid set themselves
+    bool copies_optional = true;   // they are too where memory lacks for the copies (else that is an error)
     gsc_b200::DilateTile tile{};          // else from dilated copies
     uint32_t ylev[gsc_b200::kYLevels] = {};
     gsc_b200::bword *dzw = nullptr, *vzw = nullptr;

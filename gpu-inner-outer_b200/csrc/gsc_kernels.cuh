@@ -243,9 +243,10 @@ struct PlanRecord {
     unsigned long long rep_rows;    // (theta, v) cells of their windows, summed
 };
 
-// Words of the dilated copies of a set for these widths and y levels.
+// Words of the dilated copies of a set for these widths and y levels (level 0
+// where there are none).
 inline uint64_t dilated_words(const GridInfo& g, const DilateArgs& d, uint32_t levels) {
-    return static_cast<uint64_t>(d.nk) * d.nl * __builtin_popcount(levels | 1u) * g.slices * g.sw;
+    return static_cast<uint64_t>(d.nk) * d.nl * __builtin_popcount(levels ? levels : 1u) * g.slices * g.sw;
 }
 // Whether the satisfaction test reads a representative's (theta, v) window
 // of D' itself (nz * nv words per staged word), and of the valid set, rather

@@ -193,6 +193,7 @@ bool advance_prep1(gsc_server* s) {
         any = true;
         gsc_problem* p = r->p.get();
         int status = q == cudaSuccess ? problem_plan(p) : GSC_ERR_CUDA;
+        p->copies_optional = nothing_in_flight(s);   // (else it waits for memory)
         if (status == GSC_OK) status = problem_stage2(p);
         if (status == GSC_ERR_OUT_OF_MEMORY && !nothing_in_flight(s)) {
             cudaStreamSynchronize(s->s_prep);

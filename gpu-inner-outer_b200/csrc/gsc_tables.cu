@@ -273,7 +273,7 @@ __global__ void __launch_bounds__(kPlaneThreads) k_axis_tables(GridInfo g, Query
             const uint32_t n = g.n[d];
             const double r = box_radius(g, q, d, vc);
             const double* nom = (d ? yn : xn) + plane * n;
-            uint32_t* out = d ? yt + plane * g.n1p : xt + plane * n;
+            uint32_t* out = d ? yt + plane * g.n[1] : xt + plane * n;
             uint32_t ref = 0, first = 0, end = 0, cells = 0;
             bool same = true;
             for (uint32_t base = 0; base < n; base += 32) {
@@ -421,7 +421,7 @@ __device__ __forceinline__ PairBox pair_box(const GridInfo& g, const uint32_t* _
     const uint32_t ja = j % g.ma, jw = j / g.ma;
     const uint64_t plane = xy_plane(g, idx[2], idx[3], j);
     const uint32_t xe = __ldg(xt + plane * g.n[0] + idx[0]);
-    const uint32_t ye = __ldg(yt + plane * g.n1p + idx[1]);
+    const uint32_t ye = __ldg(yt + plane * g.n[1] + idx[1]);
     const uint32_t ze = __ldg(zt + idx[2] * g.mw + jw);
     const uint32_t we = __ldg(wt + idx[3] * g.ma + ja);
     bool src = true;
@@ -613,7 +613,7 @@ __device__ __forceinline__ bool same_rows(const GridInfo& g, const uint32_t* __r
     if (ys && (a.y != b.y || a.z != b.z)) return false;
     bool eq = true;
     for (uint32_t i = lane; !xs && i < g.n[0]; i += lanes) eq = eq && xt[pa * g.n[0] + i] == xt[pb * g.n[0] + i];
-    for (uint32_t i = lane; !ys && i < g.n[1]; i += lanes) eq = eq && yt[pa * g.n1p + i] == yt[pb * g.n1p + i];
+    for (uint32_t i = lane; !ys && i < g.n[1]; i += lanes) eq = eq && yt[pa * g.n[1] + i] == yt[pb * g.n[1] + i];
     return lanes == 1 ? eq : __all_sync(0xFFFFFFFFu, eq) != 0;
 }
 

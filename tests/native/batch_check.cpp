@@ -31,7 +31,7 @@ struct Instance {
         g.n[2] = 2;
         g.n[3] = 1;
         g.W = 1;
-        g.sw = g.n1p = 8;
+        g.sw = 8;
         g.slices = 2;
         g.rows = 16;
         g.S = 512;

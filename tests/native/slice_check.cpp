@@ -41,7 +41,6 @@ int check(int argc, char** argv) {
     g.n[3] = 2;
     g.W = W;
     g.sw = (n1 * W + 3) & ~3u;
-    g.n1p = (n1 + 3) & ~3u;
     g.slices = 8;
     g.rows = static_cast<uint64_t>(n1) * g.slices;
     g.S = g.rows * n0;
