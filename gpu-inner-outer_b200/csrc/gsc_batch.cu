@@ -127,7 +127,6 @@ struct gsc_batch {
     // uploads do not wait for the set-up queued before them.
     InstanceDesc* hdesc_pin = nullptr;
     uint32_t* hlist_pin = nullptr;   // [2][work_list_words(count)]
-    bool lists_uploaded = false;
     void* pin_early = nullptr;   // hplans, hrunning, hfc (from the context's pinned cache)
     void* pin_late = nullptr;    // hstats, hdesc_pin, hlist_pin (from the context's pinned cache)
     size_t pin_early_bytes = 0, pin_late_bytes = 0;
@@ -188,8 +187,9 @@ uint32_t log2_ceil(uint64_t v) {
     return l;
 }
 
-// Work lists with `chunk` word positions per task: the small instances'
-// (the batched kernels) and every instance's (init and status).
+// Work lists with `chunk` word positions per init task: the small instances'
+// (the batched kernels) and every instance's (init and status).  Once a batch:
+// its pinned copies are not written again.
 int upload_list(gsc_batch* b, uint32_t chunk) {
     std::vector<const gsc_problem*> probs;
     std::vector<uint32_t> slots;
@@ -206,9 +206,6 @@ int upload_list(gsc_batch* b, uint32_t chunk) {
         slots.push_back(i);
     }
     build_work_list(probs, slots, chunk, b->hlist_all, b->tot_all);
-    // A new upload (autotuning) waits until the previous one has read the
-    // pinned lists; the first does not wait.
-    if (b->lists_uploaded) GSC_CU(b->ctx, cudaStreamSynchronize(b->ctx->stream));
     const size_t words = work_list_words(b->probs.size());
     uint32_t* pin_small = b->hlist_pin;
     uint32_t* pin_all = b->hlist_pin + words;
@@ -217,7 +214,6 @@ int upload_list(gsc_batch* b, uint32_t chunk) {
     GSC_CU(b->ctx, cudaMemcpyAsync(b->dlist, pin_small, b->hlist.size() * 4, cudaMemcpyHostToDevice, b->ctx->stream));
     GSC_CU(b->ctx, cudaMemcpyAsync(b->dlist_all, pin_all, b->hlist_all.size() * 4, cudaMemcpyHostToDevice,
                                    b->ctx->stream));
-    b->lists_uploaded = true;
     b->wl = device_work_list(b->dlist, static_cast<uint32_t>(b->small.size()), chunk, nullptr, b->drunning);
     b->wl_all = device_work_list(b->dlist_all, static_cast<uint32_t>(b->probs.size()), chunk, b->hfc_dev, b->drunning);
     return GSC_OK;
@@ -237,10 +233,11 @@ int enqueue_iterations(gsc_batch* b, uint32_t count, uint32_t* launches) {
 // Time the solve from a fresh start (up to kTuneIterations iterations,
 // checked every kTuneChunk: the first iterations test every pair, the later
 // ones only the pairs near states that left D', and the best shape differs
-// between the two) under each candidate shape; keep the fastest.  Candidates: one task per block (64 / 128 / 256
-// threads) and one task per warp (4 or 8 warps a block), each with one
-// block per task or a persistent grid, and chunks of 256 or 1,024 words; a
-// warp shape whose staging does not fit a block's shared memory is left out.
+// between the two) under each candidate shape; keep the fastest.  Candidates:
+// one task per block (64 / 128 / 256 threads) and one task per warp (4 or 8
+// warps a block), each with one block per task or a persistent grid; a warp
+// shape whose staging does not fit a block's shared memory is left out.  The
+// chunk of init tasks stays as it was asked for: no iteration depends on it.
 // A single trial of a few iterations varies by a few percent between runs,
 // so the three fastest shapes are timed twice more and each keeps its best
 // time.
@@ -252,17 +249,11 @@ int autotune(gsc_batch* b) {
     };
     const Trial trials[] = {{64, 0}, {128, 0}, {256, 0}, {128, 1}, {256, 1}};
     const uint32_t per_sm[] = {0, 4, 8, 16};
-    const uint32_t chunks[] = {256, 1024};
     constexpr uint32_t kTuneChunk = 8, kTuneIterations = 32;
     cudaEvent_t e0, e1;
     GSC_CU(ctx, cudaEventCreate(&e0));
     GSC_CU(ctx, cudaEventCreate(&e1));
-    uint32_t listed = 0;   // chunk of the uploaded work lists
     auto time_shape = [&](const BatchShape& cand, float* ms) -> int {
-        if (cand.chunk != listed) {
-            GSC_TRY(upload_list(b, cand.chunk));
-            listed = cand.chunk;
-        }
         b->shape = cand;
         cudaError_t e = launch_batch_init(b->ddesc, b->wl, b->tot, sms, ctx->stream);
         if (e == cudaSuccess) e = cudaEventRecord(e0, ctx->stream);
@@ -283,17 +274,15 @@ int autotune(gsc_batch* b) {
     };
     std::vector<std::pair<float, BatchShape>> timed;
     int status = GSC_OK;
-    for (uint32_t ch : chunks) {
-        for (const Trial& tr : trials) {
-            for (uint32_t ps : per_sm) {
-                const BatchShape cand{tr.threads, ps * static_cast<uint32_t>(sms), ch, tr.warp};
-                if (!shape_admitted(cand, b->smem)) continue;
-                float ms = 0.f;
-                status = time_shape(cand, &ms);
-                if (status != GSC_OK) break;
-                timed.emplace_back(ms, cand);
-            }
+    const uint32_t chunk = b->shape.chunk;
+    for (const Trial& tr : trials) {
+        for (uint32_t ps : per_sm) {
+            const BatchShape cand{tr.threads, ps * static_cast<uint32_t>(sms), chunk, tr.warp};
+            if (!shape_admitted(cand, b->smem)) continue;
+            float ms = 0.f;
+            status = time_shape(cand, &ms);
             if (status != GSC_OK) break;
+            timed.emplace_back(ms, cand);
         }
         if (status != GSC_OK) break;
     }
@@ -319,7 +308,7 @@ int autotune(gsc_batch* b) {
                                        [](const std::pair<float, BatchShape>& x,
                                           const std::pair<float, BatchShape>& y) { return x.first < y.first; });
     b->shape = best->second;
-    return upload_list(b, b->shape.chunk);
+    return GSC_OK;
 }
 
 void release_batch_graph(gsc_batch* b) {
@@ -610,12 +599,13 @@ int batch_finish(gsc_batch* b, const gsc_batch_options* opt) {
             std::lock_guard<std::mutex> lk(g_tune_mu);
             auto it = g_tuned.find(key);
             if (it != g_tuned.end()) {
+                const uint32_t chunk = b->shape.chunk;
                 b->shape = it->second;
+                b->shape.chunk = chunk;
                 hit = true;
             }
         }
         if (hit) {
-            GSC_TRY(upload_list(b, b->shape.chunk));
             b->t.tuned = 2;
         } else {
             const auto t0 = std::chrono::steady_clock::now();

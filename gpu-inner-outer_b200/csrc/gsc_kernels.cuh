@@ -385,7 +385,7 @@ struct BatchClass {
 struct BatchShape {
     uint32_t sat_threads;   // threads per satisfaction block
     uint32_t sat_blocks;    // persistent satisfaction blocks (0 = one per task)
-    uint32_t chunk;         // word positions per dilate / finalize task
+    uint32_t chunk;         // word positions per init task
     uint32_t warp;          // 1: one satisfaction task per warp (smem per task, sat_threads / 32 of them)
 };
 

@@ -406,7 +406,8 @@ typedef struct {
     uint32_t sat_threads;         /* threads per satisfaction block: 64, 128, 256 (0 = 128)  */
     uint32_t sat_blocks_per_sm;   /* persistent satisfaction blocks per SM (0 = one block
                                      per task)                                             */
-    uint32_t chunk_words;         /* word positions per dilate / finalize task (0 = 2048)  */
+    uint32_t chunk_words;         /* word positions per task of a solve's start (0 = 2048;
+                                     a multiple of 256)                                    */
     uint32_t sat_warp_tasks;      /* 1: each warp of a satisfaction block runs its own task
                                      (sat_threads / 32 tasks per block, no block barriers);
                                      0: the whole block runs one task                       */
