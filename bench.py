@@ -369,21 +369,33 @@ def issue_roofline(kernel, workload, per_launch_ms, sm_mhz, sms):
             "warp_instructions_per_launch": inst}
 
 
-def algorithmic_bytes(method, g, timings):
-    """Bytes one satisfaction launch must move, from the counters of a profiled
-    solve.  stored: 8 B per streamed (state, input) box + valid, candidate,
-    reachable (1 B each) and controller (4 B) per state.  fused: the x and y
-    box-table rows of every processed (slice, input) plane task (4 B per entry)
-    + four passes over the 32-bit bit-sliced sets (active, hit, previous and
-    next reachable) per launch."""
-    n0, n1, n2, n3 = g["shape"]
-    S = n0 * n1 * n2 * n3
+def satisfaction_kernel(method, shape, table_passes):
+    """The kernel that tests the pairs: the stored method looks boxes up in a
+    bit table built in one pass where that is exact, and counts them on prefix
+    sums built in two or four passes elsewhere."""
+    if method == 2:
+        return "k_slice"
+    if table_passes == 1:
+        return "k_sat_bits"
+    return "k_sat_stored_wide" if max(shape) > 255 else "k_sat_stored"
+
+
+def algorithmic_bytes(kernel, shape, timings):
+    """Bytes one launch of the satisfaction kernel must move, on average over a
+    profiled solve.  k_slice: the active set and D' read once (4 B a word of
+    32 cells, rows padded to words and slices to four) and the 32-byte records
+    of the representative inputs of every slice with an active state (the
+    solve's auxiliary count); planes whose boxes are not alike read table rows
+    on top, which are left out.  Stored: the streamed boxes (16 B a pair for
+    k_sat_stored_wide, else 8) and valid, candidate, reachable (1 B each) and
+    controller (4 B) per state."""
+    n0, n1, n2, n3 = shape
     L = max(timings["sat_launches"], 1)
-    if method == 1:
-        return (8.0 * timings["pair_tests"] + 7.0 * S * L) / L
-    W = (n0 + 31) // 32
-    words = n1 * n2 * n3 * W
-    return (4.0 * (n0 + n1) * timings["aux_count"] + 16.0 * words * L) / L
+    if kernel == "k_slice":
+        words = n2 * n3 * ((n1 * ((n0 + 31) // 32) + 3) // 4 * 4)
+        return (32.0 * timings["aux_count"] + 8.0 * words * L) / L
+    pair = 16.0 if kernel == "k_sat_stored_wide" else 8.0
+    return pair * timings["pair_tests"] / L + 7.0 * n0 * n1 * n2 * n3
 
 
 def gpu_uuid(torch, dev):
@@ -938,13 +950,13 @@ def main():
     phases = {"prefix_or_dilation_us": 1e3 * ph["prefix_build_total_ms"] / nit,
               "pass_us": [1e3 * v / nit for v in ph["scan_axis_ms"] if v > 0],
               "satisfaction_us": 1e3 * ph["pair_satisfaction_ms"] / nit,
-              "finalize_or_control_us": 1e3 * ph["reduce_inputs_ms"] / nit,
+              "control_us": 1e3 * ph["reduce_inputs_ms"] / nit,
               "note": "per iteration of one host-loop solve, its launches queued behind a short hold so that they "
                       "run back to back, with CUDA events between the phases (each event adds about 2.5 us)"}
     used = tp["method"]
-    kname = "k_sat_bits" if used == G.METHOD_STORED else "k_slice"
+    kname = satisfaction_kernel(used, shape, len(phases["pass_us"]))
     per_launch_ms = tp["sat_kernel_ms"] / max(tp["sat_launches"], 1)
-    alg = algorithmic_bytes(used, {"shape": shape}, tp)
+    alg = algorithmic_bytes(kname, shape, tp)
     peak, peak_kind = measured_peak()
     achieved = alg / (per_launch_ms * 1e-3) / 1e9
     traffic = ncu_traffic(kname, case["name"])
