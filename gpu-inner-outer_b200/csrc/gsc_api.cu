@@ -920,21 +920,20 @@ int problem_stage2(gsc_problem* p) {
         if (!p->needv) GSC_TRY(palloc(p, &p->needv, words_v));
     }
     give_back(p, &p->shorts);
-    // The dilated copies last: without room for them, D' is read directly.
-    if (!p->direct) {
-        const uint64_t copies = dilated_words(g, p->dil, p->tile.levels);
-        int s = palloc(p, &p->dzw, copies);
-        if (s == GSC_OK && p->need_valid) s = palloc(p, &p->vzw, copies);
-        if (s != GSC_OK) {
-            give_back(p, &p->dzw);
-            if (s != GSC_ERR_OUT_OF_MEMORY || !p->copies_optional) return s;
-            ctx->last_error.clear();
-            p->direct = true;
-        }
+    // The dilated copies last: without room for them, the sets are read directly.
+    const uint64_t copies = dilated_words(g, p->dil, p->tile.levels);
+    int s = GSC_OK;
+    if (!p->direct) s = palloc(p, &p->dzw, copies);
+    if (s == GSC_OK && p->need_valid && dilated_offsets_fit(g, p->dil, p->tile.levels)) s = palloc(p, &p->vzw, copies);
+    if (s != GSC_OK) {
+        give_back(p, &p->dzw);
+        if (s != GSC_ERR_OUT_OF_MEMORY || !p->copies_optional) return s;
+        ctx->last_error.clear();
+        p->direct = true;
     }
     GSC_CU(ctx, launch_rep_offsets(g, p->kidx, p->lidx, p->dil.nl, fused_args(p, 0, 0), p->reps, st));
     if (p->need_valid) {
-        if (!p->direct) GSC_CU(ctx, launch_dilate(g, p->validb, p->validb, p->vzw, p->dil, p->tile, nullptr, nullptr, 0, st));
+        if (p->vzw) GSC_CU(ctx, launch_dilate(g, p->validb, p->validb, p->vzw, p->dil, p->tile, nullptr, nullptr, 0, st));
         GSC_CU(ctx, launch_need_valid(g, fused_args(p, 0, 0), rowvoid, p->reps, p->needv, st));
     }
     return GSC_OK;

@@ -328,19 +328,12 @@ __device__ __forceinline__ void box_rows(const FusedFixArgs& a, const bword* Z, 
     }
 }
 
-// Row i1's box rows of the valid set under a representative (as box_rows): from
-// its dilated copies where D' has such copies too, else from the set itself
-// (DIRECT: as a.direct; 2 = decided at run time).
-template <int W, int DIRECT>
-__device__ __forceinline__ void valid_rows(const GridInfo& g, const FusedFixArgs& a, uint4 rp, uint32_t hx, uint32_t hy,
-                                           uint32_t i1, uint32_t ye, bword (&V)[W]) {
-    if (DIRECT == 2 ? !a.direct : !DIRECT) {
-        box_rows<W>(a, a.vzw, rp.w, hx, hy, i1, ye, V);
-        return;
-    }
-    // Row by row, in few registers: few states come here.
-    const uint32_t ylo = hx & kBoxY ? i1 + static_cast<int8_t>(hy >> 8) : lo16(ye);
-    const uint32_t words = (hx & kBoxY ? hy & 0xFFu : hi16(ye) - ylo + 1) * W;
+// Rows of the valid set in a representative's (theta, v) window, ORed: row by
+// row, out of line and in few registers, since only grids without dilated
+// copies of the valid set come here.
+template <int W>
+__device__ __noinline__ void valid_window(const GridInfo& g, const bword* validb, uint4 rp, uint32_t ylo, uint32_t ny,
+                                          bword (&V)[W]) {
 #pragma unroll
     for (int w = 0; w < W; ++w) V[w] = 0;
     uint32_t z = lo16(rp.y);
@@ -348,15 +341,31 @@ __device__ __forceinline__ void valid_rows(const GridInfo& g, const FusedFixArgs
     for (uint32_t i = 0; i < hi16(rp.y); ++i) {
 #pragma unroll 1
         for (uint32_t v = 0; v < (hi16(rp.z) & 0x7FFFu); ++v) {
-            const bword* row = a.validb + static_cast<uint64_t>(z + g.n[2] * (lo16(rp.z) + v)) * g.sw + ylo * W;
+            const bword* row = validb + static_cast<uint64_t>(z + g.n[2] * (lo16(rp.z) + v)) * g.sw + ylo * W;
 #pragma unroll 1
-            for (uint32_t e = 0; e < words; e += W) {
+            for (uint32_t e = 0; e < ny * W; e += W) {
 #pragma unroll
                 for (int w = 0; w < W; ++w) V[w] |= row[e + w];
             }
         }
         z = (z + 1 == g.n[2]) ? 0 : z + 1;
     }
+}
+
+// Row i1's box rows of the valid set under a representative (as box_rows): from
+// its dilated copies, or from the set itself where it has none, which is only
+// where D' is read directly (DIRECT: as a.direct; 2 = decided at run time).
+// Copies beside direct reads: 65x65x38x25 x 36 inputs with obstacles takes 629
+// us with them and 679 without.
+template <int W, int DIRECT>
+__device__ __forceinline__ void valid_rows(const GridInfo& g, const FusedFixArgs& a, uint4 rp, uint32_t hx, uint32_t hy,
+                                           uint32_t i1, uint32_t ye, bword (&V)[W]) {
+    if (DIRECT == 0 || a.vzw) {
+        box_rows<W>(a, a.vzw, rp.w, hx, hy, i1, ye, V);
+        return;
+    }
+    const uint32_t ylo = hx & kBoxY ? i1 + static_cast<int8_t>(hy >> 8) : lo16(ye);
+    valid_window<W>(g, a.validb, rp, ylo, hx & kBoxY ? hy & 0xFFu : hi16(ye) - ylo + 1, V);
 }
 
 // Of the states m of row i1 of a slice, those whose box under the slice's

@@ -146,8 +146,8 @@ struct gsc_problem {
     uint32_t* nreps = nullptr;
     uint32_t pass = 1, sat_threads = 128;   // of the satisfaction kernel (FusedFixArgs)
     uint32_t* needv = nullptr;
-    bool direct = false;        // windows are read from D' and the valid set themselves
-    bool copies_optional = true;   // they are too where memory lacks for the copies (else that is an error)
+    bool direct = false;        // D' windows are read from D' itself
+    bool copies_optional = true;   // also where memory lacks for dilated copies (else that is an error)
     gsc_b200::DilateTile tile{};          // else from dilated copies
     uint32_t ylev[gsc_b200::kYLevels] = {};
     gsc_b200::bword *dzw = nullptr, *vzw = nullptr;

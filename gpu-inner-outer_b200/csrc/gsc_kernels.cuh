@@ -248,13 +248,16 @@ struct PlanRecord {
 inline uint64_t dilated_words(const GridInfo& g, const DilateArgs& d, uint32_t levels) {
     return static_cast<uint64_t>(d.nk) * d.nl * __builtin_popcount(levels ? levels : 1u) * g.slices * g.sw;
 }
+// Whether a set may have dilated copies: offsets into them (SliceRep::off,
+// ylev) are 32-bit.
+inline bool dilated_offsets_fit(const GridInfo& g, const DilateArgs& d, uint32_t levels) {
+    return dilated_words(g, d, levels) < 0xFFFFFFFFull;
+}
 // Whether the satisfaction test reads a representative's (theta, v) window
-// of D' itself (nz * nv words per staged word), and of the valid set, rather
-// than one word of a dilated copy that a kernel of its own brings up to date
-// every iteration.
+// of D' itself (nz * nv words per staged word), rather than one word of a
+// dilated copy that a kernel of its own brings up to date every iteration.
 inline bool reads_windows_directly(const GridInfo& g, const PlanRecord& pl) {
-    // Offsets into the dilated copies (SliceRep::off, ylev) are 32-bit.
-    if (dilated_words(g, pl.dil, pl.ylevels) >= 0xFFFFFFFFull) return true;
+    if (!dilated_offsets_fit(g, pl.dil, pl.ylevels)) return true;
     return pl.rep_rows <= 4 * pl.reps && (pl.rep_rows - pl.reps) * g.sw * 4ull <= 32ull << 20;
 }
 
@@ -295,7 +298,7 @@ struct FusedFixArgs {
     const uint32_t* nreps;     // [slices]
     uint32_t pass;             // representatives whose records and changed rows are in shared memory at a time
     uint32_t sat_threads;      // threads per block
-    uint32_t direct;           // 1: windows are read from D' and the valid set themselves, 0: from dzw and vzw
+    uint32_t direct;           // 1: D' windows are read from D' itself, 0: from dzw
     bword* dzw;                // (y, theta, v)-dilated copies of D' (DilateTile), brought up to date each iteration
     uint32_t ylev[kYLevels];   // word offset of each y level in dzw
     DilateTile tile;
@@ -304,7 +307,7 @@ struct FusedFixArgs {
                                // iteration k reads [k & 1] and writes the other
     uint32_t rl_words;         // slices * W1 + 1
     // When validity is more than safety:
-    const bword* vzw;          // the dilated copies of the valid set (not with direct, which reads validb)
+    const bword* vzw;          // the dilated copies of the valid set (or null with direct: validb itself is read)
     const uint32_t* needv;     // [slices][M][W1] bit per representative and row: some state's box may hold no
                                // valid cell
     DilateArgs dil;
