@@ -793,7 +793,7 @@ int problem_plan(gsc_problem* p) {
         if (admitted > kFusedSmemMax) fused_ok = false;
         p->direct = reads_windows_directly(g, pl);
         p->pass = fused_pass(g, pl.slice_reps);
-        p->sat_threads = fused_sat_threads(g, pl.slice_reps);
+        p->shape = slice_shape(g, pl.slice_reps);
         p->tile = dilate_tile_of(g, pl.dil, pl.ylevels);
         uint32_t rank = 0;
         for (uint32_t l = 0; l < static_cast<uint32_t>(kYLevels); ++l)
@@ -995,7 +995,7 @@ FusedFixArgs fused_args(const gsc_problem* p, cudaGraphConditionalHandle cond, i
     a.reps = p->reps;
     a.nreps = p->nreps;
     a.pass = p->pass;
-    a.sat_threads = p->sat_threads;
+    a.shape = p->shape;
     a.direct = p->direct ? 1u : 0u;
     a.dzw = p->dzw;
     a.rowlost = p->rowlost;
@@ -1113,7 +1113,7 @@ int gsc_problem_create(gsc_context* ctx, const gsc_abstraction* abs, const gsc_q
     p->timings.method = p->method;
     if (p->method == GSC_METHOD_FUSED) {
         p->timings.max_reps = p->max_reps;
-        p->timings.sat_threads = p->sat_threads;
+        p->timings.sat_threads = p->shape.threads;
     }
     *out = p.release();
     return GSC_OK;

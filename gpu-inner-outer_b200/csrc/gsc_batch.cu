@@ -54,7 +54,7 @@ std::vector<BatchClass> batch_classes(const std::vector<const gsc_problem*>& pro
         BatchClass& c = out.back();
         c.end = k + 1;
         c.tasks += p->g.slices;
-        c.smem = std::max(c.smem, fused_smem_bytes(p->g, p->pass));
+        c.smem = std::max(c.smem, fused_smem_bytes(p->g, p->pass, p->g.n[1]));
     }
     return out;
 }

@@ -11,9 +11,10 @@
 // valid cell already reachable) and, when validity is more than safety, at
 // least one valid cell.
 //
-// One iteration is one launch: k_slice, one block per (theta, v) slice, tests
-// every active state of the slice against the slice's representative inputs
-// and updates the slice (slice_task); its last block applies the stop rules.
+// One iteration is one launch: k_slice, one block per (theta, v) slice (or part
+// of its rows, where slices are few), tests every active state of the slice
+// against the slice's representative inputs and updates the slice (slice_task);
+// its last block applies the stop rules.
 // Where the boxes' (theta, v) windows are wide, k_dilate first brings the
 // dilated copies of D' up to date, and k_slice reads one word of those in
 // place of a window of D'.
@@ -35,7 +36,7 @@ inline unsigned int blocks_for(uint64_t n, int threads) {
 using namespace fused;
 
 // Most threads of a satisfaction block: at most kSliceThreadsMax at 48
-// registers (40 warps an SM), or, where few slices share an SM,
+// registers (40 warps an SM), or, where few slices share an SM (wide),
 // kSliceThreadsWide at 64 (32 warps).
 constexpr uint32_t kSliceThreadsMax = 256, kSliceThreadsWide = 512;
 
@@ -258,8 +259,8 @@ __global__ void __launch_bounds__(256) k_need_valid(const __grid_constant__ Grid
     }
 }
 
-// One block per (theta, v) slice (slice_task); a sharded solve launches the
-// shard's slices only.  The last block to finish applies the stop rules
+// One block per (theta, v) slice (slice_task), or per part of its rows with WIDE
+// (blockIdx.y); a sharded solve launches the shard's slices only.  The last block to finish applies the stop rules
 // (reachability.hpp:133-144), except in a sharded solve.
 template <int W, int SHARED, int DIRECT, bool WIDE>
 __global__ void __launch_bounds__(WIDE ? kSliceThreadsWide : kSliceThreadsMax, WIDE ? 2 : 5)
@@ -267,11 +268,13 @@ __global__ void __launch_bounds__(WIDE ? kSliceThreadsWide : kSliceThreadsMax, W
     extern __shared__ __align__(16) bword smem[];
     __shared__ uint32_t s_meta[3];
     FixControl* fc = a.fc;
-    const int done = slice_task<W, SHARED, DIRECT, false, true>(g, a, blockIdx.x + a.shard_begin, smem, s_meta);
+    const int done =
+        slice_task<W, SHARED, DIRECT, false, true, WIDE>(g, a, blockIdx.x + a.shard_begin, blockIdx.y, smem, s_meta);
     if (!done) {
         // Already stopped (e.g. max_iterations == 0): the graph loop must still end.
-        if (a.use_cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(a.cond, 0u);
-        if (a.mirror && blockIdx.x == 0 && threadIdx.x == 0) write_mirror(a.mirror, fc);
+        const bool first = blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0;
+        if (a.use_cond && first) cudaGraphSetConditional(a.cond, 0u);
+        if (a.mirror && first) write_mirror(a.mirror, fc);
         return;
     }
     if (a.shard_slices) return;
@@ -282,7 +285,7 @@ __global__ void __launch_bounds__(WIDE ? kSliceThreadsWide : kSliceThreadsMax, W
     if (done == 2) __syncthreads();
     if (threadIdx.x != 0) return;
     if (done == 2) __threadfence();
-    if (atomicAdd(&fc->ticket, 1u) != gridDim.x - 1) return;
+    if (atomicAdd(&fc->ticket, 1u) != gridDim.x * gridDim.y - 1) return;
     __threadfence();
     fc->ticket = 0;
     const uint32_t it = __ldcg(&fc->iter) + 1;
@@ -308,13 +311,13 @@ cudaError_t launch_slice_v(const GridInfo& g, const FusedFixArgs& a, cudaStream_
     const cudaError_t e = allow_smem(k_slice<W, SHARED, DIRECT, WIDE>);
     if (e != cudaSuccess) return e;
     const uint32_t slices = a.shard_slices ? a.shard_slices : g.slices;
-    return launch_pdl(k_slice<W, SHARED, DIRECT, WIDE>, dim3(slices), dim3(a.sat_threads), fused_smem_bytes(g, a.pass),
-                      st, g, a);
+    return launch_pdl(k_slice<W, SHARED, DIRECT, WIDE>, dim3(slices, WIDE ? a.shape.parts(g.n[1]) : 1u),
+                      dim3(a.shape.threads), fused_smem_bytes(g, a.pass, a.shape.part_rows), st, g, a);
 }
 
 template <int W, int SHARED, int DIRECT>
 cudaError_t launch_slice_t(const GridInfo& g, const FusedFixArgs& a, cudaStream_t st) {
-    return a.sat_threads > kSliceThreadsMax ? launch_slice_v<W, SHARED, DIRECT, true>(g, a, st)
+    return a.shape.wide ? launch_slice_v<W, SHARED, DIRECT, true>(g, a, st)
                                             : launch_slice_v<W, SHARED, DIRECT, false>(g, a, st);
 }
 
@@ -326,15 +329,38 @@ cudaError_t launch_slice_w(const GridInfo& g, const FusedFixArgs& a, cudaStream_
 
 }  // namespace
 
-uint32_t fused_sat_threads(const GridInfo& g, uint32_t slice_reps) {
+SliceShape slice_shape(const GridInfo& g, uint32_t slice_reps) {
+    SliceShape s{};
+    s.part_rows = g.n[1];
+    const uint64_t items = static_cast<uint64_t>(g.n[1]) * std::max(1u, slice_reps);
+    // Few slices with much to test each: parts of at least 16 rows, two a slice
+    // or as many as give two blocks an SM, and about 750 threads an SM in all.
+    // Measured, us a solve with one block a slice and so: 16x400x12x6 57.7 and
+    // 53.6, 16x1000x8x4 57.6 and 47.1, 48x48x16x8 x 192 inputs 189 and 156,
+    // 60x60x30x10 x 36 1,477 and 1,379, 100x100x30x10 x 36 1,590 and 1,495.  But
+    // with little to test (100x100x20x12, 4 representatives) 357 and 363 in two
+    // parts, and above 300 slices (47x83x29x17) 439 and 460.
+    if (g.slices <= 300 && items * g.W > 2048) {
+        const uint32_t parts = std::max(2u, 288u / g.slices);
+        s.part_rows = std::min(g.n[1], std::max(16u, ((g.n[1] + parts - 1) / parts + 7) & ~7u));
+    }
+    if (s.part_rows < g.n[1]) {
+        s.wide = 1;
+        const uint64_t blocks = static_cast<uint64_t>(g.slices) * s.parts(g.n[1]);
+        const uint64_t each = static_cast<uint64_t>(s.part_rows) * std::max(1u, slice_reps);
+        s.threads = static_cast<uint32_t>(
+            std::min<uint64_t>({384, (110000 / blocks + 31) & ~uint64_t(31), (each + 31) & ~uint64_t(31)}));
+        return s;
+    }
     // A packed row of the slice per thread, for several representatives side
     // by side.  As wide as lets every slice's block be resident at once (a
     // second wave of a few blocks doubles an iteration), and at least 128.
     const uint32_t per_sm = (g.slices + 147) / 148;
     uint32_t most = per_sm <= 2 ? kSliceThreadsWide / per_sm * 2 : per_sm <= 10 ? 40 / per_sm * 32 : 128;
     most = std::min(per_sm <= 2 ? kSliceThreadsWide : kSliceThreadsMax, std::max(128u, most));
-    const uint64_t items = static_cast<uint64_t>(g.n[1]) * std::max(1u, slice_reps);
-    return static_cast<uint32_t>(std::min<uint64_t>(most, (items + 31) & ~31ull));
+    s.threads = static_cast<uint32_t>(std::min<uint64_t>(most, (items + 31) & ~31ull));
+    s.wide = s.threads > kSliceThreadsMax;
+    return s;
 }
 
 size_t fused_admission_bytes(const GridInfo& g, int need_valid, uint32_t max_reps) {
@@ -349,10 +375,11 @@ size_t fused_admission_bytes(const GridInfo& g, int need_valid, uint32_t max_rep
     return static_cast<size_t>(sizeof(bword) * std::max(words, bulk));
 }
 
-size_t fused_smem_bytes(const GridInfo& g, uint32_t pass) {
+size_t fused_smem_bytes(const GridInfo& g, uint32_t pass, uint32_t rows) {
     const uint64_t w1 = (g.n[1] + 31) / 32;
-    return sizeof(bword) * static_cast<size_t>(
-                               (8ull * pass + g.sw + pass * w1 + 2 * w1 + kHitNotes * (g.W + 1) + (g.n[1] <= kPackedRows ? (g.n[1] + 1) / 2 : 0) + 3) & ~3ull);
+    const uint64_t words = 8ull * pass + static_cast<uint64_t>(rows) * g.W + (pass + 2) * w1 + kHitNotes * (g.W + 1) +
+                           (rows <= kPackedRows ? (rows + 1) / 2 : 0);
+    return sizeof(bword) * static_cast<size_t>((words + 3) & ~3ull);
 }
 
 uint32_t fused_pass(const GridInfo& g, uint32_t slice_reps) {

@@ -423,12 +423,13 @@ __device__ __forceinline__ void window_rows(const GridInfo& g, const bword* cur,
     }
 }
 
-// One (theta, v) slice of one iteration, by one group: the satisfaction test
-// of every active state against every representative input, the lowest
-// satisfied input, and the state update.  A slice's states are updated by
-// its own group alone and D' is double-buffered (this iteration reads
-// dp[iter & 1] and writes its slice of the other), so the update needs no
-// further kernel, and an iteration is one launch (two with the dilation).
+// One (theta, v) slice of one iteration, or with PARTS one part of its rows
+// (SliceShape::part_rows), by one group: the satisfaction test of every active
+// state against every representative input, the lowest satisfied input, and
+// the state update.  A row's states are updated by its own group alone and D'
+// is double-buffered (this iteration reads dp[iter & 1] and writes its rows of
+// the other), so the update needs no further kernel, and an iteration is one
+// launch (two with the dilation).
 //
 // A thread takes a row of the slice and every kpar-th of its representatives
 // (launch_slice_reps).  For each, F = D' ORed over the box's y, theta and v
@@ -451,7 +452,7 @@ __device__ __forceinline__ void window_rows(const GridInfo& g, const bword* cur,
 // lost one are recorded for the next iteration.
 //
 // Bound: latency and issue, with every slice's block resident at once
-// (fused_sat_threads).  Rows are read from L2 straight into registers: staged
+// (slice_shape).  Rows are read from L2 straight into registers: staged
 // in shared memory in chunks of representatives (bulk copies on an mbarrier,
 // double-buffered, or OR-ed there), three block barriers a chunk and 45 M warp
 // instructions took 85 us an iteration on the published demo; so, 16 M take
@@ -465,13 +466,16 @@ __device__ __forceinline__ void window_rows(const GridInfo& g, const bword* cur,
 // the whole group.  s_meta: [0] iteration | incremental << 31, or all ones once
 // stopped, [1] rows packed, [2] hits noted.  SHARED: the slice has one x / y plane (xy_plane); DIRECT: as
 // a.direct; 2 = decided at run time.
-template <int W, int SHARED, int DIRECT, bool WARP, bool PDL>
-__device__ __forceinline__ int slice_task(const GridInfo& g, const FusedFixArgs& a, uint32_t slice, bword* smem,
-                                           uint32_t* s_meta) {
+template <int W, int SHARED, int DIRECT, bool WARP, bool PDL, bool PARTS>
+__device__ __forceinline__ int slice_task(const GridInfo& g, const FusedFixArgs& a, uint32_t slice, uint32_t part,
+                                           bword* smem, uint32_t* s_meta) {
     const uint32_t n0 = g.n[0], n1 = g.n[1], n2 = g.n[2];
     const uint32_t sw = g.sw, W1 = (n1 + 31) / 32;
+    // Rows [y0, y0 + np1), whose row-lost bits are in the words from yw0 on.
+    const uint32_t y0 = PARTS ? part * a.shape.part_rows : 0u, np1 = PARTS ? min(a.shape.part_rows, n1 - y0) : n1;
+    const uint32_t yw0 = PARTS ? y0 >> 5 : 0u, W1p = PARTS ? ((y0 + np1 + 31) >> 5) - yw0 : W1;
     const uint32_t i2 = slice % n2, i3 = slice / n2;
-    const uint64_t wbase = static_cast<uint64_t>(slice) * sw;
+    const uint64_t wbase = static_cast<uint64_t>(slice) * sw + y0 * W;   // of row y0
     const uint32_t tid = WARP ? (threadIdx.x & 31u) : threadIdx.x;
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t bd = WARP ? 32u : blockDim.x;
@@ -479,18 +483,18 @@ __device__ __forceinline__ int slice_task(const GridInfo& g, const FusedFixArgs&
     const bool direct = DIRECT == 2 ? a.direct != 0 : DIRECT == 1;
     const uint32_t pass = a.pass;
     uint4* reps = reinterpret_cast<uint4*>(smem);            // [pass][2] SliceRep
-    bword* hits = smem + 8 * pass;                           // [sw] states satisfied now
-    uint32_t* rowchg = hits + sw;                            // [pass][W1]
-    uint32_t* lostown = rowchg + pass * W1;                  // [W1] rows of this slice that lost a cell
-    uint32_t* lostnew = lostown + W1;                        // [W1] that lose one now
-    uint32_t* notes = lostnew + W1;                          // [kHitNotes][W + 1] hits: row | representative << 16, states
-    uint16_t* rows = reinterpret_cast<uint16_t*>(notes + kHitNotes * (W + 1));   // [n1] rows with an active state, up to kPackedRows
+    bword* hits = smem + 8 * pass;                           // [np1 * W] states satisfied now
+    uint32_t* rowchg = hits + np1 * W;                        // [pass][W1]
+    uint32_t* lostown = rowchg + pass * W1;                  // [W1p] rows of this slice that lost a cell
+    uint32_t* lostnew = lostown + W1p;                       // [W1p] that lose one now
+    uint32_t* notes = lostnew + W1p;                         // [kHitNotes][W + 1] hits: row | representative << 16, states
+    uint16_t* rows = reinterpret_cast<uint16_t*>(notes + kHitNotes * (W + 1));   // [np1] rows with an active state, up to kPackedRows
 
     // Tables that no iteration changes, before waiting for the last one.
     const uint32_t nrep = a.nreps[slice];
     const uint4* list = reinterpret_cast<const uint4*>(a.reps) + static_cast<uint64_t>(slice) * g.M * 2;
     for (uint32_t r = tid; r < 2 * min(pass, nrep); r += bd) reps[r] = list[r];
-    for (uint32_t e = tid; e < sw; e += bd) hits[e] = 0;
+    for (uint32_t e = tid; e < np1 * W; e += bd) hits[e] = 0;
     if (tid == 0) s_meta[1] = s_meta[2] = 0;
     group_sync<WARP>();
     if (PDL) pdl_wait();
@@ -503,12 +507,12 @@ __device__ __forceinline__ int slice_task(const GridInfo& g, const FusedFixArgs&
     }
     // The rows with an active state, packed (in no particular order), so that
     // every thread of the group has as many items.
-    const bool packed = n1 <= kPackedRows;
+    const bool packed = np1 <= kPackedRows;
     int any = 0;
-    for (uint32_t y0 = tid & ~31u; y0 < n1; y0 += bd) {
-        const uint32_t y = y0 + lane;
+    for (uint32_t yb = tid & ~31u; yb < np1; yb += bd) {
+        const uint32_t y = yb + lane;   // (from y0)
         bword v[W], o = 0;
-        if (y < n1) {
+        if (y < np1) {
             load_row<W>(v, a.active + wbase + y * W);
 #pragma unroll
             for (int w = 0; w < W; ++w) o |= v[w];
@@ -550,8 +554,8 @@ __device__ __forceinline__ int slice_task(const GridInfo& g, const FusedFixArgs&
         }
     };
     if (it) changed_rows(min(pass, nrep));
-    for (uint32_t e = tid; e < W1; e += bd) {
-        lostown[e] = it ? rl[static_cast<uint64_t>(slice) * W1 + e] : 0u;
+    for (uint32_t e = tid; e < W1p; e += bd) {
+        lostown[e] = it ? rl[static_cast<uint64_t>(slice) * W1 + yw0 + e] : 0u;
         lostnew[e] = 0;
     }
     any = group_sync_or<WARP>(any);
@@ -559,7 +563,7 @@ __device__ __forceinline__ int slice_task(const GridInfo& g, const FusedFixArgs&
     if (ctl == 0xFFFFFFFFu) return 0;
     const bool incremental = (ctl >> 31) != 0;
     // Threads = rows x kpar; a group smaller than the rows strides over them.
-    const uint32_t nrows = packed ? s_meta[1] : n1;
+    const uint32_t nrows = packed ? s_meta[1] : np1;
     const uint32_t kpar = any && nrows < bd ? bd / nrows : 1u;
     const uint32_t kk = any && nrows < bd ? tid / nrows : 0u;
     unsigned long long ntest = 0;
@@ -576,9 +580,9 @@ __device__ __forceinline__ int slice_task(const GridInfo& g, const FusedFixArgs&
             }
         }
         for (uint32_t row = tid - kk * nrows; row < nrows && kk < kpar; row += bd) {
-            const uint32_t i1 = packed ? rows[row] : row;
+            const uint32_t ir = packed ? rows[row] : row, i1 = y0 + ir;
             bword open[W], anyo = 0;
-            load_row<W>(open, a.active + wbase + i1 * W);
+            load_row<W>(open, a.active + wbase + ir * W);
             uint32_t states = 0;
 #pragma unroll
             for (int w = 0; w < W; ++w) {
@@ -664,11 +668,11 @@ __device__ __forceinline__ int slice_task(const GridInfo& g, const FusedFixArgs&
                 const uint32_t at = atomicAdd(s_meta + 2, 1u);
                 if (at < kHitNotes) {
                     uint32_t* note = notes + at * (W + 1);
-                    note[0] = i1 | (k << 16);
+                    note[0] = ir | (k << 16);
 #pragma unroll
                     for (int w = 0; w < W; ++w) note[1 + w] = sm[w];
                 } else {
-                    take_hits<W>(a, (static_cast<uint64_t>(slice) * n1 + i1) * n0, rp.x, hits + i1 * W, sm);
+                    take_hits<W>(a, (static_cast<uint64_t>(slice) * n1 + i1) * n0, rp.x, hits + ir * W, sm);
                 }
                 anyo = 0;
                 states = 0;
@@ -688,12 +692,12 @@ __device__ __forceinline__ int slice_task(const GridInfo& g, const FusedFixArgs&
             const uint32_t n = min(s_meta[2], kHitNotes);
             for (uint32_t e = tid; e < n; e += bd) {
                 const uint32_t* note = notes + e * (W + 1);
-                const uint32_t i1 = note[0] & 0xFFFFu;
+                const uint32_t ir = note[0] & 0xFFFFu;
                 bword sm[W];
 #pragma unroll
                 for (int w = 0; w < W; ++w) sm[w] = note[1 + w];
-                take_hits<W>(a, (static_cast<uint64_t>(slice) * n1 + i1) * n0, reps[2 * (note[0] >> 16)].x, hits + i1 * W,
-                             sm);
+                take_hits<W>(a, (static_cast<uint64_t>(slice) * n1 + y0 + ir) * n0, reps[2 * (note[0] >> 16)].x,
+                             hits + ir * W, sm);
             }
             group_sync<WARP>();
             if (tid == 0) s_meta[2] = 0;
@@ -701,7 +705,7 @@ __device__ __forceinline__ int slice_task(const GridInfo& g, const FusedFixArgs&
             // from the active set: `hits` may be written at once by a thread of
             // a pass while another, with a lower input, begins the same row.
             if (p0 + pass < nrep) {
-                for (uint32_t e = tid; e < n1 * W; e += bd)
+                for (uint32_t e = tid; e < np1 * W; e += bd)
                     if (hits[e]) a.active[wbase + e] &= ~hits[e];
             }
         }
@@ -710,10 +714,10 @@ __device__ __forceinline__ int slice_task(const GridInfo& g, const FusedFixArgs&
     bword* next = odd ? a.dp[0] : a.dp[1];
     unsigned long long nr = 0, nc = 0;
     const uint32_t step = it + 1;
-    for (uint32_t e = tid; e < n1 * W; e += bd) {
-        const uint32_t y = e / W, yb = 1u << (y & 31);
+    for (uint32_t e = tid; e < np1 * W; e += bd) {
+        const uint32_t y = y0 + e / W, yw = (y >> 5) - yw0, yb = 1u << (y & 31);
         const bword h = hit_any ? hits[e] : 0u;
-        if (!h && !(lostown[y >> 5] & yb)) continue;
+        if (!h && !(lostown[yw] & yb)) continue;
         const bword d = cur[wbase + e];
         next[wbase + e] = d & ~h;
         if (!h) continue;
@@ -723,13 +727,21 @@ __device__ __forceinline__ int slice_task(const GridInfo& g, const FusedFixArgs&
         nr += __popc(fresh);
         nc += __popc(h & ~d);
         if (fresh) {
-            atomicOr(lostnew + (y >> 5), yb);
-            const uint64_t srow = (static_cast<uint64_t>(slice) * n1 + y) * n0 + (e - y * W) * kBits;
+            atomicOr(lostnew + yw, yb);
+            const uint64_t srow = (static_cast<uint64_t>(slice) * n1 + y) * n0 + (e % W) * kBits;
             for (bword m = fresh; m; m &= m - 1) a.reach_step[srow + __ffs(m) - 1] = step;
         }
     }
     if (hit_any) group_sync<WARP>();
-    for (uint32_t e = tid; e < W1; e += bd) rlnext[static_cast<uint64_t>(slice) * W1 + e] = lostnew[e];
+    if (PARTS) {
+        // A part's rows are whole bytes of the row-lost words, the last part's to the end.
+        uint8_t* bytes = reinterpret_cast<uint8_t*>(rlnext + static_cast<uint64_t>(slice) * W1);
+        const uint32_t end = y0 + np1 == n1 ? 4 * W1 : (y0 + np1) >> 3;
+        for (uint32_t e = (y0 >> 3) + tid; e < end; e += bd)
+            bytes[e] = static_cast<uint8_t>(lostnew[(e >> 2) - yw0] >> (8 * (e & 3u)));
+    } else {
+        for (uint32_t e = tid; e < W1; e += bd) rlnext[static_cast<uint64_t>(slice) * W1 + e] = lostnew[e];
+    }
     if (any) {   // else nothing was tested
         unsigned long long* row = a.stats + kStatsCols * step;
         for (int off = 16; off > 0; off >>= 1) ntest += __shfl_down_sync(0xFFFFFFFFu, ntest, off);
@@ -828,7 +840,7 @@ __device__ __forceinline__ void batch_slices(const InstanceDesc* __restrict__ de
             stopped = __ldcg(&sd.a.fc->stop) != 0;
         }
         if (stopped) continue;
-        const int done = slice_task<W, 2, 2, WARP, false>(sd.g, sd.a, t - wl.sat_off[k], smem, s_meta);
+        const int done = slice_task<W, 2, 2, WARP, false, false>(sd.g, sd.a, t - wl.sat_off[k], 0, smem, s_meta);
         // The counters are atomics; the barrier orders the group's before its
         // first thread's fence (cumulative) and ticket.
         group_sync<WARP>();

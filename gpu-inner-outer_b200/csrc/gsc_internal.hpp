@@ -144,7 +144,8 @@ struct gsc_problem {
     uint32_t max_reps = 0;      // most representative accelerations of one omega column
     gsc_b200::SliceRep* reps = nullptr;
     uint32_t* nreps = nullptr;
-    uint32_t pass = 1, sat_threads = 128;   // of the satisfaction kernel (FusedFixArgs)
+    uint32_t pass = 1;                  // of the satisfaction kernel (FusedFixArgs)
+    gsc_b200::SliceShape shape{};
     uint32_t* needv = nullptr;
     bool direct = false;        // D' windows are read from D' itself
     bool copies_optional = true;   // also where memory lacks for dilated copies (else that is an error)

@@ -278,6 +278,14 @@ struct __align__(16) SliceRep {
     uint32_t hx, hy, yr, xr;
 };
 
+// Launch shape of k_slice: threads a block, rows of a slice a block takes (a
+// multiple of 8, or all of them), and whether it is the kernel for few slices
+// (more registers a thread; the only one that splits slices).
+struct SliceShape {
+    uint32_t threads, part_rows, wide;
+    uint32_t parts(uint32_t n1) const { return (n1 + part_rows - 1) / part_rows; }
+};
+
 struct FusedFixArgs {
     const uint32_t *xt, *yt;
     const bword* validb;
@@ -297,7 +305,7 @@ struct FusedFixArgs {
     const SliceRep* reps;      // [slices][M]: each slice's representatives, in input order
     const uint32_t* nreps;     // [slices]
     uint32_t pass;             // representatives whose records and changed rows are in shared memory at a time
-    uint32_t sat_threads;      // threads per block
+    SliceShape shape;          // of k_slice
     uint32_t direct;           // 1: D' windows are read from D' itself, 0: from dzw
     bword* dzw;                // (y, theta, v)-dilated copies of D' (DilateTile), brought up to date each iteration
     uint32_t ylev[kYLevels];   // word offset of each y level in dzw
@@ -333,10 +341,9 @@ size_t fused_admission_bytes(const GridInfo& g, int need_valid, uint32_t max_rep
 constexpr uint32_t kPackedRows = 8192;   // more rows a slice than this are all tested
 constexpr uint32_t kHitNotes = 384;      // (row, representative) hits noted at a time
 uint32_t fused_pass(const GridInfo& g, uint32_t slice_reps);
-size_t fused_smem_bytes(const GridInfo& g, uint32_t pass);
+size_t fused_smem_bytes(const GridInfo& g, uint32_t pass, uint32_t rows);
 DilateTile dilate_tile_of(const GridInfo& g, const DilateArgs& d, uint32_t levels);
-// Threads per block for a problem.
-uint32_t fused_sat_threads(const GridInfo& g, uint32_t slice_reps);
+SliceShape slice_shape(const GridInfo& g, uint32_t slice_reps);
 // Dilated copies of src into dst.  With fc and rowlost (during a fixpoint,
 // after its first iteration) only tiles whose windows hold a row that lost a
 // D' cell are recomputed, and src is src0 or src1 by the iteration's parity.

@@ -3,7 +3,7 @@
 // state:
 //   slice_check <order seed: 0 ascending, 1 descending, else shuffled> <seed>
 //               <rows> <x cells> <inputs> <inputs a pass> <group: 32 = a warp>
-//               <hits: 1 = no input of the first pass hits, all later do> <valid test>
+//               <hits: 1 = no input of the first pass hits, all later do> <valid test> <rows a block>
 // Prints the first difference and returns 1.
 #include <random>
 
@@ -156,6 +156,7 @@ int check(int argc, char** argv) {
     a.nreps = nreps.data();
     a.pass = pass;
     a.direct = 1;
+    a.shape.part_rows = argc > 10 ? std::atoi(argv[10]) : n1;
     a.rowlost = rowlost.data();
     a.rl_words = g.slices * W1 + 1;
     a.needv = needv.data();
@@ -167,11 +168,12 @@ int check(int argc, char** argv) {
     for (uint32_t i = 0; i < threads; ++i) order[i] = order_seed == 1 ? threads - 1 - i : i;
     std::mt19937_64 shuffle(order_seed);
     if (order_seed > 1) std::shuffle(order.begin(), order.end(), shuffle);
-    const bool ended = emu::run_block(threads, order, [&] {
+    bool ended = true;
+    for (uint32_t part = 0; ended && part < a.shape.parts(n1); ++part) ended = emu::run_block(threads, order, [&] {
         if (threads == 32)
-            fused::slice_task<W, 1, 1, true, false>(g, a, slice, reinterpret_cast<bword*>(smem.data()), meta);
+            fused::slice_task<W, 1, 1, true, false, false>(g, a, slice, 0, reinterpret_cast<bword*>(smem.data()), meta);
         else
-            fused::slice_task<W, 1, 1, false, false>(g, a, slice, reinterpret_cast<bword*>(smem.data()), meta);
+            fused::slice_task<W, 1, 1, false, false, true>(g, a, slice, part, reinterpret_cast<bword*>(smem.data()), meta);
     });
     if (!ended) {
         std::printf("the threads wait for one another\n");
@@ -188,6 +190,16 @@ int check(int argc, char** argv) {
     if (!same) {
         std::printf("the sets differ\n");
         return 1;
+    }
+    // The rows that lost a cell, and nothing past the last.
+    for (uint32_t y = 0; y < 32 * W1; ++y) {
+        bool lost = false;
+        for (uint32_t w = 0; y < n1 && w < W; ++w)
+            lost |= D[slice * g.sw + y * W + w] != reinterpret_cast<const bword*>(wantD.data())[slice * g.sw + y * W + w];
+        if (((rowlost[a.rl_words + slice * W1 + y / 32] >> (y % 32)) & 1u) != lost) {
+            std::printf("row %u is recorded wrongly\n", y);
+            return 1;
+        }
     }
     std::printf("ok %llu\n", static_cast<unsigned long long>(hits));
     return 0;

@@ -65,6 +65,17 @@ def test_valid_cells_of_windows_read_directly(slice_check, seed, rows, cells, in
     assert run(slice_check, seed, seed, rows, cells, inputs, per_pass, threads, 0, 1) > 0
 
 
+@pytest.mark.parametrize("order", range(3))
+@pytest.mark.parametrize("rows,cells,inputs,per_pass,threads,block_rows", [
+    (70, 40, 24, 8, 256, 16), (70, 40, 24, 8, 256, 24), (33, 20, 24, 24, 64, 8), (64, 33, 24, 8, 128, 32),
+    (9, 20, 24, 8, 64, 8), (64, 40, 24, 8, 128, 40),
+])
+def test_rows_of_a_slice_in_several_blocks(slice_check, order, rows, cells, inputs, per_pass, threads, block_rows):
+    """Blocks of whole bytes of row-lost bits, the last one shorter: each
+    updates its rows alone and records them, and no other's."""
+    assert run(slice_check, order, 2, rows, cells, inputs, per_pass, threads, 0, order % 2, block_rows) > 0
+
+
 @pytest.fixture(scope="module")
 def batch_check(tmp_path_factory):
     return compiled(tmp_path_factory, "batch_check")
