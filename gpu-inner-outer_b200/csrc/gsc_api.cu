@@ -791,7 +791,7 @@ int problem_plan(gsc_problem* p) {
         if (static_cast<uint64_t>(pl.dil.nk) * pl.dil.nl * g.rows * g.W >= 0xFFFFFFFFull) fused_ok = false;
         const size_t admitted = fused_admission_bytes(g, p->need_valid, p->max_reps);
         if (admitted > kFusedSmemMax) fused_ok = false;
-        p->direct = reads_windows_directly(g, pl);
+        p->direct = reads_windows_directly(g, pl, p->batched && !is_big_instance(g));
         p->pass = fused_pass(g, pl.slice_reps);
         p->shape = slice_shape(g, pl.slice_reps);
         p->tile = dilate_tile_of(g, pl.dil, pl.ylevels);

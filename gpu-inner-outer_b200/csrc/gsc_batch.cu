@@ -487,6 +487,7 @@ int batch_begin(gsc_batch* b, uint32_t count, const gsc_model_desc* models, cons
         p->pool = b->pool;
         p->stream = ss.of(i);
         p->method = GSC_METHOD_FUSED;
+        p->batched = true;
         p->hplan = b->hplans + i;
         p->hplan_dev = b->hplans_dev + i;
         const int s = problem_stage1(p.get(), &queries[i]);

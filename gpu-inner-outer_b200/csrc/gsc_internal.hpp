@@ -148,6 +148,7 @@ struct gsc_problem {
     gsc_b200::SliceShape shape{};
     uint32_t* needv = nullptr;
     bool direct = false;        // D' windows are read from D' itself
+    bool batched = false;       // an instance of a batch or a server
     bool copies_optional = true;   // also where memory lacks for dilated copies (else that is an error)
     gsc_b200::DilateTile tile{};          // else from dilated copies
     uint32_t ylev[gsc_b200::kYLevels] = {};

@@ -256,9 +256,26 @@ inline bool dilated_offsets_fit(const GridInfo& g, const DilateArgs& d, uint32_t
 // Whether the satisfaction test reads a representative's (theta, v) window
 // of D' itself (nz * nv words per staged word), rather than one word of a
 // dilated copy that a kernel of its own brings up to date every iteration.
-inline bool reads_windows_directly(const GridInfo& g, const PlanRecord& pl) {
+// Directly where the windows' further words, over all representatives, are
+// few: up to 17 MB, and up to 32 MB for windows of four cells.  Measured, us a
+// solve with copies and directly (MB): 20x20x16x10 50.0 and 43.1 (0.4);
+// hyperbolic 30x30x16x6 71 and 62 (1.2); 200x64x20x6 630 and 543 (6.2);
+// 256x40x20x10 787 and 659 (8.3); 47x83x29x17 487 and 419 (12); hyperbolic
+// 45x41x30x9 860 and 824 (14), 60x60x30x10 with obstacles 1,480 and 1,361 (16),
+// 20x20x63x13 209 and 216 (17), 80x80x30x8 1,756 and 1,912 (22), 70x70x63x13
+// 737 and 1,182 (177); 128x128x72x48 9,291 and 13,452 (725); of four cells
+// 65x65x38x25 717 and 645 (16), 128x128x40x20 1,408 and 1,200 (18), but
+// 48x48x16x8 x 192 inputs 163 and 175 (13).  With tests of few states an
+// iteration direct reads stay ahead for longer (64x64x72x48 x 36: 2,179 and
+// 1,839 at 71).
+// batched: the instances of a batch or server keep the line at four cells: the
+// dilations of all of them are one launch a step, which callers count among its
+// launches (32 small instances 7.8 ms a call so, 7.4 with the wider line; a
+// served burst's runs differ by more).
+inline bool reads_windows_directly(const GridInfo& g, const PlanRecord& pl, bool batched) {
     if (!dilated_offsets_fit(g, pl.dil, pl.ylevels)) return true;
-    return pl.rep_rows <= 4 * pl.reps && (pl.rep_rows - pl.reps) * g.sw * 4ull <= 32ull << 20;
+    const uint64_t further = (pl.rep_rows - pl.reps) * g.sw * sizeof(bword);
+    return (!batched && further <= 17ull << 20) || (pl.rep_rows <= 4 * pl.reps && further <= 32ull << 20);
 }
 
 // A representative input of a (theta, v) slice: the lowest of the inputs

@@ -148,6 +148,7 @@ bool admit(gsc_server* s) {
         p->pool = s->pool.get();
         p->stream = s->s_prep;
         p->method = GSC_METHOD_FUSED;
+        p->batched = true;
         p->hplan = s->hplans + r->slot;
         p->hplan_dev = s->hplans_dev + r->slot;
         int status = problem_stage1(p, &r->q);

@@ -1,5 +1,5 @@
 // Host rules of the fused plan, for a grid and the box widths in use:
-//   plan_check <n0> <n1> <n2> <n3> <theta widths> <v widths> <y levels (mask)> <windows a representative>
+//   plan_check <n0> <n1> <n2> <n3> <theta widths> <v widths> <y levels (mask)> <cells a window> <batched>
 // Prints whether windows are read directly, and the words of a set's dilated copies.
 #include <iostream>
 
@@ -8,7 +8,7 @@
 using namespace gsc_b200;
 
 int main(int argc, char** argv) {
-    if (argc < 9) return 2;
+    if (argc < 10) return 2;
     GridInfo g{};
     for (int d = 0; d < 4; ++d) g.n[d] = static_cast<uint32_t>(std::atoi(argv[1 + d]));
     g.W = (g.n[0] + kBits - 1) / kBits;
@@ -20,6 +20,6 @@ int main(int argc, char** argv) {
     pl.ylevels = std::atoi(argv[7]);
     pl.reps = g.slices;
     pl.rep_rows = pl.reps * std::strtoull(argv[8], nullptr, 10);
-    std::cout << reads_windows_directly(g, pl) << " " << dilated_words(g, pl.dil, pl.ylevels) << "\n";
+    std::cout << reads_windows_directly(g, pl, std::atoi(argv[9]) != 0) << " " << dilated_words(g, pl.dil, pl.ylevels) << "\n";
     return 0;
 }

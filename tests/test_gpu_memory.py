@@ -63,8 +63,8 @@ def test_fused_query_stays_within_its_bound(case):
 def test_without_room_for_the_dilated_copies():
     """Budgets a little below what the query takes otherwise: fewer launches an
     iteration, the same result."""
-    case = obstacles(hyperbolic((41, 37, 20, 8), (5, 5)))
-    case["max_iterations"] = 30
+    case = obstacles(hyperbolic((48, 40, 31, 12), (8, 8)))
+    case["max_iterations"] = 4
     want = O.solve(case)
     with G.Context(0) as c:
         c.set_memory_budget((64 << 20) - 1)   # below a full-size region of the pool

@@ -20,9 +20,24 @@ def plan_check(tmp_path_factory):
 ])
 def test_dilated_copies_stay_within_their_offsets(plan_check, shape, nk, nl, levels, windows, direct):
     """Where a set has dilated copies, every word of them has a 32-bit offset."""
-    out = subprocess.run([plan_check] + [str(v) for v in (*shape, nk, nl, levels, windows)], capture_output=True,
+    out = subprocess.run([plan_check] + [str(v) for v in (*shape, nk, nl, levels, windows, 0)], capture_output=True,
                          text=True, check=True).stdout.split()
     assert bool(int(out[0])) == direct
     words = nk * nl * bin(levels).count("1") * shape[2] * shape[3] * ((shape[1] * ((shape[0] + 31) // 32) + 3) // 4 * 4)
     assert int(out[1]) == words
     assert direct or words < 2**32
+
+
+@pytest.mark.parametrize("shape,cells,batched,direct", [
+    ((20, 20, 16, 10), 6, 0, True),       # few further words: directly, whatever the window
+    ((20, 20, 16, 10), 6, 1, False),      # beside others: windows of four cells only
+    ((20, 20, 16, 10), 4, 1, True),
+    ((65, 65, 100, 56), 5, 0, True),      # 16.7 MiB
+    ((65, 65, 100, 57), 5, 0, False),     # 17.04
+    ((65, 65, 100, 140), 4, 0, True),     # 31.4, of four cells
+    ((65, 65, 100, 150), 4, 0, False),
+])
+def test_windows_read_directly(plan_check, shape, cells, batched, direct):
+    out = subprocess.run([plan_check] + [str(v) for v in (*shape, 2, 2, 2, cells, batched)], capture_output=True,
+                         text=True, check=True).stdout.split()
+    assert bool(int(out[0])) == direct
