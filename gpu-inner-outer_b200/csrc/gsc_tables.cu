@@ -669,16 +669,28 @@ __global__ void __launch_bounds__(kThreadsReps) k_plane_reps(GridInfo g, const u
 // One block per slice (theta i2, v i3), one thread per input: a column
 // representative of k_plane_reps is one of the slice unless one of an earlier
 // column has the same theta box, v box and rows; the list is in input order.
-__global__ void __launch_bounds__(kThreadsReps) k_slice_reps(GridInfo g, const uint32_t* __restrict__ xt,
+// An input is compared with the columns of its theta box alone, which a chain
+// back from its column lists (up to kChainColumns columns; beyond, every earlier
+// column is looked at).  With one plane a slice (one substep) all columns of a
+// theta box are alike, so the first has them all.  Measured, us, with all earlier
+// columns looked at by 128 threads, and so: 24x24x12x8 x
+// 900 inputs (32 substeps) 187 and 61, 16x16x12x6 x 4,000 584 and 29,
+// 32x32x24x16 x 400 (32 substeps) 44 and 29, 65x65x38x25 x 100 9 and 9.
+constexpr uint32_t kChainColumns = 2048;
+__global__ void __launch_bounds__(1024) k_slice_reps(GridInfo g, const uint32_t* __restrict__ xt,
                                                              const uint32_t* __restrict__ yt,
                                                              const uint32_t* __restrict__ zt,
                                                              const uint32_t* __restrict__ wt,
                                                              const uint4* __restrict__ shorts,
                                                              const uint8_t* __restrict__ xrep, SliceRep* reps,
                                                              uint32_t* nreps, PlanRecord* plan) {
-    __shared__ uint32_t s_count[kThreadsReps / 32];
+    __shared__ uint32_t s_count[32];
+    __shared__ uint32_t s_z[kChainColumns], s_w[256];
+    __shared__ uint16_t s_prev[kChainColumns];   // the last earlier column with the same theta box, or kNoColumn
+    constexpr uint32_t kNoColumn = 0xFFFFu;
     const uint32_t tid = threadIdx.x, lane = tid & 31, wib = tid >> 5;
     const uint32_t n2 = g.n[2], ma = g.ma, mw = g.mw;
+    const bool chained = mw <= kChainColumns;
     uint32_t most = 0;
     unsigned long long total = 0, rows = 0;
     for (uint32_t s = blockIdx.x; s < g.slices; s += gridDim.x) {
@@ -686,20 +698,35 @@ __global__ void __launch_bounds__(kThreadsReps) k_slice_reps(GridInfo g, const u
         SliceRep* list = reps + static_cast<uint64_t>(s) * g.M;
         const uint8_t* col = xrep + (static_cast<uint64_t>(i2) * g.n[3] + i3) * g.M;
         const uint32_t *zs = zt + i2 * mw, *ws = wt + i3 * ma;
+        for (uint32_t k = tid; k < ma; k += blockDim.x) s_w[k] = ws[k];
+        for (uint32_t k = tid; chained && k < mw; k += blockDim.x) s_z[k] = zs[k];
+        __syncthreads();
+        for (uint32_t k = tid; chained && k < mw; k += blockDim.x) {
+            const uint32_t z = s_z[k];
+            uint32_t p = k;
+            while (p > 0 && s_z[p - 1] != z) --p;
+            s_prev[k] = static_cast<uint16_t>(p ? p - 1 : kNoColumn);
+        }
+        __syncthreads();
         uint32_t n = 0;
-        for (uint32_t j0 = 0; j0 < g.M; j0 += kThreadsReps) {
+        for (uint32_t j0 = 0; j0 < g.M; j0 += blockDim.x) {
             const uint32_t j = j0 + tid, jw = j / ma, ja = j - jw * ma;
             bool keep = false;
             uint32_t ze = 0, w = 0;
             if (j < g.M) {
                 ze = zs[jw];
-                w = ws[ja];
+                w = s_w[ja];
                 keep = w != kReject && col[j] == ja;
             }
-            for (uint32_t kw = 0; keep && kw < jw; ++kw) {
-                if (zs[kw] != ze) continue;
+            uint32_t kw = !keep ? kNoColumn : chained ? s_prev[jw] : jw ? jw - 1 : kNoColumn;
+            if (chained && g.xy_planes == 1) {
+                keep = keep && kw == kNoColumn;
+                kw = kNoColumn;
+            }
+            for (; keep && kw != kNoColumn; kw = chained ? s_prev[kw] : kw ? kw - 1 : kNoColumn) {
+                if (!chained && zs[kw] != ze) continue;
                 for (uint32_t ka = 0; keep && ka < ma; ++ka)
-                    if (ws[ka] == w && col[kw * ma + ka] == ka &&
+                    if (s_w[ka] == w && col[kw * ma + ka] == ka &&
                         same_rows(g, xt, yt, shorts, xy_plane(g, i2, i3, j), xy_plane(g, i2, i3, ka + ma * kw), 0, 1))
                         keep = false;
             }
@@ -707,7 +734,7 @@ __global__ void __launch_bounds__(kThreadsReps) k_slice_reps(GridInfo g, const u
             if (lane == 0) s_count[wib] = __popc(m);
             __syncthreads();
             uint32_t before = n, all = 0;
-            for (uint32_t k = 0; k < kThreadsReps / 32; ++k) {
+            for (uint32_t k = 0; k < (blockDim.x >> 5); ++k) {
                 if (k < wib) before += s_count[k];
                 all += s_count[k];
             }
@@ -840,8 +867,9 @@ cudaError_t launch_plane_reps(const GridInfo& g, const uint32_t* xt, const uint3
 cudaError_t launch_slice_reps(const GridInfo& g, const uint32_t* xt, const uint32_t* yt, const uint32_t* zt,
                               const uint32_t* wt, const uint4* shorts, const uint8_t* xrep, SliceRep* reps,
                               uint32_t* nreps, PlanRecord* plan, cudaStream_t st) {
-    k_slice_reps<<<std::min(g.slices, 148u * 16u), kThreadsReps, 0, st>>>(g, xt, yt, zt, wt, shorts, xrep, reps, nreps,
-                                                                      plan);
+    // A thread an input, up to 1,024.
+    const uint32_t threads = std::min(1024u, (g.M + kThreadsReps - 1) / kThreadsReps * kThreadsReps);
+    k_slice_reps<<<std::min(g.slices, 148u * 16u), threads, 0, st>>>(g, xt, yt, zt, wt, shorts, xrep, reps, nreps, plan);
     return cudaGetLastError();
 }
 
