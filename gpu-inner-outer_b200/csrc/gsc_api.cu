@@ -601,6 +601,14 @@ static void give_back(gsc_problem* p, T** ptr) {
     *ptr = nullptr;
 }
 
+// Words of the class records' table: every input's share without the records'
+// padding where a slice has a single plane.
+static uint64_t class_table_words(const GridInfo& g) {
+    if (g.xy_planes != 1) return table_planes(g) * class_words(g);
+    return std::max<uint64_t>(static_cast<uint64_t>(g.slices) * class_words(g),
+                              table_planes(g) * (4 + (kShiftMax + 1) * g.W));
+}
+
 // `count` elements in the part of the class records that no plane uses (a
 // slice with a single plane has its share for every input: table_planes), or
 // null where they do not fit.  So a one-substep query's lists take no memory of
@@ -610,7 +618,7 @@ static T* spare_records(gsc_problem* p, uint64_t count) {
     const uint64_t record = class_words(p->g) * sizeof(bword);
     const uint64_t at = std::max(p->xcls_used, static_cast<uint64_t>(p->g.slices) * p->g.xy_planes * record);
     const uint64_t end = at + (count * sizeof(T) + 15) / 16 * 16;
-    if (end > table_planes(p->g) * record) return nullptr;
+    if (end > class_table_words(p->g) * sizeof(bword)) return nullptr;
     p->xcls_used = end;
     return reinterpret_cast<T*>(reinterpret_cast<char*>(p->xcls) + at);
 }
@@ -724,7 +732,7 @@ int problem_stage1(gsc_problem* p, const gsc_query_desc* qd) {
     GSC_TRY(palloc(p, &p->wt, static_cast<uint64_t>(g.n[3]) * g.ma));
     GSC_TRY(palloc(p, &p->dplan, 1));
     if (p->fused_candidate) {
-        GSC_TRY(palloc(p, &p->xcls, planes * class_words(g)));
+        GSC_TRY(palloc(p, &p->xcls, class_table_words(g)));
         GSC_TRY(palloc(p, &p->xrep, planes));
         GSC_TRY(palloc(p, &p->kidx, static_cast<uint64_t>(g.n[2]) + 1));
         GSC_TRY(palloc(p, &p->lidx, static_cast<uint64_t>(g.n[3]) + 1));

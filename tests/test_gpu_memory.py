@@ -20,7 +20,7 @@ def bound(case, problem_widths, need_valid):
     S, M = int(np.prod(n)), m[0] * m[1]
     slices, W = n[2] * n[3], (n[0] + 31) // 32
     planes, words = slices * M, slices * n[1] * W
-    classes = (4 + 9 * W + 3) // 4 * 4
+    classes = 4 + 9 * W if case["integration_substeps"] == 1 else (4 + 9 * W + 3) // 4 * 4
     copies = problem_widths * words * (2 if need_valid else 1)
     safe = n[0] * n[1] if case["constraint"] != "none" else 0
     return (15 * S + 4 * (8 * words + copies) + planes * (4 * (n[0] + n[1]) + 4 * classes + 1) + safe +
@@ -42,6 +42,7 @@ def hyperbolic(n, m):
 
 
 CASES = [
+    C.unicycle_grid_case((24, 24, 16, 8), (50, 50)), C.unicycle_grid_case((16, 16, 12, 6), (250, 16)),
     C.small_case(), obstacles(C.small_case()), C.unicycle_grid_case((24, 24, 12, 8), (21, 17)),
     obstacles(C.unicycle_grid_case((24, 24, 12, 8), (21, 17))), obstacles(C.unicycle_grid_case((16, 16, 16, 16), (10, 10))),
     obstacles(C.unicycle_grid_case((17, 130, 9, 5), (3, 3))), hyperbolic((40, 40, 20, 8), (5, 5)),
