@@ -801,7 +801,8 @@ int problem_plan(gsc_problem* p) {
         if (admitted > kFusedSmemMax) fused_ok = false;
         p->direct = reads_windows_directly(g, pl, p->batched && !is_big_instance(g));
         p->pass = fused_pass(g, pl.slice_reps);
-        p->shape = slice_shape(g, pl.slice_reps);
+        p->slice_reps = pl.slice_reps;
+        p->shape = slice_shape(g, g.slices, pl.slice_reps);
         p->tile = dilate_tile_of(g, pl.dil, pl.ylevels);
         uint32_t rank = 0;
         for (uint32_t l = 0; l < static_cast<uint32_t>(kYLevels); ++l)
@@ -1003,7 +1004,7 @@ FusedFixArgs fused_args(const gsc_problem* p, cudaGraphConditionalHandle cond, i
     a.reps = p->reps;
     a.nreps = p->nreps;
     a.pass = p->pass;
-    a.shape = p->shape;
+    a.shape = p->shard_slices ? p->shard_shape : p->shape;
     a.direct = p->direct ? 1u : 0u;
     a.dzw = p->dzw;
     a.rowlost = p->rowlost;
@@ -1291,6 +1292,7 @@ int gsc_problem_shard_begin(gsc_problem* p, uint32_t slice_begin, uint32_t slice
     GSC_CU(ctx, cudaStreamSynchronize(ctx->stream));
     p->shard_begin = slice_begin;
     p->shard_slices = slice_end - slice_begin;
+    p->shard_shape = slice_shape(p->g, p->shard_slices, p->slice_reps);
     p->shard_iter = 0;
     p->shard_stopped = p->q.max_iterations == 0;
     return GSC_OK;

@@ -329,7 +329,7 @@ cudaError_t launch_slice_w(const GridInfo& g, const FusedFixArgs& a, cudaStream_
 
 }  // namespace
 
-SliceShape slice_shape(const GridInfo& g, uint32_t slice_reps) {
+SliceShape slice_shape(const GridInfo& g, uint32_t slices, uint32_t slice_reps) {
     SliceShape s{};
     s.part_rows = g.n[1];
     const uint64_t items = static_cast<uint64_t>(g.n[1]) * std::max(1u, slice_reps);
@@ -340,13 +340,13 @@ SliceShape slice_shape(const GridInfo& g, uint32_t slice_reps) {
     // 60x60x30x10 x 36 1,477 and 1,379, 100x100x30x10 x 36 1,590 and 1,495.  But
     // with little to test (100x100x20x12, 4 representatives) 357 and 363 in two
     // parts, and above 300 slices (47x83x29x17) 439 and 460.
-    if (g.slices <= 300 && items * g.W > 2048) {
-        const uint32_t parts = std::max(2u, 288u / g.slices);
+    if (slices <= 300 && items * g.W > 2048) {
+        const uint32_t parts = std::max(2u, 288u / slices);
         s.part_rows = std::min(g.n[1], std::max(16u, ((g.n[1] + parts - 1) / parts + 7) & ~7u));
     }
     if (s.part_rows < g.n[1]) {
         s.wide = 1;
-        const uint64_t blocks = static_cast<uint64_t>(g.slices) * s.parts(g.n[1]);
+        const uint64_t blocks = static_cast<uint64_t>(slices) * s.parts(g.n[1]);
         const uint64_t each = static_cast<uint64_t>(s.part_rows) * std::max(1u, slice_reps);
         s.threads = static_cast<uint32_t>(
             std::min<uint64_t>({384, (110000 / blocks + 31) & ~uint64_t(31), (each + 31) & ~uint64_t(31)}));
@@ -355,7 +355,7 @@ SliceShape slice_shape(const GridInfo& g, uint32_t slice_reps) {
     // A packed row of the slice per thread, for several representatives side
     // by side.  As wide as lets every slice's block be resident at once (a
     // second wave of a few blocks doubles an iteration), and at least 128.
-    const uint32_t per_sm = (g.slices + 147) / 148;
+    const uint32_t per_sm = (slices + 147) / 148;
     uint32_t most = per_sm <= 2 ? kSliceThreadsWide / per_sm * 2 : per_sm <= 10 ? 40 / per_sm * 32 : 128;
     most = std::min(per_sm <= 2 ? kSliceThreadsWide : kSliceThreadsMax, std::max(128u, most));
     s.threads = static_cast<uint32_t>(std::min<uint64_t>(most, (items + 31) & ~31ull));

@@ -145,7 +145,8 @@ struct gsc_problem {
     gsc_b200::SliceRep* reps = nullptr;
     uint32_t* nreps = nullptr;
     uint32_t pass = 1;                  // of the satisfaction kernel (FusedFixArgs)
-    gsc_b200::SliceShape shape{};
+    uint32_t slice_reps = 0;            // most representatives of a slice
+    gsc_b200::SliceShape shape{}, shard_shape{};
     uint32_t* needv = nullptr;
     bool direct = false;        // D' windows are read from D' itself
     bool batched = false;       // an instance of a batch or a server

@@ -360,7 +360,8 @@ constexpr uint32_t kHitNotes = 384;      // (row, representative) hits noted at 
 uint32_t fused_pass(const GridInfo& g, uint32_t slice_reps);
 size_t fused_smem_bytes(const GridInfo& g, uint32_t pass, uint32_t rows);
 DilateTile dilate_tile_of(const GridInfo& g, const DilateArgs& d, uint32_t levels);
-SliceShape slice_shape(const GridInfo& g, uint32_t slice_reps);
+// For a launch over `slices` slices of at most slice_reps representatives.
+SliceShape slice_shape(const GridInfo& g, uint32_t slices, uint32_t slice_reps);
 // Dilated copies of src into dst.  With fc and rowlost (during a fixpoint,
 // after its first iteration) only tiles whose windows hold a row that lost a
 // D' cell are recomputed, and src is src0 or src1 by the iteration's parity.
