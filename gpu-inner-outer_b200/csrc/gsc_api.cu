@@ -633,7 +633,8 @@ static int method_tables(gsc_problem* p, bool stored_ok) {
         for (bword** set : {&p->validb, &p->unsafeb, &p->srcb, &p->candb})
             if (s == GSC_OK) s = palloc(p, set, words);
         if (s == GSC_OK) s = palloc(p, &p->shorts, static_cast<uint64_t>(g.slices) * g.xy_planes);
-        if (s == GSC_OK && !(p->reps = spare_records<SliceRep>(p, table_planes(g)))) s = palloc(p, &p->reps, table_planes(g));
+        if (s == GSC_OK && !(p->reps = spare_records<SliceRep>(p, table_planes(g))))
+            s = palloc(p, &p->reps, table_planes(g));
         if (s == GSC_OK) s = palloc(p, &p->nreps, g.slices);
         if (s == GSC_OK) return s;
         for (bword** set : {&p->validb, &p->unsafeb, &p->srcb, &p->candb}) give_back(p, set);
@@ -806,7 +807,8 @@ int problem_plan(gsc_problem* p) {
         p->tile = dilate_tile_of(g, pl.dil, pl.ylevels);
         uint32_t rank = 0;
         for (uint32_t l = 0; l < static_cast<uint32_t>(kYLevels); ++l)
-            if ((p->tile.levels >> l) & 1u) p->ylev[l] = static_cast<uint32_t>(rank++ * pl.dil.nk * pl.dil.nl * g.slices * g.sw);
+            if ((p->tile.levels >> l) & 1u)
+                p->ylev[l] = static_cast<uint32_t>(rank++ * pl.dil.nk * pl.dil.nl * g.slices * g.sw);
     }
     uint32_t method = p->method;
     if (method == GSC_METHOD_AUTO) method = fused_ok ? GSC_METHOD_FUSED : (stored_ok ? GSC_METHOD_STORED : 0);
@@ -906,11 +908,9 @@ int problem_stage2(gsc_problem* p) {
     const uint64_t words = static_cast<uint64_t>(g.slices) * g.sw;
     GSC_TRY(palloc(p, &p->dp[0], words));
     GSC_TRY(palloc(p, &p->dp[1], words));
+    // Updated in place: no iteration reads another slice's reachable words (the
+    // satisfaction test reads D' only).
     GSC_TRY(palloc(p, &p->reach0, words));
-    // One reachable set, updated in place: no iteration reads another slice's
-    // reachable words (the satisfaction test reads D' only), so reach1 names
-    // the same buffer and every parity choice picks it.
-    p->reach1 = p->reach0;
     GSC_TRY(palloc(p, &p->active, words));
     const uint64_t w1 = (g.n[1] + 31) / 32;
     p->rl_words = static_cast<uint32_t>(g.slices * w1 + 1);
@@ -942,7 +942,8 @@ int problem_stage2(gsc_problem* p) {
     }
     GSC_CU(ctx, launch_rep_offsets(g, p->kidx, p->lidx, p->dil.nl, fused_args(p, 0, 0), p->reps, st));
     if (p->need_valid) {
-        if (p->vzw) GSC_CU(ctx, launch_dilate(g, p->validb, p->validb, p->vzw, p->dil, p->tile, nullptr, nullptr, 0, st));
+        if (p->vzw)
+            GSC_CU(ctx, launch_dilate(g, p->validb, p->validb, p->vzw, p->dil, p->tile, nullptr, nullptr, 0, st));
         GSC_CU(ctx, launch_need_valid(g, fused_args(p, 0, 0), rowvoid, p->reps, p->needv, st));
     }
     return GSC_OK;
@@ -998,7 +999,6 @@ FusedFixArgs fused_args(const gsc_problem* p, cudaGraphConditionalHandle cond, i
     a.reach_step = p->reach_step;
     a.fc = p->fc;
     a.stats = p->stats;
-    a.need_valid = p->need_valid;
     a.xcls = p->xcls;
     a.cls_words = class_words(p->g);
     a.reps = p->reps;
@@ -1201,9 +1201,8 @@ int gsc_problem_solve(gsc_problem* p, uint32_t flags) {
         // iteration's last kernel, no copy in the stream), so the device
         // never waits for the host, and at most kLoopAhead iterations
         // (kernels that return at once on the stop flag) run past the stop.
-        // When the stream has drained and the word shows no stop (a stop set
-        // by a bounded device wait that gave up), the record in device memory
-        // decides.
+        // When the stream has drained and the word shows no stop, the record in
+        // device memory decides.
         constexpr uint32_t kLoopAhead = 2;
         GSC_CU(ctx, loop_resources(ctx));
         volatile unsigned long long* word = ctx->loop_word;
@@ -1370,7 +1369,7 @@ int gsc_problem_read(gsc_problem* p, gsc_result* r) {
     if (r->candidate_mask) GSC_CU(ctx, cudaMemcpyAsync(r->candidate_mask, p->cand, g.S, cudaMemcpyDeviceToHost, st));
     if (r->reachable_mask) {
         if (p->method == GSC_METHOD_FUSED)
-            GSC_CU(ctx, launch_unpack_bits(g, (fc.iter & 1) ? p->reach1 : p->reach0, p->reach8, st));
+            GSC_CU(ctx, launch_unpack_bits(g, p->reach0, p->reach8, st));
         GSC_CU(ctx, cudaMemcpyAsync(r->reachable_mask, p->reach8, g.S, cudaMemcpyDeviceToHost, st));
     }
     if (r->controller)

@@ -889,7 +889,7 @@ int gsc_batch_run(gsc_context* ctx, uint32_t count, const gsc_model_desc* models
         for (uint32_t i = 0; i < n; ++i) {
             gsc_problem* p = b->probs[i].get();
             if (results[f + i].reachable_mask)
-                GSC_CU(ctx, launch_unpack_reach(p->g, p->fc, p->reach0, p->reach1, p->reach8, solve));
+                GSC_CU(ctx, launch_unpack_bits(p->g, p->reach0, p->reach8, solve));
         }
         cudaEvent_t ev = nullptr;
         GSC_CU(ctx, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
@@ -929,7 +929,7 @@ int gsc_batch_read_all(gsc_batch* b, gsc_result* out) {
     for (size_t i = 0; i < b->probs.size(); ++i) {
         gsc_problem* p = b->probs[i].get();
         if (out[i].reachable_mask)
-            GSC_CU(ctx, launch_unpack_bits(p->g, (b->hfc[i].iter & 1) ? p->reach1 : p->reach0, p->reach8, st));
+            GSC_CU(ctx, launch_unpack_bits(p->g, p->reach0, p->reach8, st));
         rows[i] = read_rows(b, out + i, i);
     }
     GSC_TRY(read_enqueue(b, out, st, rows));

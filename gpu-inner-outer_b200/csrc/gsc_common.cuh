@@ -52,8 +52,10 @@ struct GridInfo {
 
 // Programmatic dependent launch (PTX griddepcontrol, sm_90 and later): wait
 // until the kernel this one was launched after has completed and its writes
-// are visible.  Called first in a kernel, before any load or store of global
-// memory.  The launch of such a kernel is prepared while its predecessor
+// are visible.  Called before any access to memory that a predecessor writes;
+// what set-up wrote, before the kernel ahead of this one was launched, may be
+// read earlier (k_slice reads its representatives).  The launch of such a
+// kernel is prepared while its predecessor
 // runs and its blocks start as the predecessor's blocks exit (no explicit
 // early trigger: releasing dependents at the start of a kernel measured
 // slower).  For a kernel launched without the programmatic-serialization
@@ -76,7 +78,7 @@ struct QueryInfo {
 // masks) of slice (i2, i3) and input j.  With one Euler substep x and y move
 // by dt * v * (cos, sin)(theta) of the source cell (model.hpp:34-41), the same
 // for every input, so a slice has one plane; with more substeps the input
-// acts on v and theta between them and every input has its own.  At
+// acts on v and theta between them and every input has its own.
 __host__ __device__ __forceinline__ uint32_t xy_planes_of(uint32_t K, uint32_t M) { return K == 1 ? 1u : M; }
 __device__ __forceinline__ uint64_t xy_plane(const GridInfo& g, uint32_t i2, uint32_t i3, uint32_t j) {
     const uint64_t q = static_cast<uint64_t>(i2) * g.n[3] + i3;

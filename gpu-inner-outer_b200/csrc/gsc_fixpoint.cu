@@ -407,8 +407,9 @@ __global__ void __launch_bounds__(256) k_sat_stored(GridInfo g, StoredFixArgs a)
 // lookup instead of 16 or 32 gathers.  One state a thread, four inputs at a
 // time, their loads in flight before the first is looked at.  The last block
 // applies the stop rules.
-// Bound: DRAM sectors that the open states of a warp (about half its lanes)
-// use in part; a profile of the two-state form read 3.4 TB/s at 42 % occupancy.
+// Bound: the latency of the streamed pairs, of whose sectors the open states of
+// a warp use a part: at 32x32x24x16 x 64 a launch reads 178 MB, where 117 are
+// needed, at 3.4 to 3.6 TB/s with three quarters of the warps resident.
 // Measured, an iteration of a graph solve with its table: 48x40x31x12 x 64
 // inputs 191 -> 70 us, 300x24x20x8 x 25 94 -> 49 us.  Two states a thread: 75
 // and 53; the next four boxes fetched ahead as well: 85 and 59 (fetched in vain

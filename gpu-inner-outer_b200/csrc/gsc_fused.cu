@@ -364,8 +364,8 @@ SliceShape slice_shape(const GridInfo& g, uint32_t slices, uint32_t slice_reps) 
 }
 
 size_t fused_admission_bytes(const GridInfo& g, int need_valid, uint32_t max_reps) {
-    // Bulk-staged (16-byte slots three words longer) or word by word,
-    // whichever is more.
+    // The rows, class records and y tables of a column's representatives, in
+    // slots of 16 bytes three words longer or word by word, whichever is more.
     auto r4 = [](uint64_t x) { return (x + 3) & ~uint64_t(3); };
     const uint64_t nw = static_cast<uint64_t>(g.n[1]) * g.W, nv = need_valid ? 2 : 1, mr = max_reps;
     const uint64_t cw = 4 + (kShiftMax + 1) * g.W, n1 = g.n[1], w1 = (n1 + 31) / 32, ma = g.ma;
@@ -478,10 +478,10 @@ cudaError_t launch_shard_control(FixControl* fc, unsigned long long* stats, unsi
     return cudaGetLastError();
 }
 
-// Device time of an iteration (dilation + satisfaction + finalize launches
-// of one block per (slice, omega column), against this):
+// Device time of an iteration, against three launches (dilation, a block per
+// slice and omega column, update) before:
 //   65x65x38x25 x 100     38 -> 17 us       published demo   88 -> 54 us
-//   128x128x72x48 x 144  518 -> 135 us      47x83x29x17 x 63  24 -> 19 us
+//   128x128x72x48 x 144  518 -> 135 us      47x83x29x17 x 63  24 -> 17 us
 cudaError_t launch_fused_iteration(const GridInfo& g, const FusedFixArgs& a, cudaStream_t st, uint32_t* launches,
                                    cudaEvent_t* ev) {
     if (ev) cudaEventRecord(ev[0], st);

@@ -439,9 +439,8 @@ __device__ __forceinline__ void window_rows(const GridInfo& g, const bword* cur,
 // OR_{d=a..b} (F >> d); with the plane's shift masks M_d (launch_x_classes)
 // that is bit i0 of OR_d ((F >> d) & M_d); a plane whose boxes are alike needs
 // no masks (SliceRep::hx), one with boxes of more than kShiftMax shifts is
-// tested state by state.  When validity is more than
-// safety, the box must also hold a valid cell (keep_valid; few rows have a box
-// that may not).
+// tested state by state.  When validity is more than safety, the box must also
+// hold a valid cell (keep_valid; few rows have a box that may not).
 // In incremental iterations a representative's rows that lost a D' cell in
 // the last iteration are gathered first, and a (representative, row) item
 // with none in its y range is left out: its states failed, and nothing they
@@ -453,19 +452,19 @@ __device__ __forceinline__ void window_rows(const GridInfo& g, const bword* cur,
 //
 // Bound: latency and issue, with every slice's block resident at once
 // (slice_shape).  Rows are read from L2 straight into registers: staged
-// in shared memory in chunks of representatives (bulk copies on an mbarrier,
-// double-buffered, or OR-ed there), three block barriers a chunk and 45 M warp
-// instructions took 85 us an iteration on the published demo; so, 16 M take
-// 51 us, where one block per (slice, omega column) with a finalize kernel of
-// its own took 88.  Hits are noted and taken after the loop: taken in it, by
+// in shared memory in chunks of representatives, three block barriers a chunk
+// and 45 M warp instructions took 85 us an iteration on the published demo; so,
+// 16 M take 51 us, where one block per (slice, omega column) with a kernel of
+// its own for the update took 88.  Hits are noted and taken after the loop: taken in it, by
 // one lane while its warp waits, the same iteration took 76 us.  Loading two
 // or four representatives ahead costs registers (resident warps) and was no
 // faster (55 to 58 us).
 //
-// Returns 0 once the solve has stopped, 2 when the group counted a hit, else 1.  Every early return is taken by
-// the whole group.  s_meta: [0] iteration | incremental << 31, or all ones once
-// stopped, [1] rows packed, [2] hits noted.  SHARED: the slice has one x / y plane (xy_plane); DIRECT: as
-// a.direct; 2 = decided at run time.
+// Returns 0 once the solve has stopped, 2 when the group counted a hit, else 1.
+// Every early return is taken by the whole group.  s_meta: [0] iteration |
+// incremental << 31, or all ones once stopped, [1] rows packed, [2] hits noted.
+// SHARED: the slice has one x / y plane (xy_plane); DIRECT: as a.direct; 2 =
+// decided at run time.
 template <int W, int SHARED, int DIRECT, bool WARP, bool PDL, bool PARTS>
 __device__ __forceinline__ int slice_task(const GridInfo& g, const FusedFixArgs& a, uint32_t slice, uint32_t part,
                                            bword* smem, uint32_t* s_meta) {

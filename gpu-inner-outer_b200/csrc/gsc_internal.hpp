@@ -137,7 +137,7 @@ struct gsc_problem {
     // fused
     gsc_b200::bword *validb = nullptr, *unsafeb = nullptr, *srcb = nullptr, *candb = nullptr;
     gsc_b200::bword* dp[2] = {nullptr, nullptr};
-    gsc_b200::bword *reach0 = nullptr, *reach1 = nullptr, *active = nullptr;
+    gsc_b200::bword *reach0 = nullptr, *active = nullptr;
     gsc_b200::bword* xcls = nullptr;
     uint64_t xcls_used = 0;     // bytes of it up to the last list placed behind its records
     uint8_t* xrep = nullptr;
@@ -178,7 +178,7 @@ struct gsc_problem {
     // Per-phase device times (gsc_problem_phase_timings).  h2d_ms: uploads of
     // the query's host arrays at creation; the rest from the last
     // GSC_SOLVE_PROFILE solve: prefix passes, satisfaction, reduction
-    // (control or finalize kernel) and stop-record reads, summed, and per
+    // (control kernel) and stop-record reads, summed, and per
     // iteration {iteration, prefix build, satisfaction, reduction incl. the
     // stop-record read}.
     bool time_h2d = false;

@@ -92,10 +92,6 @@ cudaError_t launch_unpack_bits(const GridInfo& g, const bword* bits, uint8_t* ou
 // n words from src to dst by one small kernel (dst may be pinned host memory
 // mapped into the device's address space).
 cudaError_t launch_store_words(const uint32_t* src, uint32_t* dst, uint32_t n, cudaStream_t st);
-// The fixpoint's current reachable set (reach0 or reach1 by fc->iter, read
-// on the device) as one byte per state.
-cudaError_t launch_unpack_reach(const GridInfo& g, const FixControl* fc, const bword* reach0, const bword* reach1,
-                                uint8_t* out, cudaStream_t st);
 
 // ---- 4-D inclusive prefix tables (int32, zero first plane per dimension) -----------------
 // mode 0: valid; 1: valid && !reach (b = reach); 2: !safe (4-D safe mask).
@@ -200,12 +196,14 @@ inline uint64_t box_table_words(const GridInfo& g, const StoredBits& b) {
 }
 // Kernels of one iteration, and those of them that rebuild the table.
 uint32_t stored_passes(const GridInfo& g, const StoredBits& b);
-inline uint32_t stored_launches(const GridInfo& g, const StoredBits& b) { return stored_passes(g, b) + (b.copies ? 1u : 2u); }
+inline uint32_t stored_launches(const GridInfo& g, const StoredBits& b) {
+    return stored_passes(g, b) + (b.copies ? 1u : 2u);
+}
 cudaError_t launch_stored_init(const GridInfo& g, const StoredFixArgs& a, cudaStream_t st);
-// ev (optional, kProfileEvents events): [0] before the prefix rebuild,
-// [1..n] after its n passes (stored_passes; events n+1 .. 4 are not recorded), [5] after the satisfaction kernel, [6] after
-// the control kernel.  The fused iteration records [0], [1] after the
-// dilation, [5] and [6] alike.
+// ev (optional, kProfileEvents events): [0] before the table's rebuild, [1..n]
+// after its n passes (stored_passes; events n+1 .. 4 are not recorded), [5]
+// after the satisfaction kernel, [6] after the control kernel, where there is
+// one.
 constexpr int kProfileEvents = 8;
 cudaError_t launch_stored_iteration(const GridInfo& g, const StoredFixArgs& a, cudaStream_t st, uint32_t* launches,
                                     cudaEvent_t* ev = nullptr);
@@ -316,7 +314,6 @@ struct FusedFixArgs {
     uint32_t* reach_step;
     FixControl* fc;
     unsigned long long* stats;
-    int need_valid;
     const bword* xcls;         // per-plane x-box classes (launch_x_classes)
     uint32_t cls_words;        // 32-bit words per class record
     const SliceRep* reps;      // [slices][M]: each slice's representatives, in input order
@@ -348,9 +345,11 @@ struct FusedFixArgs {
 };
 
 constexpr int kShiftMax = 8;   // most shifts d of a plane's shift-mask record
-// Which problems the fused method takes is a rule on the staging of one
-// (slice, omega column) task with max_reps representative accelerations
-// (fused_admission_bytes at most kFusedSmemMax); a slice's task needs less.
+// Which problems the fused method takes, and which launch shapes a batch may
+// use, is a rule on the shared memory that a task of max_reps representative
+// accelerations once staged (fused_admission_bytes at most kFusedSmemMax).  A
+// slice's task takes less (fused_smem_bytes); the rule stays because it decides
+// which calls by method or launch shape are refused.
 constexpr size_t kFusedSmemMax = 200 * 1024;
 size_t fused_admission_bytes(const GridInfo& g, int need_valid, uint32_t max_reps);
 // Representatives kept in shared memory at a time, and the shared memory of a

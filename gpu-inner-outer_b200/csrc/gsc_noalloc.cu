@@ -145,7 +145,7 @@ __device__ __forceinline__ uint32_t nq16(const int32_t* __restrict__ P, const Gr
 
 // The corners of a (min_flat, max_flat) pair in the reference's flat layout
 // (prefix_sum.hpp:87-105).  Division by a grid extent n is the high half of a
-// product with floor(2^64 / n) + 1, which is exact for 32-bit numerators
+// product with ceil(2^64 / n), which is exact for 32-bit numerators
 // (Lemire, Kaser and Kurz, "Faster remainder by direct computation", 2019).
 struct FlatDiv {
     unsigned long long m[3];

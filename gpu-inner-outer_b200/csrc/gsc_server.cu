@@ -267,7 +267,7 @@ void start_copy(gsc_server* s, Req* r) {
     if (e == cudaSuccess && out->candidate_mask)
         e = cudaMemcpyAsync(out->candidate_mask, p->cand, g.S, cudaMemcpyDeviceToHost, cs);
     if (e == cudaSuccess && out->reachable_mask) {
-        e = launch_unpack_bits(g, (r->fc.iter & 1) ? p->reach1 : p->reach0, p->reach8, cs);
+        e = launch_unpack_bits(g, p->reach0, p->reach8, cs);
         if (e == cudaSuccess) e = cudaMemcpyAsync(out->reachable_mask, p->reach8, g.S, cudaMemcpyDeviceToHost, cs);
     }
     if (e == cudaSuccess && out->controller)

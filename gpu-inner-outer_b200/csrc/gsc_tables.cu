@@ -51,8 +51,9 @@ __device__ __forceinline__ bool in_rect(const double* lb, const double* ub, cons
 // ---- nominal successors -----------------------------------------------------------------
 
 // One warp per plane (xy_plane: (i2*n3 + i3)*M + j, or i2*n3 + i3 with one
-// substep, whose terms input 0 stands for); lanes over the x then the y cells.  The plane's trajectory terms dt * (v * cos theta)
-// and dt * (v * sin theta) do not depend on the cell, so each is computed once
+// substep, whose terms input 0 stands for); lanes over the x then the y cells.
+// The plane's trajectory terms dt * (v * cos theta) and dt * (v * sin theta) do
+// not depend on the cell, so each is computed once
 // (staged in shared memory for up to kTermsMax substeps) and added to the
 // cell centre in the reference's order (model.hpp:34-45).
 constexpr int kPlaneThreads = 256;
@@ -266,7 +267,7 @@ __global__ void __launch_bounds__(kPlaneThreads) k_axis_tables(GridInfo g, Query
          plane < planes; plane += wstride) {
         const uint32_t i3 = static_cast<uint32_t>((plane / g.xy_planes) % g.n[3]);
         const double vc = centre(g, 3, i3);
-        // The plane's boxes in short (ShortBox): one ballot, shuffle and vote a 32 cells.
+        // The plane's boxes in short (launch_axis_tables): one ballot, shuffle and vote a 32 cells.
         uint32_t ab[2] = {0, 0}, range[2] = {0, 0};
         bool alike[2];
         for (int d = 0; d < 2; ++d) {
@@ -342,12 +343,9 @@ __global__ void k_store_words(const uint32_t* __restrict__ src, uint32_t* __rest
     for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) dst[i] = src[i];
 }
 
-// One warp per x-row.  With fc, the set is the fixpoint's current
-// reachable buffer (bits when fc->iter is even, odd otherwise).
+// One warp per x-row.
 __global__ void __launch_bounds__(kPlaneThreads) k_unpack_bits(GridInfo g, const bword* __restrict__ bits,
-                                                              uint8_t* __restrict__ out, const FixControl* fc,
-                                                              const bword* __restrict__ odd) {
-    if (fc && (fc->iter & 1)) bits = odd;
+                                                              uint8_t* __restrict__ out) {
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t wstride = static_cast<uint64_t>(gridDim.x) * (blockDim.x >> 5);
     for (uint64_t r = blockIdx.x * static_cast<uint64_t>(blockDim.x >> 5) + (threadIdx.x >> 5); r < g.rows;
@@ -533,7 +531,7 @@ __global__ void k_export(GridInfo g, ExportArgs a) {
 // One thread per plane; a block first copies its planes' x rows (contiguous)
 // into shared memory in one coalesced round, then each thread scans its row
 // there twice (a row stride of n0 words): the shift range, then the masks.
-// Planes whose boxes are alike need no record (ShortBox) and get none.
+// Planes whose boxes are alike (kBoxX) need no record and get none.
 __global__ void k_x_classes(GridInfo g, const uint32_t* __restrict__ xt, const uint4* __restrict__ shorts,
                             bword* __restrict__ out) {
     extern __shared__ uint32_t s_xrows[];
@@ -814,18 +812,12 @@ cudaError_t launch_axis_tables(const GridInfo& g, const QueryInfo& q, const doub
 }
 
 cudaError_t launch_unpack_bits(const GridInfo& g, const bword* bits, uint8_t* out, cudaStream_t st) {
-    k_unpack_bits<<<warp_blocks(g.rows), kPlaneThreads, 0, st>>>(g, bits, out, nullptr, nullptr);
+    k_unpack_bits<<<warp_blocks(g.rows), kPlaneThreads, 0, st>>>(g, bits, out);
     return cudaGetLastError();
 }
 
 cudaError_t launch_store_words(const uint32_t* src, uint32_t* dst, uint32_t n, cudaStream_t st) {
     k_store_words<<<1, 32, 0, st>>>(src, dst, n);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_unpack_reach(const GridInfo& g, const FixControl* fc, const bword* reach0, const bword* reach1,
-                                uint8_t* out, cudaStream_t st) {
-    k_unpack_bits<<<warp_blocks(g.rows), kPlaneThreads, 0, st>>>(g, reach0, out, fc, reach1);
     return cudaGetLastError();
 }
 

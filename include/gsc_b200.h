@@ -460,7 +460,7 @@ int gsc_batch_run(gsc_context* ctx, uint32_t count, const gsc_model_desc* models
  * fits the server's budget; admitted queries are set up on a second stream
  * while the running ones iterate, and join the running set at the next
  * iteration step (continuous batching: every step runs one batched fixpoint
- * iteration -- or iterations_per_step -- of every running query in four
+ * iteration -- or iterations_per_step -- of every running query in a few
  * launches).  A query that stops leaves the set, its results are copied to
  * the caller's buffers on a third stream, and its memory and slot go to the
  * next query.  Each query's result is bit-identical to its own gsc_problem

@@ -151,7 +151,6 @@ int check(int argc, char** argv) {
     a.reach_step = step.data();
     a.fc = &fc;
     a.stats = stats.data();
-    a.need_valid = need_valid;
     a.reps = reps.data();
     a.nreps = nreps.data();
     a.pass = pass;
