@@ -35,11 +35,6 @@ inline unsigned int blocks_for(uint64_t n, int threads) {
 
 using namespace fused;
 
-// Most threads of a satisfaction block: at most kSliceThreadsMax at 48
-// registers (40 warps an SM), or, where few slices share an SM (wide),
-// kSliceThreadsWide at 64 (32 warps).
-constexpr uint32_t kSliceThreadsMax = 256, kSliceThreadsWide = 512;
-
 __global__ void k_fused_init(GridInfo g, FusedFixArgs a, const uint8_t* __restrict__ cand) {
     const uint64_t words = static_cast<uint64_t>(g.slices) * g.sw;
     for (uint64_t e = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; e < words;
@@ -328,40 +323,6 @@ cudaError_t launch_slice_w(const GridInfo& g, const FusedFixArgs& a, cudaStream_
 }
 
 }  // namespace
-
-SliceShape slice_shape(const GridInfo& g, uint32_t slices, uint32_t slice_reps) {
-    SliceShape s{};
-    s.part_rows = g.n[1];
-    const uint64_t items = static_cast<uint64_t>(g.n[1]) * std::max(1u, slice_reps);
-    // Few slices with much to test each: parts of at least 16 rows, two a slice
-    // or as many as give two blocks an SM, and about 750 threads an SM in all.
-    // Measured, us a solve with one block a slice and so: 16x400x12x6 57.7 and
-    // 53.6, 16x1000x8x4 57.6 and 47.1, 48x48x16x8 x 192 inputs 189 and 156,
-    // 60x60x30x10 x 36 1,477 and 1,379, 100x100x30x10 x 36 1,590 and 1,495.  But
-    // with little to test (100x100x20x12, 4 representatives) 357 and 363 in two
-    // parts, and above 300 slices (47x83x29x17) 439 and 460.
-    if (slices <= 300 && items * g.W > 2048) {
-        const uint32_t parts = std::max(2u, 288u / slices);
-        s.part_rows = std::min(g.n[1], std::max(16u, ((g.n[1] + parts - 1) / parts + 7) & ~7u));
-    }
-    if (s.part_rows < g.n[1]) {
-        s.wide = 1;
-        const uint64_t blocks = static_cast<uint64_t>(slices) * s.parts(g.n[1]);
-        const uint64_t each = static_cast<uint64_t>(s.part_rows) * std::max(1u, slice_reps);
-        s.threads = static_cast<uint32_t>(
-            std::min<uint64_t>({384, (110000 / blocks + 31) & ~uint64_t(31), (each + 31) & ~uint64_t(31)}));
-        return s;
-    }
-    // A packed row of the slice per thread, for several representatives side
-    // by side.  As wide as lets every slice's block be resident at once (a
-    // second wave of a few blocks doubles an iteration), and at least 128.
-    const uint32_t per_sm = (slices + 147) / 148;
-    uint32_t most = per_sm <= 2 ? kSliceThreadsWide / per_sm * 2 : per_sm <= 10 ? 40 / per_sm * 32 : 128;
-    most = std::min(per_sm <= 2 ? kSliceThreadsWide : kSliceThreadsMax, std::max(128u, most));
-    s.threads = static_cast<uint32_t>(std::min<uint64_t>(most, (items + 31) & ~31ull));
-    s.wide = s.threads > kSliceThreadsMax;
-    return s;
-}
 
 size_t fused_admission_bytes(const GridInfo& g, int need_valid, uint32_t max_reps) {
     // The rows, class records and y tables of a column's representatives, in

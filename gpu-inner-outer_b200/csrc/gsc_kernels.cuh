@@ -1,6 +1,7 @@
 // gsc_kernels.cuh -- launch wrappers shared between the kernel files and the C ABI layer.
 #pragma once
 
+#include <algorithm>
 #include <cstdint>
 #include <mutex>
 #include <set>
@@ -359,8 +360,50 @@ constexpr uint32_t kHitNotes = 384;      // (row, representative) hits noted at 
 uint32_t fused_pass(const GridInfo& g, uint32_t slice_reps);
 size_t fused_smem_bytes(const GridInfo& g, uint32_t pass, uint32_t rows);
 DilateTile dilate_tile_of(const GridInfo& g, const DilateArgs& d, uint32_t levels);
+// Most threads of a satisfaction block: at most kSliceThreadsMax at 48
+// registers (40 warps an SM), or, where few slices share an SM (wide),
+// kSliceThreadsWide at 64 (32 warps).
+constexpr uint32_t kSliceThreadsMax = 256, kSliceThreadsWide = 512;
 // For a launch over `slices` slices of at most slice_reps representatives.
-SliceShape slice_shape(const GridInfo& g, uint32_t slices, uint32_t slice_reps);
+inline SliceShape slice_shape(const GridInfo& g, uint32_t slices, uint32_t slice_reps) {
+    SliceShape s{};
+    s.part_rows = g.n[1];
+    const uint64_t items = static_cast<uint64_t>(g.n[1]) * std::max(1u, slice_reps);
+    // Few slices with much to test each: parts of at least 16 rows, two a slice
+    // or as many as give two blocks an SM.
+    // Measured, us a solve with one block a slice and so: 16x400x12x6 57.7 and
+    // 53.6, 16x1000x8x4 57.6 and 47.1, 48x48x16x8 x 192 inputs 189 and 156,
+    // 60x60x30x10 x 36 1,477 and 1,379, 100x100x30x10 x 36 1,590 and 1,495.  But
+    // with little to test (100x100x20x12, 4 representatives) 357 and 363 in two
+    // parts, and above 300 slices (47x83x29x17) 439 and 460.
+    if (slices <= 300 && items * g.W > 2048) {
+        const uint32_t parts = std::max(2u, 288u / slices);
+        s.part_rows = std::min(g.n[1], std::max(16u, ((g.n[1] + parts - 1) / parts + 7) & ~7u));
+    }
+    if (s.part_rows < g.n[1]) {
+        s.wide = 1;
+        // Every block resident at once (1,024 threads an SM at 64 registers), up
+        // to 384 threads.  Measured, us a solve with 110,000 threads in all, which
+        // left a second wave of a few blocks at 149 to 184 slices, and so:
+        // hyperbolic 64x64x24x7 x 36 inputs 876 and 745, 108x46x24x7 x 35 1,122 and
+        // 1,030, 48x96x20x8 x 36 617 and 529, 45x41x30x9 x 36 2,077 and 2,020.
+        const uint32_t per_sm = (slices * s.parts(g.n[1]) + 147) / 148;
+        const uint64_t each = static_cast<uint64_t>(s.part_rows) * std::max(1u, slice_reps);
+        s.threads = static_cast<uint32_t>(
+            std::min<uint64_t>({384, kSliceThreadsWide * 2 / per_sm & ~31u, (each + 31) & ~uint64_t(31)}));
+        return s;
+    }
+    // A packed row of the slice per thread, for several representatives side
+    // by side.  As wide as lets every slice's block be resident at once (a
+    // second wave of a few blocks doubles an iteration), and at least 128.
+    const uint32_t per_sm = (slices + 147) / 148;
+    uint32_t most = per_sm <= 2 ? kSliceThreadsWide / per_sm * 2 : per_sm <= 10 ? 40 / per_sm * 32 : 128;
+    most = std::min(per_sm <= 2 ? kSliceThreadsWide : kSliceThreadsMax, std::max(128u, most));
+    s.threads = static_cast<uint32_t>(std::min<uint64_t>(most, (items + 31) & ~31ull));
+    s.wide = s.threads > kSliceThreadsMax;
+    return s;
+}
+
 // Dilated copies of src into dst.  With fc and rowlost (during a fixpoint,
 // after its first iteration) only tiles whose windows hold a row that lost a
 // D' cell are recomputed, and src is src0 or src1 by the iteration's parity.

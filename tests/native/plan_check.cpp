@@ -1,13 +1,25 @@
 // Host rules of the fused plan, for a grid and the box widths in use:
 //   plan_check <n0> <n1> <n2> <n3> <theta widths> <v widths> <y levels (mask)> <cells a window> <batched>
 // Prints whether windows are read directly, and the words of a set's dilated copies.
+//   plan_check shape <n0> <n1> <slices> <representatives a slice>
+// Prints the threads, rows a part, parts and kernel of a launch.
 #include <iostream>
+#include <string>
 
 #include "device_emulation.hpp"
 
 using namespace gsc_b200;
 
 int main(int argc, char** argv) {
+    if (argc == 6 && std::string(argv[1]) == "shape") {
+        GridInfo g{};
+        g.n[0] = std::atoi(argv[2]);
+        g.n[1] = std::atoi(argv[3]);
+        g.W = (g.n[0] + kBits - 1) / kBits;
+        const SliceShape s = slice_shape(g, std::atoi(argv[4]), std::atoi(argv[5]));
+        std::cout << s.threads << " " << s.part_rows << " " << s.parts(g.n[1]) << " " << s.wide << "\n";
+        return 0;
+    }
     if (argc < 10) return 2;
     GridInfo g{};
     for (int d = 0; d < 4; ++d) g.n[d] = static_cast<uint32_t>(std::atoi(argv[1 + d]));

@@ -41,3 +41,16 @@ def test_windows_read_directly(plan_check, shape, cells, batched, direct):
     out = subprocess.run([plan_check] + [str(v) for v in (*shape, 2, 2, 2, cells, batched)], capture_output=True,
                          text=True, check=True).stdout.split()
     assert bool(int(out[0])) == direct
+
+
+@pytest.mark.parametrize("n0,n1,reps", [(64, 64, 36), (108, 46, 35), (45, 41, 36), (17, 300, 9), (250, 17, 36)])
+@pytest.mark.parametrize("slices", [1, 7, 72, 143, 144, 148, 149, 168, 184, 185, 222, 223, 275, 296, 297, 300])
+def test_parts_of_slices_are_resident_at_once(plan_check, n0, n1, reps, slices):
+    """The parts that slices are split into (whole bytes of row bits) are one
+    wave: at 64 registers a thread an SM holds 1,024 threads."""
+    out = subprocess.run([plan_check, "shape"] + [str(v) for v in (n0, n1, slices, reps)], capture_output=True,
+                         text=True, check=True).stdout.split()
+    threads, rows, parts, wide = map(int, out)
+    assert parts > 1 and wide and rows % 8 == 0 and (parts - 1) * rows < n1 <= parts * rows
+    assert threads % 32 == 0 and 32 <= threads <= 384
+    assert -(-slices * parts // 148) * threads <= 1024
