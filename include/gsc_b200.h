@@ -50,7 +50,7 @@ typedef enum {
     GSC_ERR_NO_DEVICE = 5,          /* no CUDA device (kernels.cu:497-502)        */
     GSC_ERR_CANDIDATE_INVALID = 6,  /* candidate set contains invalid states
                                        (abstraction.hpp:268-272)                  */
-    GSC_ERR_TIMEOUT = 7             /* a bounded device-side wait ran out         */
+    GSC_ERR_TIMEOUT = 7             /* a bounded wait ran out                     */
 } gsc_status;
 
 /* Fixpoint outcome, reachability.hpp:133-152 (messages kept verbatim by
@@ -179,7 +179,8 @@ typedef struct {
                                        input) tests, summed over iterations       */
     uint64_t aux_count;             /* stored: box counts evaluated; fused:
                                        (slice, representative input) planes
-                                       staged, summed over iterations             */
+                                       staged (by each block of a slice that is
+                                       split), summed over iterations             */
     uint32_t sat_threads;           /* fused: threads per satisfaction block      */
     uint32_t max_reps;              /* fused: most representative accelerations
                                        of one omega column                        */
